@@ -24,11 +24,13 @@
 
 #include <cuda_bf16.h>
 
+#include "unet_dw.cuh"
 #include "unet_tc.cuh"
 
 #include <cmath>
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace fg {
@@ -121,86 +123,69 @@ __global__ void __launch_bounds__(128) k_conv3(const bf16* __restrict__ in, int 
   }
 }
 
-// dW[t][o][i] += sum_p g[p][o] * in[p + off(t)][i]  (FP32; one tap per block row)
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_conv3_dw(const bf16* __restrict__ in, int in_stride,
-                                                  int in_off, const bf16* __restrict__ gout,
-                                                  int g_stride, int g_off, float* __restrict__ dW,
-                                                  int nx, int ny, int nz, size_t chunk) {
-  constexpr int TP = 32;
-  __shared__ float gs[TP][COUT];
-  __shared__ float is[TP][CIN];
-  const int tap = blockIdx.x;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  const size_t n = (size_t)nx * ny * nz;
-  const size_t p0 = blockIdx.y * chunk, p1 = min(n, p0 + chunk);
-  constexpr int NOUT = COUT * CIN;
-  constexpr int PER = (NOUT + 255) / 256;
-  float acc[PER];
-#pragma unroll
-  for (int q = 0; q < PER; ++q) acc[q] = 0.f;
-  for (size_t pt = p0; pt < p1; pt += TP) {
-    for (int e = threadIdx.x; e < TP * COUT; e += 256) {
-      const int pp = e / COUT, o = e % COUT;
-      const size_t p = pt + pp;
-      gs[pp][o] = p < p1 ? __bfloat162float(gout[p * g_stride + g_off + o]) : 0.f;
-    }
-    for (int e = threadIdx.x; e < TP * CIN; e += 256) {
-      const int pp = e / CIN, i = e % CIN;
-      const size_t p = pt + pp;
-      float v = 0.f;
-      if (p < p1) {
-        const int x = (int)(p % nx), y = (int)((p / nx) % ny), z = (int)(p / ((size_t)nx * ny));
-        const int xx = x + dx, yy = y + dy, zz = z + dz;
-        if (xx >= 0 && xx < nx && yy >= 0 && yy < ny && zz >= 0 && zz < nz)
-          v = __bfloat162float(in[((size_t)xx + (size_t)nx * ((size_t)yy + (size_t)ny * zz)) *
-                                      in_stride + in_off + i]);
-      }
-      is[pp][i] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int e = threadIdx.x + q * 256;
-      if (e < NOUT) {
-        const int o = e / CIN, i = e % CIN;
-        float s = acc[q];
-#pragma unroll 8
-        for (int pp = 0; pp < TP; ++pp) s = fmaf(gs[pp][o], is[pp][i], s);
-        acc[q] = s;
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int e = threadIdx.x + q * 256;
-    if (e < NOUT) atomicAdd(&dW[(size_t)tap * NOUT + e], acc[q]);
-  }
-}
-
-// db[o] += sum_p g[p][o]
-__global__ void k_bias_grad(const bf16* __restrict__ g, int g_stride, int g_off, int cout,
-                            size_t n, float* __restrict__ db) {
-  __shared__ float s[64];
-  if (threadIdx.x < 64) s[threadIdx.x] = 0.f;
-  __syncthreads();
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n;
-       p += (size_t)gridDim.x * blockDim.x)
-    for (int o = 0; o < cout; ++o) atomicAdd(&s[o], __bfloat162float(g[p * g_stride + g_off + o]));
-  __syncthreads();
-  if (threadIdx.x < cout) atomicAdd(&db[threadIdx.x], s[threadIdx.x]);
-}
-
-// grad *= (act > 0)
-__global__ void k_relu_bwd(bf16* __restrict__ g, int g_stride, int g_off,
-                           const bf16* __restrict__ act, int a_stride, int a_off, int c, size_t n) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n * c;
+// The gradient of one layer's activations made ready for the layer's weight and data gradients,
+// in one pass: g *= (act > 0) in place and db[c] += sum_p g[p][c]; POOL: first
+// g += gp[pool(p)] / 8, the gradient that arrives through the 2x2x2 pooling (rounded to BF16
+// before the mask, as a stored sum).  One thread per pixel and group of 8 channels (16-byte
+// accesses); the group is the same for all of a thread's pixels (256 and the grid stride are
+// multiples of C / 8), so the channel sums stay in registers and one atomic per channel and
+// block adds them.  Bound by memory: 6 C bytes
+// per pixel, 11 us for 1M pixels of 16 channels (a mask and a sum with shared-memory atomics
+// were 37 + 212 us).
+template <int C, bool POOL>
+__global__ void __launch_bounds__(256) k_grad_mask(bf16* __restrict__ g, int g_stride, int g_off,
+                                                   const bf16* __restrict__ act, int a_stride,
+                                                   int a_off, const bf16* __restrict__ gp, int nx,
+                                                   int ny, size_t n, float* __restrict__ db) {
+  constexpr int G = C / 8;
+  const int cg = threadIdx.x % G;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n * G;
        e += (size_t)gridDim.x * blockDim.x) {
-    const size_t p = e / c;
-    const int ch = (int)(e % c);
-    if (!(__bfloat162float(act[p * a_stride + a_off + ch]) > 0.f))
-      g[p * g_stride + g_off + ch] = __float2bfloat16(0.f);
+    const size_t p = e / G;
+    uint4* gq = reinterpret_cast<uint4*>(g + p * g_stride + g_off + 8 * cg);
+    uint4 v = *gq;
+    const uint4 av = *reinterpret_cast<const uint4*>(act + p * a_stride + a_off + 8 * cg);
+    uint4 pv = make_uint4(0u, 0u, 0u, 0u);
+    if (POOL) {
+      const uint32_t q = (uint32_t)p, x = q % (uint32_t)nx, yz = q / (uint32_t)nx;
+      const uint32_t y = yz % (uint32_t)ny, z = yz / (uint32_t)ny;
+      const size_t c = (x >> 1) + (size_t)(nx / 2) * ((y >> 1) + (size_t)(ny / 2) * (z >> 1));
+      pv = *reinterpret_cast<const uint4*>(gp + c * C + 8 * cg);
+    }
+    uint32_t* vw = reinterpret_cast<uint32_t*>(&v);
+    const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&av);
+    const __nv_bfloat162* ph = reinterpret_cast<const __nv_bfloat162*>(&pv);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&vw[u]));
+      if (POOL) {
+        const float2 h = __bfloat1622float2(ph[u]);
+        f.x = __bfloat162float(__float2bfloat16(f.x + 0.125f * h.x));
+        f.y = __bfloat162float(__float2bfloat16(f.y + 0.125f * h.y));
+      }
+      const float2 a = __bfloat1622float2(ah[u]);
+      if (!(a.x > 0.f)) f.x = 0.f;
+      if (!(a.y > 0.f)) f.y = 0.f;
+      vw[u] = pack2(f.x, f.y);
+      s[2 * u] += f.x;
+      s[2 * u + 1] += f.y;
+    }
+    *gq = v;
+  }
+  // lanes with the same channel group, then the block's warps
+  __shared__ float sh[8][G][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    for (int off = 16; off >= G; off >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], off);
+    if (lane < G) sh[warp][lane][u] = s[u];
+  }
+  __syncthreads();
+  if (threadIdx.x < C) {
+    float t = 0.f;
+    for (int w = 0; w < 8; ++w) t += sh[w][threadIdx.x / 8][threadIdx.x % 8];
+    atomicAdd(&db[threadIdx.x], t);
   }
 }
 
@@ -239,22 +224,6 @@ __global__ void k_pool(const bf16* __restrict__ in, int in_stride, int in_off, b
   }
 }
 
-// gradient of pooling, added to an existing gradient slice: gin[p] += gout[pool(p)] / 8
-__global__ void k_pool_bwd_add(const bf16* __restrict__ gout, bf16* __restrict__ gin,
-                               int gin_stride, int gin_off, int c, int nx, int ny, int nz) {
-  const size_t n = (size_t)nx * ny * nz;
-  const int cx = nx / 2, cy = ny / 2;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n * c;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t p = e / c;
-    const int ch = (int)(e % c);
-    const int x = (int)(p % nx), y = (int)((p / nx) % ny), z = (int)(p / ((size_t)nx * ny));
-    const size_t q = (size_t)(x / 2) + (size_t)cx * ((size_t)(y / 2) + (size_t)cy * (z / 2));
-    bf16* d = gin + p * gin_stride + gin_off + ch;
-    *d = __float2bfloat16(__bfloat162float(*d) + 0.125f * __bfloat162float(gout[q * c + ch]));
-  }
-}
-
 // nearest 2x upsampling of a coarse field (stride c) into a channel slice of a fine buffer
 __global__ void k_up(const bf16* __restrict__ in, bf16* __restrict__ out, int out_stride,
                      int out_off, int c, int nx, int ny, int nz) {
@@ -274,23 +243,36 @@ __global__ void k_up(const bf16* __restrict__ in, bf16* __restrict__ out, int ou
   }
 }
 
-// gradient of upsampling: gin[q] = sum of the 8 children of a fine gradient slice
+// gradient of upsampling: gin[q] = sum of the 8 children of a fine gradient slice; one thread per
+// coarse cell and group of 8 channels (16-byte accesses)
 __global__ void k_up_bwd(const bf16* __restrict__ gout, int g_stride, int g_off,
                          bf16* __restrict__ gin, int c, int nx, int ny, int nz) {
-  const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
-  const size_t nc = (size_t)cx * cy * cz;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nc * c;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t q = e / c;
-    const int ch = (int)(e % c);
-    const int x = (int)(q % cx), y = (int)((q / cx) % cy), z = (int)(q / ((size_t)cx * cy));
-    float s = 0.f;
+  const uint32_t cx = nx / 2, cy = ny / 2, cz = nz / 2;
+  const uint32_t g = (uint32_t)c / 8;
+  const uint64_t tot = (uint64_t)cx * cy * cz * g;
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < tot;
+       e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t q = (uint32_t)(e / g), cg = (uint32_t)(e - (uint64_t)q * g);
+    const uint32_t x = q % cx, yz = q / cx, y = yz % cy, z = yz / cy;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const size_t p = (size_t)(2 * x + (k & 1)) + (size_t)nx * ((size_t)(2 * y + ((k >> 1) & 1)) +
-                                                                   (size_t)ny * (2 * z + (k >> 2)));
-      s += __bfloat162float(gout[p * g_stride + g_off + ch]);
+      const uint32_t p = (2 * x + (k & 1)) + (uint32_t)nx * ((2 * y + ((k >> 1) & 1)) +
+                                                             (uint32_t)ny * (2 * z + (k >> 2)));
+      const uint4 v = *reinterpret_cast<const uint4*>(gout + (size_t)p * g_stride + g_off + 8 * cg);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 f = __bfloat1622float2(h[u]);
+        s[2 * u] += f.x;
+        s[2 * u + 1] += f.y;
+      }
     }
-    gin[q * c + ch] = __float2bfloat16(s);
+    uint4 o;
+    uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ow[u] = pack2(s[2 * u], s[2 * u + 1]);
+    *reinterpret_cast<uint4*>(gin + (size_t)q * c + 8 * cg) = o;
   }
 }
 
@@ -368,12 +350,18 @@ __global__ void k_out(const bf16* __restrict__ d1, const float* __restrict__ wo,
   }
 }
 
-// loss = mean((y - t)^2); gy = 2 (y - t) / n; plus the output-layer gradients and dL/dd1
-__global__ void k_out_bwd(const bf16* __restrict__ d1, const float* __restrict__ wo,
-                          const float* __restrict__ y, const float* __restrict__ tgt,
-                          const float* __restrict__ tscale, size_t n, float weight,
-                          bf16* __restrict__ gd1, float* __restrict__ gwo,
-                          double* __restrict__ loss) {
+// loss = mean((y - t)^2); gy = 2 (y - t) / n; plus the output-layer gradients and dL/dd1.  The
+// 18 sums are added up over the block before one atomic each (per warp, 330,000 atomics on 18
+// addresses took most of the
+// kernel's time at 1M cells: 379 us against 17).
+__global__ void __launch_bounds__(256) k_out_bwd(const bf16* __restrict__ d1,
+                                                 const float* __restrict__ wo,
+                                                 const float* __restrict__ y,
+                                                 const float* __restrict__ tgt,
+                                                 const float* __restrict__ tscale, size_t n,
+                                                 float weight, bf16* __restrict__ gd1,
+                                                 float* __restrict__ gwo,
+                                                 double* __restrict__ loss) {
   const float ts = *tscale;
   float lw[17];
 #pragma unroll
@@ -385,24 +373,47 @@ __global__ void k_out_bwd(const bf16* __restrict__ d1, const float* __restrict__
     const float e = y[p] - tgt[p] * ts;
     ls += (double)weight * e * e;
     const float gy = 2.0f * weight * e * inv_n;
-    uint32_t* o = reinterpret_cast<uint32_t*>(gd1 + p * 16);
+    const uint4* dv = reinterpret_cast<const uint4*>(d1 + p * 16);
+    uint4* o4 = reinterpret_cast<uint4*>(gd1 + p * 16);
 #pragma unroll
-    for (int c = 0; c < 16; c += 2) {
-      const float a = __bfloat162float(d1[p * 16 + c]), b = __bfloat162float(d1[p * 16 + c + 1]);
-      lw[c] = fmaf(gy, a, lw[c]);
-      lw[c + 1] = fmaf(gy, b, lw[c + 1]);
-      o[c / 2] = pack2(gy * wo[c], gy * wo[c + 1]);
+    for (int half = 0; half < 2; ++half) {
+      const uint4 w = dv[half];
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
+      uint4 o;
+      uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = 8 * half + 2 * u;
+        const float2 f = __bfloat1622float2(h[u]);
+        lw[c] = fmaf(gy, f.x, lw[c]);
+        lw[c + 1] = fmaf(gy, f.y, lw[c + 1]);
+        ow[u] = pack2(gy * wo[c], gy * wo[c + 1]);
+      }
+      o4[half] = o;
     }
     lw[16] += gy;
   }
+  __shared__ float sh[8][17];
+  __shared__ double shl[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int c = 0; c < 17; ++c) {
     float v = lw[c];
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&gwo[c], v);
+    if (lane == 0) sh[warp][c] = v;
   }
   ls = warp_sum(ls);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, ls / (double)n);
+  if (lane == 0) shl[warp] = ls;
+  __syncthreads();
+  if (threadIdx.x < 17) {
+    float t = 0.f;
+    for (int w = 0; w < 8; ++w) t += sh[w][threadIdx.x];
+    atomicAdd(&gwo[threadIdx.x], t);
+  } else if (threadIdx.x == 32) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += shl[w];
+    atomicAdd(loss, t / (double)n);
+  }
 }
 
 // mirrored-and-transposed weights for the data gradient: Wt[t'][i][o] = W[26-t'][o][i]
@@ -460,6 +471,11 @@ static int blocks_for(size_t n) {
   size_t b = (n + 255) / 256;
   if (b > (size_t)kNumSMs * 16) b = (size_t)kNumSMs * 16;
   return (int)(b < 1 ? 1 : b);
+}
+
+// blocks of a kernel that ends with a few atomics per block
+static int red_blocks(size_t n) {
+  return (int)std::min<size_t>(std::max<size_t>(1, (n + 255) / 256), (size_t)kNumSMs * 8);
 }
 
 // the error word of the tensor-core convolutions (a bounded wait ran out), one per process
@@ -539,15 +555,23 @@ static void conv_sync(const bf16* in, int in_stride, int in_off, const bf16* W,
                                            out_off, nx, ny, nz, relu ? 1 : 0);
 }
 
+// Weight gradient: as many blocks as the device holds at once, dealt to the groups of 16 input
+// channels; z columns of 16 planes (two extra input planes each), shorter on small grids until
+// there are items enough for every block.
 template <int CIN, int COUT>
 static void conv_dw(const bf16* in, int in_stride, int in_off, const bf16* g, int g_stride,
                     int g_off, float* dW, int nx, int ny, int nz, cudaStream_t st) {
-  const size_t n = (size_t)nx * ny * nz;
-  const int chunks = (int)std::max<size_t>(1, std::min<size_t>(64, n / 256));
-  const size_t chunk = (n + chunks - 1) / chunks;
-  dim3 grid(27, chunks);
-  k_conv3_dw<CIN, COUT><<<grid, 256, 0, st>>>(in, in_stride, in_off, g, g_stride, g_off, dW, nx,
-                                               ny, nz, chunk);
+  using S = DwShape<COUT>;
+  // set on every launch: the attribute belongs to the current device, and the call is cheap
+  cudaFuncSetAttribute(k_conv3_dw<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+  const long tiles = (long)((nx + kDwT - 1) / kDwT) * ((ny + kDwT - 1) / kDwT);
+  const long want = std::max<long>(1, (long)kNumSMs * S::BLOCKS / (CIN / 16));
+  int zc = 16;
+  while (zc > 4 && tiles * ((nz + zc - 1) / zc) < want) zc /= 2;
+  const long items = tiles * ((nz + zc - 1) / zc);
+  const dim3 grid((unsigned)std::min(items, want), CIN / 16);
+  k_conv3_dw<CIN, COUT><<<grid, kDwThreads, S::SMEM, st>>>(in, in_stride, in_off, g, g_stride,
+                                                           g_off, dW, nx, ny, nz, zc);
 }
 
 }  // namespace unet
@@ -720,63 +744,56 @@ int backward(frehg_unet* net, const float* target, cudaStream_t st) {
   FG_CUDA(cudaMemsetAsync(G, 0, net->nparam * sizeof(float), st));
   FG_CUDA(cudaMemsetAsync(net->loss, 0, sizeof(double), st));
   // normalised target: t * (1/rms r); y holds the unscaled network output
-  k_out_bwd<<<blocks_for(n1), 256, 0, st>>>(net->d1, M + net->ooff, net->y, target, net->scal,
+  k_out_bwd<<<red_blocks(n1), 256, 0, st>>>(net->d1, M + net->ooff, net->y, target, net->scal,
                                             n1, net->loss_weight, net->g_d1, G + net->ooff,
                                             net->loss);
-  auto relu_b = [&](bf16* g, int gs, int go, const bf16* a, int as, int ao, int c, size_t n) {
-    k_relu_bwd<<<blocks_for(n * c), 256, 0, st>>>(g, gs, go, a, as, ao, c, n);
+  // mask by the layer's activations and bias gradient of layer l (C channels, grid gx x gy)
+  auto mask = [&](auto cc, bf16* g, int gs, int go, const bf16* a, int as, int ao, size_t n, int l) {
+    constexpr int C = decltype(cc)::value;
+    k_grad_mask<C, false><<<red_blocks(n * (C / 8)), 256, 0, st>>>(g, gs, go, a, as, ao, nullptr, 0, 0,
+                                                                   n, G + net->boff[l]);
   };
-  auto bias_g = [&](const bf16* g, int gs, int go, int c, size_t n, int l) {
-    k_bias_grad<<<blocks_for(n), 256, 0, st>>>(g, gs, go, c, n, G + net->boff[l]);
-  };
+  constexpr std::integral_constant<int, 16> c16{};
+  constexpr std::integral_constant<int, 32> c32{};
+  constexpr std::integral_constant<int, 64> c64{};
   // level 1 decoder
-  relu_b(net->g_d1, 16, 0, net->d1, 16, 0, 16, n1);
+  mask(c16, net->g_d1, 16, 0, net->d1, 16, 0, n1, 9);
   conv_dw<16, 16>(net->d1a, 16, 0, net->g_d1, 16, 0, G + net->woff[9], nx, ny, nz, st);
-  bias_g(net->g_d1, 16, 0, 16, n1, 9);
   conv<16, 16>(net->g_d1, 16, 0, T + net->wboff[9], nullptr, net->g_d1a, 16, 0, nx, ny, nz, false, st);
-  relu_b(net->g_d1a, 16, 0, net->d1a, 16, 0, 16, n1);
+  mask(c16, net->g_d1a, 16, 0, net->d1a, 16, 0, n1, 8);
   conv_dw<48, 16>(net->cat1, 48, 0, net->g_d1a, 16, 0, G + net->woff[8], nx, ny, nz, st);
-  bias_g(net->g_d1a, 16, 0, 16, n1, 8);
   conv<16, 48>(net->g_d1a, 16, 0, T + net->wboff[8], nullptr, net->g_cat1, 48, 0, nx, ny, nz, false, st);
   // level 2 decoder
-  k_up_bwd<<<blocks_for(n2 * 32), 256, 0, st>>>(net->g_cat1, 48, 0, net->g_d2, 32, nx, ny, nz);
-  relu_b(net->g_d2, 32, 0, net->d2, 32, 0, 32, n2);
+  k_up_bwd<<<blocks_for(n2 * 4), 256, 0, st>>>(net->g_cat1, 48, 0, net->g_d2, 32, nx, ny, nz);
+  mask(c32, net->g_d2, 32, 0, net->d2, 32, 0, n2, 7);
   conv_dw<32, 32>(net->d2a, 32, 0, net->g_d2, 32, 0, G + net->woff[7], x2, y2, z2, st);
-  bias_g(net->g_d2, 32, 0, 32, n2, 7);
   conv<32, 32>(net->g_d2, 32, 0, T + net->wboff[7], nullptr, net->g_d2a, 32, 0, x2, y2, z2, false, st);
-  relu_b(net->g_d2a, 32, 0, net->d2a, 32, 0, 32, n2);
+  mask(c32, net->g_d2a, 32, 0, net->d2a, 32, 0, n2, 6);
   conv_dw<96, 32>(net->cat2, 96, 0, net->g_d2a, 32, 0, G + net->woff[6], x2, y2, z2, st);
-  bias_g(net->g_d2a, 32, 0, 32, n2, 6);
   conv<32, 96>(net->g_d2a, 32, 0, T + net->wboff[6], nullptr, net->g_cat2, 96, 0, x2, y2, z2, false, st);
   // level 3
-  k_up_bwd<<<blocks_for(n3 * 64), 256, 0, st>>>(net->g_cat2, 96, 0, net->g_e3, 64, x2, y2, z2);
-  relu_b(net->g_e3, 64, 0, net->e3, 64, 0, 64, n3);
+  k_up_bwd<<<blocks_for(n3 * 8), 256, 0, st>>>(net->g_cat2, 96, 0, net->g_e3, 64, x2, y2, z2);
+  mask(c64, net->g_e3, 64, 0, net->e3, 64, 0, n3, 5);
   conv_dw<64, 64>(net->a3, 64, 0, net->g_e3, 64, 0, G + net->woff[5], x3, y3, z3, st);
-  bias_g(net->g_e3, 64, 0, 64, n3, 5);
   conv<64, 64>(net->g_e3, 64, 0, T + net->wboff[5], nullptr, net->g_a3, 64, 0, x3, y3, z3, false, st);
-  relu_b(net->g_a3, 64, 0, net->a3, 64, 0, 64, n3);
+  mask(c64, net->g_a3, 64, 0, net->a3, 64, 0, n3, 4);
   conv_dw<32, 64>(net->p2, 32, 0, net->g_a3, 64, 0, G + net->woff[4], x3, y3, z3, st);
-  bias_g(net->g_a3, 64, 0, 64, n3, 4);
   conv<64, 32>(net->g_a3, 64, 0, T + net->wboff[4], nullptr, net->g_p2, 32, 0, x3, y3, z3, false, st);
   // level 2 encoder: e2 gradient = skip part + pooling part
-  k_pool_bwd_add<<<blocks_for(n2 * 32), 256, 0, st>>>(net->g_p2, net->g_cat2, 96, 64, 32, x2, y2, z2);
-  relu_b(net->g_cat2, 96, 64, net->cat2, 96, 64, 32, n2);
+  k_grad_mask<32, true><<<red_blocks(n2 * 4), 256, 0, st>>>(
+      net->g_cat2, 96, 64, net->cat2, 96, 64, net->g_p2, x2, y2, n2, G + net->boff[3]);
   conv_dw<32, 32>(net->a2, 32, 0, net->g_cat2, 96, 64, G + net->woff[3], x2, y2, z2, st);
-  bias_g(net->g_cat2, 96, 64, 32, n2, 3);
   conv<32, 32>(net->g_cat2, 96, 64, T + net->wboff[3], nullptr, net->g_a2, 32, 0, x2, y2, z2, false, st);
-  relu_b(net->g_a2, 32, 0, net->a2, 32, 0, 32, n2);
+  mask(c32, net->g_a2, 32, 0, net->a2, 32, 0, n2, 2);
   conv_dw<16, 32>(net->p1, 16, 0, net->g_a2, 32, 0, G + net->woff[2], x2, y2, z2, st);
-  bias_g(net->g_a2, 32, 0, 32, n2, 2);
   conv<32, 16>(net->g_a2, 32, 0, T + net->wboff[2], nullptr, net->g_p1, 16, 0, x2, y2, z2, false, st);
   // level 1 encoder: e1 gradient = skip part + pooling part
-  k_pool_bwd_add<<<blocks_for(n1 * 16), 256, 0, st>>>(net->g_p1, net->g_cat1, 48, 32, 16, nx, ny, nz);
-  relu_b(net->g_cat1, 48, 32, net->cat1, 48, 32, 16, n1);
+  k_grad_mask<16, true><<<red_blocks(n1 * 2), 256, 0, st>>>(
+      net->g_cat1, 48, 32, net->cat1, 48, 32, net->g_p1, nx, ny, n1, G + net->boff[1]);
   conv_dw<16, 16>(net->a1, 16, 0, net->g_cat1, 48, 32, G + net->woff[1], nx, ny, nz, st);
-  bias_g(net->g_cat1, 48, 32, 16, n1, 1);
   conv<16, 16>(net->g_cat1, 48, 32, T + net->wboff[1], nullptr, net->g_a1, 16, 0, nx, ny, nz, false, st);
-  relu_b(net->g_a1, 16, 0, net->a1, 16, 0, 16, n1);
+  mask(c16, net->g_a1, 16, 0, net->a1, 16, 0, n1, 0);
   conv_dw<16, 16>(net->x0, 16, 0, net->g_a1, 16, 0, G + net->woff[0], nx, ny, nz, st);
-  bias_g(net->g_a1, 16, 0, 16, n1, 0);
   FG_CUDA(cudaGetLastError());
   return FREHG_OK;
 }

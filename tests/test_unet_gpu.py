@@ -156,3 +156,33 @@ def test_flop_count(gpu_lib):
     n = 256 * 256 * 128
     per_cell = f.value / n
     assert 1.0e5 < per_cell < 2.0e5
+
+
+@pytest.mark.parametrize("shape", [(8, 20, 36), (20, 16, 4), (4, 36, 68), (36, 8, 16)])
+def test_gradients_at_tile_edges(gpu_lib, shape):
+    """Weight and bias gradients where the weight-gradient kernel's 16 x 16-pixel tiles and its z
+    columns (4 to 16 planes) end inside the grid, at all three levels.  Same bound as
+    test_forward_and_gradients_match_reference: the statement rounds to BF16 where the GPU
+    does, FP32 sums differ in order and BF16 ties."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(sum(shape))
+    r, lnk, tgt = (rng.standard_normal(shape).astype(np.float32) for _ in range(3))
+    cap = rng.uniform(0, 1, shape).astype(np.float32)
+    params = U.init_params(6)
+    h = net_with(gpu_lib, params)
+    nz, ny, nx = shape
+    tr, tk, tc, tt = dev(torch, r), dev(torch, lnk), dev(torch, cap), dev(torch, tgt)
+    loss = C.c_double()
+    g = np.zeros(params.size, dtype=np.float32)
+    assert gpu_lib.frehg_unet_loss_grad(h, nx, ny, nz, tr.data_ptr(), tk.data_ptr(),
+                                        tc.data_ptr(), tt.data_ptr(), C.byref(loss),
+                                        g.ctypes.data_as(C.POINTER(C.c_float)), None) == 0
+    lref, gref = U.loss_grad(params, r, lnk, cap, tgt)
+    assert abs(loss.value - lref) <= 1e-3 * abs(lref)
+    woff, boff, ooff, ntot = U.layout()
+    for l in range(10):
+        end = woff[l + 1] if l < 9 else ooff
+        for a, b in ((woff[l], boff[l]), (boff[l], end)):
+            assert np.linalg.norm(g[a:b] - gref[a:b]) <= 2e-2 * np.linalg.norm(gref[a:b]) + 1e-12, l
+    assert np.linalg.norm(g[ooff:] - gref[ooff:]) <= 2e-2 * np.linalg.norm(gref[ooff:])
+    gpu_lib.frehg_unet_destroy(h)
