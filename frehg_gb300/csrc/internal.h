@@ -248,15 +248,18 @@ class KrylovSolver {
   int rnorm_slot = 1;
   size_t cap_line = 0;
   float *lkf = nullptr, *dinvf = nullptr, *uf = nullptr;
-  // PCSOR (pc_type "sor", precision 0): 1/d, the preconditioned residual, iteration graph
-  int ensure_sor(size_t n);
-  size_t cap_sor = 0;
-  double *invd = nullptr, *zs = nullptr;
+  // PCSOR (pc_type "sor", precision 0): 1/d, the preconditioned residual, the sweeps' operands in
+  // the order its warps take them, iteration graph
+  int ensure_sor(size_t n, size_t slots);
+  size_t cap_sor = 0, cap_slots = 0;
+  double *invd = nullptr, *zs = nullptr, *sor_slots = nullptr;
   cudaGraphExec_t gsor = nullptr;
   const void* gsor_key = nullptr;
   const void* gsor_key2 = nullptr;
+  const void* gsor_key3 = nullptr;
   cudaStream_t gsor_stream = nullptr;
   size_t gsor_n = 0;
+  int gsor_dims[3] = {0, 0, 0};
   int g32_line = 0;
   const void* g32_key = nullptr;
   cudaStream_t g_stream = nullptr;

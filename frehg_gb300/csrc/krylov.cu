@@ -514,6 +514,7 @@ KrylovSolver::~KrylovSolver() {
   if (gsor) cudaGraphExecDestroy(gsor);
   cudaFree(invd);
   cudaFree(zs);
+  cudaFree(sor_slots);
   cudaFree(x);
   cudaFree(r);
   cudaFree(p);

@@ -10,17 +10,38 @@
 // with 1/d formed once as PETSc's MatSOR does (a zero diagonal entry taken as 1), the product
 // d y formed as y / (1/d), and the neighbour terms in the reference's column order.
 //
-// Lexicographic Gauss-Seidel is sequential in row order, but on the 7-point stencil a cell
-// depends only on its -1 neighbours along each axis (forward) or +1 neighbours (backward), so
-// all cells of one hyperplane a0 + a1 + a2 = w are independent once the planes before it are
-// done: sweeping the planes in order reproduces the sequential result exactly.  Small systems
-// run both sweeps in one block, the planes separated by __syncthreads (one launch per
-// application, no inter-block synchronisation); larger ones launch one kernel per plane, all
-// captured in the iteration graph.  The Krylov part is the unscaled PETSc KSPSolve_CG: the
-// operator keeps its diagonal (SOR needs D and L, not D^-1/2 A D^-1/2).
+// Evaluation.  With v = D y the two sweeps need one fused multiply-add per neighbour and cell:
+//   v_c = r_c - sum e_m v_m        (m the lower neighbours, e_m = a_m / d_m at the neighbour)
+//   z_c = v_c / d_c - sum e_c z_u  (u the upper neighbours, e_c = a_c / d_c at the cell)
+// with the same e = a / d for both, formed once per solve (a zero diagonal entry taken as 1, as
+// MatSOR does).  This is the same preconditioner as the product / difference / scaling sequence
+// of MatSOR to rounding; on GB300 a warp issues one FP64 instruction per 64 clocks however few of
+// its lanes are active, so the dependent FP64 instructions per cell are what the sweeps cost
+// (three instead of seven, and no division).
+//
+// Schedule.  A cell depends only on its lower (backward: upper) neighbours, so the sequential
+// order is a wavefront.  One warp owns a tile of 32 lines (lines run along the longest axis, the
+// tile spans the other two): in step t, lane (l1, l2) takes the cell at position t - l1 - l2 of
+// its line.  Neighbours inside the tile are the values two lanes computed one step earlier (warp
+// shuffles), the line's own previous value is a register, and the values of the neighbouring
+// tiles are read from memory, where the value itself is the signal that it is there: before a
+// sweep the array holds kSorWait (a NaN that no arithmetic produces), a reader repeats its load
+// until that is gone (bounded).  The loads run a group of steps ahead of
+// their use.  No barrier,
+// no fence and no flag: a handover costs one trip through the L2.
+//   n <= kSorSolveCells: the whole CG solve in one block with its vectors in shared memory.
+//   larger: one cooperative launch (all tiles' blocks resident) per preconditioner application
+//   and the CG kernels around it, captured as graphs.
+// Measured on GB300, one application (both sweeps): 405,000 cells (90 x 75 x 60) 244 us against
+// 1.1 ms for a launch per hyperplane; 4,096 cells 45 us; a whole solve of a 100-cell column
+// (four applications, three iterations) 59 us, of a 50 x 30 section 93 us, where one block with a
+// barrier and an L2 round trip per hyperplane took 168 and 228 us for each application.  A step
+// costs about 85 clocks per dependent FP64 instruction, a handover to the next tile about 10,000
+// clocks (the tile's skew, a group of steps and the trip through the L2).
 #include "internal.h"
 #include "reduce.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -28,134 +49,390 @@ namespace fg {
 
 namespace {
 
+// a quiet NaN with a payload: FP64 arithmetic on the device returns the canonical NaN, never this
+constexpr unsigned long long kSorWait = 0x7ff85eed5eed5eedull;
+constexpr long kSorPolls = 1L << 22;  // polls of one value before a sweep gives up (seconds)
+// largest system solved in one block: eight shared arrays of FP64 (64 bytes a cell, 227 KB)
+constexpr int kSorSolveCells = 3600;
+constexpr int kSorSolveThreads = 256;
+
 struct SorGeom {
+  // line axis, then the two tile axes: extents and strides
   int n[3];
-  size_t stride[3];
-  int ord[3];  // axes from the slowest to the fastest of the reference's row order
-  int w_end;   // number of hyperplanes, n0 + n1 + n2 - 2
+  long s[3];
+  int ax[3];     // which axis of the operator each is
+  int t1, t2;    // lines of a tile along the two tile axes (t1 t2 = 32)
+  int nb1, nb2;  // tiles along them
+  int steps;     // steps of a full tile
+  int axes;      // tile axes of more than one cell (one: the first)
 };
 
 SorGeom sor_geom(const Stencil64& A) {
+  const int n[3] = {A.n0, A.n1, A.n2};
+  const long st[3] = {1, A.n0, (long)A.n0 * A.n1};
+  int la = 0;
+  for (int q = 1; q < 3; ++q)
+    if (n[q] > n[la]) la = q;
+  int x1 = la == 0 ? 1 : 0, x2 = la == 2 ? 1 : 2;
+  if (n[x1] == 1) std::swap(x1, x2);  // an axis of one cell last
   SorGeom g;
-  g.n[0] = A.n0;
-  g.n[1] = A.n1;
-  g.n[2] = A.n2;
-  g.stride[0] = 1;
-  g.stride[1] = (size_t)A.n0;
-  g.stride[2] = (size_t)A.n0 * A.n1;
-  for (int q = 0; q < 3; ++q) g.ord[q] = A.ref_order[q];
-  g.w_end = A.n0 + A.n1 + A.n2 - 2;
+  const int ord[3] = {la, x1, x2};
+  for (int q = 0; q < 3; ++q) {
+    g.n[q] = n[ord[q]];
+    g.s[q] = st[ord[q]];
+    g.ax[q] = ord[q];
+  }
+  // 8 x 4 lines; along an axis with fewer than that, as many as it has (rounded up to a power of
+  // two), and the others along its partner
+  g.axes = (g.n[1] > 1) + (g.n[2] > 1);
+  g.t2 = 4;
+  while (g.t2 > 1 && g.t2 / 2 >= g.n[2]) g.t2 /= 2;
+  g.t1 = 32 / g.t2;
+  while (g.t1 > 8 && g.t2 < g.n[2] && g.t1 / 2 >= g.n[1]) {
+    g.t1 /= 2;
+    g.t2 *= 2;
+  }
+  while (g.t1 > 1 && g.t1 / 2 >= g.n[1] && g.t2 < g.n[2]) {
+    g.t1 /= 2;
+    g.t2 *= 2;
+  }
+  g.nb1 = (g.n[1] + g.t1 - 1) / g.t1;
+  g.nb2 = (g.n[2] + g.t2 - 1) / g.t2;
+  g.steps = g.n[0] + g.t1 + g.t2 - 2;
   return g;
 }
 
-__device__ __forceinline__ const double* coupling(const double* a0, const double* a1,
-                                                  const double* a2, int ax) {
-  return ax == 0 ? a0 : (ax == 1 ? a1 : a2);
+__device__ __forceinline__ double sor_peek(const double* p) {
+  return *reinterpret_cast<const volatile double*>(p);
 }
 
-// forward update of one cell: z_c = (r_c - sum of lower terms) * invd_c
-__device__ __forceinline__ void sor_fwd_cell(const SorGeom& g, const int (&idx)[3], size_t c,
-                                             const double* __restrict__ a0,
-                                             const double* __restrict__ a1,
-                                             const double* __restrict__ a2,
-                                             const double* __restrict__ invd,
-                                             const double* __restrict__ r, double* z) {
-  double sum = r[c];
+__device__ __forceinline__ bool sor_missing(double v) {
+  return __double2hiint(v) == (int)(kSorWait >> 32);
+}
+
+// The lane's line of a tile.  Loads of a lane outside its line (before its first and after its
+// last step) go to the line's end cells and are not used.
+struct SorLane {
+  int l1, l2;       // position in the tile
+  int x1, x2;       // the tile's extent (less than t1, t2 in the last tiles)
+  bool line;        // the lane has a line
+  int i1, i2;
+  __device__ __forceinline__ SorLane(const SorGeom& g, int b1, int b2) {
+    const int lane = threadIdx.x & 31;
+    l1 = lane % g.t1;
+    l2 = lane / g.t1;
+    x1 = min(g.t1, g.n[1] - b1 * g.t1);
+    x2 = min(g.t2, g.n[2] - b2 * g.t2);
+    line = l1 < x1 && l2 < x2;
+    i1 = b1 * g.t1 + (line ? l1 : 0);
+    i2 = b2 * g.t2 + (line ? l2 : 0);
+  }
+};
+
+// The operands of N consecutive steps of one lane: start value, couplings over d with the
+// neighbours one step back along the line and the two tile axes, the scale of the start value
+// (global form), and the values of neighbouring tiles.
+template <int N>
+struct SorSet {
+  double a[N], c0[N], c1[N], c2[N], w[N], f1[N], f2[N];
+};
+
+// One tile of one sweep by one warp.  In step q the lane takes position q - l1 - l2 of its line,
+// backward from the far ends in the reverse of the forward steps.  P loads the operands of a
+// step, tells where the neighbouring tiles' values are and takes the result.  Operands are loaded
+// a group of steps ahead into the other of two register sets; a group starts when the
+// neighbouring tiles' values it needs are there, so a wait costs a trip to the L2 per group and
+// not per step.  AXES: tile axes of more than one cell (one: the first); the products of the
+// others are left out.  Returns false when a wait ran out.
+template <bool FWD, int AXES, class P>
+__device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, const P& ops,
+                                         int* abort_word) {
+  constexpr int N = P::kGroup;
+  const int lane = threadIdx.x & 31;
+  const int steps = g.n[0] + L.x1 + L.x2 - 2;
+  const bool edge1 = FWD ? L.l1 == 0 : L.l1 == L.x1 - 1;
+  const bool edge2 = FWD ? L.l2 == 0 : L.l2 == L.x2 - 1;
+  const bool far1 = AXES > 0 && L.line && edge1 && (FWD ? L.i1 > 0 : L.i1 + 1 < g.n[1]);
+  const bool far2 = AXES > 1 && L.line && edge2 && (FWD ? L.i2 > 0 : L.i2 + 1 < g.n[2]);
+  const bool any_far = AXES > 0 && __any_sync(0xffffffffu, far1 || far2);
+  const int from1 = (FWD ? lane - 1 : lane + 1) & 31, from2 = (FWD ? lane - g.t1 : lane + g.t1) & 31;
+  // position of step 0, and per step; a lane without a line has no position in [0, len)
+  const int len = g.n[0], start = (FWD ? 0 : steps - 1) - L.l1 - L.l2;
+  const unsigned len_on = L.line ? (unsigned)len : 0u;
+  auto at = [&](int q) { return FWD ? start + q : start - q; };
+  auto clamp = [&](int i0) { return min(max(i0, 0), len - 1); };
+  auto fetch = [&](int q0, SorSet<N>& S) {
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const int ax = g.ord[q];
-    if (idx[ax] > 0) {
-      const size_t m = c - g.stride[ax];
-      sum = __dsub_rn(sum, __dmul_rn(coupling(a0, a1, a2, ax)[m], __ldcg(&z[m])));
+    for (int u = 0; u < N; ++u) {
+      const int i0 = at(q0 + u), ic = clamp(i0);
+      ops.template load<FWD, AXES>(min(q0 + u, steps - 1), steps, ic, S.a[u], S.c0[u], S.c1[u], S.c2[u],
+                                   S.w[u]);
+      if (any_far) {
+        S.f1[u] = far1 && (unsigned)i0 < len_on ? sor_peek(ops.template near1<FWD>(ic)) : 0.0;
+        if (AXES > 1)
+          S.f2[u] = far2 && (unsigned)i0 < len_on ? sor_peek(ops.template near2<FWD>(ic)) : 0.0;
+      } else {
+        S.f1[u] = 0.0;
+        S.f2[u] = 0.0;
+      }
     }
-  }
-  z[c] = __dmul_rn(sum, invd[c]);
-}
-
-// backward update: z_c = (z_c / invd_c - sum of upper terms) * invd_c
-__device__ __forceinline__ void sor_bwd_cell(const SorGeom& g, const int (&idx)[3], size_t c,
-                                             const double* __restrict__ a0,
-                                             const double* __restrict__ a1,
-                                             const double* __restrict__ a2,
-                                             const double* __restrict__ invd, double* z) {
-  const double id = invd[c];
-  double sum = __ddiv_rn(__ldcg(&z[c]), id);
+  };
+  auto missing = [&](const SorSet<N>& S) {
+    bool m = false;
 #pragma unroll
-  for (int q = 2; q >= 0; --q) {
-    const int ax = g.ord[q];
-    if (idx[ax] + 1 < g.n[ax]) {
-      sum = __dsub_rn(sum, __dmul_rn(coupling(a0, a1, a2, ax)[c], __ldcg(&z[c + g.stride[ax]])));
+    for (int u = 0; u < N; ++u) {
+      m = m || sor_missing(S.f1[u]);
+      if (AXES > 1) m = m || sor_missing(S.f2[u]);
+    }
+    return m;
+  };
+  bool ok = true;
+  double v = 0.0;
+  // the set's loads are complete and the neighbouring tiles' values there
+  auto arrive = [&](int q0, SorSet<N>& S) {
+    // a use of every operand: the next set's loads are issued only behind it.  A load's
+    // completion is tracked by one of a few counters; with both sets' loads outstanding on the
+    // same ones, the first use of this set would wait for the next set's as well, a trip to the L2
+    // per group (222 against 238 ns a step).
+    int t = 0;
+#pragma unroll
+    for (int u = 0; P::kGlobal && u < N; ++u) {
+      t ^= __double2loint(S.a[u]) ^ __double2loint(S.c0[u]);
+      if (AXES > 0) t ^= __double2loint(S.c1[u]);
+      if (AXES > 1) t ^= __double2loint(S.c2[u]);
+    }
+    if (P::kGlobal && t == 0x5eed5eed) __nanosleep(0);
+    if (any_far) {
+      for (long k = 0; ok && __any_sync(0xffffffffu, missing(S)); ++k) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+          const int ic = clamp(at(q0 + u));
+          if (sor_missing(S.f1[u])) S.f1[u] = sor_peek(ops.template near1<FWD>(ic));
+          if (AXES > 1 && sor_missing(S.f2[u])) S.f2[u] = sor_peek(ops.template near2<FWD>(ic));
+        }
+        // (warp-uniform: every lane sees the same k, and the abort word is voted on)
+        if (k > kSorPolls ||
+            ((k & 1023) == 1023 &&
+             __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(abort_word) != 0)))
+          ok = false;
+      }
+    }
+  };
+  auto compute = [&](int q0, SorSet<N>& S) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const int i0 = at(q0 + u);
+      double x = P::kGlobal && !FWD ? S.w[u] * S.a[u] : S.a[u];
+      // the line's first cell has no coupling back: v is still 0 there
+      x = fma(-S.c0[u], v, x);
+      if (AXES > 0) {
+        const double y = __shfl_sync(0xffffffffu, v, from1);
+        x = fma(-S.c1[u], edge1 ? S.f1[u] : y, x);
+      }
+      if (AXES > 1) {
+        const double y = __shfl_sync(0xffffffffu, v, from2);
+        x = fma(-S.c2[u], edge2 ? S.f2[u] : y, x);
+      }
+      const bool on = (unsigned)i0 < len_on;
+      v = on ? x : v;
+      if (on) ops.template store<FWD>(q0 + u, i0, x);
+    }
+  };
+  SorSet<N> A, B;
+  fetch(0, A);
+  for (int q0 = 0; q0 < steps && ok; q0 += 2 * N) {
+    arrive(q0, A);
+    fetch(q0 + N, B);
+    compute(q0, A);
+    arrive(q0 + N, B);
+    fetch(q0 + 2 * N, A);
+    compute(q0 + N, B);
+  }
+  return ok;
+}
+
+// the vectors in shared memory in cell order: src r (forward) or v / d, out v or z, e the couplings
+// over d
+struct SorShared {
+  static constexpr bool kGlobal = false;
+  static constexpr int kGroup = 2;  // 8 % faster than 4 on a 100-cell column
+  const double *src, *e0, *e1, *e2;  // e shifted to the neighbour's (forward)
+  double* out;
+  int first, s0, o1, o2;
+  __device__ __forceinline__ SorShared(bool fwd, const SorGeom& g, const SorLane& L,
+                                       const double* src_, const double* e0_, const double* e1_,
+                                       const double* e2_, double* out_)
+      : src(src_), e0(e0_), e1(e1_), e2(e2_), out(out_) {
+    s0 = (int)g.s[0];
+    o1 = fwd ? -(int)g.s[1] : (int)g.s[1];
+    o2 = fwd ? -(int)g.s[2] : (int)g.s[2];
+    first = L.i1 * (int)g.s[1] + L.i2 * (int)g.s[2];
+    if (fwd && L.i1 > 0) e1 += o1;
+    if (fwd && L.i2 > 0) e2 += o2;
+  }
+  template <bool FWD, int AXES>
+  __device__ __forceinline__ void load(int, int, int ic, double& a, double& c0, double& c1,
+                                       double& c2, double&) const {
+    const int c = first + s0 * ic;
+    a = src[c];
+    c0 = e0[FWD ? c - (ic > 0 ? s0 : 0) : c];
+    if (AXES > 0) c1 = e1[c];
+    if (AXES > 1) c2 = e2[c];
+  }
+  template <bool FWD>
+  __device__ __forceinline__ const double* near1(int ic) const { return out + (first + s0 * ic + o1); }
+  template <bool FWD>
+  __device__ __forceinline__ const double* near2(int ic) const { return out + (first + s0 * ic + o2); }
+  template <bool FWD>
+  __device__ __forceinline__ void store(int, int i0, double x) const {
+    *reinterpret_cast<volatile double*>(out + (first + s0 * i0)) = x;
+  }
+};
+
+// Larger systems keep the sweeps' operands in the order the warps take them ("slots"):
+// slot = (tile * steps + t) * 32 + lane, so a step's loads are consecutive.
+struct SorSlots {
+  double2* f01;  // forward: couplings over d with the line's previous cell and along tile axis 1
+  double* f2;    // and along tile axis 2 (0 where there is no neighbour)
+  double2* e01;  // backward, the same
+  double2* e2d;  // backward: along tile axis 2, and 1 / d
+  double* v;     // forward values
+};
+
+// The far neighbours' values: forward in the slot array (the last lane of the tile before took
+// the same position t1 - 1 or t2 - 1 steps later), backward in z.
+struct SorGlobal {
+  static constexpr bool kGlobal = true;
+  static constexpr int kGroup = 4;  // 2: 20 % slower, the loads' latency shows
+  const SorSlots& S;
+  const double* r;
+  double* z;
+  long first, s0, s1, s2;
+  size_t slot0;
+  const double *p1, *p2;
+  __device__ __forceinline__ SorGlobal(const SorSlots& S_, const SorGeom& g, const SorLane& L,
+                                       int tile, const double* r_, double* z_)
+      : S(S_), r(r_), z(z_) {
+    s0 = g.s[0];
+    s1 = g.s[1];
+    s2 = g.s[2];
+    first = (long)L.i1 * s1 + (long)L.i2 * s2;
+    slot0 = (size_t)tile * g.steps * 32 + (threadIdx.x & 31);
+    p1 = S.v + ((size_t)(tile - 1) * g.steps + (g.t1 - 1) + L.l2) * 32 + (g.t1 - 1) + g.t1 * L.l2;
+    p2 = S.v + ((size_t)(tile - g.nb1) * g.steps + (g.t2 - 1) + L.l1) * 32 + L.l1 +
+         g.t1 * (g.t2 - 1);
+  }
+  template <bool FWD, int AXES>
+  __device__ __forceinline__ void load(int q, int steps, int ic, double& a, double& c0, double& c1,
+                                       double& c2, double& w) const {
+    const size_t slot = slot0 + (size_t)(FWD ? q : steps - 1 - q) * 32;
+    if (FWD) {
+      a = __ldg(r + first + s0 * ic);
+      const double2 f = __ldg(S.f01 + slot);
+      c0 = f.x;
+      c1 = f.y;
+      if (AXES > 1) c2 = __ldg(S.f2 + slot);
+    } else {
+      a = S.v[slot];
+      const double2 e = __ldg(S.e01 + slot), d = __ldg(S.e2d + slot);
+      c0 = e.x;
+      c1 = e.y;
+      c2 = d.x;
+      w = d.y;
     }
   }
-  z[c] = __dmul_rn(sum, id);
-}
+  template <bool FWD>
+  __device__ __forceinline__ const double* near1(int ic) const {
+    return FWD ? p1 + 32L * ic : z + (first + s0 * ic + s1);
+  }
+  template <bool FWD>
+  __device__ __forceinline__ const double* near2(int ic) const {
+    return FWD ? p2 + 32L * ic : z + (first + s0 * ic + s2);
+  }
+  template <bool FWD>
+  __device__ __forceinline__ void store(int q, int i0, double x) const {
+    double* o = FWD ? S.v + slot0 + (size_t)q * 32 : z + first + s0 * i0;
+    *reinterpret_cast<volatile double*>(o) = x;
+  }
+};
 
-// cells of hyperplane w: one per (a1, a2) pair with a0 = w - a1 - a2 inside the box
-__device__ __forceinline__ bool plane_cell(const SorGeom& g, int w, long t, int (&idx)[3],
-                                           size_t& c) {
-  idx[1] = (int)(t % g.n[1]);
-  idx[2] = (int)(t / g.n[1]);
-  idx[0] = w - idx[1] - idx[2];
-  if (idx[0] < 0 || idx[0] >= g.n[0]) return false;
-  c = (size_t)idx[0] + g.stride[1] * idx[1] + g.stride[2] * idx[2];
-  return true;
-}
-
-// both sweeps in one block (small systems)
-__global__ void k_sor_block(SorGeom g, const double* __restrict__ a0,
-                            const double* __restrict__ a1, const double* __restrict__ a2,
-                            const double* __restrict__ invd, const double* __restrict__ r,
-                            double* z, const CgDevState* st) {
+// Both sweeps over all tiles, one warp per block, every block resident (cooperative launch).  A
+// block's tiles are in row order forward and in the reverse order backward, so each tile comes
+// after the tiles it reads from wherever they run.
+template <int AXES>
+__global__ void __launch_bounds__(32) k_sor_sweeps(SorGeom g, SorSlots S,
+                                                   const double* __restrict__ r, double* z,
+                                                   CgDevState* st) {
   if (st->status) return;
-  const long cols = (long)g.n[1] * g.n[2];
-  for (int w = 0; w < g.w_end + 1; ++w) {
-    for (long t = threadIdx.x; t < cols; t += blockDim.x) {
-      int idx[3];
-      size_t c;
-      if (plane_cell(g, w, t, idx, c)) sor_fwd_cell(g, idx, c, a0, a1, a2, invd, r, z);
-    }
-    __syncthreads();
+  const int tiles = g.nb1 * g.nb2;
+  bool ok = true;
+  int last = -1;
+  for (int b = blockIdx.x; b < tiles && ok; b += gridDim.x) {
+    const SorLane L(g, b % g.nb1, b / g.nb1);
+    ok = sor_tile<true, AXES>(g, L, SorGlobal(S, g, L, b, r, z), &st->bar_timeout);
+    last = b;
   }
-  for (int w = g.w_end; w >= 0; --w) {
-    for (long t = threadIdx.x; t < cols; t += blockDim.x) {
-      int idx[3];
-      size_t c;
-      if (plane_cell(g, w, t, idx, c)) sor_bwd_cell(g, idx, c, a0, a1, a2, invd, z);
-    }
-    __syncthreads();
+  __syncwarp();
+  for (int b = last; b >= 0 && ok; b -= gridDim.x) {
+    const SorLane L(g, b % g.nb1, b / g.nb1);
+    ok = sor_tile<false, AXES>(g, L, SorGlobal(S, g, L, b, r, z), &st->bar_timeout);
   }
-}
-
-// one hyperplane of one sweep (larger systems; one launch per plane)
-template <bool FWD>
-__global__ void k_sor_plane(SorGeom g, int w, const double* __restrict__ a0,
-                            const double* __restrict__ a1, const double* __restrict__ a2,
-                            const double* __restrict__ invd, const double* __restrict__ r,
-                            double* z, const CgDevState* st) {
-  if (st->status) return;
-  const long cols = (long)g.n[1] * g.n[2];
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < cols;
-       t += (long)gridDim.x * blockDim.x) {
-    int idx[3];
-    size_t c;
-    if (!plane_cell(g, w, t, idx, c)) continue;
-    if (FWD)
-      sor_fwd_cell(g, idx, c, a0, a1, a2, invd, r, z);
-    else
-      sor_bwd_cell(g, idx, c, a0, a1, a2, invd, z);
+  if (!ok && threadIdx.x == 0) {
+    atomicExch(&st->bar_timeout, 1);
+    atomicExch(&st->status, (int)kGridBarrierTimeout);
   }
 }
 
-// 1/d (a zero diagonal entry replaced by 1, MatSOR / PCJacobi), x = 0, r = b
+__device__ __forceinline__ double sor_wait_value() {
+  return __longlong_as_double((long long)kSorWait);
+}
+
+// 1/d (a zero diagonal entry replaced by 1, MatSOR / PCJacobi), x = 0, r = b, and z set to "not
+// there yet"
 __global__ void k_sor_prep(const double* __restrict__ d, const double* __restrict__ b,
                            double* __restrict__ invd, double* __restrict__ x,
-                           double* __restrict__ r, size_t n) {
+                           double* __restrict__ r, double* __restrict__ z, size_t n) {
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
     const double dc = d[c];
     invd[c] = 1.0 / (dc == 0.0 ? 1.0 : dc);
     x[c] = 0.0;
     r[c] = b[c];
+    z[c] = sor_wait_value();
+  }
+}
+
+// the sweeps' operands in slot order, and v set to "not there yet"; a0, a1, a2 in the order of the
+// geometry's axes
+__global__ void k_sor_slots(SorGeom g, SorSlots S, const double* __restrict__ a0,
+                            const double* __restrict__ a1, const double* __restrict__ a2,
+                            const double* __restrict__ invd, size_t slots) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < slots;
+       e += (size_t)gridDim.x * blockDim.x) {
+    const int lane = (int)(e & 31);
+    const unsigned row = (unsigned)(e >> 5), tile = row / (unsigned)g.steps;
+    const int t = (int)(row - tile * (unsigned)g.steps);
+    const int b1 = (int)(tile % (unsigned)g.nb1), b2 = (int)(tile / (unsigned)g.nb1);
+    const int l1 = lane % g.t1, l2 = lane / g.t1;
+    const int i0 = t - l1 - l2, i1 = b1 * g.t1 + l1, i2 = b2 * g.t2 + l2;
+    double2 f = make_double2(0.0, 0.0), h = f, w = f;
+    double f2 = 0.0;
+    if (i0 >= 0 && i0 < g.n[0] && i1 < g.n[1] && i2 < g.n[2]) {
+      const size_t c = (size_t)i0 * g.s[0] + (size_t)i1 * g.s[1] + (size_t)i2 * g.s[2];
+      const double id = invd[c];
+      if (i0 > 0) f.x = a0[c - g.s[0]] * invd[c - g.s[0]];
+      if (i1 > 0) f.y = a1[c - g.s[1]] * invd[c - g.s[1]];
+      if (i2 > 0) f2 = a2[c - g.s[2]] * invd[c - g.s[2]];
+      if (i0 + 1 < g.n[0]) h.x = a0[c] * id;
+      if (i1 + 1 < g.n[1]) h.y = a1[c] * id;
+      if (i2 + 1 < g.n[2]) w.x = a2[c] * id;
+      w.y = id;
+    }
+    S.f01[e] = f;
+    S.f2[e] = f2;
+    S.e01[e] = h;
+    S.e2d[e] = w;
+    S.v[e] = sor_wait_value();
   }
 }
 
@@ -164,6 +441,58 @@ __device__ __forceinline__ int sor_converged(CgDevState* s, double rnorm) {
   if (rnorm <= s->ttol) return rnorm < s->atol ? kConvergedAtol : kConvergedRtol;
   if (s->divtol > 0.0 && rnorm >= s->divtol * s->rnorm0) return kDivergedDtol;
   return 0;
+}
+
+// KSPSolve_CG's scalar steps after a preconditioner application (||z||^2 = zz, z.r = zr): the
+// stopping test and the next direction's coefficient; INIT: before the first iteration.
+template <bool INIT>
+__device__ __forceinline__ void sor_scalars(CgDevState* st, double zz, double zr) {
+  const double dp = sqrt(zz);
+  st->dp = dp;
+  if (INIT) {
+    st->rnorm0 = dp;
+    st->ttol = fmax(st->rtol * dp, st->atol);
+    st->its = 0;
+    st->iter = 0;
+    st->dpi = 0.0;
+    st->status = sor_converged(st, dp);
+    if (st->status) return;
+    st->beta = zr;
+    st->its = 1;
+    if (st->beta == 0.0) st->status = kConvergedAtol;
+    return;
+  }
+  const int reason = sor_converged(st, dp);
+  if (reason) {
+    st->status = reason;
+    return;
+  }
+  st->betaold = st->beta;
+  st->beta = zr;
+  st->iter += 1;
+  if (st->iter >= st->max_it) {
+    st->status = kDivergedIts;
+    return;
+  }
+  st->its = st->iter + 1;
+  if (st->beta == 0.0) {
+    st->status = kConvergedAtol;
+    return;
+  }
+  st->bcoef = st->beta / st->betaold;
+  if (st->bcoef < 0.0) st->status = kDivergedIndefinitePc;
+}
+
+// p.w known: the iteration's alpha, or the end of the solve
+__device__ __forceinline__ void sor_alpha(CgDevState* st, double dpi) {
+  st->its = st->iter + 1;
+  if (dpi == 0.0 || (st->iter > 0 && ((dpi > 0.0) != (st->dpi > 0.0))) || isnan(dpi)) {
+    st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
+    return;
+  }
+  st->dpiold = st->dpi;
+  st->dpi = dpi;
+  st->a = st->beta / dpi;
 }
 
 // ||z|| and beta = z.r after a preconditioner application; the last block runs
@@ -181,41 +510,7 @@ __global__ void k_sor_dots(const double* __restrict__ z, const double* __restric
   }
   double tot[2];
   if (!grid_sum<2>(v, partials, &st->arrive[3], tot)) return;
-  if (flat_tid() != 0) return;
-  const double dp = sqrt(tot[0]);
-  st->dp = dp;
-  if (INIT) {
-    st->rnorm0 = dp;
-    st->ttol = fmax(st->rtol * dp, st->atol);
-    st->its = 0;
-    st->iter = 0;
-    st->dpi = 0.0;
-    st->status = sor_converged(st, dp);
-    if (st->status) return;
-    st->beta = tot[1];
-    st->its = 1;
-    if (st->beta == 0.0) st->status = kConvergedAtol;
-    return;
-  }
-  const int reason = sor_converged(st, dp);
-  if (reason) {
-    st->status = reason;
-    return;
-  }
-  st->betaold = st->beta;
-  st->beta = tot[1];
-  st->iter += 1;
-  if (st->iter >= st->max_it) {
-    st->status = kDivergedIts;
-    return;
-  }
-  st->its = st->iter + 1;
-  if (st->beta == 0.0) {
-    st->status = kConvergedAtol;
-    return;
-  }
-  st->bcoef = st->beta / st->betaold;
-  if (st->bcoef < 0.0) st->status = kDivergedIndefinitePc;
+  if (flat_tid() == 0) sor_scalars<INIT>(st, tot[0], tot[1]);
 }
 
 // p = z (first iteration) or z + (beta/betaold) p
@@ -242,9 +537,9 @@ __global__ void __launch_bounds__(256) k_sor_spmv(const double* __restrict__ d,
   double acc[1] = {0.0};
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
-    const int i0 = (int)(c % s1);
-    const int i1 = (int)((c / s1) % n1);
-    const int i2 = (int)(c / s2);
+    const unsigned line = (unsigned)c / (unsigned)n0;  // fewer than 2^31 cells
+    const int i0 = (int)((unsigned)c - line * (unsigned)n0);
+    const int i2 = (int)(line / (unsigned)n1), i1 = (int)(line - (unsigned)i2 * (unsigned)n1);
     const double pc = p[c];
     double v = d[c] * pc;
     if (i0 > 0) v = fma(a0[c - 1], p[c - 1], v);
@@ -258,22 +553,13 @@ __global__ void __launch_bounds__(256) k_sor_spmv(const double* __restrict__ d,
   }
   double tot[1];
   if (!grid_sum<1>(acc, partials, &st->arrive[1], tot)) return;
-  if (flat_tid() == 0) {
-    const double dpi = tot[0];
-    st->its = st->iter + 1;
-    if (dpi == 0.0 || (st->iter > 0 && ((dpi > 0.0) != (st->dpi > 0.0))) || isnan(dpi)) {
-      st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
-      return;
-    }
-    st->dpiold = st->dpi;
-    st->dpi = dpi;
-    st->a = st->beta / dpi;
-  }
+  if (flat_tid() == 0) sor_alpha(st, tot[0]);
 }
 
-// x += a p, r -= a w
+// x += a p, r -= a w, and the sweeps' arrays set to "not there yet"
 __global__ void k_sor_update(double* __restrict__ x, double* __restrict__ r,
                              const double* __restrict__ p, const double* __restrict__ w,
+                             double* __restrict__ v, size_t slots, double* __restrict__ z,
                              size_t n, const CgDevState* st) {
   if (st->status) return;
   const double a = st->a;
@@ -281,45 +567,172 @@ __global__ void k_sor_update(double* __restrict__ x, double* __restrict__ r,
        c += (size_t)gridDim.x * blockDim.x) {
     x[c] = fma(a, p[c], x[c]);
     r[c] = fma(-a, w[c], r[c]);
+    z[c] = sor_wait_value();
+  }
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < slots;
+       c += (size_t)gridDim.x * blockDim.x)
+    v[c] = sor_wait_value();
+}
+
+// The whole solve of a small system in one block: the same iteration with every vector that the
+// sweeps or the neighbours read in shared memory (e, 1/d, r, v, z, p), the operator and x in
+// global memory (each thread its own cells).  w = A p lives where v does (v is written by the next
+// sweep).  x_out receives the solution of a converged solve.
+template <int AXES>
+__global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
+    SorGeom g, const double* __restrict__ d, const double* __restrict__ a0,
+    const double* __restrict__ a1, const double* __restrict__ a2, const double* __restrict__ b,
+    double* __restrict__ x, double* __restrict__ x_out, int n0, int n1, int n2, double rtol,
+    double atol, double divtol, int max_it, CgDevState* dst) {
+  extern __shared__ double sor_sh[];
+  __shared__ CgDevState st;
+  __shared__ double red[64];
+  const int n = n0 * n1 * n2, tid = threadIdx.x, warp = tid >> 5;
+  constexpr int kWarps = kSorSolveThreads / 32;
+  double *e0 = sor_sh, *e1 = e0 + n, *e2 = e1 + n, *invd = e2 + n, *r = invd + n, *v = r + n,
+         *z = v + n, *p = z + n;
+  // the couplings in the order of the geometry's axes
+  const double *g0 = sor_sh + g.ax[0] * n, *g1 = sor_sh + g.ax[1] * n, *g2 = sor_sh + g.ax[2] * n;
+  if (tid == 0) {
+    st.rtol = rtol;
+    st.atol = atol;
+    st.divtol = divtol;
+    st.max_it = max_it;
+    st.status = 0;
+    st.bar_timeout = 0;
+    st.bcoef = st.beta = st.betaold = st.dp = st.dpiold = 0.0;
+  }
+  for (int c = tid; c < n; c += kSorSolveThreads) {
+    const double dc = d[c];
+    const double id = 1.0 / (dc == 0.0 ? 1.0 : dc);
+    invd[c] = id;
+    e0[c] = a0[c] * id;
+    e1[c] = a1[c] * id;
+    e2[c] = a2[c] * id;
+    x[c] = 0.0;
+    r[c] = b[c];
+    v[c] = sor_wait_value();
+    z[c] = sor_wait_value();
+  }
+  __syncthreads();
+  const int tiles = g.nb1 * g.nb2;
+  // z = M r and (z.z, z.r) into the scalar steps; block-uniform
+  auto apply = [&](bool init) {
+    bool ok = true;
+    for (int t = warp; t < tiles && ok; t += kWarps) {
+      const SorLane L(g, t % g.nb1, t / g.nb1);
+      ok = sor_tile<true, AXES>(g, L, SorShared(true, g, L, r, g0, g1, g2, v), &st.bar_timeout);
+    }
+    if (!ok) atomicExch(&st.bar_timeout, 1);
+    __syncthreads();
+    // v / d by all threads: in the sweep it would be one more FP64 instruction per step
+    for (int c = tid; c < n; c += kSorSolveThreads) v[c] *= invd[c];
+    __syncthreads();
+    for (int t = warp + (tiles - 1 - warp) / kWarps * kWarps; warp < tiles && t >= 0 && ok;
+         t -= kWarps) {
+      const SorLane L(g, t % g.nb1, t / g.nb1);
+      ok = sor_tile<false, AXES>(g, L, SorShared(false, g, L, v, g0, g1, g2, z), &st.bar_timeout);
+    }
+    if (!ok) atomicExch(&st.bar_timeout, 1);
+    __syncthreads();
+    double s[2] = {0.0, 0.0};
+    for (int c = tid; c < n; c += kSorSolveThreads) {
+      s[0] = fma(z[c], z[c], s[0]);
+      s[1] = fma(z[c], r[c], s[1]);
+    }
+    block_sum<2>(s, red);
+    if (tid == 0) {
+      if (st.bar_timeout)
+        st.status = kGridBarrierTimeout;
+      else if (init)
+        sor_scalars<true>(&st, s[0], s[1]);
+      else
+        sor_scalars<false>(&st, s[0], s[1]);
+    }
+    __syncthreads();
+  };
+  apply(true);
+  const int s1 = n0, s2 = n0 * n1;
+  while (st.status == 0) {
+    const double bc = st.bcoef;
+    const bool first = st.iter == 0;
+    for (int c = tid; c < n; c += kSorSolveThreads) p[c] = first ? z[c] : fma(bc, p[c], z[c]);
+    __syncthreads();
+    double acc[1] = {0.0};
+    double* w = v;
+    for (int c = tid; c < n; c += kSorSolveThreads) {
+      const int i0 = c % n0, q = c / n0, i1 = q % n1, i2 = q / n1;
+      const double pc = p[c];
+      double y = d[c] * pc;
+      if (i0 > 0) y = fma(a0[c - 1], p[c - 1], y);
+      if (i0 + 1 < n0) y = fma(a0[c], p[c + 1], y);
+      if (i1 > 0) y = fma(a1[c - s1], p[c - s1], y);
+      if (i1 + 1 < n1) y = fma(a1[c], p[c + s1], y);
+      if (i2 > 0) y = fma(a2[c - s2], p[c - s2], y);
+      if (i2 + 1 < n2) y = fma(a2[c], p[c + s2], y);
+      w[c] = y;
+      acc[0] = fma(pc, y, acc[0]);
+    }
+    block_sum<1>(acc, red);
+    if (tid == 0) sor_alpha(&st, acc[0]);
+    __syncthreads();
+    if (st.status) break;
+    const double a = st.a;
+    for (int c = tid; c < n; c += kSorSolveThreads) {
+      x[c] = fma(a, p[c], x[c]);
+      r[c] = fma(-a, w[c], r[c]);
+      v[c] = sor_wait_value();
+      z[c] = sor_wait_value();
+    }
+    __syncthreads();
+    apply(false);
+  }
+  if (st.status > 0 && x_out != x)
+    for (int c = tid; c < n; c += kSorSolveThreads) x_out[c] = x[c];
+  if (tid == 0) {
+    dst->its = st.its;
+    dst->iter = st.iter;
+    dst->status = st.status;
+    dst->dp = st.dp;
+    dst->bar_timeout = st.bar_timeout;
   }
 }
 
-// systems up to this many unknowns sweep in one block
-constexpr size_t kSorBlockMax = 1u << 16;
+// blocks of a cooperative k_sor_sweeps launch: one per tile, at most what the device holds at once
+// (0: no cooperative launch)
+int sor_sweep_blocks(const SorGeom& g, const void* kernel) {
+  int dev = 0, coop = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (!coop) return 0;
+  return (int)std::min<long>((long)g.nb1 * g.nb2, (long)per_sm * sms);
+}
 
 }  // namespace
 
-int KrylovSolver::ensure_sor(size_t n) {
-  if (n <= cap_sor && invd) return FREHG_OK;
-  cudaFree(invd);
-  cudaFree(zs);
-  invd = zs = nullptr;
-  FG_CUDA(cudaMalloc(&invd, n * sizeof(double)));
-  FG_CUDA(cudaMalloc(&zs, n * sizeof(double)));
-  cap_sor = n;
-  return FREHG_OK;
-}
-
-// one preconditioner application r -> z on stream st
-static void sor_apply(const SorGeom& g, const Stencil64& A, const double* invd, const double* r,
-                      double* z, const CgDevState* dst, cudaStream_t st, Profiler* prof) {
-  const size_t n = A.n;
-  const long cols = (long)g.n[1] * g.n[2];
-  if (n <= kSorBlockMax) {
-    int bs = (int)((cols + 31) / 32 * 32);
-    bs = bs < 32 ? 32 : (bs > 1024 ? 1024 : bs);
-    FG_LAUNCH(prof, st, "k_sor_block", 56.0 * (double)n,
-              k_sor_block<<<1, bs, 0, st>>>(g, A.a0, A.a1, A.a2, invd, r, z, dst));
-    return;
+int KrylovSolver::ensure_sor(size_t n, size_t slots) {
+  if (n > cap_sor || !invd) {
+    cudaFree(invd);
+    cudaFree(zs);
+    invd = zs = nullptr;
+    cap_sor = 0;
+    FG_CUDA(cudaMalloc(&invd, n * sizeof(double)));
+    FG_CUDA(cudaMalloc(&zs, n * sizeof(double)));
+    cap_sor = n;
   }
-  const int nb = (int)((cols + 255) / 256);
-  for (int w = 0; w <= g.w_end; ++w)
-    FG_LAUNCH(prof, st, "k_sor_plane_fwd", 48.0 * (double)n / (g.w_end + 1),
-              k_sor_plane<true><<<nb, 256, 0, st>>>(g, w, A.a0, A.a1, A.a2, invd, r, z, dst));
-  for (int w = g.w_end; w >= 0; --w)
-    FG_LAUNCH(prof, st, "k_sor_plane_bwd", 48.0 * (double)n / (g.w_end + 1),
-              k_sor_plane<false><<<nb, 256, 0, st>>>(g, w, A.a0, A.a1, A.a2, invd, nullptr, z,
-                                                     dst));
+  if (slots > cap_slots || !sor_slots) {
+    cudaFree(sor_slots);
+    sor_slots = nullptr;
+    cap_slots = 0;
+    FG_CUDA(cudaMalloc(&sor_slots, slots * 8 * sizeof(double)));
+    cap_slots = slots;
+  }
+  return FREHG_OK;
 }
 
 int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_config& cfg,
@@ -329,8 +742,54 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     return FREHG_ERR_STATE;
   }
   const size_t n = A.n;
-  FG_TRY(ensure_sor(n));
   const SorGeom g = sor_geom(A);
+  const double dn = (double)n;
+  auto finish = [&]() -> int {
+    res->its = hst->its;
+    res->reason = hst->status;
+    res->rnorm = hst->dp;
+    res->inner_its = hst->its;
+    res->ir_its = 0;
+    if (hst->bar_timeout || hst->status == kGridBarrierTimeout) {
+      set_error("SOR sweep: a bounded wait for a neighbouring tile ran out after %d iterations",
+                hst->its);
+      return FREHG_ERR_CUDA;
+    }
+    if (hst->status < 0) {
+      set_error("KSP diverged (reason %d) after %d iterations, residual norm %g", hst->status,
+                hst->its, hst->dp);
+      return hst->status == kDivergedNanOrInf ? FREHG_ERR_NONFINITE : FREHG_ERR_NOT_CONVERGED;
+    }
+    return FREHG_OK;
+  };
+  if (n <= (size_t)kSorSolveCells) {
+    const int smem = 8 * (int)n * (int)sizeof(double);
+    // on every solve: the attribute belongs to the current device, and the call is cheap
+    auto kernel = g.axes == 2 ? k_sor_solve<2> : (g.axes == 1 ? k_sor_solve<1> : k_sor_solve<0>);
+    FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 8 * kSorSolveCells * (int)sizeof(double)));
+    FG_LAUNCH(prof, st, "k_sor_solve", 48.0 * dn,
+              kernel<<<1, kSorSolveThreads, smem, st>>>(
+                  g, A.s, A.a0, A.a1, A.a2, A.b, x, x_out ? x_out : x, A.n0, A.n1, A.n2, cfg.rtol,
+                  cfg.atol, 1.0e4, cfg.max_it, dst));
+    FG_CUDA(cudaGetLastError());
+    FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
+    FG_CUDA(cudaStreamSynchronize(st));
+    if (prof && prof->on) FG_TRY(prof->flush());
+    return finish();
+  }
+  const size_t slots = (size_t)g.nb1 * g.nb2 * g.steps * 32;
+  FG_TRY(ensure_sor(n, slots));
+  SorSlots S;
+  S.f01 = reinterpret_cast<double2*>(sor_slots);
+  S.e01 = S.f01 + slots;
+  S.e2d = S.e01 + slots;
+  S.f2 = reinterpret_cast<double*>(S.e2d + slots);
+  S.v = S.f2 + slots;
+  // one block (all tiles in order, nothing to wait for) where the device refuses cooperative
+  // launches
+  auto kernel = g.axes == 2 ? k_sor_sweeps<2> : (g.axes == 1 ? k_sor_sweeps<1> : k_sor_sweeps<0>);
+  const int sweep_blocks = coop_failed ? 1 : std::max(1, sor_sweep_blocks(g, (const void*)kernel));
   CgDevState init;
   memset(&init, 0, sizeof(init));
   init.rtol = cfg.rtol;
@@ -339,44 +798,69 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   init.max_it = cfg.max_it;
   FG_CUDA(cudaMemcpyAsync(dst, &init, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
   const int nb = reduction_blocks(n, 256, 4);
-  const double dn = (double)n;
   double* xs = x;  // the graph keeps fixed pointers; x_out receives a copy
-  FG_LAUNCH(prof, st, "k_sor_prep", 40.0 * dn,
-            k_sor_prep<<<nb, 256, 0, st>>>(A.s, A.b, invd, xs, r, n));
-  sor_apply(g, A, invd, r, zs, dst, st, prof);
+  auto sweeps = [&](cudaStream_t s) -> cudaError_t {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)sweep_blocks);
+    lc.blockDim = dim3(32);
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = sweep_blocks > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, kernel, g, S, (const double*)r, zs, dst);
+  };
+  FG_LAUNCH(prof, st, "k_sor_prep", 48.0 * dn,
+            k_sor_prep<<<nb, 256, 0, st>>>(A.s, A.b, invd, xs, r, zs, n));
+  const double* ax[3] = {A.a0, A.a1, A.a2};
+  FG_LAUNCH(prof, st, "k_sor_slots", 32.0 * dn + 64.0 * (double)slots,
+            k_sor_slots<<<reduction_blocks(slots, 256, 1), 256, 0, st>>>(
+                g, S, ax[g.ax[0]], ax[g.ax[1]], ax[g.ax[2]], invd, slots));
+  cudaError_t le = cudaSuccess;
+  FG_LAUNCH(prof, st, "k_sor_sweeps", 16.0 * dn + 72.0 * (double)slots, le = sweeps(st));
+  if (le != cudaSuccess && sweep_blocks > 1) {
+    cudaGetLastError();
+    coop_failed = true;
+    return solve_sor(A, x_out, cfg, st, res);
+  }
+  FG_CUDA(le);
   FG_LAUNCH(prof, st, "k_sor_dots", 16.0 * dn,
             k_sor_dots<true><<<nb, 256, 0, st>>>(zs, r, n, dst, partials));
   FG_CUDA(cudaGetLastError());
 
   // one iteration: p, w = A p (alpha), x/r update, z = M r, norms and beta
-  auto iteration = [&](cudaStream_t s, Profiler* pr) {
+  auto iteration = [&](cudaStream_t s, Profiler* pr) -> int {
     FG_LAUNCH(pr, s, "k_sor_p", 24.0 * dn, k_sor_p<<<nb, 256, 0, s>>>(zs, p, n, dst));
     FG_LAUNCH(pr, s, "k_sor_spmv", 48.0 * dn,
               k_sor_spmv<<<nb, 256, 0, s>>>(A.s, A.a0, A.a1, A.a2, p, w, A.n0, A.n1, A.n2, dst,
                                             partials));
-    FG_LAUNCH(pr, s, "k_sor_update", 48.0 * dn,
-              k_sor_update<<<nb, 256, 0, s>>>(xs, r, p, w, n, dst));
-    sor_apply(g, A, invd, r, zs, dst, s, pr);
+    FG_LAUNCH(pr, s, "k_sor_update", 56.0 * dn + 8.0 * (double)slots,
+              k_sor_update<<<nb, 256, 0, s>>>(xs, r, p, w, S.v, slots, zs, n, dst));
+    FG_LAUNCH(pr, s, "k_sor_sweeps", 16.0 * dn + 72.0 * (double)slots, FG_CUDA(sweeps(s)));
     FG_LAUNCH(pr, s, "k_sor_dots", 16.0 * dn,
               k_sor_dots<false><<<nb, 256, 0, s>>>(zs, r, n, dst, partials));
+    return FREHG_OK;
   };
-  const int per_it = 4 + (n <= kSorBlockMax ? 1 : 2 * (g.w_end + 1));
-  int chunk = 4096 / per_it;
-  chunk = chunk < 1 ? 1 : (chunk > 32 ? 32 : chunk);
+  // iterations between two reads of the status: few, as a solve takes from 1 to a few tens of
+  // iterations and an idle one costs five launches (about 6 us)
+  const int per_it = 5, chunk = 4;
 
-  FG_CUDA(cudaMemcpyAsync(hst, dst, sizeof(CgDevState), cudaMemcpyDeviceToHost, st));
+  FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
   FG_CUDA(cudaStreamSynchronize(st));
   if (prof && prof->on) {
+    FG_TRY(prof->flush());
     for (int q = 0; q < cfg.max_it + 1 && hst->status == 0; ++q) {
-      iteration(st, prof);
+      FG_TRY(iteration(st, prof));
       FG_CUDA(cudaGetLastError());
-      FG_CUDA(cudaMemcpyAsync(hst, dst, sizeof(CgDevState), cudaMemcpyDeviceToHost, st));
+      FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
       FG_CUDA(cudaStreamSynchronize(st));
       FG_TRY(prof->flush());
     }
   } else if (hst->status == 0) {
-    const bool rebuild = !gsor || gsor_key != (const void*)A.a0 || gsor_key2 != (const void*)invd ||
-                         gsor_stream != st || gsor_n != n;
+    const int dims[3] = {A.n0, A.n1, A.n2};
+    const bool rebuild = !gsor || gsor_key != (const void*)A.a0 || gsor_key2 != (const void*)sor_slots || gsor_key3 != (const void*)invd ||
+                         gsor_stream != st || gsor_n != n || memcmp(gsor_dims, dims, sizeof(dims));
     if (rebuild) {
       if (gsor) cudaGraphExecDestroy(gsor);
       gsor = nullptr;
@@ -384,11 +868,14 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
       FG_CUDA(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking));
       cudaGraph_t graph;
       FG_CUDA(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
-      for (int q = 0; q < chunk; ++q) iteration(cap_st, nullptr);
+      int rc = FREHG_OK;
+      for (int q = 0; q < chunk && rc == FREHG_OK; ++q) rc = iteration(cap_st, nullptr);
       cudaError_t e = cudaStreamEndCapture(cap_st, &graph);
       cudaStreamDestroy(cap_st);
-      if (e != cudaSuccess) {
-        set_error("SOR graph capture failed: %s", cudaGetErrorString(e));
+      if (rc != FREHG_OK || e != cudaSuccess) {
+        if (rc == FREHG_OK) set_error("SOR graph capture failed: %s", cudaGetErrorString(e));
+        else if (e == cudaSuccess) cudaGraphDestroy(graph);
+        cudaGetLastError();
         return FREHG_ERR_CUDA;
       }
       e = cudaGraphInstantiate(&gsor, graph, 0);
@@ -398,16 +885,18 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
         return FREHG_ERR_CUDA;
       }
       gsor_key = A.a0;
-      gsor_key2 = invd;
+      gsor_key2 = sor_slots;
+      gsor_key3 = invd;
       gsor_stream = st;
       gsor_n = n;
+      memcpy(gsor_dims, dims, sizeof(dims));
     }
     const int max_launch = cfg.max_it / chunk + 2;
     int q = 0;
     for (; q < max_launch; ++q) {
       FG_CUDA(cudaGraphLaunch(gsor, st));
       if (prof) prof->launches += (int64_t)per_it * chunk;
-      FG_CUDA(cudaMemcpyAsync(hst, dst, sizeof(CgDevState), cudaMemcpyDeviceToHost, st));
+      FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
       FG_CUDA(cudaStreamSynchronize(st));
       if (hst->status != 0) break;
     }
@@ -417,16 +906,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
       return FREHG_ERR_STATE;
     }
   }
-  res->its = hst->its;
-  res->reason = hst->status;
-  res->rnorm = hst->dp;
-  res->inner_its = hst->its;
-  res->ir_its = 0;
-  if (hst->status < 0) {
-    set_error("KSP diverged (reason %d) after %d iterations, residual norm %g", hst->status,
-              hst->its, hst->dp);
-    return hst->status == kDivergedNanOrInf ? FREHG_ERR_NONFINITE : FREHG_ERR_NOT_CONVERGED;
-  }
+  FG_TRY(finish());
   if (x_out && x_out != x)
     FG_CUDA(cudaMemcpyAsync(x_out, x, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
   return FREHG_OK;
