@@ -145,7 +145,9 @@ struct CgDevState {
   // the flag a block sets when its bounded wait ran out
   unsigned int bar_count, bar_gen;
   int bar_timeout;
-  int pad_;
+  // inner FP32 solve: below ttol_soft (0: unused) it runs kSoftIterations more at most towards ttol
+  int soft_its;
+  double ttol_soft;
 };
 
 // KSPConvergedReason values

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) k_ir_residual(
       ir->rscale = rs0;
       in->beta = tot[0];
       in->rnorm0 = sqrt(tot[0]);
-      in->ttol = inner_rtol * in->rnorm0;
+      set_inner_tolerance<INV_S>(in, inner_rtol, rn, fmax(ir_rtol * ir->ir_bnorm, ir->atol));
       in->iter = 0;
       in->its = 0;
       in->dpi = 0.0;
@@ -447,7 +447,7 @@ __global__ void k32_update(float* __restrict__ e, float* __restrict__ r,
     st->iter += 1;
     if (isnan(rn)) {
       st->status = kDivergedNanOrInf;
-    } else if (rn <= st->ttol) {
+    } else if (inner_converged(st, rn)) {
       st->status = kConvergedRtol;
     } else if (st->iter >= st->max_it) {
       st->status = kDivergedIts;
