@@ -139,8 +139,9 @@ struct CgDevState {
   unsigned int arrive[8];
   double ir_bnorm, ir_rnorm;  // refinement loop norms (mixed precision)
   double rscale;              // the inner right-hand side is r~ / rscale (mixed precision)
-  int ir_its;
-  int rhs_rescale;  // k_prep_ff: its power-of-two scaled right-hand side needs k_ir_scale instead
+  int ir_its;       // complete refinement sweeps (its: their inner iterations)
+  int pad_;
+  double first_a;   // ||r~|| of the first sweep
   // grid barrier of the one-launch CG iteration (k_cg_iter): arrival count, generation, and
   // the flag a block sets when its bounded wait ran out
   unsigned int bar_count, bar_gen;
@@ -159,8 +160,11 @@ enum {
   kDivergedIndefinitePc = -8,
   kDivergedNanOrInf = -9,
   kDivergedIndefiniteMat = -10,
-  // not a PETSc reason: a grid barrier of the one-launch CG iteration did not complete in time
+  // not PETSc reasons: a grid barrier of the one-launch CG iteration did not complete in time;
+  // k_prep_ff's power-of-two scaled right-hand side left the FP32 margin and has to be formed in
+  // FP64 (k_ir_residual<true>, k_ir_scale)
   kGridBarrierTimeout = -90,
+  kRescaleRhs = 1,
 };
 
 struct CgResult {
@@ -216,7 +220,6 @@ class KrylovSolver {
   // graphs
   cudaGraphExec_t g64 = nullptr;
   cudaGraphExec_t g32 = nullptr;
-  cudaGraphExec_t g32s = nullptr;  // first, short chunk of the inner solve
   const void* g64_key = nullptr;
   const void* g64_key2 = nullptr;
   // the FP64 Jacobi-PCG iteration as one cooperative launch (k_cg_iter) rather than three
@@ -237,19 +240,21 @@ class KrylovSolver {
   bool keep_scaled = false;
   const double* scale_vector(const Stencil64& A) const { return A.s_in_r ? r : A.s; }
   float* zf = nullptr;
-  // vertical-line preconditioner (FP32 factors and sweep scratch)
+  // vertical-line preconditioner (FP32 factors, the preconditioned residual, the direction's second
+  // buffer)
   int ensure_line(size_t n);
   // scaling of the operator for the mixed path (sq = D^1/2 into r, FP32 copy, line factors)
   int prep_mixed(Stencil64& A, cudaStream_t st, bool line, const frehg_solver_config& cfg);
   bool first_done = false;  // prep_mixed formed the first refinement residual and its state
-  bool first_line_done = false;  // ... and the line preconditioner's first application
   // first residual norms of earlier solves, the scale of the next one's: slot 0 for the first
   // solve of a time step (its residual is orders of magnitude above the previous step's last
   // one), slot 1 for the later (Picard) solves; the caller picks the slot
   double first_rnorm[2] = {0.0, 0.0};
   int rnorm_slot = 1;
+  // inner iterations launched at once: what recent first and later sweeps took
+  int spec32[2] = {1, 1};
   size_t cap_line = 0;
-  float *lkf = nullptr, *dinvf = nullptr, *uf = nullptr;
+  float *lkf = nullptr, *dinvf = nullptr, *uf = nullptr, *pf2 = nullptr;
   // PCSOR (pc_type "sor", precision 0): 1/d, the preconditioned residual, the sweeps' operands in
   // the order its warps take them, iteration graph
   int ensure_sor(size_t n, size_t slots);
@@ -262,7 +267,6 @@ class KrylovSolver {
   cudaStream_t gsor_stream = nullptr;
   size_t gsor_n = 0;
   int gsor_dims[3] = {0, 0, 0};
-  int g32_line = 0;
   const void* g32_key = nullptr;
   cudaStream_t g_stream = nullptr;
   size_t g_n = 0;
@@ -296,6 +300,9 @@ int reduction_blocks(size_t n, int threads, int per_thread);
 // alloc_mapped), so that they do not queue on the copy engines behind a bulk result copy in
 // flight.  The caller synchronises st before reading.  bytes: a multiple of 4.
 int fetch_small(void* host_mapped, const void* dev, size_t bytes, cudaStream_t st);
+// two of them by one launch, of the same size
+int fetch_small2(void* host_mapped, const void* dev, void* host_mapped2, const void* dev2,
+                 size_t bytes, cudaStream_t st);
 int alloc_mapped(void** host, size_t bytes);
 
 }  // namespace fg

@@ -88,6 +88,29 @@ int fetch_small(void* host_mapped, const void* dev, size_t bytes, cudaStream_t s
   return FREHG_OK;
 }
 
+namespace {
+__global__ void k_fetch_words2(const unsigned* __restrict__ src, unsigned* __restrict__ dst,
+                               const unsigned* __restrict__ src2, unsigned* __restrict__ dst2,
+                               int words) {
+  for (int i = threadIdx.x; i < words; i += blockDim.x) {
+    dst[i] = src[i];
+    dst2[i] = src2[i];
+  }
+}
+}  // namespace
+
+int fetch_small2(void* host_mapped, const void* dev, void* host_mapped2, const void* dev2,
+                 size_t bytes, cudaStream_t st) {
+  void *d = nullptr, *d2 = nullptr;
+  FG_CUDA(cudaHostGetDevicePointer(&d, host_mapped, 0));
+  FG_CUDA(cudaHostGetDevicePointer(&d2, host_mapped2, 0));
+  k_fetch_words2<<<1, 32, 0, st>>>(static_cast<const unsigned*>(dev), static_cast<unsigned*>(d),
+                                   static_cast<const unsigned*>(dev2), static_cast<unsigned*>(d2),
+                                   (int)(bytes / 4));
+  FG_CUDA(cudaGetLastError());
+  return FREHG_OK;
+}
+
 int reduction_blocks(size_t n, int threads, int per_thread) {
   size_t b = (n + (size_t)threads * per_thread - 1) / ((size_t)threads * per_thread);
   if (b < 1) b = 1;
@@ -510,7 +533,6 @@ void Stencil32::release() {
 KrylovSolver::~KrylovSolver() {
   if (g64) cudaGraphExecDestroy(g64);
   if (g32) cudaGraphExecDestroy(g32);
-  if (g32s) cudaGraphExecDestroy(g32s);
   if (gsor) cudaGraphExecDestroy(gsor);
   cudaFree(invd);
   cudaFree(zs);
@@ -533,6 +555,7 @@ KrylovSolver::~KrylovSolver() {
   cudaFree(lkf);
   cudaFree(dinvf);
   cudaFree(uf);
+  cudaFree(pf2);
   op32.release();
 }
 

@@ -14,18 +14,19 @@
 // r . z = sum_k y_k^2 / d_k = sum_k y_k u_k comes out of the forward sweep, so the backward
 // sweep needs neither r nor a reduction and can form the next search direction in place.
 //
-// PCG iteration (3 kernels, no separate direction kernel):
-//   k32_spmv_v4 / k32_spmv : w = A~ p,  alpha = (r.z) / (p.w)
-//   k32_line_fwd<true>     : x += alpha p, r -= alpha w, u = D^-1 L^-1 r, r.z, r.r, test, beta
-//   k32_line_bwd           : z = L^-T u and p = z + beta p in the same sweep
+// PCG iteration, two kernels:
+//   k32_dir_spmv(_v4) : p = z + beta p_old and w = A~ p in one pass (the neighbours' directions are
+//                       formed again from z and p_old, so p goes from one buffer into the other),
+//                       alpha = (r.z) / (p.w)
+//   k32_line_step     : x += alpha p, r -= alpha w, z = M^-1 r with both sweeps, r.z, r.r, test, beta
 #pragma once
 
 #include "internal.h"
 #include "reduce.cuh"
 
-namespace fg {
+#include <algorithm>
 
-constexpr int kLineBatch = 4;  // levels whose loads are issued together
+namespace fg {
 
 // The inner solve's tolerance in a refinement sweep whose true residual is rn (target: the
 // refinement's own).  A sweep that can end the refinement aims at it: kSweepMargin below the
@@ -37,7 +38,7 @@ constexpr int kLineBatch = 4;  // levels whose loads are issued together
 // On the 768x768x96 combined workload (line solve: one iteration reduces the residual by about
 // 1e-6) a third sweep, 1.8 ms, was needed in 14 of 26 solves because the second ended 2 to 30
 // times above the target; on 256x256x128 loam that sweep took 5 to 26 inner iterations for a
-// factor 1e-4 where 2 was missing (three steps: 52.1 -> 46.5 ms; the combined workload 273 -> 266).
+// factor 1e-4 where 2 was missing (two steps: 52.1 -> 46.5 ms; the combined workload 273 -> 266).
 constexpr double kSweepMargin = 0.1;
 constexpr double kSweepReach = 1e-7;
 constexpr int kSoftIterations = 2;
@@ -87,128 +88,250 @@ __global__ void k_line_factor(const double* __restrict__ a2, float* __restrict__
   }
 }
 
-// Forward sweep.  UPDATE: first x += alpha p, r -= alpha w (the CG update of this iteration);
-// then u = D^-1 L^-1 r and the sums r.z (as y.u) and r.r.  The last block runs the inner
-// convergence test (on ||r||) and forms beta = (r.z)_new / (r.z)_old.  Without UPDATE it is
-// the initial application: st->beta = r0.z0.
-template <bool UPDATE>
-__global__ void __launch_bounds__(128) k32_line_fwd(float* __restrict__ x, float* __restrict__ r,
-                                                    const float* __restrict__ p,
-                                                    const float* __restrict__ w,
-                                                    const float* __restrict__ lk,
-                                                    const float* __restrict__ dinv,
-                                                    float* __restrict__ u, int ncol, int nz,
-                                                    CgDevState* st, double* partials) {
+// The scalar end of k32_line_step (last block).  FIRST: the first application, z0 = M^-1 r0.
+template <bool FIRST>
+__device__ __forceinline__ void line_step_tail(CgDevState* st, double rzn, double rr) {
+  if (FIRST) {
+    st->beta = rzn;
+    st->bcoef = 0.0;
+    if (!(rzn > 0.0)) st->status = rzn == 0.0 ? kConvergedAtol : kDivergedIndefinitePc;
+    return;
+  }
+  const double rn = sqrt(rr);
+  st->dp = rn;
+  st->iter += 1;
+  if (isnan(rn) || isnan(rzn)) {
+    st->status = kDivergedNanOrInf;
+  } else if (inner_converged(st, rn)) {
+    st->status = kConvergedRtol;
+  } else if (st->iter >= st->max_it) {
+    st->status = kDivergedIts;
+  } else if (!(rzn > 0.0)) {
+    st->status = kDivergedIndefinitePc;
+  } else {
+    st->bcoef = rzn / st->beta;
+    st->beta = rzn;
+    st->its = st->iter + 1;
+  }
+}
+
+// FIRST: z = M^-1 r.  Else the CG update x += alpha p, r -= alpha w, then z = M^-1 r.
+// p0, p1: the direction's two buffers; iteration `iter` wrote p1 when iter is even.
+// A block owns 32 neighbouring columns; its W warps split the levels, each thread
+// holding its at most L levels of r, l, 1/d in registers, so that all of a column's loads are in
+// flight at once (a march down the column with one thread has a few levels in flight and needs
+// more columns than small grids have).  Both sweeps are affine recurrences: a warp runs its
+// levels with a zero carry and the product of the factors, the warps' ends are combined through
+// shared memory (W - 1 steps), and the carry's share is added.  36 B/cell.
+// 768 x 768 x 96: 324 us, 0.93 of the copy peak (the two sweeps as marches with one thread per
+// column were 318 + 157, and 28 of 36 bytes more); 256 x 256 x 128: 72 us against 69 + 40.  16
+// warps: 8 with twice the levels fit fewer blocks (573 us), 32 lengthen the carry's chain (610).
+template <bool FIRST, int W, int L>
+__global__ void __launch_bounds__(32 * W, L > 8 ? 1 : 2) k32_line_step(
+    float* __restrict__ x, float* __restrict__ r, const float* __restrict__ p0,
+    const float* __restrict__ p1, const float* __restrict__ w, const float* __restrict__ lk,
+    const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
+    double* partials) {
   if (st->status) return;
-  const float a = UPDATE ? (float)st->a : 0.0f;
-  // the first update writes x = alpha p (x is not initialised)
-  const bool xfirst = UPDATE && st->iter == 0;
+  __shared__ float2 fwd[W][32], bwd[W][32];
+  __shared__ float lfirst[W + 1][32];
+  const float a = FIRST ? 0.0f : (float)st->a;
+  const int iter = st->iter;
+  const float* p = (iter & 1) ? p0 : p1;
+  const bool xfirst = iter == 0;  // the first update writes x = alpha p (x is not initialised)
   const size_t sk = (size_t)ncol;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int len = (nz + W - 1) / W;  // levels per warp, <= L
+  const int k0 = warp * len, nk = max(0, min(len, nz - k0));
+  if (warp == 0) lfirst[W][lane] = 0.0f;
   Kahan32 rz, rr;
-  for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
-       col += gridDim.x * blockDim.x) {
-    float y = 0.0f;
-    for (int k0 = 0; k0 < nz; k0 += kLineBatch) {
-      float rv[kLineBatch], lv[kLineBatch], dv[kLineBatch], xv[kLineBatch], pv[kLineBatch],
-          wv[kLineBatch];
+  const int groups = (ncol + 31) / 32;
+  // FIRST: the next group's loads are issued before this group's sweeps (the update has its own
+  // loads in flight then, and no registers to spare)
+  float ny[FIRST ? L : 1], nl[FIRST ? L : 1], nd[FIRST ? L : 1];
+  auto load = [&](int g, float* ry, float* rl, float* rd) {
+    const int col = g * 32 + lane;
+    const int n = col < ncol ? nk : 0;
+    const size_t base = (size_t)min(col, ncol - 1) + sk * min(k0, nz - 1);
 #pragma unroll
-      for (int q = 0; q < kLineBatch; ++q) {
-        if (k0 + q < nz) {
-          const size_t c = (size_t)col + sk * (k0 + q);
-          rv[q] = r[c];
-          lv[q] = lk[c];
-          dv[q] = dinv[c];
-          if (UPDATE) {
-            xv[q] = xfirst ? 0.0f : x[c];
-            pv[q] = p[c];
-            wv[q] = w[c];
-          }
+    for (int q = 0; q < L; ++q) {
+      ry[q] = rl[q] = rd[q] = 0.0f;
+      if (q < n) {
+        const size_t c = base + sk * q;
+        ry[q] = r[c];
+        rl[q] = lk[c];
+        rd[q] = dinv[c];
+      }
+    }
+  };
+  if (FIRST) load(blockIdx.x, ny, nl, nd);
+  for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+    const int col = g * 32 + lane;
+    const int n = col < ncol ? nk : 0;
+    const size_t base = (size_t)min(col, ncol - 1) + sk * min(k0, nz - 1);
+    float y[L], l[L], d[L];
+    if (FIRST) {
+#pragma unroll
+      for (int q = 0; q < L; ++q) {
+        y[q] = ny[FIRST ? q : 0];
+        l[q] = nl[FIRST ? q : 0];
+        d[q] = nd[FIRST ? q : 0];
+      }
+      if (g + (int)gridDim.x < groups) load(g + gridDim.x, ny, nl, nd);
+    } else {
+      load(g, y, l, d);
+    }
+    if (!FIRST) {
+      // all loads before the first store: the compiler may not move them across it
+      float pv[L], wv[L], xv[L];
+#pragma unroll
+      for (int q = 0; q < L; ++q) {
+        pv[q] = wv[q] = xv[q] = 0.0f;
+        if (q < n) {
+          const size_t c = base + sk * q;
+          pv[q] = p[c];
+          wv[q] = w[c];
+          if (!xfirst) xv[q] = x[c];
         }
       }
 #pragma unroll
-      for (int q = 0; q < kLineBatch; ++q) {
-        if (k0 + q < nz) {
-          const size_t c = (size_t)col + sk * (k0 + q);
-          float rk = rv[q];
-          if (UPDATE) {
-            x[c] = fmaf(a, pv[q], xv[q]);
-            rk = fmaf(-a, wv[q], rk);
-            r[c] = rk;
-          }
-          y = fmaf(-lv[q], y, rk);
-          const float uk = y * dv[q];
-          u[c] = uk;
-          rz.add(y * uk);
-          rr.add(rk * rk);
+      for (int q = 0; q < L; ++q) {
+        y[q] = fmaf(-a, wv[q], y[q]);
+        if (q < n) {
+          const size_t c = base + sk * q;
+          x[c] = fmaf(a, pv[q], xv[q]);
+          r[c] = y[q];
         }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < L; ++q) rr.add(y[q] * y[q]);
+    // forward, zero carry: y_k = r_k - l_k y_{k-1}; the carry enters with the product of -l
+    float prod = 1.0f;
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      if (q < n) {
+        if (q > 0) y[q] = fmaf(-l[q], y[q - 1], y[q]);
+        prod *= -l[q];
+      }
+    }
+    float end = 0.0f;
+#pragma unroll
+    for (int q = 0; q < L; ++q)
+      if (q == n - 1) end = y[q];
+    fwd[warp][lane] = make_float2(end, n > 0 ? prod : 1.0f);
+    lfirst[warp][lane] = l[0];
+    __syncthreads();
+    float carry = 0.0f;
+    for (int v = 0; v < warp; ++v) carry = fmaf(fwd[v][lane].y, carry, fwd[v][lane].x);
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      if (q < n) {
+        carry *= -l[q];
+        const float yk = y[q] + carry;
+        y[q] = yk * d[q];  // u
+        rz.add(yk * y[q]);
+      }
+    }
+    // backward: z_k = u_k - l_{k+1} z_{k+1}
+    const float lnext = lfirst[warp + 1][lane];
+    prod = 1.0f;
+#pragma unroll
+    for (int q = L - 1; q >= 0; --q) {
+      if (q < n) {
+        if (q + 1 < n) y[q] = fmaf(-l[min(q + 1, L - 1)], y[min(q + 1, L - 1)], y[q]);
+        prod *= -(q + 1 < n ? l[min(q + 1, L - 1)] : lnext);
+      }
+    }
+    bwd[warp][lane] = make_float2(y[0], n > 0 ? prod : 1.0f);
+    __syncthreads();
+    carry = 0.0f;
+    for (int v = W - 1; v > warp; --v)
+      carry = fmaf(bwd[v][lane].y, carry, bwd[v][lane].x);
+#pragma unroll
+    for (int q = L - 1; q >= 0; --q) {
+      if (q < n) {
+        carry *= -(q + 1 < n ? l[min(q + 1, L - 1)] : lnext);
+        z[base + sk * q] = y[q] + carry;
       }
     }
   }
   double loc[2] = {rz.value(), rr.value()};
   double tot[2];
   if (!grid_sum<2>(loc, partials, &st->arrive[2], tot)) return;
-  if (flat_tid() == 0) {
-    const double rzn = tot[0];
-    const double rn = sqrt(tot[1]);
-    if (!UPDATE) {
-      st->beta = rzn;
-      st->bcoef = 0.0;
-      if (!(rzn > 0.0)) st->status = rzn == 0.0 ? kConvergedAtol : kDivergedIndefinitePc;
-      return;
-    }
-    st->dp = rn;
-    st->iter += 1;
-    if (isnan(rn) || isnan(rzn)) {
-      st->status = kDivergedNanOrInf;
-    } else if (inner_converged(st, rn)) {
-      st->status = kConvergedRtol;
-    } else if (st->iter >= st->max_it) {
-      st->status = kDivergedIts;
-    } else if (!(rzn > 0.0)) {
-      st->status = kDivergedIndefinitePc;
-    } else {
-      st->bcoef = rzn / st->beta;
-      st->beta = rzn;
-      st->its = st->iter + 1;
-    }
-  }
+  if (flat_tid() == 0) line_step_tail<FIRST>(st, tot[0], tot[1]);
 }
 
-// Backward sweep z = L^-T u fused with the direction update p = z + beta p (p = z on the first
-// iteration).
-__global__ void __launch_bounds__(128) k32_line_bwd(const float* __restrict__ u,
-                                                    const float* __restrict__ lk,
-                                                    float* __restrict__ p, int ncol, int nz,
-                                                    const CgDevState* st) {
+// The same step with one thread per column, for columns longer than k32_line_step's registers
+// hold (256 levels): the forward sweep leaves u in z, the backward sweep overwrites it.
+template <bool FIRST>
+__global__ void __launch_bounds__(128) k32_line_step_long(
+    float* __restrict__ x, float* __restrict__ r, const float* __restrict__ p0,
+    const float* __restrict__ p1, const float* __restrict__ w, const float* __restrict__ lk,
+    const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
+    double* partials) {
   if (st->status) return;
-  const float bc = (float)st->bcoef;
-  const bool first = st->iter == 0;
+  const float a = FIRST ? 0.0f : (float)st->a;
+  const float* p = (st->iter & 1) ? p0 : p1;
+  const bool xfirst = st->iter == 0;
   const size_t sk = (size_t)ncol;
+  Kahan32 rz, rr;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
        col += gridDim.x * blockDim.x) {
-    float z = 0.0f, lnext = 0.0f;
-    for (int k0 = nz - 1; k0 >= 0; k0 -= kLineBatch) {
-      float uv[kLineBatch], lv[kLineBatch], pv[kLineBatch];
-#pragma unroll
-      for (int q = 0; q < kLineBatch; ++q) {
-        if (k0 - q >= 0) {
-          const size_t c = (size_t)col + sk * (k0 - q);
-          uv[q] = u[c];
-          lv[q] = lk[c];
-          pv[q] = first ? 0.0f : p[c];
-        }
+    float y = 0.0f;
+    size_t c = (size_t)col;
+#pragma unroll 4
+    for (int k = 0; k < nz; ++k, c += sk) {
+      float rk = r[c];
+      if (!FIRST) {
+        x[c] = fmaf(a, p[c], xfirst ? 0.0f : x[c]);
+        rk = fmaf(-a, w[c], rk);
+        r[c] = rk;
       }
-#pragma unroll
-      for (int q = 0; q < kLineBatch; ++q) {
-        if (k0 - q >= 0) {
-          const size_t c = (size_t)col + sk * (k0 - q);
-          z = fmaf(-lnext, z, uv[q]);
-          lnext = lv[q];
-          p[c] = first ? z : fmaf(bc, pv[q], z);
-        }
-      }
+      y = fmaf(-lk[c], y, rk);
+      const float uk = y * dinv[c];
+      z[c] = uk;
+      rz.add(y * uk);
+      rr.add(rk * rk);
+    }
+    float zz = 0.0f, lnext = 0.0f;
+#pragma unroll 4
+    for (int k = nz - 1; k >= 0; --k) {
+      c -= sk;
+      zz = fmaf(-lnext, zz, z[c]);
+      lnext = lk[c];
+      z[c] = zz;
     }
   }
+  double loc[2] = {rz.value(), rr.value()};
+  double tot[2];
+  if (!grid_sum<2>(loc, partials, &st->arrive[2], tot)) return;
+  if (flat_tid() == 0) line_step_tail<FIRST>(st, tot[0], tot[1]);
+}
+
+// Launch of the step: the register form's level count per warp by the number of levels.
+template <bool FIRST>
+inline void launch_line_step(float* x, float* r, const float* p0, const float* p1, const float* w,
+                             const float* lk, const float* dinv, float* z, int ncol, int nz,
+                             CgDevState* dst, double* partials, cudaStream_t s) {
+  const int groups = (ncol + 31) / 32;
+  // the resident blocks (two per SM) walk the groups: a block's end costs a reduction on the FP64
+  // pipe (about 3,000 clocks of it per block; one block per group took 0.5 ms instead of 0.2 on
+  // 768 x 768 columns), and a third block per SM would wait for a second wave
+#define FG_LINE_STEP(W, LEV)                                                              \
+  k32_line_step<FIRST, W, LEV><<<std::min(groups, (LEV > 8 ? 1 : 2) * kNumSMs), 32 * W, 0, s>>>(x, r, p0, p1, w, lk, dinv, z, ncol, nz, \
+                                                         dst, partials)
+  if (nz <= 32) FG_LINE_STEP(16, 2);
+  else if (nz <= 64) FG_LINE_STEP(16, 4);
+  else if (nz <= 96) FG_LINE_STEP(16, 6);
+  else if (nz <= 128) FG_LINE_STEP(16, 8);
+  else if (nz <= 256) FG_LINE_STEP(16, 16);
+  else {
+    const int lb = (ncol + 127) / 128;
+    k32_line_step_long<FIRST><<<lb < kMaxRedBlocks ? lb : kMaxRedBlocks, 128, 0, s>>>(
+        x, r, p0, p1, w, lk, dinv, z, ncol, nz, dst, partials);
+  }
+#undef FG_LINE_STEP
 }
 
 // z (+)= M^-1 r for the flexible-CG path (u is scratch).

@@ -26,14 +26,6 @@
 
 namespace fg {
 
-// The inner state after the line preconditioner's first application, z0 = M^-1 r0, as
-// k32_line_fwd<false> leaves it: beta = r0 . z0, no direction yet.
-__device__ __forceinline__ void line_first_state(CgDevState* in, double rz) {
-  in->beta = rz;
-  in->bcoef = 0.0;
-  if (!(rz > 0.0)) in->status = rz == 0.0 ? kConvergedAtol : kDivergedIndefinitePc;
-}
-
 // r~ = s b - A~ x~ (FP64); sums of r~^2 (scale of the inner system),
 // (r~/s)^2 = (sq r~)^2 for the true residual (sq = 1/s) and b^2 for ||b||.  The last block
 // runs the refinement test.  The inner solution e needs no zeroing: the inner solve's first
@@ -45,9 +37,8 @@ __device__ __forceinline__ void line_first_state(CgDevState* in, double rz) {
 // difference of nearly equal terms, and the refinement converges only as far as this product
 // is accurate (a float-float form, 2^-48, was both slower here and short of 1e-12 on
 // ill-conditioned systems).
-// (Applying the line preconditioner to the new right-hand side in the same column march, as
-// k_prep_ff does for the first sweep, made this kernel slower by more than the separate
-// k32_line_fwd<false> takes.)
+// The inner iterations and k_ir_update are launched ahead of the host's knowledge of the inner
+// solve's state: as long as it runs (in->status == 0) this kernel returns at once.
 template <bool FIRST, bool INV_S = false>
 __global__ void __launch_bounds__(256) k_ir_residual(
     const double* __restrict__ a0, const double* __restrict__ a1, const double* __restrict__ a2,
@@ -55,7 +46,7 @@ __global__ void __launch_bounds__(256) k_ir_residual(
     double* __restrict__ x, double* __restrict__ rres, int n0, int n1, int n2, int planes,
     int tiles, CgDevState* ir, double* partials, double ir_rtol,
     float* __restrict__ rfo = nullptr, CgDevState* in = nullptr, double inner_rtol = 0.0) {
-  if (ir->status) return;
+  if (ir->status || (!FIRST && in->status == 0)) return;
   const int t0 = (n0 + 31) / 32;
   const size_t s01 = (size_t)n0 * n1;
   double v[3] = {0.0, 0.0, 0.0};
@@ -115,12 +106,18 @@ __global__ void __launch_bounds__(256) k_ir_residual(
   if (!grid_sum<3>(v, partials, &ir->arrive[0], tot)) return;
   if (flat_tid() == 0) {
     const double rn = sqrt(tot[1]);
-    if (ir->ir_its == 0) ir->ir_bnorm = sqrt(tot[2]);
+    if (FIRST) {
+      ir->ir_bnorm = sqrt(tot[2]);
+    } else {
+      ir->ir_its += 1;  // a sweep is complete
+      ir->its += in->its;
+    }
     ir->ir_rnorm = rn;
     ir->dp = rn;
     // ||r~||; later sweeps summed (r~ / rs0)^2, the FP32 right-hand side they wrote
     const double rs0 = FIRST ? 1.0 : pow2d(pow2_above(ir->a));
     ir->a = sqrt(tot[0]) * rs0;
+    if (FIRST) ir->first_a = ir->a;
     if (isnan(rn) || isinf(rn)) {
       ir->status = kDivergedNanOrInf;
     } else if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol) || tot[0] == 0.0) {
@@ -146,7 +143,10 @@ __global__ void __launch_bounds__(256) k_ir_residual(
 __global__ void k_ir_scale(const double* __restrict__ rres, float* __restrict__ rf, size_t n,
                            CgDevState* ir, CgDevState* in, double* partials,
                            double inner_rtol) {
-  if (ir->status) return;
+  if (ir->status) {  // the inner iterations launched ahead have nothing to do
+    if (blockIdx.x == 0 && threadIdx.x == 0) in->status = kConvergedAtol;
+    return;
+  }
   // 2^-k with 2^(k-1) <= ||r~|| < 2^k: the right-hand side's norm in [1/2, 1), and the scale
   // a power of two (exact, and the refinement update forms rscale e without FP64 arithmetic)
   const int k = pow2_above(ir->a);
@@ -217,6 +217,17 @@ __global__ void k32_p(const float* __restrict__ r, float* __restrict__ p, size_t
   }
 }
 
+// p.w known: alpha, or the end of the inner solve (breakdown or NaN; the refinement decides)
+__device__ __forceinline__ void spmv32_tail(CgDevState* st, double dpi) {
+  st->its = st->iter + 1;
+  if (!(dpi > 0.0)) {
+    st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
+    return;
+  }
+  st->dpi = dpi;
+  st->a = st->beta / dpi;
+}
+
 __global__ void __launch_bounds__(256) k32_spmv(const float* __restrict__ a0,
                                                 const float* __restrict__ a1,
                                                 const float* __restrict__ a2,
@@ -260,16 +271,7 @@ __global__ void __launch_bounds__(256) k32_spmv(const float* __restrict__ a0,
   double loc[1] = {acc.value()};
   double tot[1];
   if (!grid_sum<1>(loc, partials, &st->arrive[1], tot)) return;
-  if (flat_tid() == 0) {
-    const double dpi = tot[0];
-    st->its = st->iter + 1;
-    if (!(dpi > 0.0)) {  // breakdown (or NaN): end the inner solve, refinement decides
-      st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
-      return;
-    }
-    st->dpi = dpi;
-    st->a = st->beta / dpi;
-  }
+  if (flat_tid() == 0) spmv32_tail(st, tot[0]);
 }
 
 // Vectorised variant for n0 % 4 == 0: a thread owns 4 consecutive cells along axis 0 (16-byte
@@ -277,6 +279,40 @@ __global__ void __launch_bounds__(256) k32_spmv(const float* __restrict__ a0,
 // the axis-2 neighbours roll in registers while the thread marches through its planes.
 __device__ __forceinline__ float4 ld4(const float* __restrict__ a, size_t c) {
   return *reinterpret_cast<const float4*>(a + c);
+}
+
+// the unit-diagonal stencil product of four neighbouring cells: pl / pr (al) the cells beside
+// them, PS / PN, pm / pp the rows and planes on either side
+__device__ __forceinline__ float4 stencil4(float4 pc, float pl, float pr, float al, float4 A0,
+                                           float4 PS, float4 AS, float4 PN, float4 A1, float4 pm,
+                                           float4 am, float4 pp, float4 A2) {
+  float4 v;
+  v.x = pc.x;
+  v.x = fmaf(al, pl, v.x);
+  v.x = fmaf(A0.x, pc.y, v.x);
+  v.y = fmaf(A0.x, pc.x, pc.y);
+  v.y = fmaf(A0.y, pc.z, v.y);
+  v.z = fmaf(A0.y, pc.y, pc.z);
+  v.z = fmaf(A0.z, pc.w, v.z);
+  v.w = fmaf(A0.z, pc.z, pc.w);
+  v.w = fmaf(A0.w, pr, v.w);
+  v.x = fmaf(AS.x, PS.x, v.x);
+  v.y = fmaf(AS.y, PS.y, v.y);
+  v.z = fmaf(AS.z, PS.z, v.z);
+  v.w = fmaf(AS.w, PS.w, v.w);
+  v.x = fmaf(A1.x, PN.x, v.x);
+  v.y = fmaf(A1.y, PN.y, v.y);
+  v.z = fmaf(A1.z, PN.z, v.z);
+  v.w = fmaf(A1.w, PN.w, v.w);
+  v.x = fmaf(am.x, pm.x, v.x);
+  v.y = fmaf(am.y, pm.y, v.y);
+  v.z = fmaf(am.z, pm.z, v.z);
+  v.w = fmaf(am.w, pm.w, v.w);
+  v.x = fmaf(A2.x, pp.x, v.x);
+  v.y = fmaf(A2.y, pp.y, v.y);
+  v.z = fmaf(A2.z, pp.z, v.z);
+  v.w = fmaf(A2.w, pp.w, v.w);
+  return v;
 }
 
 __global__ void __launch_bounds__(128) k32_spmv_v4(const float* __restrict__ a0,
@@ -324,32 +360,7 @@ __global__ void __launch_bounds__(128) k32_spmv_v4(const float* __restrict__ a0,
         al = l ? a0[c - 1] : 0.f;
       }
       if (lane == 31) pr = (act && i0 + 4 < n0) ? p[c + 4] : 0.f;
-      float4 v;
-      v.x = pc.x;
-      v.x = fmaf(al, pl, v.x);
-      v.x = fmaf(A0.x, pc.y, v.x);
-      v.y = fmaf(A0.x, pc.x, pc.y);
-      v.y = fmaf(A0.y, pc.z, v.y);
-      v.z = fmaf(A0.y, pc.y, pc.z);
-      v.z = fmaf(A0.z, pc.w, v.z);
-      v.w = fmaf(A0.z, pc.z, pc.w);
-      v.w = fmaf(A0.w, pr, v.w);
-      v.x = fmaf(AS.x, PS.x, v.x);
-      v.y = fmaf(AS.y, PS.y, v.y);
-      v.z = fmaf(AS.z, PS.z, v.z);
-      v.w = fmaf(AS.w, PS.w, v.w);
-      v.x = fmaf(A1.x, PN.x, v.x);
-      v.y = fmaf(A1.y, PN.y, v.y);
-      v.z = fmaf(A1.z, PN.z, v.z);
-      v.w = fmaf(A1.w, PN.w, v.w);
-      v.x = fmaf(am.x, pm.x, v.x);
-      v.y = fmaf(am.y, pm.y, v.y);
-      v.z = fmaf(am.z, pm.z, v.z);
-      v.w = fmaf(am.w, pm.w, v.w);
-      v.x = fmaf(A2.x, pp.x, v.x);
-      v.y = fmaf(A2.y, pp.y, v.y);
-      v.z = fmaf(A2.z, pp.z, v.z);
-      v.w = fmaf(A2.w, pp.w, v.w);
+      const float4 v = stencil4(pc, pl, pr, al, A0, PS, AS, PN, A1, pm, am, pp, A2);
       if (act) {
         *reinterpret_cast<float4*>(w + c) = v;
         acc.add(pc.x * v.x);
@@ -366,16 +377,155 @@ __global__ void __launch_bounds__(128) k32_spmv_v4(const float* __restrict__ a0,
   double loc[1] = {acc.value()};
   double tot[1];
   if (!grid_sum<1>(loc, partials, &st->arrive[1], tot)) return;
-  if (flat_tid() == 0) {
-    const double dpi = tot[0];
-    st->its = st->iter + 1;
-    if (!(dpi > 0.0)) {
-      st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
-      return;
+  if (flat_tid() == 0) spmv32_tail(st, tot[0]);
+}
+
+// Line-PCG: p = z + bcoef p_old (p = z in iteration 0) and w = A~ p, p.w in one pass.  The
+// direction goes from one buffer (iteration parity) into the other, since neighbouring blocks
+// read p_old; the neighbours' new directions are formed from z and p_old again (two loads
+// instead of one for each cell beside the tile's own, from L1 and L2).  28 B/cell, against 36
+// for a direction pass and a product: 260 us at 768 x 768 x 96, 0.90 of the copy peak (the product
+// alone was 210, the direction's pass 160).
+__global__ void __launch_bounds__(256) k32_dir_spmv(
+    const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
+    const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
+    float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
+    double* partials) {
+  if (st->status) return;
+  const bool first = st->iter == 0, odd = st->iter & 1;
+  const float bc = first ? 0.0f : (float)st->bcoef;
+  const float* __restrict__ po = odd ? p1 : p0;
+  float* __restrict__ pn = odd ? p0 : p1;
+  auto dir = [&](size_t c) { return first ? z[c] : fmaf(bc, po[c], z[c]); };
+  const int t0 = (n0 + 31) / 32, lane = threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const size_t s01 = (size_t)n0 * n1;
+  Kahan32 acc;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int i0 = (tile % t0) * 32 + lane;
+    const int i1 = (tile / t0) * 8 + threadIdx.y;
+    const bool act = i0 < n0 && i1 < n1;
+    const int kb = blockIdx.y * planes, ke = min(n2, kb + planes);
+    size_t c = act ? (size_t)i0 + (size_t)n0 * i1 + s01 * kb : 0;
+    float pm = 0.0f, am = 0.0f;
+    if (act && kb > 0) {
+      pm = dir(c - s01);
+      am = a2[c - s01];
     }
-    st->dpi = dpi;
-    st->a = st->beta / dpi;
+    float pc = act ? dir(c) : 0.0f;
+    for (int k = kb; k < ke; ++k) {
+      const float pp = act && k + 1 < n2 ? dir(c + s01) : 0.0f;
+      const float ac = act ? a2[c] : 0.0f, ax = act ? a0[c] : 0.0f;
+      float pl = __shfl_up_sync(full, pc, 1), al = __shfl_up_sync(full, ax, 1);
+      float pr = __shfl_down_sync(full, pc, 1);
+      if (act) {
+        if (lane == 0 && i0 > 0) {
+          pl = dir(c - 1);
+          al = a0[c - 1];
+        }
+        if (lane == 31 && i0 + 1 < n0) pr = dir(c + 1);
+        float v = pc;
+        if (i0 > 0) v = fmaf(al, pl, v);
+        if (i0 + 1 < n0) v = fmaf(ax, pr, v);
+        if (i1 > 0) v = fmaf(a1[c - n0], dir(c - n0), v);
+        if (i1 + 1 < n1) v = fmaf(a1[c], dir(c + n0), v);
+        v = fmaf(am, pm, v);
+        v = fmaf(ac, pp, v);
+        pn[c] = pc;
+        w[c] = v;
+        acc.add(pc * v);
+      }
+      pm = pc;
+      pc = pp;
+      am = ac;
+      c += s01;
+    }
   }
+  double loc[1] = {acc.value()};
+  double tot[1];
+  if (!grid_sum<1>(loc, partials, &st->arrive[1], tot)) return;
+  if (flat_tid() == 0) spmv32_tail(st, tot[0]);
+}
+
+// n0 a multiple of 4: four cells per thread, 16-byte accesses
+__global__ void __launch_bounds__(128) k32_dir_spmv_v4(
+    const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
+    const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
+    float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
+    double* partials) {
+  if (st->status) return;
+  const bool first = st->iter == 0, odd = st->iter & 1;
+  const float bc = first ? 0.0f : (float)st->bcoef;
+  const float* __restrict__ po = odd ? p1 : p0;
+  float* __restrict__ pn = odd ? p0 : p1;
+  auto dir4 = [&](size_t c) {
+    float4 v = ld4(z, c);
+    if (!first) {
+      const float4 o = ld4(po, c);
+      v.x = fmaf(bc, o.x, v.x);
+      v.y = fmaf(bc, o.y, v.y);
+      v.z = fmaf(bc, o.z, v.z);
+      v.w = fmaf(bc, o.w, v.w);
+    }
+    return v;
+  };
+  auto dir = [&](size_t c) { return first ? z[c] : fmaf(bc, po[c], z[c]); };
+  const int t0 = (n0 + 127) / 128;
+  const int lane = threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const size_t s01 = (size_t)n0 * n1;
+  Kahan32 acc;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int i0 = (tile % t0) * 128 + lane * 4;
+    const int i1 = (tile / t0) * 4 + threadIdx.y;
+    const bool act = i0 < n0 && i1 < n1;
+    const int kb = blockIdx.y * planes, ke = min(n2, kb + planes);
+    size_t c = act ? (size_t)i0 + (size_t)n0 * i1 + s01 * kb : 0;
+    float4 pc = act ? dir4(c) : z4;
+    float4 pm = z4, am = z4;
+    if (act && kb > 0) {
+      pm = dir4(c - s01);
+      am = ld4(a2, c - s01);
+    }
+    for (int k = kb; k < ke; ++k) {
+      const bool up = act && k + 1 < n2;
+      const float4 pp = up ? dir4(c + s01) : z4;
+      const float4 A0 = act ? ld4(a0, c) : z4;
+      const float4 A1 = act ? ld4(a1, c) : z4;
+      const float4 A2 = act ? ld4(a2, c) : z4;
+      const bool hs = act && i1 > 0, hn = act && i1 + 1 < n1;
+      const float4 PS = hs ? dir4(c - n0) : z4;
+      const float4 AS = hs ? ld4(a1, c - n0) : z4;
+      const float4 PN = hn ? dir4(c + n0) : z4;
+      float pl = __shfl_up_sync(full, pc.w, 1);
+      float al = __shfl_up_sync(full, A0.w, 1);
+      float pr = __shfl_down_sync(full, pc.x, 1);
+      if (lane == 0) {
+        const bool l = act && i0 > 0;
+        pl = l ? dir(c - 1) : 0.f;
+        al = l ? a0[c - 1] : 0.f;
+      }
+      if (lane == 31) pr = (act && i0 + 4 < n0) ? dir(c + 4) : 0.f;
+      const float4 v = stencil4(pc, pl, pr, al, A0, PS, AS, PN, A1, pm, am, pp, A2);
+      if (act) {
+        *reinterpret_cast<float4*>(pn + c) = pc;
+        *reinterpret_cast<float4*>(w + c) = v;
+        acc.add(pc.x * v.x);
+        acc.add(pc.y * v.y);
+        acc.add(pc.z * v.z);
+        acc.add(pc.w * v.w);
+      }
+      pm = pc;
+      pc = pp;
+      am = A2;
+      c += s01;
+    }
+  }
+  double loc[1] = {acc.value()};
+  double tot[1];
+  if (!grid_sum<1>(loc, partials, &st->arrive[1], tot)) return;
+  if (flat_tid() == 0) spmv32_tail(st, tot[0]);
 }
 
 // launch geometry of k32_spmv_v4: (32 x 4) threads cover 128 x 4 cells of a plane
@@ -383,7 +533,10 @@ static StencilLaunch launch_v4(int n0, int n1, int n2) {
   StencilLaunch L;
   L.block = dim3(32, 4, 1);
   const long tiles = (long)((n0 + 127) / 128) * ((n1 + 3) / 4);
-  const long target = (long)kNumSMs * 16 * 2;
+  // one wave of eight 128-thread blocks per SM: each z chunk reads two more planes and each block
+  // ends with a reduction on the FP64 pipe (line-PCG product at 256 x 256 x 128: 56 us, 65 with
+  // four times the blocks; the same at 768 x 768 x 96)
+  const long target = (long)kNumSMs * 8;
   long z = target / (tiles > 0 ? tiles : 1);
   if (z < 1) z = 1;
   if (z > n2) z = n2;
@@ -459,36 +612,29 @@ __global__ void k32_update(float* __restrict__ e, float* __restrict__ r,
   }
 }
 
-// x~ += rscale e (the inner system was solved for the residual divided by rscale); FIRST:
-// x~ = rscale e (x~ was 0 and is not read).  The inner solve's first update writes e without
+// x~ += rscale e (the inner system was solved for the residual divided by rscale); the first
+// sweep: x~ = rscale e (x~ was 0 and is not read).  The inner solve's first update writes e without
 // reading it, so e holds nothing before it: an inner solve that stopped before its first
 // iteration (in->iter == 0) contributes e = 0.  Four cells per step with 16-byte loads and
 // stores (the buffers are whole cudaMalloc allocations: 256-byte aligned).
 // rscale is a power of two 2^k: rscale e is formed by integer operations (f2d_scaled), which
-// leaves FIRST without FP64 instructions and the others with one addition per cell.
+// leaves the first sweep without FP64 instructions and the others with one addition per cell.
+// Nothing is done while the inner solve runs or after the refinement has ended.
 template <bool FIRST>
-__device__ __forceinline__ double ir_step(int k, float e, double x) {
-  const double v = f2d_scaled(e, k);
-  return FIRST ? v : x + v;
-}
-
-template <bool FIRST>
-__global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e, size_t n,
-                            const CgDevState* ir, const CgDevState* in) {
+__device__ __forceinline__ void ir_update_cells(double* __restrict__ x,
+                                                const float* __restrict__ e, size_t n, double rs,
+                                                int scale) {
   const size_t gid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
-  if (in->iter == 0) {
-    if (FIRST)
-      for (size_t c = gid; c < n; c += stride) x[c] = 0.0;
-    return;
-  }
-  const double rs = ir->rscale;
-  const int scale = pow2_above(rs) - 1;  // rscale = 2^scale
   if (rs != pow2d(scale)) {  // not a power of two (no path sets one): FP64 arithmetic
     for (size_t c = gid; c < n; c += stride)
       x[c] = FIRST ? rs * (double)e[c] : fma(rs, (double)e[c], x[c]);
     return;
   }
+  auto step = [&](float ev, double xv) {
+    const double v = f2d_scaled(ev, scale);
+    return FIRST ? v : xv + v;
+  };
   const float4* e4 = reinterpret_cast<const float4*>(e);
   double2* x2 = reinterpret_cast<double2*>(x);
   for (size_t q = gid; q < n / 4; q += stride) {
@@ -498,15 +644,33 @@ __global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e,
       lo = x2[2 * q];
       hi = x2[2 * q + 1];
     }
-    lo.x = ir_step<FIRST>(scale, ev.x, lo.x);
-    lo.y = ir_step<FIRST>(scale, ev.y, lo.y);
-    hi.x = ir_step<FIRST>(scale, ev.z, hi.x);
-    hi.y = ir_step<FIRST>(scale, ev.w, hi.y);
+    lo.x = step(ev.x, lo.x);
+    lo.y = step(ev.y, lo.y);
+    hi.x = step(ev.z, hi.x);
+    hi.y = step(ev.w, hi.y);
     x2[2 * q] = lo;
     x2[2 * q + 1] = hi;
   }
-  for (size_t c = (n & ~(size_t)3) + gid; c < n; c += stride)
-    x[c] = ir_step<FIRST>(scale, e[c], FIRST ? 0.0 : x[c]);
+  for (size_t c = (n & ~(size_t)3) + gid; c < n; c += stride) x[c] = step(e[c], FIRST ? 0.0 : x[c]);
+}
+
+__global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e, size_t n,
+                            const CgDevState* ir, const CgDevState* in) {
+  if (ir->status || in->status == 0) return;
+  const bool first = ir->ir_its == 0;
+  if (in->iter == 0) {
+    if (first)
+      for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
+           c += (size_t)gridDim.x * blockDim.x)
+        x[c] = 0.0;
+    return;
+  }
+  const double rs = ir->rscale;
+  const int scale = pow2_above(rs) - 1;  // rscale = 2^scale
+  if (first)
+    ir_update_cells<true>(x, e, n, rs, scale);
+  else
+    ir_update_cells<false>(x, e, n, rs, scale);
 }
 
 __global__ void k_to_f32(const double* __restrict__ a0, const double* __restrict__ a1,
@@ -581,10 +745,6 @@ int KrylovSolver::ensure32(size_t n) {
   if (g32) {
     cudaGraphExecDestroy(g32);
     g32 = nullptr;
-  }
-  if (g32s) {
-    cudaGraphExecDestroy(g32s);
-    g32s = nullptr;
   }
   FG_CUDA(cudaMalloc(&xf, n * sizeof(float)));
   FG_CUDA(cudaMalloc(&rf, n * sizeof(float)));
@@ -699,7 +859,7 @@ __global__ void __launch_bounds__(128) k_scale_mixed(double* __restrict__ a0,
 // previous solve's first residual, which keeps the scaled values and their squares far from
 // the FP32 range limits (a power of two changes no rounding).  When a scaled sum of squares
 // leaves [2^-60, 2^60] (the first solve, a jump in scale) the last block sets
-// ir->rhs_rescale and the host runs k_ir_residual<true> and k_ir_scale instead (FP64).  The
+// the status kRescaleRhs and the host runs k_ir_residual<true> and k_ir_scale instead (FP64).  The
 // kernel has no FP64 arithmetic: GB300's FP64 pipe would bound it.
 // This replaces k_diag_rsqrt_sq, k_scale_mixed, the first k_ir_residual and k_ir_scale: the
 // diagonal, the couplings and b are read once.  The assembly wrote
@@ -714,18 +874,17 @@ __global__ void __launch_bounds__(128) k_prep_ff(
     float* __restrict__ f1, float* __restrict__ f2, float* __restrict__ lk,
     float* __restrict__ dinv, int n0, int n1, int n2, int line, CgDevState* ir,
     double* partials, double ir_rtol, float* __restrict__ rf, CgDevState* in, int sig_exp,
-    double inner_rtol, float* __restrict__ u) {
+    double inner_rtol) {
   const int ncol = n0 * n1;
   const size_t sk = (size_t)ncol;
   const ff zero = ff_make(0.0f);
   const float sig = pow2f_of(-sig_exp);
-  Kahan32 kq, kb, kz;
+  Kahan32 kq, kb;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
        col += gridDim.x * blockDim.x) {
     const int i0 = col % n0, i1 = col / n0;
     const bool hx = i0 + 1 < n0, hy = i1 + 1 < n1;
     ff inv_d = ff_make(1.0f), aprev = zero;
-    float y = 0.0f;  // u != nullptr: forward substitution of the first right-hand side
     size_t c = (size_t)col;
     // level k's inputs are loaded one level ahead (two levels of loads in flight per thread)
     float sc = scale_of(dg[c]);
@@ -778,24 +937,18 @@ __global__ void __launch_bounds__(128) k_prep_ff(
       rf[c] = q;
       kq.add(q * q);
       kb.add(qb * qb);
-      if (u) {  // the line preconditioner's first application (k32_line_fwd<false>)
-        y = fmaf(-l.h, y, q);
-        const float uk = y * inv_d.h;
-        u[c] = uk;
-        kz.add(y * uk);
-      }
       sc = sb;
     }
   }
-  double v[3] = {kq.value(), kb.value(), kz.value()};
-  double tot[3];
-  if (!grid_sum<3>(v, partials, &ir->arrive[0], tot)) return;
+  double v[2] = {kq.value(), kb.value()};
+  double tot[2];
+  if (!grid_sum<2>(v, partials, &ir->arrive[0], tot)) return;
   if (flat_tid() == 0) {
-    ir->rhs_rescale = 0;
     if (!(tot[0] >= 0x1p-60 && tot[0] <= 0x1p60 && tot[1] >= 0x1p-60 && tot[1] <= 0x1p60)) {
       // the scaled sums left the FP32 margin (or are 0, inf, NaN): the host recomputes this
       // sweep's residual, norms and test in FP64 (k_ir_residual<true>, k_ir_scale)
-      ir->rhs_rescale = 1;
+      ir->status = kRescaleRhs;
+      in->status = kConvergedAtol;  // the inner iterations launched ahead have nothing to do
       return;
     }
     const double inv_sig = pow2d(sig_exp);
@@ -804,6 +957,7 @@ __global__ void __launch_bounds__(128) k_prep_ff(
     ir->ir_rnorm = rn;
     ir->dp = rn;
     ir->a = sqrt(tot[0]) * inv_sig;
+    ir->first_a = ir->a;
     if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol))
       ir->status = rn < ir->atol ? kConvergedAtol : kConvergedRtol;
     if (ir->status == 0) {
@@ -815,7 +969,8 @@ __global__ void __launch_bounds__(128) k_prep_ff(
       in->its = 0;
       in->dpi = 0.0;
       in->status = 0;
-      if (u) line_first_state(in, tot[2]);
+    } else {
+      in->status = kConvergedAtol;
     }
   }
 }
@@ -837,7 +992,6 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
   const int ncol = A.n0 * A.n1;
   const int lb = (int)std::min<long>((ncol + 127) / 128, kMaxRedBlocks);
   first_done = false;
-  first_line_done = false;
   if (A.f32_entries && (A.scaled || !ff_operator)) {
     set_error("FP32-form operator outside the float-float preparation");
     return FREHG_ERR_STATE;
@@ -860,18 +1014,14 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
       // the first inner right-hand side's scale: 2^-e with 2^(e-1) <= the previous solve's
       // first residual norm < 2^e
       const int sig_exp = pow2_above(first_rnorm[rnorm_slot & 1]);
-      // the line preconditioner's first application as well, unless the network runs
-      const bool first_line = line && net.net == nullptr;
       FG_LAUNCH(prof, st, "k_prep_ff",
-                (4.0 + 12.0 + 8.0 + 24.0 + 12.0 + 8.0 + 4.0 + (line ? 8.0 : 0.0) +
-                 (first_line ? 4.0 : 0.0)) * dn,
+                (4.0 + 12.0 + 8.0 + 24.0 + 12.0 + 8.0 + 4.0 + (line ? 8.0 : 0.0)) * dn,
                 k_prep_ff<<<lb, 128, 0, st>>>(A.a0, A.a1, A.a2, reinterpret_cast<const float*>(A.s),
                                               A.b, r, op32.a0, op32.a1, op32.a2, lkf, dinvf,
                                               A.n0, A.n1, A.n2, line ? 1 : 0, dst, partials,
-                                              cfg.ir_rtol, rf, dst32, sig_exp, cfg.inner_rtol,
-                                              first_line ? uf : nullptr));
+                                              cfg.ir_rtol, rf, dst32, sig_exp,
+                                              cfg.inner_rtol));
       FG_CUDA(cudaGetLastError());
-      first_line_done = first_line;
       A.scaled = true;
       A.s_in_r = true;
       A.f32_entries = false;
@@ -905,10 +1055,12 @@ int KrylovSolver::ensure_line(size_t n) {
   cudaFree(lkf);
   cudaFree(dinvf);
   cudaFree(uf);
-  lkf = dinvf = uf = nullptr;
+  cudaFree(pf2);
+  lkf = dinvf = uf = pf2 = nullptr;
   FG_CUDA(cudaMalloc(&lkf, n * sizeof(float)));
   FG_CUDA(cudaMalloc(&dinvf, n * sizeof(float)));
   FG_CUDA(cudaMalloc(&uf, n * sizeof(float)));
+  FG_CUDA(cudaMalloc(&pf2, n * sizeof(float)));
   cap_line = n;
   return FREHG_OK;
 }
@@ -926,29 +1078,23 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
   // inner preconditioner: Jacobi (unit diagonal, z = r) or vertical lines
   const bool line = !strcmp(cfg.pc_type, "line");
   const int ncol = A.n0 * A.n1, nzl = A.n2;
-  const int lb = (int)std::min<long>((ncol + 127) / 128, kMaxRedBlocks);
-  CgDevState ir0, in0;
-  memset(&ir0, 0, sizeof(ir0));
-  memset(&in0, 0, sizeof(in0));
-  ir0.atol = cfg.atol;
-  in0.max_it = cfg.max_it;
-  // prep_mixed may have formed the first sweep's residual and its state already, and the
-  // line preconditioner's first application to it
+  // prep_mixed may have formed the first sweep's residual and its state already
   const bool first_done_here = first_done;
-  const bool first_line_here = first_line_done;
   first_done = false;
-  first_line_done = false;
   if (!first_done_here) {
+    CgDevState ir0, in0;
+    memset(&ir0, 0, sizeof(ir0));
+    memset(&in0, 0, sizeof(in0));
+    ir0.atol = cfg.atol;
+    in0.max_it = cfg.max_it;
     FG_CUDA(cudaMemcpyAsync(dst, &ir0, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaMemcpyAsync(dst32, &in0, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
   }
   // where the scale factors are: A.s, or r (as floats) after the float-float preparation
   const double* sv = A.s_in_r ? r : A.s;
+  const char* spmv_name = vec4 ? "k32_spmv_v4" : "k32_spmv";
+  const char* dir_name = vec4 ? "k32_dir_spmv_v4" : "k32_dir_spmv";
 
-  const int chunk = 32;
-  const long shape_key = (long)A.n0 * 1000003L + A.n1;
-  const bool rebuild = !g32 || g32_key != (const void*)op32.a0 || g_stream32 != st || g_n32 != n ||
-                       g32_shape != shape_key || g32_line != (line ? 1 : 0);
   auto spmv32 = [&](cudaStream_t s) {
     if (vec4)
       k32_spmv_v4<<<L4.grid, L4.block, 0, s>>>(op32.a0, op32.a1, op32.a2, pf, wf, A.n0, A.n1,
@@ -957,121 +1103,124 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
       k32_spmv<<<L.grid, L.block, 0, s>>>(op32.a0, op32.a1, op32.a2, pf, wf, A.n0, A.n1, A.n2,
                                           L.planes, L.tiles, dst32, partials);
   };
-  // inner iterations run as CUDA graphs: a first chunk of 4 (easy systems converge in a few),
-  // then chunks of 32; iterations after convergence return at once
-  const int chunk0 = 4;
-  auto capture = [&](int iters, cudaGraphExec_t* out) -> int {
-    if (*out) cudaGraphExecDestroy(*out);
-    *out = nullptr;
+  // one inner iteration; returns at once on the device when the inner solve has ended
+  auto iteration = [&](cudaStream_t s, Profiler* pr) {
+    if (line) {
+      FG_LAUNCH(pr, s, dir_name, 28.0 * dn, {
+        if (vec4)
+          k32_dir_spmv_v4<<<L4.grid, L4.block, 0, s>>>(op32.a0, op32.a1, op32.a2, uf, pf, pf2, wf,
+                                                       A.n0, A.n1, A.n2, L4.planes, L4.tiles,
+                                                       dst32, partials);
+        else
+          k32_dir_spmv<<<L.grid, L.block, 0, s>>>(op32.a0, op32.a1, op32.a2, uf, pf, pf2, wf,
+                                                  A.n0, A.n1, A.n2, L.planes, L.tiles, dst32,
+                                                  partials);
+      });
+      FG_LAUNCH(pr, s, "k32_line_step", 36.0 * dn,
+                launch_line_step<false>(xf, rf, pf, pf2, wf, lkf, dinvf, uf, ncol, nzl, dst32,
+                                        partials, s));
+    } else {
+      FG_LAUNCH(pr, s, "k32_p", 12.0 * dn, k32_p<<<nb, 256, 0, s>>>(rf, pf, n, dst32));
+      FG_LAUNCH(pr, s, spmv_name, 20.0 * dn, spmv32(s));
+      FG_LAUNCH(pr, s, "k32_update", 24.0 * dn,
+                k32_update<<<nb, 256, 0, s>>>(xf, rf, pf, wf, n, dst32, partials));
+    }
+  };
+  // Jacobi: long inner solves, captured in chunks (the line solves' few iterations are launched
+  // one by one)
+  const int chunk = 32;
+  const bool graphs = !line && !(prof && prof->on);
+  const long shape_key = (long)A.n0 * 1000003L + A.n1;
+  if (graphs && (!g32 || g32_key != (const void*)op32.a0 || g_stream32 != st || g_n32 != n ||
+                 g32_shape != shape_key)) {
+    if (g32) cudaGraphExecDestroy(g32);
+    g32 = nullptr;
     cudaStream_t cap_st;
     FG_CUDA(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking));
     cudaGraph_t graph;
     FG_CUDA(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
-    for (int q = 0; q < iters; ++q) {
-      if (line) {
-        spmv32(cap_st);
-        k32_line_fwd<true><<<lb, 128, 0, cap_st>>>(xf, rf, pf, wf, lkf, dinvf, uf, ncol, nzl,
-                                                   dst32, partials);
-        k32_line_bwd<<<lb, 128, 0, cap_st>>>(uf, lkf, pf, ncol, nzl, dst32);
-      } else {
-        k32_p<<<nb, 256, 0, cap_st>>>(rf, pf, n, dst32);
-        spmv32(cap_st);
-        k32_update<<<nb, 256, 0, cap_st>>>(xf, rf, pf, wf, n, dst32, partials);
-      }
-    }
+    for (int q = 0; q < chunk; ++q) iteration(cap_st, nullptr);
     cudaError_t e = cudaStreamEndCapture(cap_st, &graph);
     cudaStreamDestroy(cap_st);
     if (e != cudaSuccess) {
       set_error("graph capture failed: %s", cudaGetErrorString(e));
       return FREHG_ERR_CUDA;
     }
-    e = cudaGraphInstantiate(out, graph, 0);
+    e = cudaGraphInstantiate(&g32, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
       set_error("graph instantiate failed: %s", cudaGetErrorString(e));
       return FREHG_ERR_CUDA;
     }
-    return FREHG_OK;
-  };
-  if (!(prof && prof->on) && rebuild) {
-    FG_TRY(capture(chunk, &g32));
-    FG_TRY(capture(chunk0, &g32s));
     g32_key = op32.a0;
     g_stream32 = st;
     g_n32 = n;
     g32_shape = shape_key;
-    g32_line = line ? 1 : 0;
   }
 
-  const int max_sweeps = 60;
-  int inner_total = 0, sweeps = 0;
-  bool fcg_fallback = false;
-  const bool dbg = getenv("FREHG_DEBUG_IR") != nullptr;
-  for (;;) {
-    // whether this sweep's right-hand side producer also applied the line preconditioner
-    // once (k32_line_fwd<false>): k_prep_ff does in the first sweep
-    bool fwd0_done = false;
-    if (sweeps == 0) {
-      if (!first_done_here)
-        FG_LAUNCH(prof, st, "k_ir_residual0", 24.0 * dn,
-                  k_ir_residual<true><<<L.grid, L.block, 0, st>>>(
-                      A.a0, A.a1, A.a2, sv, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes,
-                      L.tiles, dst, partials, cfg.ir_rtol));
-      else
-        fwd0_done = first_line_here;
-    } else if (A.s_in_r) {
-      FG_LAUNCH(prof, st, "k_ir_residual", 52.0 * dn,
-                (k_ir_residual<false, true><<<L.grid, L.block, 0, st>>>(
-                    A.a0, A.a1, A.a2, sv, sv, A.b, x, rres, A.n0, A.n1, A.n2, L.planes,
-                    L.tiles, dst, partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol)));
-    } else {
-      FG_LAUNCH(prof, st, "k_ir_residual", 52.0 * dn,
-                k_ir_residual<false><<<L.grid, L.block, 0, st>>>(
-                    A.a0, A.a1, A.a2, A.s, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes,
-                    L.tiles, dst, partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol));
-    }
-    // the first sweep's right-hand side (norm in [1/2, 1); k_prep_ff wrote it already); later
-    // residual kernels write theirs
-    if (sweeps == 0 && !first_done_here)
-      FG_LAUNCH(prof, st, "k_ir_scale", 12.0 * dn,
-                k_ir_scale<<<nb, 256, 0, st>>>(rres, rf, n, dst, dst32, partials,
-                                               cfg.inner_rtol));
+  // both states at the host
+  auto fetch = [&]() -> int {
     FG_CUDA(cudaGetLastError());
-    FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
+    FG_TRY(fetch_small2(hst, dst, hst32, dst32, sizeof(CgDevState), st));
     FG_CUDA(cudaStreamSynchronize(st));
     if (prof && prof->on) FG_TRY(prof->flush());
-    if (sweeps == 0 && first_done_here && hst->rhs_rescale) {
-      // k_prep_ff's scale left the FP32 margin: this sweep's residual, norms and test in FP64
-      fwd0_done = false;
-      FG_LAUNCH(prof, st, "k_ir_residual0", 24.0 * dn,
-                k_ir_residual<true><<<L.grid, L.block, 0, st>>>(
-                    A.a0, A.a1, A.a2, sv, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes,
-                    L.tiles, dst, partials, cfg.ir_rtol));
-      FG_LAUNCH(prof, st, "k_ir_scale", 12.0 * dn,
-                k_ir_scale<<<nb, 256, 0, st>>>(rres, rf, n, dst, dst32, partials,
-                                               cfg.inner_rtol));
-      FG_CUDA(cudaGetLastError());
-      FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
-      FG_CUDA(cudaStreamSynchronize(st));
-      if (prof && prof->on) FG_TRY(prof->flush());
-    }
-    if (sweeps == 0 && hst->a > 0.0 && std::isfinite(hst->a))
-      first_rnorm[rnorm_slot & 1] = hst->a;
-    if (hst->status != 0) break;
-    if (sweeps >= max_sweeps) break;
-    // inner FP32 solve: flexible CG with the learned preconditioner, or Jacobi CG
-    FG_TRY(fetch_small(hst32, dst32, sizeof(CgDevState), st));
-    FG_CUDA(cudaStreamSynchronize(st));
+    return FREHG_OK;
+  };
+  // the first sweep's residual, norms and test in FP64, and its right-hand side
+  auto first_residual = [&]() {
+    FG_LAUNCH(prof, st, "k_ir_residual0", 24.0 * dn,
+              k_ir_residual<true><<<L.grid, L.block, 0, st>>>(
+                  A.a0, A.a1, A.a2, sv, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes, L.tiles,
+                  dst, partials, cfg.ir_rtol));
+    FG_LAUNCH(prof, st, "k_ir_scale", 12.0 * dn,
+              k_ir_scale<<<nb, 256, 0, st>>>(rres, rf, n, dst, dst32, partials, cfg.inner_rtol));
+  };
+  // the inner solve's start: z0 = M^-1 r0 and r0.z0
+  auto line_first = [&]() {
+    if (line)
+      FG_LAUNCH(prof, st, "k32_line_first", 16.0 * dn,
+                launch_line_step<true>(xf, rf, pf, pf2, wf, lkf, dinvf, uf, ncol, nzl, dst32,
+                                       partials, st));
+  };
+  // x~ += 2^k e and the next true residual with the next inner system (both return at once on the
+  // device while the inner solve still runs)
+  auto sweep_end = [&]() {
+    FG_LAUNCH(prof, st, "k_ir_update", 20.0 * dn,
+              k_ir_update<<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
+    FG_LAUNCH(prof, st, "k_ir_residual", 52.0 * dn, {
+      if (A.s_in_r)
+        k_ir_residual<false, true><<<L.grid, L.block, 0, st>>>(
+            A.a0, A.a1, A.a2, sv, sv, A.b, x, rres, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
+            partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol);
+      else
+        k_ir_residual<false><<<L.grid, L.block, 0, st>>>(
+            A.a0, A.a1, A.a2, A.s, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
+            partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol);
+    });
+  };
+
+  // Rounds of: the inner solve's start (on a new sweep), some inner iterations, the sweep's end,
+  // and one read-back of both states.  The host launches ahead of what it knows: every kernel
+  // returns at once when it has nothing to do, and what a round did is read off the states after
+  // it.  The iterations launched are those that recent sweeps took (spec32: first sweeps, later
+  // ones); a sweep that takes more goes on in the next round.
+  const int max_sweeps = 60;
+  bool fcg_fallback = false;
+  const bool dbg = getenv("FREHG_DEBUG_IR") != nullptr;
+  if (!first_done_here) first_residual();
+  if (net.net != nullptr) FG_TRY(fetch());  // the network's loop is host-driven
+  int sweeps = 0;     // complete sweeps
+  int round = 0;      // rounds of the current sweep
+  int total = 0, sweep_its = 0;
+  for (;;) {
+    int launched = 0;
     // a sweep that starts with the network's budget (twice the reference solve's inner
     // iterations) spent runs without it, as do the later ones
-    if (net.net != nullptr && !fcg_fallback && net.max_inner > 0 &&
-        inner_total >= net.max_inner)
+    if (net.net != nullptr && !fcg_fallback && net.max_inner > 0 && total >= net.max_inner)
       fcg_fallback = true;
-    const bool use_net = net.net != nullptr && !fcg_fallback;
-    if (use_net) {
-      if (!zf) {
-        FG_CUDA(cudaMalloc(&zf, cap32 * sizeof(float)));
-      }
+    if (net.net != nullptr && !fcg_fallback && hst->status == 0) {
+      if (!zf) FG_CUDA(cudaMalloc(&zf, cap32 * sizeof(float)));
+      const int lb = (int)std::min<long>((ncol + 127) / 128, kMaxRedBlocks);
       const int check = 4;
       for (int it = 0; it < cfg.max_it && hst32->status == 0; ++it) {
         FG_TRY(unet_apply(net.net, A.n0, A.n1, A.n2, rf, net.lnk, net.cap, zf, st));
@@ -1084,101 +1233,82 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
                   k_fcg_beta<<<nb, 256, 0, st>>>(zf, wf, n, dst32, partials));
         FG_LAUNCH(prof, st, "k_fcg_p", 16.0 * dn,
                   k_fcg_p<<<nb, 256, 0, st>>>(zf, pf, rf, n, dst32, partials));
-        FG_LAUNCH(prof, st, vec4 ? "k32_spmv_v4" : "k32_spmv", 20.0 * dn, spmv32(st));
+        FG_LAUNCH(prof, st, spmv_name, 20.0 * dn, spmv32(st));
         FG_LAUNCH(prof, st, "k32_update", 24.0 * dn,
                   k32_update<<<nb, 256, 0, st>>>(xf, rf, pf, wf, n, dst32, partials));
         FG_CUDA(cudaGetLastError());
         if ((it + 1) % check == 0) {
-          FG_TRY(fetch_small(hst32, dst32, sizeof(CgDevState), st));
-          FG_CUDA(cudaStreamSynchronize(st));
-          if (prof && prof->on) FG_TRY(prof->flush());
-          if (net.max_inner > 0 && inner_total + hst32->its > net.max_inner) {
-            fcg_fallback = true;  // too slow: Jacobi CG from here on (the iterate is kept)
+          FG_TRY(fetch());
+          if (net.max_inner > 0 && total + hst32->its > net.max_inner) {
+            fcg_fallback = true;  // too slow: plain CG from the next sweep on (the iterate is kept)
             break;
           }
         }
       }
-      FG_TRY(fetch_small(hst32, dst32, sizeof(CgDevState), st));
-      FG_CUDA(cudaStreamSynchronize(st));
-      if (prof && prof->on) FG_TRY(prof->flush());
-    }
-    if (!use_net && line) {
-      // z0 = M^-1 r0, r0.z0 (unless the right-hand side's producer formed them) and p0 = z0
-      if (!fwd0_done)
-        FG_LAUNCH(prof, st, "k32_line_fwd0", 16.0 * dn,
-                  (k32_line_fwd<false><<<lb, 128, 0, st>>>(xf, rf, pf, wf, lkf, dinvf, uf, ncol,
-                                                           nzl, dst32, partials)));
-      FG_LAUNCH(prof, st, "k32_line_bwd", 12.0 * dn,
-                k32_line_bwd<<<lb, 128, 0, st>>>(uf, lkf, pf, ncol, nzl, dst32));
-      FG_CUDA(cudaGetLastError());
-    }
-    for (int q = 0; !use_net && q < cfg.max_it / chunk + 2 && hst32->status == 0; ++q) {
-      const int iters = q == 0 ? chunk0 : chunk;
-      const int its_before = hst32->its;
-      if (prof && prof->on) {
-        for (int it = 0; it < iters; ++it) {
-          if (line) {
-            FG_LAUNCH(prof, st, vec4 ? "k32_spmv_v4" : "k32_spmv", 20.0 * dn, spmv32(st));
-            FG_LAUNCH(prof, st, "k32_line_fwd", 36.0 * dn,
-                      (k32_line_fwd<true><<<lb, 128, 0, st>>>(xf, rf, pf, wf, lkf, dinvf, uf,
-                                                              ncol, nzl, dst32, partials)));
-            FG_LAUNCH(prof, st, "k32_line_bwd", 16.0 * dn,
-                      k32_line_bwd<<<lb, 128, 0, st>>>(uf, lkf, pf, ncol, nzl, dst32));
-          } else {
-            FG_LAUNCH(prof, st, "k32_p", 12.0 * dn,
-                      k32_p<<<nb, 256, 0, st>>>(rf, pf, n, dst32));
-            FG_LAUNCH(prof, st, vec4 ? "k32_spmv_v4" : "k32_spmv", 20.0 * dn, spmv32(st));
-            FG_LAUNCH(prof, st, "k32_update", 24.0 * dn,
-                      k32_update<<<nb, 256, 0, st>>>(xf, rf, pf, wf, n, dst32, partials));
-          }
-        }
-        FG_CUDA(cudaGetLastError());
+      if (fcg_fallback && hst32->status == 0) {  // this sweep's inner solve ends here
+        const int stop = kDivergedIts;
+        FG_CUDA(cudaMemcpyAsync(&dst32->status, &stop, sizeof(int), cudaMemcpyHostToDevice, st));
+      }
+    } else {
+      if (round == 0) line_first();
+      const int spec = spec32[sweeps > 0];
+      if (graphs && (round > 0 || spec > 8)) {
+        FG_CUDA(cudaGraphLaunch(g32, st));
+        if (prof) prof->launches += 3 * chunk;
+        launched = chunk;
       } else {
-        FG_CUDA(cudaGraphLaunch(q == 0 ? g32s : g32, st));
-        if (prof) prof->launches += 3 * iters;
-      }
-      FG_TRY(fetch_small(hst32, dst32, sizeof(CgDevState), st));
-      FG_CUDA(cudaStreamSynchronize(st));
-      if (prof && prof->on) {
-        FG_TRY(prof->flush());
-        // the chunk's iterations after convergence returned at once (the line solve's backward
-        // sweep of the converging iteration too: the forward sweep's kernel ran the test)
-        const int done = std::min(iters, std::max(0, hst32->its - its_before));
-        const int64_t idle = iters - done;
-        if (line) {
-          prof->idle(vec4 ? "k32_spmv_v4" : "k32_spmv", idle);
-          prof->idle("k32_line_fwd", idle);
-          prof->idle("k32_line_bwd", std::min<int64_t>(iters, idle + (hst32->status != 0 &&
-                                                                       done > 0 ? 1 : 0)));
-        } else {
-          prof->idle("k32_p", idle);
-          prof->idle(vec4 ? "k32_spmv_v4" : "k32_spmv", idle);
-          prof->idle("k32_update", idle);
-        }
+        launched = round == 0 ? std::max(1, std::min(spec, 8)) : 4 << std::min(round - 1, 3);
+        for (int q = 0; q < launched; ++q) iteration(st, prof);
       }
     }
-    inner_total += hst32->its;
+    sweep_end();
+    FG_TRY(fetch());
+    if (hst->status == kRescaleRhs) {
+      // the preparation could not scale its right-hand side: FP64, and the sweep again
+      const int zero = 0;
+      FG_CUDA(cudaMemcpyAsync(&dst->status, &zero, sizeof(int), cudaMemcpyHostToDevice, st));
+      first_residual();
+      if (net.net != nullptr) FG_TRY(fetch());
+      continue;
+    }
+    if (hst->first_a > 0.0 && std::isfinite(hst->first_a))
+      first_rnorm[rnorm_slot & 1] = hst->first_a;
+    const bool ended = hst->ir_its > sweeps || hst->status != 0;
+    const int done = hst->its + (ended ? 0 : hst32->its) - total;
+    if (prof && prof->on && launched > 0) {
+      const int64_t idle = std::max(0, launched - std::max(0, done));
+      if (line) {
+        prof->idle(dir_name, idle);
+        prof->idle("k32_line_step", idle);
+      } else {
+        prof->idle("k32_p", idle);
+        prof->idle(spmv_name, idle);
+        prof->idle("k32_update", idle);
+      }
+      if (hst->ir_its == sweeps) {
+        prof->idle("k_ir_update", 1);
+        prof->idle("k_ir_residual", 1);
+      }
+    }
     if (dbg)
-      fprintf(stderr, "ir sweep %d: true |r| %.3e / |b| %.3e ; inner its %d status %d |r0| %.3e -> %.3e\n",
-              sweeps, hst->ir_rnorm, hst->ir_bnorm, hst32->its, hst32->status, hst32->rnorm0,
-              hst32->dp);
-    if (sweeps == 0)
-      FG_LAUNCH(prof, st, "k_ir_update", 12.0 * dn,
-                k_ir_update<true><<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
-    else
-      FG_LAUNCH(prof, st, "k_ir_update", 20.0 * dn,
-                k_ir_update<false><<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
-    FG_CUDA(cudaGetLastError());
-    ++sweeps;
-    // next sweep's residual kernel re-arms the refinement bookkeeping
-    FG_CUDA(cudaMemcpyAsync(&dst->ir_its, &sweeps, sizeof(int), cudaMemcpyHostToDevice, st));
+      fprintf(stderr, "ir sweep %d round %d: launched %d done %d; true |r| %.3e / |b| %.3e status %d\n",
+              sweeps, round, launched, done, hst->ir_rnorm, hst->ir_bnorm, hst->status);
+    total += done;
+    sweep_its += done;
+    ++round;
+    if (ended) {
+      if (launched > 0) spec32[sweeps > 0] = std::max(sweep_its, spec32[sweeps > 0] - 1);
+      sweeps = hst->ir_its;
+      round = sweep_its = 0;
+    }
+    if (hst->status != 0 || sweeps >= max_sweeps) break;
   }
   // stopped before the first update: x~ = 0
   if (sweeps == 0)
     FG_LAUNCH(prof, st, "k_zero64", 8.0 * dn, k_zero64<<<nb, 256, 0, st>>>(x, n));
   FG_TRY(finish64(A, x_out, st, res, nb));
-  res->its = inner_total;
-  res->inner_its = inner_total;
+  res->its = total;
+  res->inner_its = total;
   res->ir_its = sweeps;
   res->fallback = fcg_fallback ? 1 : 0;
   res->rnorm = hst->ir_rnorm;
