@@ -269,7 +269,7 @@ __global__ void k_theta_of_h(ReArgs a, const double* __restrict__ h, double* __r
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < a.n;
        c += (size_t)gridDim.x * blockDim.x) {
     const CellSoil s = soil_of(a.soil, c, c % a.ncol);
-    w[c] = vg_theta(s, h[c]);
+    w[c] = vg_theta_initial(s, h[c]);
   }
 }
 __global__ void k_h_of_theta(ReArgs a, const double* __restrict__ w, double* __restrict__ h) {
@@ -339,6 +339,16 @@ __global__ void k_volume(ReArgs a, const double* __restrict__ w, double* out) {
 }  // namespace
 
 static int nblocks(size_t n) { return reduction_blocks(n, 256, 4); }
+
+// Launch of the per-cell FP64 kernels without reductions: they are bound by the SMs' FP64 units (19
+// clocks per warp instruction, one unit per SM), so the warps are spread evenly over the SMs: one
+// cell per thread in blocks of two warps, up to as many threads as fit.  In blocks of 256 threads
+// with four cells each, 1,500 cells ran on two SMs (k_kr 30 us, now 11) and 160,000 on one
+// block per SM (75 us, now 46).
+constexpr int kSpreadThreads = 64;
+static int spread_blocks(size_t n) {
+  return (int)std::min<size_t>((n + kSpreadThreads - 1) / kSpreadThreads, (size_t)kNumSMs * 32);
+}
 
 namespace {
 // Surface-water exchange through the top face (Coupling::exchange, src/coupling/Coupling.cpp:
@@ -587,7 +597,8 @@ static int pca_step(frehg_re* re) {
   FG_LAUNCH(prof, st, "k_step_begin", 0.0, k_step_begin<<<1, 1, 0, st>>>(re->sc));
   // computeKFace inputs at h^n
   FG_LAUNCH(prof, st, "k_kr", (24.0 + sb) * n,
-            (k_constit<false, true><<<nb, 256, 0, st>>>(a, a.h_old, re->kr, nullptr, re->cap)));
+            (k_constit<false, true><<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(
+                a, a.h_old, re->kr, nullptr, re->cap)));
   // groundwaterMatCoeff + groundwaterRhs + assembly
   const StencilLaunch L = stencil_launch(re->nx, re->ny, re->nz);
   re->A.scaled = false;
@@ -606,7 +617,8 @@ static int pca_step(frehg_re* re) {
   re->cnt.ir_sweeps += res.ir_its;
   if (rc != FREHG_OK) return rc;
   // enforceHeadBc + computeKFace + updateDiagnostics at h^{n+1} (the solve wrote h^{n+1})
-  FG_LAUNCH(prof, st, "k_post", (24.0 + sb) * n, k_post<<<nb, 256, 0, st>>>(a));
+  FG_LAUNCH(prof, st, "k_post", (24.0 + sb) * n,
+            k_post<<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(a));
   FG_CUDA(cudaGetLastError());
   // groundwaterFlux + updateWaterContent (+ dq of adaptiveTimeStep, boundary budgets)
   FG_LAUNCH(prof, st, "k_correct", (73.0 + sb) * n,
@@ -779,8 +791,8 @@ static int picard_step(frehg_re* re) {
     for (its = 0; its < re->p.picard_max_it; ++its) {
       if (!picard_ff(re))
         FG_LAUNCH(prof, st, "k_kr", (32.0 + sb) * n,
-                  (k_constit<true, true><<<nb, 256, 0, st>>>(a, a.h_new, re->kr, re->wch,
-                                                             re->cap)));
+                  (k_constit<true, true><<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(
+                      a, a.h_new, re->kr, re->wch, re->cap)));
       else if (constit_ready) {
       } else if (all_ff)
         FG_LAUNCH(prof, st, "k_kr_ff", (32.0 + sb) * n,
@@ -1176,7 +1188,7 @@ int frehg_re_set_initial_head(frehg_re* re, const double* h) {
   FG_CUDA(cudaStreamSynchronize(re->stream));
   FG_CUDA(cudaMemcpy(re->H[re->cur], h, re->n * sizeof(double), cudaMemcpyHostToDevice));
   ReArgs a = make_args(re);
-  k_theta_of_h<<<nblocks(re->n), 256, 0, re->stream>>>(a, re->H[re->cur], re->W[re->cur]);
+  k_theta_of_h<<<spread_blocks(re->n), kSpreadThreads, 0, re->stream>>>(a, re->H[re->cur], re->W[re->cur]);
   FG_CUDA(cudaGetLastError());
   FG_CUDA(cudaStreamSynchronize(re->stream));
   re->have_state = true;
@@ -1191,7 +1203,7 @@ int frehg_re_set_initial_water_content(frehg_re* re, const double* wc) {
   FG_CUDA(cudaStreamSynchronize(re->stream));
   FG_CUDA(cudaMemcpy(re->W[re->cur], wc, re->n * sizeof(double), cudaMemcpyHostToDevice));
   ReArgs a = make_args(re);
-  k_h_of_theta<<<nblocks(re->n), 256, 0, re->stream>>>(a, re->W[re->cur], re->H[re->cur]);
+  k_h_of_theta<<<spread_blocks(re->n), kSpreadThreads, 0, re->stream>>>(a, re->W[re->cur], re->H[re->cur]);
   FG_CUDA(cudaGetLastError());
   FG_CUDA(cudaStreamSynchronize(re->stream));
   re->have_state = true;
@@ -1774,7 +1786,8 @@ int frehg_re_training_pairs(frehg_re* re, int npairs, const int* iters, int targ
   const size_t n = re->n;
   // the next step's system at the current state (nothing advances)
   k_step_begin<<<1, 1, 0, st>>>(re->sc);
-  k_constit<false, true><<<nb, 256, 0, st>>>(a, a.h_old, re->kr, nullptr, re->cap);
+  k_constit<false, true><<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(a, a.h_old, re->kr,
+                                                                          nullptr, re->cap);
   const StencilLaunch L = stencil_launch(re->nx, re->ny, re->nz);
   re->A.scaled = false;
   re->A.s_in_r = false;
