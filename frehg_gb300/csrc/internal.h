@@ -229,6 +229,9 @@ class KrylovSolver {
   int fused64 = -1;
   int g64_form = -1;
   bool coop_failed = false;
+  // the one-launch solve's exchange words and the number of solves that have used them
+  void* solve_words = nullptr;
+  unsigned long long solve_count = 0;
   Profiler* prof = nullptr;  // owner's profiler (launch counts, optional event timing)
   NetPrecond net;            // learned preconditioner (FCG inner solves when set)
   // the mixed path's scaled couplings in float-float (2^-48) instead of FP64 products: for

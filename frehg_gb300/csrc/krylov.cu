@@ -11,10 +11,11 @@
 //    is Jacobi-PCG on A (x~ = D^1/2 x, r~ = D^-1/2 r, beta = r.z = r~.r~, p'Ap = p~'A~p~,
 //    ||B r|| = ||s r~|| with s = D^-1/2), so the diagonal is never stored or multiplied and
 //    no divisions remain in the loop.
-//  * Three phases per iteration (p-update, stencil SpMV + p.w, update + two norms), as one
-//    cooperative launch (k_cg_iter, the phases separated by two bounded grid barriers; by
-//    default for systems of up to kFusedAutoCells unknowns) or as three kernels (larger
-//    systems, or devices without cooperative launch); the last reduction ends in the
+//  * Three phases per iteration (p-update, stencil SpMV + p.w, update + two norms).  By default
+//    the whole loop is one cooperative launch with its vectors in registers (k_cg_solve, up to
+//    622,592 unknowns).  Larger systems, and on request or under profiling all, run iterations as
+//    one cooperative launch each (k_cg_iter, the phases separated by two bounded grid barriers;
+//    by default up to kFusedAutoCells unknowns) or as three kernels; the last reduction ends in the
 //    last-arriving block, which also runs the scalar part of the algorithm (beta, stopping
 //    test) on the device.  Launches of a converged solve return at once, so
 //    iterations are captured in a CUDA graph of `chunk` iterations and the host only reads
@@ -226,6 +227,18 @@ __device__ __forceinline__ Acc spmv_cell(const T* __restrict__ p, const T* __res
   return v;
 }
 
+// p.w known: the iteration's alpha, or the end of the solve
+__device__ __forceinline__ void cg_alpha(CgDevState* st, double dpi) {
+  st->its = st->iter + 1;
+  if (dpi == 0.0 || (st->iter > 0 && ((dpi > 0.0) != (st->dpi > 0.0))) || isnan(dpi)) {
+    st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
+    return;
+  }
+  st->dpiold = st->dpi;
+  st->dpi = dpi;
+  st->a = st->beta / dpi;
+}
+
 __global__ void __launch_bounds__(256) k_cg_spmv(const double* __restrict__ a0,
                                                  const double* __restrict__ a1,
                                                  const double* __restrict__ a2,
@@ -266,17 +279,7 @@ __global__ void __launch_bounds__(256) k_cg_spmv(const double* __restrict__ a0,
   }
   double tot[1];
   if (!grid_sum<1>(acc, partials, &st->arrive[1], tot)) return;
-  if (flat_tid() == 0) {
-    const double dpi = tot[0];
-    st->its = st->iter + 1;
-    if (dpi == 0.0 || (st->iter > 0 && ((dpi > 0.0) != (st->dpi > 0.0))) || isnan(dpi)) {
-      st->status = isnan(dpi) ? kDivergedNanOrInf : kDivergedIndefiniteMat;
-      return;
-    }
-    st->dpiold = st->dpi;
-    st->dpi = dpi;
-    st->a = st->beta / dpi;
-  }
+  if (flat_tid() == 0) cg_alpha(st, tot[0]);
 }
 
 // The scalar end of an iteration (last block): ||B r|| = sqrt(tot[1]) and the stopping test,
@@ -477,6 +480,335 @@ __global__ void __launch_bounds__(256) k_cg_iter(const double* __restrict__ a0,
   if (flat_tid() == 0) cg_update_tail(st, tot);
 }
 
+// The whole loop of a solve in one cooperative launch: every block owns blockDim x K consecutive
+// cells, each thread K of them, whose x, r, p and w stay in its registers; the operator comes
+// from L1 (32 bytes a cell, read-only: it stays there for the block's cells), and the neighbours'
+// values go through the L2.  A reduction ends in every block: after its barrier each sums the
+// same partials in the same order and runs the same scalar steps, so nothing is waited for
+// twice.  Same arithmetic per cell as the three kernels; an absent neighbour's product is with
+// the zero coupling that the operator holds there.
+//   REDIR: two grid-wide exchanges an iteration (p.w; the norms, behind which r is there): the
+//   neighbours' directions are formed from r and the previous directions, six more FP64
+//   instructions per cell.  Else the directions are written and the blocks that own neighbouring
+//   cells waited for.
+// An exchange between a few blocks is one trip through the L2: each block writes its partial sum
+// and the exchange's number as one 16-byte word, and a warp of each block reads all blocks' words
+// until they carry that number (numbers are never reused: the solver counts its solves).  With
+// many blocks the readers hold up the writers (32,768 cells, 128 blocks: 14.2 us an iteration),
+// and a counter with one reader per block comes first (9.7).
+// The FP64 unit of an SM (19 clocks per warp instruction, 64 and more in a chain) sets the
+// shape: few warps per block (a reduction costs each of them five steps), as many cells per thread
+// as fill the SMs evenly, no square root and no FP64 comparison in the loop (the norms' squares
+// are compared as integers), and the division for beta done ahead by another warp.
+// A solve with 73 to 96 iterations, this / three kernels in graph chunks: 512 cells 0.51 / 1.3 ms,
+// 4,096 0.80 / 1.7, 32,768 1.03 / 1.86, 160,000 1.65 / 2.56, 412,000 2.1 / 3.6, 524,288 2.3 / 4.0.
+constexpr int kSolveThreads = 512;  // at most
+constexpr int kSolveCells = 8;      // per thread, at most
+constexpr int kSolveBlocks = 160;   // at most (five words per lane)
+constexpr int kSolveWordBlocks = 16;  // blocks that exchange without the counter, at most
+constexpr long kSolvePolls = 1L << 22;
+
+// all blocks have arrived: a count that only grows within a launch (bar_count, zero before it)
+__device__ __forceinline__ bool solve_arrive_wait(CgDevState* st, unsigned target) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
+  unsigned v = 0;
+  for (long q = 0; v < target; ++q) {
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->bar_count) : "memory");
+    if (q >= kSolvePolls) {
+      atomicExch(&st->bar_timeout, 1);
+      return false;
+    }
+  }
+  return true;
+}
+
+struct alignas(16) SolveWord {
+  double v;
+  unsigned long long epoch;
+};
+
+__device__ __forceinline__ void word_put(SolveWord* p, double v, unsigned long long epoch) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}"
+               ::"l"(p), "l"(__double_as_longlong(v)), "l"(epoch)
+               : "memory");
+}
+
+__device__ __forceinline__ bool word_get(const SolveWord* p, unsigned long long epoch, double* v) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  *v = __longlong_as_double((long long)lo);
+  return hi == epoch;
+}
+
+// words w[b], b = first + lane + 32 j up to last, until all carry `epoch` (one warp); the sum of
+// this lane's, in order of b.  *ok false when the wait ran out.
+__device__ __forceinline__ double words_wait(const SolveWord* w, int first, int last,
+                                             unsigned long long epoch, bool* ok, CgDevState* st) {
+  const int lane = threadIdx.x & 31;
+  double v[kSolveBlocks / 32];
+  for (long q = 0;; ++q) {
+    bool have = true;
+#pragma unroll
+    for (int j = 0; j < kSolveBlocks / 32; ++j) {
+      v[j] = 0.0;
+      const int b = first + lane + 32 * j;
+      if (b <= last && !word_get(w + b, epoch, &v[j])) have = false;
+    }
+    if (__all_sync(0xffffffffu, have)) break;
+    if (q >= kSolvePolls) {
+      *ok = false;
+      if (lane == 0) atomicExch(&st->bar_timeout, 1);
+      break;
+    }
+  }
+  double t = v[0];
+#pragma unroll
+  for (int j = 1; j < kSolveBlocks / 32; ++j)
+    if (32 * j <= last - first) t += v[j];
+  return t;
+}
+
+// the block's copy of the solve's scalars
+struct SolveScalars {
+  double bcoef, a, beta, inv_beta, dpi, dp0, zz;  // dp0: ||B b||
+  double ttol, ttol2, atol, atol2, div, div2;
+  int iter, its, max_it, status, squares, ok;
+};
+
+// grid totals of NV values, in sh[16 q]: value q by warp q.  RELEASE: what the block wrote
+// before is visible to the other blocks behind it.
+template <int NV, bool RELEASE>
+__device__ __forceinline__ bool solve_sum(double (&v)[NV], SolveWord* words, CgDevState* st,
+                                          unsigned long long epoch, unsigned target, double* sh,
+                                          int* ok_sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    v[q] = warp_sum(v[q]);
+    if (lane == 0) sh[q * 16 + warp] = v[q];
+  }
+  __syncthreads();
+  const bool counter = gridDim.x > kSolveWordBlocks;
+  double t = 0.0;
+  if (warp < NV) {
+    // the block's warps, at most 16
+    t = lane < warps ? sh[warp * 16 + lane] : 0.0;
+    for (int o = 8; o > 0; o >>= 1)
+      if (o < warps) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (gridDim.x > 1 && lane == 0) {
+      if (RELEASE && !counter) __threadfence();
+      word_put(words + warp * kSolveBlocks + blockIdx.x, t, epoch);
+    }
+  }
+  if (counter) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (!solve_arrive_wait(st, target)) *ok_sh = 0;
+    }
+    __syncthreads();
+  }
+  if (warp < NV) {
+    if (gridDim.x > 1) {
+      bool ok = true;
+      t = warp_sum(words_wait(words + warp * kSolveBlocks, 0, (int)gridDim.x - 1, epoch, &ok, st));
+      if (RELEASE) __threadfence();
+      if (!ok) *ok_sh = 0;
+    }
+    if (lane == 0) sh[warp * 16] = t;
+  }
+  __syncthreads();
+  return *ok_sh != 0;
+}
+
+// cg_alpha and cg_update_tail on the block's scalars; non-negative doubles order like their bits
+__device__ __forceinline__ long long solve_bits(double v) { return __double_as_longlong(v); }
+
+__device__ __forceinline__ void solve_alpha(SolveScalars& s, double dpi) {
+  s.its = s.iter + 1;
+  const long long b = solve_bits(dpi) & 0x7fffffffffffffffll;
+  if (b == 0 || (s.iter > 0 && (solve_bits(dpi) < 0) != (solve_bits(s.dpi) < 0)) ||
+      b > 0x7ff0000000000000ll) {
+    s.status = b > 0x7ff0000000000000ll ? kDivergedNanOrInf : kDivergedIndefiniteMat;
+    return;
+  }
+  s.dpi = dpi;
+  s.a = s.beta / dpi;
+}
+
+__device__ __forceinline__ void solve_tail(SolveScalars& s, double rr, double zz) {
+  s.zz = zz;
+  const long long bz = solve_bits(zz);
+  if ((bz & 0x7fffffffffffffffll) >= 0x7ff0000000000000ll) {
+    s.status = kDivergedNanOrInf;
+    return;
+  }
+  bool done, small, far;
+  if (s.squares) {
+    done = bz <= solve_bits(s.ttol2);
+    small = bz < solve_bits(s.atol2);
+    far = bz >= solve_bits(s.div2);
+  } else {  // tolerances whose squares leave the normal range
+    const double dp = sqrt(zz);
+    done = dp <= s.ttol;
+    small = dp < s.atol;
+    far = dp >= s.div;
+  }
+  if (done) {
+    s.status = small ? kConvergedAtol : kConvergedRtol;
+    return;
+  }
+  if (s.div > 0.0 && far) {
+    s.status = kDivergedDtol;
+    return;
+  }
+  s.beta = rr;
+  s.iter += 1;
+  if (s.iter >= s.max_it) {
+    s.status = kDivergedIts;
+    return;
+  }
+  s.its = s.iter + 1;
+  if (solve_bits(rr) == 0) {
+    s.status = kConvergedAtol;
+    return;
+  }
+  s.bcoef = rr * s.inv_beta;
+  if (solve_bits(s.bcoef) < 0) s.status = kDivergedIndefinitePc;
+}
+
+template <int K, bool REDIR>
+__global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
+    const double* __restrict__ a0, const double* __restrict__ a1, const double* __restrict__ a2,
+    const double* __restrict__ s, double* __restrict__ x_out, double* r_io, double* p0, double* p1,
+    unsigned n, unsigned s1, unsigned s2, CgDevState* st, SolveWord* words,
+    unsigned long long epoch) {
+  __shared__ SolveScalars ss;
+  __shared__ double sh[32];
+  if (threadIdx.x == 0) {
+    ss.status = st->status;
+    ss.beta = st->beta;
+    ss.bcoef = ss.dpi = ss.a = 0.0;
+    ss.dp0 = st->rnorm0;
+    ss.zz = st->rnorm0 * st->rnorm0;
+    ss.ttol = st->ttol;
+    ss.ttol2 = ss.ttol * ss.ttol;
+    ss.atol = st->atol;
+    ss.atol2 = ss.atol * ss.atol;
+    ss.div = st->divtol > 0.0 ? st->divtol * st->rnorm0 : 0.0;
+    ss.div2 = ss.div * ss.div;
+    ss.iter = ss.its = 0;
+    ss.max_it = st->max_it;
+    ss.squares = ss.ttol > 1e-140 && ss.atol >= 0.0 && ss.div < 1e150;
+    ss.ok = 1;
+  }
+  __syncthreads();
+  if (ss.status) return;
+  const unsigned nt = blockDim.x;
+  const unsigned c0 = blockIdx.x * (K * nt) + threadIdx.x;
+  double x[K], r[K], p[K], w[K];
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const unsigned c = c0 + q * nt;
+    x[q] = p[q] = w[q] = 0.0;
+    r[q] = c < n ? __ldcg(r_io + c) : 0.0;
+  }
+  const int reach = (int)((s2 + K * nt - 1) / (K * nt));  // blocks on either side with neighbours
+  unsigned target = 0;
+  bool ok = true;
+  for (;;) {
+    const double bc = ss.bcoef;
+    const bool first = ss.iter == 0;
+    const double* po = (ss.iter & 1) ? p0 : p1;
+    double* pn = (ss.iter & 1) ? p1 : p0;
+    if (threadIdx.x == nt - 1) ss.inv_beta = 1.0 / ss.beta;  // read behind the norms' exchange
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      const unsigned c = c0 + q * nt;
+      p[q] = first ? r[q] : fma(bc, p[q], r[q]);
+      if (c < n) __stcg(pn + c, p[q]);
+    }
+    if (!REDIR) {
+      ++epoch;
+      __syncthreads();
+      if (threadIdx.x < 32 && gridDim.x > 1) {
+        bool there = true;
+        if (threadIdx.x == 0) {
+          __threadfence();
+          word_put(words + 3 * kSolveBlocks + blockIdx.x, 0.0, epoch);
+        }
+        const int b = (int)blockIdx.x;
+        words_wait(words + 3 * kSolveBlocks, max(0, b - reach), min((int)gridDim.x - 1, b + reach),
+                   epoch, &there, st);
+        __threadfence();
+        if (!there) ss.ok = 0;
+      }
+      __syncthreads();
+      if (!(ok = ss.ok != 0)) break;
+    }
+    auto dir = [&](unsigned c) {
+      if (!REDIR) return __ldcg(pn + c);
+      const double rc = __ldcg(r_io + c);
+      return first ? rc : fma(bc, __ldcg(po + c), rc);
+    };
+    double acc[1] = {0.0};
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      const unsigned c = c0 + q * nt;
+      if (c < n) {
+        double v = p[q];
+        if (c >= 1) v = fma(a0[c - 1], dir(c - 1), v);
+        if (c + 1 < n) v = fma(a0[c], dir(c + 1), v);
+        if (c >= s1) v = fma(a1[c - s1], dir(c - s1), v);
+        if (c + s1 < n) v = fma(a1[c], dir(c + s1), v);
+        if (c >= s2) v = fma(a2[c - s2], dir(c - s2), v);
+        if (c + s2 < n) v = fma(a2[c], dir(c + s2), v);
+        w[q] = v;
+        acc[0] = fma(p[q], v, acc[0]);
+      }
+    }
+    if (!(ok = solve_sum<1, false>(acc, words + 2 * kSolveBlocks, st, ++epoch, target += gridDim.x,
+                                   sh, &ss.ok)))
+      break;
+    if (threadIdx.x == 0) solve_alpha(ss, sh[0]);
+    __syncthreads();
+    if (ss.status) break;
+    const double a = ss.a;
+    double v[2] = {0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      const unsigned c = c0 + q * nt;
+      if (c < n) {
+        x[q] = fma(a, p[q], x[q]);
+        r[q] = fma(-a, w[q], r[q]);
+        if (REDIR) __stcg(r_io + c, r[q]);
+        v[0] = fma(r[q], r[q], v[0]);
+        const double z = s[c] * r[q];
+        v[1] = fma(z, z, v[1]);
+      }
+    }
+    if (!(ok = solve_sum<2, REDIR>(v, words, st, ++epoch, target += gridDim.x, sh, &ss.ok)))
+      break;
+    if (threadIdx.x == 0) solve_tail(ss, sh[0], sh[16]);
+    __syncthreads();
+    if (ss.status) break;
+  }
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const unsigned c = c0 + q * nt;
+    if (c < n) x_out[c] = x[q];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->its = ss.its;
+    st->iter = ss.iter;
+    st->dp = sqrt(ss.zz);
+    st->status = ok ? ss.status : (int)kGridBarrierTimeout;
+  }
+}
+
 __global__ void k_unscale(const double* __restrict__ s, const double* __restrict__ xs,
                           double* __restrict__ x, size_t n) {
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
@@ -542,6 +874,7 @@ KrylovSolver::~KrylovSolver() {
   cudaFree(p);
   cudaFree(w);
   cudaFree(partials);
+  cudaFree(solve_words);
   cudaFree(dst);
   cudaFreeHost(hst);
   cudaFree(xf);
@@ -579,6 +912,8 @@ int KrylovSolver::ensure(size_t n) {
     FG_CUDA(cudaMalloc(&dst, sizeof(CgDevState)));
     FG_CUDA(cudaMemset(dst, 0, sizeof(CgDevState)));
     FG_TRY(alloc_mapped(reinterpret_cast<void**>(&hst), sizeof(CgDevState)));
+    FG_CUDA(cudaMalloc(&solve_words, 4 * kSolveBlocks * sizeof(SolveWord)));
+    FG_CUDA(cudaMemset(solve_words, 0, 4 * kSolveBlocks * sizeof(SolveWord)));
   }
   cap = n;
   return FREHG_OK;
@@ -707,6 +1042,78 @@ static cudaError_t launch_cg_iter(const StencilLaunch& L, cudaStream_t st, const
                             A.n2, L.planes, L.tiles, dst, partials);
 }
 
+// Launch shape of k_cg_solve: cells per thread, threads and blocks.  False where the system is too
+// large (more than 512 x 8 cells per SM) or cooperative launches are absent.
+struct SolveShape {
+  int cells, threads, blocks;
+  bool redir;
+};
+
+static bool solve_shape(size_t n, SolveShape* sh) {
+  int dev = 0, coop = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  sms = std::min(sms, kSolveBlocks);
+  if (!coop || sms < 1 || n > (size_t)sms * kSolveThreads * kSolveCells) return false;
+  // least FP64 work of the fullest SM: 13 instructions per warp and cell, and the reductions' 15
+  // per warp; at least 4 warps (one per scheduler)
+  const size_t per_sm = (n + sms - 1) / sms;
+  long best = LONG_MAX;
+  for (int k = 1; k <= kSolveCells; ++k) {
+    const long warps = std::max<long>(4, (long)((per_sm + 32 * k - 1) / (32 * k)));
+    if (warps * 32 > kSolveThreads) continue;
+    const long cost = warps * (13 * k + 15);
+    if (cost < best) {
+      best = cost;
+      sh->cells = k;
+      sh->threads = (int)warps * 32;
+    }
+  }
+  const size_t per = (size_t)sh->cells * sh->threads;
+  sh->blocks = (int)((n + per - 1) / per);
+  // the wait for the neighbouring blocks costs about 1,500 clocks, forming their directions
+  // 6 x 19 per warp and cell
+  sh->redir = sh->blocks > 1 && 6 * 19 * sh->cells * (sh->threads / 32) < 1500;
+  return true;
+}
+
+static cudaError_t launch_cg_solve(const SolveShape& sh, cudaStream_t st, const Stencil64& A,
+                                   double* x, double* r, double* p, double* p2, CgDevState* dst,
+                                   void* words, unsigned long long epoch) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)sh.blocks);
+  cfg.blockDim = dim3((unsigned)sh.threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = sh.blocks > 1 ? 1 : 0;
+  auto go = [&](auto kernel) {
+    return cudaLaunchKernelEx(&cfg, kernel, (const double*)A.a0, (const double*)A.a1,
+                              (const double*)A.a2, (const double*)A.s, x, r, p, p2, (unsigned)A.n,
+                              (unsigned)A.n0, (unsigned)(A.n0 * A.n1), dst,
+                              static_cast<SolveWord*>(words), epoch);
+  };
+#define FG_SOLVE_CASE(KK) \
+  case KK: return sh.redir ? go(k_cg_solve<KK, true>) : go(k_cg_solve<KK, false>);
+  switch (sh.cells) {
+    FG_SOLVE_CASE(1)
+    FG_SOLVE_CASE(2)
+    FG_SOLVE_CASE(3)
+    FG_SOLVE_CASE(4)
+    FG_SOLVE_CASE(5)
+    FG_SOLVE_CASE(6)
+    FG_SOLVE_CASE(7)
+    default: return go(k_cg_solve<8, false>);
+  }
+#undef FG_SOLVE_CASE
+}
+
 static int chunk_for(size_t n) {
   if (n >= (size_t)4 << 20) return 16;
   if (n >= (size_t)1 << 18) return 32;
@@ -730,6 +1137,24 @@ int KrylovSolver::solve64(Stencil64& A, double* x_out, const frehg_solver_config
             k_cg_init<<<nb, 256, 0, st>>>(A.s, A.b, x, r, n, dst, partials));
   FG_CUDA(cudaGetLastError());
 
+  // by default the whole loop in one launch, where the system fits (and no per-kernel times are
+  // asked for)
+  if (fused64 < 0 && !coop_failed && !(prof && prof->on)) {
+    SolveShape sh;
+    if (solve_shape(n, &sh)) {
+      const cudaError_t e = launch_cg_solve(sh, st, A, x, r, p, w, dst, solve_words,
+                                            ++solve_count << 32);
+      if (e == cudaSuccess) {
+        if (prof) prof->launches += 1;
+        FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
+        FG_CUDA(cudaStreamSynchronize(st));
+        return finish64(A, x_out, st, res, nb);
+      }
+      // the cooperative launch was refused (e.g. under MPS): three kernels from now on
+      cudaGetLastError();
+      coop_failed = true;
+    }
+  }
   const int chunk = chunk_for(n);
   const StencilLaunch L = stencil_launch(A.n0, A.n1, A.n2);
   StencilLaunch LF;
