@@ -50,9 +50,13 @@ StencilLaunch stencil_launch(int n0, int n1, int n2) {
   L.block = dim3(32, 8, 1);
   const int t0 = (n0 + 31) / 32, t1 = (n1 + 7) / 8;
   const long tiles = (long)t0 * t1;
-  // about two waves of 8 resident (32 x 8)-thread blocks per SM; the launch shape, and with
-  // it the summation tree of the reductions, depends on the grid sizes only
-  const long target = (long)kNumSMs * 8 * 2;
+  // about two waves of 8 resident (32 x 8)-thread blocks per SM, fewer on small grids: 8 cells per
+  // thread, down to two blocks per SM, since each block's sums and its uneven share cost the FP64
+  // pipe more than the cells do (FP64 assembly of 101 x 77 x 53: 159 us with 1 to 2 cells per
+  // thread, 106 with 8; the FP32 product of 203 x 149 x 96 prefers more blocks, 32 against 33); the
+  // launch shape, and with it the summation tree of the reductions, depends on the grid sizes only
+  const long want = (long)n0 * n1 * n2 / 2048;
+  const long target = std::min((long)kNumSMs * 8 * 2, std::max((long)kNumSMs * 2, want));
   long z = target / (tiles > 0 ? tiles : 1);
   if (z < 1) z = 1;
   if (z > n2) z = n2;
@@ -428,7 +432,7 @@ __global__ void __launch_bounds__(256) k_cg_iter(const double* __restrict__ a0,
       c += s01;
     }
   }
-  __shared__ double sh[32];
+  __shared__ double sh[256];
   __shared__ double dpi_sh;
   double* pw = partials + 3 * (size_t)kMaxRedBlocks;
   block_sum<1>(acc, sh);

@@ -49,8 +49,9 @@ __global__ void __launch_bounds__(256) k_ir_residual(
   if (ir->status || (!FIRST && in->status == 0)) return;
   const int t0 = (n0 + 31) / 32;
   const size_t s01 = (size_t)n0 * n1;
-  double v[3] = {0.0, 0.0, 0.0};
-  if (FIRST) {
+  double v[FIRST ? 3 : 2] = {};
+  double unscale = 1.0;
+  if constexpr (FIRST) {
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
       const int i0 = (tile % t0) * 32 + threadIdx.x;
       const int i1 = (tile / t0) * 8 + threadIdx.y;
@@ -100,13 +101,14 @@ __global__ void __launch_bounds__(256) k_ir_residual(
       }
     }
     v[0] = k0.value();
-    v[1] = k1.value() * rs1 * rs1;
+    v[1] = k1.value();
+    unscale = rs1;
   }
-  double tot[3];
-  if (!grid_sum<3>(v, partials, &ir->arrive[0], tot)) return;
+  double tot[FIRST ? 3 : 2];
+  if (!grid_sum<FIRST ? 3 : 2>(v, partials, &ir->arrive[0], tot)) return;
   if (flat_tid() == 0) {
-    const double rn = sqrt(tot[1]);
-    if (FIRST) {
+    const double rn = FIRST ? sqrt(tot[1]) : sqrt(tot[1]) * unscale;
+    if constexpr (FIRST) {
       ir->ir_bnorm = sqrt(tot[2]);
     } else {
       ir->ir_its += 1;  // a sweep is complete
@@ -867,112 +869,194 @@ __global__ void __launch_bounds__(128) k_scale_mixed(double* __restrict__ a0,
 // place by the scaled FP32 copies, and the FP64 scaled couplings go to a0-a2.
 __device__ __forceinline__ float scale_of(float d) { return rsqrtf(d == 0.0f ? 1.0f : d); }
 
+// One cell of the preparation: scale factors sc (its own), sx, sy, sz (the +1 neighbours'), the
+// unscaled couplings e0-e2 (0 towards absent neighbours); writes the scaled operator, s and the
+// first right-hand side and returns the scaled axis-2 coupling.
+struct PrepOut {
+  double *a0, *a1, *a2, *s;
+  float *f0, *f1, *f2, *rf;
+};
+__device__ __forceinline__ ff prep_cell(const PrepOut& o, size_t c, float e0, float e1, float e2,
+                                        float sc, float sx, float sy, float sz, bool hx, bool hy,
+                                        bool hz, double bc, float sig, Kahan32& kq, Kahan32& kb) {
+  const ff zero = ff_make(0.0f);
+  o.s[c] = f2d_scaled(sc, 0);
+  ff v0 = zero, v1 = zero, v2 = zero;
+  if (hx) v0 = scaled_coupling_f(e0, o.a0, c, sc, sx);
+  else o.a0[c] = 0.0;
+  if (hy) v1 = scaled_coupling_f(e1, o.a1, c, sc, sy);
+  else o.a1[c] = 0.0;
+  if (hz) v2 = scaled_coupling_f(e2, o.a2, c, sc, sz);
+  else o.a2[c] = 0.0;
+  o.f0[c] = v0.h;
+  o.f1[c] = v1.h;
+  o.f2[c] = v2.h;
+  // first sweep: x~ = 0 (the first k_ir_update writes x~ without reading it), r~ = s b,
+  // kept only as its FP32 form r~ 2^-e (the inner right-hand side), with the sums of
+  // squares of r~ 2^-e and b 2^-e (with x~ = 0 the true residual is b) compensated in FP32
+  const float qb = ff_hi_of(bc) * sig;
+  const float q = sc * qb;
+  o.rf[c] = q;
+  kq.add(q * q);
+  kb.add(qb * qb);
+  return v2;
+}
+
+// the line factors of level k > 0: l = aprev / d_{k-1}, inv_d = 1 / d_k
+__device__ __forceinline__ ff prep_factor(ff aprev, ff& inv_d) {
+  const ff l = ff_mul(aprev, inv_d);
+  ff d = ff_add_f(ff_neg(ff_mul(l, aprev)), 1.0f);
+  if (!(d.h > 1e-30f)) d = ff_make(1.0f);  // not SPD: that row falls back to Jacobi
+  inv_d = ff_div(ff_make(1.0f), d);
+  return l;
+}
+
+// The scalar end of the preparation (last block): norms, test and the first inner system.
+__device__ __forceinline__ void prep_tail(CgDevState* ir, CgDevState* in, const double (&tot)[2],
+                                          int sig_exp, double ir_rtol, double inner_rtol) {
+  if (!(tot[0] >= 0x1p-60 && tot[0] <= 0x1p60 && tot[1] >= 0x1p-60 && tot[1] <= 0x1p60)) {
+    // the scaled sums left the FP32 margin (or are 0, inf, NaN): the host recomputes this
+    // sweep's residual, norms and test in FP64 (k_ir_residual<true>, k_ir_scale)
+    ir->status = kRescaleRhs;
+    in->status = kConvergedAtol;  // the inner iterations launched ahead have nothing to do
+    return;
+  }
+  const double inv_sig = pow2d(sig_exp);
+  const double rn = sqrt(tot[1]) * inv_sig;
+  ir->ir_bnorm = rn;
+  ir->ir_rnorm = rn;
+  ir->dp = rn;
+  ir->a = sqrt(tot[0]) * inv_sig;
+  ir->first_a = ir->a;
+  if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol))
+    ir->status = rn < ir->atol ? kConvergedAtol : kConvergedRtol;
+  if (ir->status == 0) {
+    ir->rscale = inv_sig;
+    in->beta = tot[0];
+    in->rnorm0 = sqrt(tot[0]);
+    in->ttol = inner_rtol * in->rnorm0;
+    in->iter = 0;
+    in->its = 0;
+    in->dpi = 0.0;
+    in->status = 0;
+  } else {
+    in->status = kConvergedAtol;
+  }
+}
+
 __global__ void __launch_bounds__(128) k_prep_ff(
-    double* __restrict__ a0, double* __restrict__ a1, double* __restrict__ a2,
-    const float* __restrict__ dg, const double* __restrict__ b, double* __restrict__ s_out,
-    float* __restrict__ f0,
-    float* __restrict__ f1, float* __restrict__ f2, float* __restrict__ lk,
-    float* __restrict__ dinv, int n0, int n1, int n2, int line, CgDevState* ir,
-    double* partials, double ir_rtol, float* __restrict__ rf, CgDevState* in, int sig_exp,
+    PrepOut o, const float* __restrict__ dg, const double* __restrict__ b,
+    float* __restrict__ lk, float* __restrict__ dinv, int n0, int n1, int n2, int line,
+    CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
     double inner_rtol) {
   const int ncol = n0 * n1;
   const size_t sk = (size_t)ncol;
-  const ff zero = ff_make(0.0f);
   const float sig = pow2f_of(-sig_exp);
   Kahan32 kq, kb;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
        col += gridDim.x * blockDim.x) {
     const int i0 = col % n0, i1 = col / n0;
     const bool hx = i0 + 1 < n0, hy = i1 + 1 < n1;
-    ff inv_d = ff_make(1.0f), aprev = zero;
+    ff inv_d = ff_make(1.0f), aprev = ff_make(0.0f);
     size_t c = (size_t)col;
     // level k's inputs are loaded one level ahead (two levels of loads in flight per thread)
     float sc = scale_of(dg[c]);
-    float q0 = f0[c], q1 = f1[c], q2 = f2[c];
+    float q0 = o.f0[c], q1 = o.f1[c], q2 = o.f2[c];
     float dx = hx ? dg[c + 1] : 1.0f, dy = hy ? dg[c + n0] : 1.0f;
     float dz = n2 > 1 ? dg[c + sk] : 1.0f;
     double bq = b[c];
     for (int k = 0; k < n2; ++k, c += sk) {
       const float e0 = q0, e1 = q1, e2 = q2, ex = dx, ey = dy, ez = dz;
       const double bc = bq;
-      if (k + 1 < n2) {
+      const bool hz = k + 1 < n2;
+      if (hz) {
         const size_t cn = c + sk;
-        q0 = f0[cn];
-        q1 = f1[cn];
-        q2 = f2[cn];
+        q0 = o.f0[cn];
+        q1 = o.f1[cn];
+        q2 = o.f2[cn];
         dx = hx ? dg[cn + 1] : 1.0f;
         dy = hy ? dg[cn + n0] : 1.0f;
         dz = k + 2 < n2 ? dg[cn + sk] : 1.0f;
         bq = b[cn];
       }
-      const float sb = (k + 1 < n2) ? scale_of(ez) : 0.0f;
-      s_out[c] = f2d_scaled(sc, 0);
-      ff v0 = zero, v1 = zero, v2 = zero;
-      if (hx) v0 = scaled_coupling_f(e0, a0, c, sc, scale_of(ex));
-      else a0[c] = 0.0;
-      if (hy) v1 = scaled_coupling_f(e1, a1, c, sc, scale_of(ey));
-      else a1[c] = 0.0;
-      if (k + 1 < n2) v2 = scaled_coupling_f(e2, a2, c, sc, sb);
-      else a2[c] = 0.0;
-      f0[c] = v0.h;
-      f1[c] = v1.h;
-      f2[c] = v2.h;
-      ff l = zero;
+      const float sb = hz ? scale_of(ez) : 0.0f;
+      const ff v2 = prep_cell(o, c, e0, e1, e2, sc, scale_of(ex), scale_of(ey), sb, hx, hy, hz, bc,
+                              sig, kq, kb);
       if (line) {
-        if (k > 0) {
-          l = ff_mul(aprev, inv_d);
-          ff d = ff_add_f(ff_neg(ff_mul(l, aprev)), 1.0f);
-          if (!(d.h > 1e-30f)) d = ff_make(1.0f);  // not SPD: that row falls back to Jacobi
-          inv_d = ff_div(ff_make(1.0f), d);
-        }
+        ff l = ff_make(0.0f);
+        if (k > 0) l = prep_factor(aprev, inv_d);
         lk[c] = l.h;
         dinv[c] = inv_d.h;
         aprev = v2;
       }
-      // first sweep: x~ = 0 (the first k_ir_update writes x~ without reading it), r~ = s b,
-      // kept only as its FP32 form r~ 2^-e (the inner right-hand side), with the sums of
-      // squares of r~ 2^-e and b 2^-e (with x~ = 0 the true residual is b) compensated in FP32
-      const float qb = ff_hi_of(bc) * sig;
-      const float q = sc * qb;
-      rf[c] = q;
-      kq.add(q * q);
-      kb.add(qb * qb);
       sc = sb;
     }
   }
   double v[2] = {kq.value(), kb.value()};
   double tot[2];
   if (!grid_sum<2>(v, partials, &ir->arrive[0], tot)) return;
-  if (flat_tid() == 0) {
-    if (!(tot[0] >= 0x1p-60 && tot[0] <= 0x1p60 && tot[1] >= 0x1p-60 && tot[1] <= 0x1p60)) {
-      // the scaled sums left the FP32 margin (or are 0, inf, NaN): the host recomputes this
-      // sweep's residual, norms and test in FP64 (k_ir_residual<true>, k_ir_scale)
-      ir->status = kRescaleRhs;
-      in->status = kConvergedAtol;  // the inner iterations launched ahead have nothing to do
-      return;
+  if (flat_tid() == 0) prep_tail(ir, in, tot, sig_exp, ir_rtol, inner_rtol);
+}
+
+// The same preparation for grids whose columns are too few for a march with one thread each to keep
+// the loads in flight (a microsecond per level): a block owns 32 columns, its eight warps take the
+// cells' part level by level in any order, and only the line factors, which need the level above,
+// are left to one warp, from shared memory. March / split: 40 x 40 x 100 107 / 35 us, 203 x 149 x
+// 96 139 / 80, 256 x 256 x 128 208 / 202; 768 x 768 x 96 846 / 1400, where the march's loads
+// already fill the memory pipe and this form's barrier between its two parts empties it.
+constexpr int kPrepWarps = 8;
+constexpr int kPrepLevels = 190;         // 48 KB of scaled couplings beside the sums' 4 KB
+constexpr int kPrepSplitGroups = 2048;   // 65,536 columns: above, the march is the faster
+__global__ void __launch_bounds__(32 * kPrepWarps) k_prep_ff_split(
+    PrepOut o, const float* __restrict__ dg, const double* __restrict__ b,
+    float* __restrict__ lk, float* __restrict__ dinv, int n0, int n1, int n2, int line,
+    CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
+    double inner_rtol) {
+  extern __shared__ float2 prep_sh[];  // [n2][32]
+  const int ncol = n0 * n1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t sk = (size_t)ncol;
+  const float sig = pow2f_of(-sig_exp);
+  Kahan32 kq, kb;
+  const int groups = (ncol + 31) / 32;
+  for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+    const int col = g * 32 + lane;
+    const bool act = col < ncol;
+    const int i0 = col % n0, i1 = col / n0;
+    const bool hx = act && i0 + 1 < n0, hy = act && i1 + 1 < n1;
+    __syncthreads();  // the previous group's factors have been read
+#pragma unroll 4
+    for (int k = warp; k < n2; k += kPrepWarps) {
+      if (act) {
+        const size_t c = (size_t)col + sk * k;
+        const bool hz = k + 1 < n2;
+        const float sc = scale_of(dg[c]);
+        const float sx = scale_of(hx ? dg[c + 1] : 1.0f), sy = scale_of(hy ? dg[c + n0] : 1.0f);
+        const float sz = scale_of(hz ? dg[c + sk] : 1.0f);
+        const ff v2 = prep_cell(o, c, o.f0[c], o.f1[c], o.f2[c], sc, sx, sy, sz, hx, hy, hz, b[c],
+                                sig, kq, kb);
+        prep_sh[k * 32 + lane] = make_float2(v2.h, v2.l);
+      }
     }
-    const double inv_sig = pow2d(sig_exp);
-    const double rn = sqrt(tot[1]) * inv_sig;
-    ir->ir_bnorm = rn;
-    ir->ir_rnorm = rn;
-    ir->dp = rn;
-    ir->a = sqrt(tot[0]) * inv_sig;
-    ir->first_a = ir->a;
-    if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol))
-      ir->status = rn < ir->atol ? kConvergedAtol : kConvergedRtol;
-    if (ir->status == 0) {
-      ir->rscale = inv_sig;
-      in->beta = tot[0];
-      in->rnorm0 = sqrt(tot[0]);
-      in->ttol = inner_rtol * in->rnorm0;
-      in->iter = 0;
-      in->its = 0;
-      in->dpi = 0.0;
-      in->status = 0;
-    } else {
-      in->status = kConvergedAtol;
+    __syncthreads();
+    if (line && warp == 0 && act) {
+      ff inv_d = ff_make(1.0f);
+      size_t c = (size_t)col;
+      lk[c] = 0.0f;
+      dinv[c] = 1.0f;
+#pragma unroll 2
+      for (int k = 1; k < n2; ++k) {
+        c += sk;
+        const float2 v = prep_sh[(k - 1) * 32 + lane];
+        const ff l = prep_factor(ff_make(v.x, v.y), inv_d);
+        lk[c] = l.h;
+        dinv[c] = inv_d.h;
+      }
     }
   }
+  double v[2] = {kq.value(), kb.value()};
+  double tot[2];
+  if (!grid_sum<2>(v, partials, &ir->arrive[0], tot)) return;
+  if (flat_tid() == 0) prep_tail(ir, in, tot, sig_exp, ir_rtol, inner_rtol);
 }
 
 // sq = 1 / s for an operator scaled earlier (s already holds D^-1/2)
@@ -1014,13 +1098,27 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
       // the first inner right-hand side's scale: 2^-e with 2^(e-1) <= the previous solve's
       // first residual norm < 2^e
       const int sig_exp = pow2_above(first_rnorm[rnorm_slot & 1]);
+      const int groups = (ncol + 31) / 32;
+      const bool split = groups <= kPrepSplitGroups && A.n2 <= kPrepLevels;
+      const size_t split_sh = (size_t)A.n2 * 32 * sizeof(float2);
+      if (split && split_sh > 40 * 1024)
+        FG_CUDA(cudaFuncSetAttribute(k_prep_ff_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)split_sh));
       FG_LAUNCH(prof, st, "k_prep_ff",
                 (4.0 + 12.0 + 8.0 + 24.0 + 12.0 + 8.0 + 4.0 + (line ? 8.0 : 0.0)) * dn,
-                k_prep_ff<<<lb, 128, 0, st>>>(A.a0, A.a1, A.a2, reinterpret_cast<const float*>(A.s),
-                                              A.b, r, op32.a0, op32.a1, op32.a2, lkf, dinvf,
-                                              A.n0, A.n1, A.n2, line ? 1 : 0, dst, partials,
-                                              cfg.ir_rtol, rf, dst32, sig_exp,
-                                              cfg.inner_rtol));
+                {
+                  const PrepOut o = {A.a0, A.a1, A.a2, r, op32.a0, op32.a1, op32.a2, rf};
+                  const float* dg = reinterpret_cast<const float*>(A.s);
+                  if (split)
+                    k_prep_ff_split<<<std::min(groups, 6 * kNumSMs), 32 * kPrepWarps, split_sh,
+                                      st>>>(
+                        o, dg, A.b, lkf, dinvf, A.n0, A.n1, A.n2, line ? 1 : 0, dst, partials,
+                        cfg.ir_rtol, dst32, sig_exp, cfg.inner_rtol);
+                  else
+                    k_prep_ff<<<lb, 128, 0, st>>>(o, dg, A.b, lkf, dinvf, A.n0, A.n1, A.n2,
+                                                  line ? 1 : 0, dst, partials, cfg.ir_rtol,
+                                                  dst32, sig_exp, cfg.inner_rtol);
+                });
       FG_CUDA(cudaGetLastError());
       A.scaled = true;
       A.s_in_r = true;

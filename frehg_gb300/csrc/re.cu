@@ -876,8 +876,7 @@ static int picard_step(frehg_re* re) {
                   k_pic_update<true><<<nb, 256, 0, st>>>(a, re->ksp.x,
                                                          re->ksp.scale_vector(re->A)));
       FG_CUDA(cudaGetLastError());
-      FG_TRY(fetch_small(&re->sc_host->dq_max, &re->sc->dq_max, sizeof(double), st));
-      FG_TRY(fetch_small(&re->sc_host->stage_err, &re->sc->stage_err, sizeof(int), st));
+      FG_TRY(fetch_small(re->sc_host, re->sc, sizeof(ReScalars), st));
       FG_CUDA(cudaStreamSynchronize(st));
       if (re->sc_host->stage_err) {
         set_error("staged Picard assembly: a bounded wait on its copy pipeline ran out (%d)",

@@ -2,6 +2,7 @@
 // no grid barrier, no spin-wait), and the bounded grid barrier of cooperative launches.
 #pragma once
 
+#include "ff32.cuh"
 #include "internal.h"
 
 namespace fg {
@@ -15,7 +16,9 @@ struct Kahan32 {
     c = (t - s) - y;
     s = t;
   }
-  __device__ __forceinline__ double value() const { return (double)s - (double)c; }
+  // the sum as a double by integer operations (each FP64 instruction of a block's threads costs
+  // the SM's FP64 unit 19 clocks per warp)
+  __device__ __forceinline__ double value() const { return ff_to_double_nb(fast_two_sum(s, -c)); }
 };
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -29,25 +32,37 @@ __device__ __forceinline__ int flat_nthreads() { return blockDim.x * blockDim.y;
 __device__ __forceinline__ int flat_bid() { return blockIdx.x + blockIdx.y * gridDim.x; }
 __device__ __forceinline__ int flat_nblocks() { return gridDim.x * gridDim.y; }
 
-// Sum NV values over the block; the result is valid in thread 0.  Uses sh[NV*32].
-template <int NV>
+// Sum NV values over the block; the result is valid in every thread.  Uses sh[NV * CAP]; a
+// __syncthreads has to come between this and the next use of sh.
+// The threads' values (folded by shuffles to CAP at most) go through shared memory to one warp
+// per value: 13 FP64 instructions per value and block of 256 threads, where shuffles in every
+// warp take 45 (the SM's one FP64 unit serves a warp instruction in 19 clocks, so the reductions at
+// the ends of the blocks cost more than many of the kernels' own work on small grids: the FP64
+// residual of 40 x 40 x 100 took 26.8 us with shuffles in every warp, 18.1 so).
+template <int NV, int CAP = 256>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
-  const int tid = flat_tid(), lane = tid & 31, wid = tid >> 5, nw = flat_nthreads() >> 5;
+  const int tid = flat_tid(), lane = tid & 31, wid = tid >> 5;
+  const int nw = flat_nthreads() >> 5;
+  int width = 32;
+  for (; nw * width > CAP; width >>= 1) {
 #pragma unroll
-  for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
-  if (lane == 0) {
+    for (int q = 0; q < NV; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], width >> 1);
+  }
+  if (lane < width) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) sh[q * 32 + wid] = v[q];
+    for (int q = 0; q < NV; ++q) sh[q * CAP + wid * width + lane] = v[q];
   }
   __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double t = lane < nw ? sh[q * 32 + lane] : 0.0;
-      v[q] = warp_sum(t);
-    }
+  const int count = nw * width;
+  for (int q = wid; q < NV; q += nw) {
+    double t = lane < count ? sh[q * CAP + lane] : 0.0;
+    for (int i = lane + 32; i < count; i += 32) t += sh[q * CAP + i];
+    t = warp_sum(t);
+    if (lane == 0) sh[q * CAP] = t;
   }
   __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = sh[q * CAP];
 }
 
 // Grid-wide sum through per-block partials; returns true in every thread of the last block
@@ -55,7 +70,7 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
 template <int NV>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* partials, unsigned int* arrive,
                          double (&tot)[NV]) {
-  __shared__ double sh[NV * 32];
+  __shared__ double sh[NV * 256];
   __shared__ unsigned int ticket;
   const int tid = flat_tid(), bid = flat_bid(), nb = flat_nblocks();
   block_sum<NV>(v, sh);

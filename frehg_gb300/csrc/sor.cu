@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     double atol, double divtol, int max_it, CgDevState* dst) {
   extern __shared__ double sor_sh[];
   __shared__ CgDevState st;
-  __shared__ double red[64];
+  __shared__ double red[128];  // (the vectors of 3,600 cells leave 2 KB)
   const int n = n0 * n1 * n2, tid = threadIdx.x, warp = tid >> 5;
   constexpr int kWarps = kSorSolveThreads / 32;
   double *e0 = sor_sh, *e1 = e0 + n, *e2 = e1 + n, *invd = e2 + n, *r = invd + n, *v = r + n,
@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
       s[0] = fma(z[c], z[c], s[0]);
       s[1] = fma(z[c], r[c], s[1]);
     }
-    block_sum<2>(s, red);
+    block_sum<2, 64>(s, red);
     if (tid == 0) {
       if (st.bar_timeout)
         st.status = kGridBarrierTimeout;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
       w[c] = y;
       acc[0] = fma(pc, y, acc[0]);
     }
-    block_sum<1>(acc, red);
+    block_sum<1, 64>(acc, red);
     if (tid == 0) sor_alpha(&st, acc[0]);
     __syncthreads();
     if (st.status) break;
