@@ -29,6 +29,7 @@
 
 #include <cmath>
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -485,64 +486,46 @@ int* tc_error_word() {
   return w;
 }
 
-// The convolutions of the network (forward and data gradient) run on the tcgen05 kernel.
-// resident blocks per SM of a kernel with `smem` dynamic bytes and `tmem_cols` tensor-memory
-// columns: shared memory (1 KB reserved per block), 16 blocks of 128 threads, and the SM's 512
-// tensor-memory columns shared by its blocks
-static int tc_blocks_per_sm(int smem, int tmem_cols) {
-  int dev = 0, smem_sm = 228 * 1024;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  return std::max(1, std::min({smem_sm / (smem + 128 + 1024), 16, 512 / tmem_cols}));
+// Output planes per z column: the smallest time of the busiest block, in input planes, over the
+// columns it walks (a column of zc output planes reads zc + 2 input planes).
+static int conv_column(long tiles, int nz, long blocks) {
+  int best = nz;
+  long best_cost = LONG_MAX;
+  for (int cols = 1; cols <= nz; ++cols) {
+    const int zc = (nz + cols - 1) / cols;
+    const long items = tiles * ((nz + zc - 1) / zc);
+    const long cost = (items + blocks - 1) / blocks * (zc + 2);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = zc;
+    }
+    if (items >= 16 * blocks) break;  // even already
+  }
+  return best;
 }
 
+// The convolutions of the network (forward and data gradient) run on the tcgen05 kernel.  Output
+// channels in one part where the stacked weights allow it: one MMA of N = 144 (72 clocks) instead
+// of three of N = 48 (44 each).  Two parts for 32 to 96 (N at most 256), 64 to 64 (221 KB of weights)
+// and 96 to 32, whose 166 KB of weights would leave less than two planes of patches (270 us in one
+// part with eleven of the twelve slices resident, 200 in two).
 template <int CIN, int COUT>
 static void conv(const bf16* in, int in_stride, int in_off, const bf16* W, const float* bias,
                  bf16* out, int out_stride, int out_off, int nx, int ny, int nz, bool relu,
                  cudaStream_t st) {
-  if constexpr (CIN <= 16 && TcPShape<CIN, COUT>::FITS) {
-    // weights resident, one MMA group per output plane (16-channel inputs)
-    using Z = TcPShape<CIN, COUT>;
-    static int per_sm = 0;
-    if (per_sm == 0) {
-      cudaFuncSetAttribute(k_conv3_tcp<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           Z::SMEM);
-      per_sm = tc_blocks_per_sm(Z::SMEM, Z::TMEM_COLS);
-    }
-    const long items = (long)tc_tiles_x(nx) * tc_tiles_y(ny) * ((nz + kTcZC - 1) / kTcZC);
-    const int grid = (int)std::min<long>(items, (long)kNumSMs * per_sm);
-    k_conv3_tcp<CIN, COUT><<<grid, 128, Z::SMEM, st>>>(in, in_stride, in_off, W, bias, out,
-                                                       out_stride, out_off, nx, ny, nz,
-                                                       relu ? 1 : 0, tc_error_word());
-    return;
-  } else if constexpr (TcZShape<CIN, COUT>::FITS) {
-    // weights resident, z columns pipelined
-    using Z = TcZShape<CIN, COUT>;
-    static int per_sm = 0;
-    if (per_sm == 0) {
-      cudaFuncSetAttribute(k_conv3_tcz<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           Z::SMEM);
-      per_sm = tc_blocks_per_sm(Z::SMEM, Z::TMEM_COLS);
-    }
-    const long items = (long)tc_tiles_x(nx) * tc_tiles_y(ny) * ((nz + Z::ZC - 1) / Z::ZC);
-    const int grid = (int)std::min<long>(items, (long)kNumSMs * per_sm);
-    k_conv3_tcz<CIN, COUT><<<grid, 128, Z::SMEM, st>>>(in, in_stride, in_off, W, bias, out,
-                                                       out_stride, out_off, nx, ny, nz,
-                                                       relu ? 1 : 0, tc_error_word());
-    return;
-  }
-  using S = TcShape<CIN, COUT>;
-  static int per_sm = 0;
-  if (per_sm == 0) {
-    cudaFuncSetAttribute(k_conv3_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         S::SMEM);
-    per_sm = tc_blocks_per_sm(S::SMEM, S::TMEM_COLS);
-  }
-  const long tiles = (long)tc_tiles_x(nx) * tc_tiles_y(ny) * nz;
-  const int grid = (int)std::min<long>(tiles, (long)kNumSMs * per_sm);
-  k_conv3_tc<CIN, COUT><<<grid, 128, S::SMEM, st>>>(in, in_stride, in_off, W, bias, out,
-                                                    out_stride, out_off, nx, ny, nz,
-                                                    relu ? 1 : 0, tc_error_word());
+  constexpr int NB = COUT == 96 ? 48 : (27 * CIN * COUT * 2 > 150 * 1024 ? COUT / 2 : COUT);
+  constexpr int PARTS = COUT / NB;
+  using S = TcShape<CIN, NB>;
+  // set on every launch: the attribute belongs to the current device, and the call is cheap
+  cudaFuncSetAttribute(k_conv3_tc<CIN, COUT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       S::SMEM);
+  const long tiles = (long)tc_tiles_x(nx) * tc_tiles_y(ny), blocks = kNumSMs / PARTS;
+  const int zc = conv_column(tiles, nz, blocks);
+  const long items = tiles * ((nz + zc - 1) / zc);
+  const int grid = (int)std::min(items, blocks) * PARTS;
+  k_conv3_tc<CIN, COUT, NB><<<grid, kTcThreads, S::SMEM, st>>>(
+      in, in_stride, in_off, W, bias, out, out_stride, out_off, nx, ny, nz, zc, relu ? 1 : 0,
+      tc_error_word());
 }
 
 // the same convolution on the mma.sync kernel (the self-check's comparison)

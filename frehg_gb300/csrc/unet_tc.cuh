@@ -3,33 +3,44 @@
 //
 // Implicit GEMM per tile of 8 x 16 pixels (x, y) of one z plane: D[128 x COUT] (FP32, in TMEM;
 // row r = 8 py + px) = sum over the 27 taps and the input channels of A[128 x 16] . B[16 x COUT],
-// one tcgen05.mma.cta_group::1.kind::f16 (BF16 operands, FP32 accumulation, M = 128, N = COUT,
-// K = 16) per tap and 16-channel slice.  Operands sit in shared memory in the no-swizzle
-// K-major core-matrix layout, which the channels-last activations reach by splitting the
-// channels into 8-channel chunks:
-//   input patch [chunk][hy][hx][8]  (the 10 x 18 pixels x0-1 .. x0+8, y0-1 .. y0+16 of a plane,
-//               zero outside the grid): a tap (dx, dy) is the view starting at pixel
-//               (dx, dy); its M-adjacent core matrices (eight pixels of one patch row) are one
-//               patch row (160 bytes) apart, its K-adjacent ones one chunk plane (2880 bytes);
-//   weights     [tap][chunk][o][8]:  N-adjacent core matrices 128 bytes apart, K-adjacent ones
-//               COUT x 16 bytes.
-// Two-dimensional tiles stage 180 pixels per plane where a 128-pixel row tile needs three rows of
-// 130, which leaves shared memory for more resident blocks and deeper copy pipelines.
-// k_conv3_tc: a block (one warpgroup) walks its tiles; per z plane it loads the plane's patch and
-// the nine taps' weights of that plane with 16-byte cp.async copies, one thread issues the plane's
-// MMAs and commits them to an mbarrier, and the block waits for them before the next plane's
-// copies reuse the buffers.  The four warps then read the accumulator lanes (tcgen05.ld 32x32b:
-// warp w owns lanes 32w .. 32w+31 = rows), add the bias, apply the ReLU and store BF16.  Several
-// blocks per SM (shared memory, tensor-memory columns permitting) overlap one block's copies with
-// another's MMAs.
+// tcgen05.mma.cta_group::1.kind::f16 (BF16 operands, FP32 accumulation, M = 128, K = 16).
+// An MMA of M = 128 takes 32 + N / 4 clocks up to N = 96 (shared-memory reads: 4 KB of A, 32 N bytes
+// of B) and N / 2 above (measured, whatever the alignment of A), so the three dz taps are stacked along N: the weights sit as [t9][chunk][rb COUT + o][8] with
+// row block rb = 2 - dz, and one group of MMAs per INPUT plane z' (9 taps x CIN/16 slices, N =
+// 3 COUT) adds W(dz=2) In(z') to out(z'-1), W(1) In(z') to out(z') and W(0) In(z') to out(z'+1):
+// a third of the MMAs of one group per output plane over three input planes, and each input plane
+// is read once per tile.
+// Operands sit in shared memory in the no-swizzle K-major core-matrix layout, which the
+// channels-last activations reach by splitting the channels into 8-channel chunks:
+//   ring slots  [chunk of 2][hy][hx][8]: 16 channels of the 10 x 18 pixels x0-1 .. x0+8,
+//               y0-1 .. y0+16 of a plane, zero outside the grid; a tap (dx, dy) is the view starting
+//               at pixel (dx, dy), its M-adjacent core matrices one patch row (160 bytes) apart, its
+//               K-adjacent ones one chunk (2880 bytes);
+//   weights     N-adjacent core matrices 128 bytes apart, K-adjacent ones 3 COUT x 16 bytes; all 27
+//               taps stay resident.
+// The accumulators of consecutive output planes lie side by side in all 512 tensor-memory columns,
+// used as a ring (two MMAs instead of one where the three planes' columns wrap round); the epilogue
+// leaves each zeroed, so every MMA accumulates.
+// One block per SM; its warps work in parallel through mbarriers: eight copy planes into a ring of
+// patches (16-byte cp.async), one issues MMAs, one runs ahead with that warp's waits, eight read
+// finished accumulators (tcgen05.ld 32x32b), free them, add the bias, apply the ReLU and store BF16.
+// A block walks z columns of zc output planes (which cost zc + 2 input planes; conv_column chooses
+// zc so that the last blocks do not work alone).  The order of the sums is (dz, t9, channel slice)
+// for every output, whatever the columns.
+// Bound by the MMAs' shared-memory reads for 16 input channels, by the copies' 32-byte sectors for
+// 48 and 96.  256 x 256 x 128, against one MMA group per output plane and per-plane barriers of one
+// warpgroup: 16 -> 16 305 -> 153 us, 48 -> 16 617 -> 372; 128 x 128 x 64: 96 -> 32 628 -> 200, 32 ->
+// 32 96 -> 61; 64 x 64 x 32: 64 -> 64 112 -> 33.
 //
-// Every wait is bounded: a wait that runs out records an error word and the block stops
-// issuing work, waits (bounded) for its MMAs in flight, frees its tensor memory and returns.
+// Every wait is bounded: a wait that runs out records an error word, the block's other waits see
+// the abort word and return, and the MMAs in flight finish (bounded) before the tensor memory is
+// freed.
 #pragma once
 
 #include <cuda_bf16.h>
 
 #include <cstdint>
+#include <type_traits>
 
 namespace fg {
 namespace unet {
@@ -38,22 +49,12 @@ constexpr int kTcM = 128;                       // pixels per tile (the MMA's M)
 constexpr int kTcTX = 8, kTcTY = 16;             // the tile: 8 x 16 pixels, row r = 8 py + px
 constexpr int kTcHX = kTcTX + 2, kTcHY = kTcTY + 2;  // with the halo
 constexpr int kTcHP = kTcHX * kTcHY;             // 180 staged pixels per plane
-constexpr long kTcSpin = 1L << 24;
+constexpr long kTcSpin = 1L << 22;
+constexpr uint32_t kTcStop = 0xffffffffu;
 
 // tiles of an nx x ny plane
 __host__ __device__ inline int tc_tiles_x(int nx) { return (nx + kTcTX - 1) / kTcTX; }
 __host__ __device__ inline int tc_tiles_y(int ny) { return (ny + kTcTY - 1) / kTcTY; }
-
-template <int CIN, int COUT>
-struct TcShape {
-  static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 128, "channel counts");
-  static constexpr int CH = CIN / 8;
-  static constexpr int PLANE = kTcHP * 16;             // one chunk plane of a patch
-  static constexpr int ROWS = CH * PLANE;              // one z plane's patch
-  static constexpr int WTS = 9 * CH * COUT * 16;       // the nine taps of one z plane
-  static constexpr int SMEM = ROWS + WTS + 128;        // + alignment slack
-  static constexpr int TMEM_COLS = COUT <= 32 ? 32 : (COUT <= 64 ? 64 : 128);
-};
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -82,47 +83,91 @@ __device__ __forceinline__ void tc_cp16(void* dst, const void* src, int bytes) {
                : "memory");
 }
 
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity) {
-  for (long q = 0; q < kTcSpin; ++q) {
-    uint32_t ok;
+__device__ __forceinline__ void tc_bar_init(uint64_t* bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(bar)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void tc_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(bar)) : "memory");
+}
+
+// this thread's copies so far arrive on the barrier when they have landed
+__device__ __forceinline__ void tc_arrive_copies(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc_smem(bar)) : "memory");
+}
+
+// whether the phase is complete (TRY: after waiting for it for a time that the hardware limits)
+template <bool TRY = false>
+__device__ __forceinline__ bool tc_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  if (TRY)
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
         " selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(tc_smem(bar)), "r"(parity)
         : "memory");
-    if (ok) return true;
-  }
-  return false;
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(tc_smem(bar)), "r"(parity)
+        : "memory");
+  return ok != 0;
 }
 
-// Copies of the patch of plane zz (pixels x0-1 .. x0+8, y0-1 .. y0+16) into dst,
-// [chunk][hy][hx][8], with zero fill outside the grid: thread t copies patch pixel t (threads
-// 0-51 also pixel 128 + t), every chunk, so the index arithmetic is per pixel, not per copy.
-template <int CH>
-__device__ __forceinline__ void tc_load_patch(unsigned char* dst, const __nv_bfloat16* in,
-                                              int in_stride, int in_off, int x0, int y0, int zz,
-                                              int nx, int ny, int nz, int tid) {
-  const bool zok = zz >= 0 && zz < nz;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int p = half ? kTcM + tid : tid;
-    if (half && p >= kTcHP) break;
-    const int xx = x0 + p % kTcHX - 1, yy = y0 + p / kTcHX - 1;
-    const bool ok = zok && xx >= 0 && xx < nx && yy >= 0 && yy < ny;
-    const __nv_bfloat16* src =
-        ok ? in + ((size_t)xx + (size_t)nx * ((size_t)yy + (size_t)ny * zz)) * in_stride + in_off
-           : in;
-    unsigned char* d = dst + p * 16;
-#pragma unroll
-    for (int c = 0; c < CH; ++c) tc_cp16(d + c * kTcHP * 16, ok ? src + 8 * c : in, ok ? 16 : 0);
+// 1: the phase is complete; 0: the wait ran out; -1: *stop was set meanwhile
+__device__ __forceinline__ int tc_wait(uint64_t* bar, uint32_t parity, const volatile int* stop) {
+  for (long q = 0; q < kTcSpin; ++q) {
+    if (tc_test<true>(bar, parity)) return 1;
+    if (stop && *stop) return -1;
   }
+  return 0;
 }
 
-// byte offset of tap (dx, dy)'s view and of 16-channel slice kc in a patch
-template <int CH>
-__host__ __device__ constexpr uint32_t tc_tap_offset(int dx, int dy, int kc) {
-  return (uint32_t)(((2 * kc) * kTcHP + dy * kTcHX + dx) * 16);
+// the published count of ready planes once it exceeds p (kTcStop: the block stops)
+__device__ __forceinline__ uint32_t tc_ready(const uint32_t* word, uint32_t p) {
+  for (long q = 0; q < 16 * kTcSpin; ++q) {
+    uint32_t r;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(r) : "r"(tc_smem(word)) : "memory");
+    if (r > p) return r;
+  }
+  return kTcStop;
+}
+
+// true in one lane of a converged warp
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}"
+               : "=r"(p));
+  return p != 0;
+}
+
+// D (tensor memory) += A B of one M128 x N x K16 product
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.eq.u32 p, 0, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc)
+      : "memory");
+}
+
+// *bar completes when every MMA issued so far has
+__device__ __forceinline__ void tc_commit(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+          tc_smem(bar))
+      : "memory");
+}
+
+// zero 16 tensor-memory columns of the warp's lanes
+__device__ __forceinline__ void tc_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+      "%1};" ::"r"(taddr),
+      "r"(0u)
+      : "memory");
 }
 
 // A descriptor advanced by a byte offset (a multiple of 16): the start address is the low
@@ -132,599 +177,337 @@ __device__ __forceinline__ uint64_t tc_desc_at(uint64_t d, uint32_t bytes) {
   return d + (uint64_t)(bytes >> 4);
 }
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16* __restrict__ in,
-                                                  int in_stride, int in_off,
-                                                  const __nv_bfloat16* __restrict__ W,
-                                                  const float* __restrict__ bias,
-                                                  __nv_bfloat16* __restrict__ out, int out_stride,
-                                                  int out_off, int nx, int ny, int nz, int relu,
-                                                  int* err) {
-  using S = TcShape<CIN, COUT>;
+// Shape of the convolution CIN -> NB output channels (of COUT, in COUT / NB parts that blocks of
+// their own compute, where the weights of all COUT do not fit or 3 COUT exceeds the MMA's N of 256).
+template <int CIN, int NB>
+struct TcShape {
+  static_assert(CIN % 16 == 0 && NB % 16 == 0 && 3 * NB <= 256, "channel counts");
+  static constexpr int KC = CIN / 16;                  // 16-channel slices of a plane
+  static constexpr int N3 = 3 * NB;                    // the stacked N
+  static constexpr int PLANE = kTcHP * 16;             // eight channels of a patch
+  static constexpr int SLOT = 2 * PLANE;               // one slice of a plane's patch
+  static constexpr int WTS = 27 * CIN * NB * 2;        // all taps, [t9][chunk][rb NB + o][8]
+  static constexpr int LIMIT = 230400;                 // of the 227 KB a block can have
+  static constexpr int FIT = (LIMIT - WTS) / SLOT;
+  static constexpr int PLANES = (FIT < 30 ? FIT : 30) / KC;  // whole planes in the ring
+  static constexpr int SMEM = WTS + PLANES * KC * SLOT + 128;  // + alignment slack
+  static constexpr int R = 512 / NB;                   // accumulators in tensor memory
+  static constexpr int COPY_WARPS = KC == 1 ? 2 : KC <= 3 ? 4 : 8;  // that copy a plane together
+  static_assert(PLANES >= 2 && R >= 4, "ring");
+};
+
+// warps 0-7 epilogue (two groups of four, one per output plane in turn), 8-15 copies, 16 MMAs,
+// 17 the MMAs' waits
+constexpr int kTcCopyWarps = 8, kTcCopy0 = 8, kTcMma = kTcCopy0 + kTcCopyWarps;
+constexpr int kTcThreads = 32 * (kTcMma + 2);
+constexpr int kTcDone = 64;  // barriers of finished input planes, more than the roles can be apart
+
+template <int CIN, int COUT, int NB>
+__global__ void __launch_bounds__(kTcThreads, 1)
+    k_conv3_tc(const __nv_bfloat16* __restrict__ in, int in_stride, int in_off,
+               const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
+               __nv_bfloat16* __restrict__ out, int out_stride, int out_off, int nx, int ny, int nz,
+               int zc, int relu, int* err) {
+  using S = TcShape<CIN, NB>;
+  constexpr int PARTS = COUT / NB;
   extern __shared__ __align__(128) unsigned char tc_dyn[];
-  unsigned char* rows = reinterpret_cast<unsigned char*>(
+  unsigned char* wts = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(tc_dyn) + 127) & ~static_cast<uintptr_t>(127));
-  unsigned char* wts = rows + S::ROWS;
-  __shared__ __align__(8) uint64_t mma_bar;
+  unsigned char* ring = wts + S::WTS;
+  __shared__ __align__(8) uint64_t full[S::PLANES];     // a plane's slices have landed
+  __shared__ __align__(8) uint64_t acc_empty[S::R];     // an accumulator is read and zero again
+  __shared__ __align__(8) uint64_t done[kTcDone + 1];   // the MMAs of an input plane (last: all)
+  __shared__ uint32_t ready_word;  // input planes whose slices and accumulators are ready
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
-  volatile int& abort_flag = abort_word;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ float bias_s[NB];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform to the compiler, too
+  const int part = blockIdx.x % PARTS, o0 = part * NB;
 
-  if (warp == 0) {
+  if (warp == kTcMma) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      tc_smem(&tmem_slot)),
-                 "r"(S::TMEM_COLS)
+                 "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&mma_bar)) : "memory");
+    for (int q = 0; q < S::PLANES; ++q) tc_bar_init(&full[q], 32 * S::COPY_WARPS);
+    for (int q = 0; q < S::R; ++q) tc_bar_init(&acc_empty[q], 4);
+    for (int q = 0; q <= kTcDone; ++q) tc_bar_init(&done[q], 1);
+    ready_word = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     abort_word = 0;
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
-  const uint32_t rows_s = tc_smem(rows), wts_s = tc_smem(wts);
-  constexpr uint32_t idesc = tc_idesc(COUT);
-  uint32_t phase = 0;
-  int pending = 0;  // MMAs committed and not yet waited for
-
-  const int xt = tc_tiles_x(nx), yt = tc_tiles_y(ny);
-  const long tiles = (long)xt * yt * nz;
-  for (long tile = blockIdx.x; tile < tiles && !abort_flag; tile += gridDim.x) {
-    const int x0 = (int)(tile % xt) * kTcTX;
-    const long yz = tile / xt;
-    const int y0 = (int)(yz % yt) * kTcTY, z = (int)(yz / yt);
-    bool first = true;
-    for (int dz = -1; dz <= 1 && !abort_flag; ++dz) {
-      const int zz = z + dz;
-      if (zz < 0 || zz >= nz) continue;  // zero padding: the plane adds nothing
-      // the plane's patch, [chunk][hy][hx][8]
-      tc_load_patch<S::CH>(rows, in, in_stride, in_off, x0, y0, zz, nx, ny, nz, tid);
-      // the plane's nine taps of W[tap][o][i], [tap][chunk][o][8]
-      for (int q = tid; q < 9 * S::CH * COUT; q += 128) {
-        const int o = q % COUT, c = (q / COUT) % S::CH, t9 = q / (COUT * S::CH);
-        const int tap = (dz + 1) * 9 + t9;
-        tc_cp16(wts + ((t9 * S::CH + c) * COUT + o) * 16,
-                W + ((size_t)tap * COUT + o) * CIN + 8 * c, 16);
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      // the copies are generic-proxy writes the tensor cores read through the async proxy
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tid == 0) {
-        const uint64_t a0 = tc_desc(rows_s, S::PLANE, kTcHX * 16);
-        const uint64_t b0 = tc_desc(wts_s, COUT * 16, 128);
-#pragma unroll
-        for (int t9 = 0; t9 < 9; ++t9) {
-          const int dy = t9 / 3, dx = t9 % 3;
-#pragma unroll
-          for (int kc = 0; kc < CIN / 16; ++kc) {
-            const uint64_t a = tc_desc_at(a0, tc_tap_offset<S::CH>(dx, dy, kc));
-            const uint64_t b = tc_desc_at(b0, (t9 * S::CH + 2 * kc) * COUT * 16);
-            const uint32_t acc = first ? 0u : 1u;
-            asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-                "l"(a), "l"(b), "r"(idesc), "r"(acc)
-                : "memory");
-            first = false;
-          }
-        }
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                tc_smem(&mma_bar))
-            : "memory");
-      }
-      first = false;
-      pending = 1;
-      // the plane's MMAs read the buffers the next plane's copies overwrite (the outcome of the
-      // wait is made block-uniform, so every thread takes the same path)
-      const bool late = __syncthreads_or(!tc_wait(&mma_bar, phase));
-      if (late) {
-        if (tid == 0) atomicExch(err, 1);
-        abort_flag = 1;
-        break;
-      }
-      pending = 0;
-      phase ^= 1u;
-    }
-    if (abort_flag) break;
-    // epilogue: warp w reads TMEM lanes 32w .. 32w+31 (its 32 pixels), 16 columns at a time
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int r = warp * 32 + lane, px = x0 + (r & 7), py = y0 + (r >> 3);
-    __nv_bfloat16* dst =
-        out + ((size_t)px + (size_t)nx * ((size_t)py + (size_t)ny * z)) * out_stride + out_off;
-#pragma unroll
-    for (int cb = 0; cb < COUT; cb += 16) {
-      uint32_t r[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-            "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cb));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      uint32_t packed[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float v0 = __uint_as_float(r[2 * q]) + (bias ? bias[cb + 2 * q] : 0.f);
-        float v1 = __uint_as_float(r[2 * q + 1]) + (bias ? bias[cb + 2 * q + 1] : 0.f);
-        if (relu) {
-          v0 = fmaxf(v0, 0.f);
-          v1 = fmaxf(v1, 0.f);
-        }
-        __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-        packed[q] = *reinterpret_cast<uint32_t*>(&h);
-      }
-      if (px < nx && py < ny) {
-        uint4* d4 = reinterpret_cast<uint4*>(dst + cb);
-        d4[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        d4[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      }
-    }
-  }
-  // MMAs still in flight (a wait that ran out) finish before the tensor memory is freed
-  if (pending) (void)tc_wait(&mma_bar, phase);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(S::TMEM_COLS)
-                 : "memory");
-}
-
-
-// ---------------------------------------------------------------------------------------------
-// Per-output-plane pipelined form, for the 16-channel-input layers: their patches and weights
-// are small, and small tensor-memory accumulators (COUT columns, two of them) let six blocks
-// share an SM, which beats the dz-stacked form below for them (2.0 against 2.6 ms per
-// 16-to-16-channel layer at 768 x 768 x 96).  The 27 taps of weights stay resident in shared
-// memory (27 x CIN x COUT x 2 bytes <= 64 KB).
-// A block walks columns of ZC tiles along z at one (x, y) tile: a ring of four slots holds
-// input planes (one patch each, [slot][chunk][hy][hx][8]); each tile needs one new plane,
-// loaded one tile ahead with cp.async while the previous tile's MMAs run, and two tensor-memory
-// accumulators let the epilogue of tile z-1 overlap the MMAs of tile z:
-//   wait for plane z+1, barrier; issue MMA(z) -> acc[z&1], commit;
-//   wait MMA(z-1); load plane z+2 into the slot of plane z-2 (free: MMA(z-1) was its last
-//   reader); epilogue(z-1) from acc[(z-1)&1] while those copies land.
-// The MMA issue is unrolled over the taps and channel slices with the descriptors advanced by
-// constant offsets.
-constexpr int kTcZC = 16;  // output planes of one z column
-
-template <int CIN, int COUT>
-struct TcPShape {
-  static_assert(CIN % 16 == 0 && COUT % 16 == 0, "channel counts");
-  static constexpr int CH = CIN / 8;
-  static constexpr int PLANE = kTcHP * 16;
-  static constexpr int SLOT = CH * PLANE;              // one input plane's patch
-  static constexpr int WTS = 27 * CH * COUT * 16;      // all taps, [tap][chunk][o][8]
-  static constexpr int SMEM = WTS + 4 * SLOT + 128;
-  static constexpr int ACC_COLS = COUT <= 16 ? 16 : (COUT <= 32 ? 32 : 64);
-  static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;
-  static constexpr bool FITS = WTS <= 64 * 1024 && COUT <= 64;
-};
-
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv3_tcp(const __nv_bfloat16* __restrict__ in,
-                                                   int in_stride, int in_off,
-                                                   const __nv_bfloat16* __restrict__ W,
-                                                   const float* __restrict__ bias,
-                                                   __nv_bfloat16* __restrict__ out,
-                                                   int out_stride, int out_off, int nx, int ny,
-                                                   int nz, int relu, int* err) {
-  using S = TcPShape<CIN, COUT>;
-  extern __shared__ __align__(128) unsigned char tcp_dyn[];
-  unsigned char* wts = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(tcp_dyn) + 127) & ~static_cast<uintptr_t>(127));
-  unsigned char* ring = wts + S::WTS;
-  __shared__ __align__(8) uint64_t mma_bar[2];
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_smem(&tmem_slot)),
-                 "r"(S::TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&mma_bar[0])) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&mma_bar[1])) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  // all 27 taps of the weights, once per block
-  for (int q = tid; q < 27 * S::CH * COUT; q += 128) {
-    const int o = q % COUT, c = (q / COUT) % S::CH, tap = q / (COUT * S::CH);
-    tc_cp16(wts + ((tap * S::CH + c) * COUT + o) * 16, W + ((size_t)tap * COUT + o) * CIN + 8 * c,
-            16);
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
-  const uint32_t wts_s = tc_smem(wts), ring_s = tc_smem(ring);
-  constexpr uint32_t idesc = tc_idesc(COUT);
-  uint32_t phase[2] = {0u, 0u};
-  int outstanding[2] = {0, 0};  // MMAs committed to mma_bar[b] and not yet waited for
-  bool failed = false;
-
-  // copies of input plane zz's patch into ring slot zz & 3, zero outside the grid
-  auto load_plane = [&](int x0, int y0, int zz) {
-    tc_load_patch<S::CH>(ring + (zz & 3) * S::SLOT, in, in_stride, in_off, x0, y0, zz, nx, ny, nz,
-                         tid);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // bias + ReLU + BF16 store of tile (x0, y0, z) from accumulator b
-  auto epilogue = [&](int x0, int y0, int z, int b) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int r = warp * 32 + lane, px = x0 + (r & 7), py = y0 + (r >> 3);
-    __nv_bfloat16* dst =
-        out + ((size_t)px + (size_t)nx * ((size_t)py + (size_t)ny * z)) * out_stride + out_off;
-#pragma unroll
-    for (int cb = 0; cb < COUT; cb += 16) {
-      uint32_t r[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-            "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * S::ACC_COLS + cb)));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      uint32_t packed[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float v0 = __uint_as_float(r[2 * q]) + (bias ? bias[cb + 2 * q] : 0.f);
-        float v1 = __uint_as_float(r[2 * q + 1]) + (bias ? bias[cb + 2 * q + 1] : 0.f);
-        if (relu) {
-          v0 = fmaxf(v0, 0.f);
-          v1 = fmaxf(v1, 0.f);
-        }
-        __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-        packed[q] = *reinterpret_cast<uint32_t*>(&h);
-      }
-      if (px < nx && py < ny) {
-        uint4* d4 = reinterpret_cast<uint4*>(dst + cb);
-        d4[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        d4[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  };
-  // block-uniform bounded wait for the MMAs committed to mma_bar[b]
-  auto wait_mma = [&](int b) -> bool {
-    const bool late = __syncthreads_or(!tc_wait(&mma_bar[b], phase[b]));
-    if (late) {
-      if (tid == 0) atomicExch(err, 2);
-      return false;
-    }
-    phase[b] ^= 1u;
-    outstanding[b] = 0;
-    return true;
-  };
-
-  const int xt = tc_tiles_x(nx), yt = tc_tiles_y(ny);
-  const int zcols = (nz + kTcZC - 1) / kTcZC;
-  const long items = (long)xt * yt * zcols;
-  for (long item = blockIdx.x; item < items && !failed; item += gridDim.x) {
-    const int x0 = (int)(item % xt) * kTcTX;
-    const long rest = item / xt;
-    const int y0 = (int)(rest % yt) * kTcTY;
-    const int zb = (int)(rest / yt) * kTcZC, ze = min(nz, zb + kTcZC);
-    load_plane(x0, y0, zb - 1);
-    load_plane(x0, y0, zb);
-    load_plane(x0, y0, zb + 1);
-    for (int z = zb; z < ze; ++z) {
-      const int b = z & 1;
-      // planes z-1, z, z+1 (and, the first time, the weights) have landed
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tid == 0) {
-        bool first = true;
-        const uint64_t b0 = tc_desc(wts_s, COUT * 16, 128);
-        const uint32_t d_tmem = tmem + (uint32_t)(b * S::ACC_COLS);
-#pragma unroll
-        for (int dz = 0; dz < 3; ++dz) {
-          const int zz = z + dz - 1;
-          if (zz < 0 || zz >= nz) continue;  // zero padding
-          const uint64_t a0 =
-              tc_desc(ring_s + (uint32_t)((zz & 3) * S::SLOT), S::PLANE, kTcHX * 16);
-#pragma unroll
-          for (int t9 = 0; t9 < 9; ++t9) {
-            const int dy = t9 / 3, dx = t9 % 3, t = dz * 9 + t9;
-#pragma unroll
-            for (int kc = 0; kc < CIN / 16; ++kc) {
-              const uint64_t a = tc_desc_at(a0, tc_tap_offset<S::CH>(dx, dy, kc));
-              const uint64_t bd = tc_desc_at(b0, (t * S::CH + 2 * kc) * COUT * 16);
-              const uint32_t acc = first ? 0u : 1u;
-              asm volatile(
-                  "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-                  "l"(a), "l"(bd), "r"(idesc), "r"(acc)
-                  : "memory");
-              first = false;
-            }
-          }
-        }
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                tc_smem(&mma_bar[b]))
-            : "memory");
-      }
-      outstanding[b] = 1;
-      if (z > zb) {  // the previous tile: its MMAs were the last readers of plane z-2's slot
-        if (!wait_mma(b ^ 1)) {
-          failed = true;
-          break;
-        }
-        // the next plane's copies first, so that they run during the epilogue
-        if (z + 1 < ze) load_plane(x0, y0, z + 2);
-        epilogue(x0, y0, z - 1, b ^ 1);
-      } else if (z + 1 < ze) {
-        load_plane(x0, y0, z + 2);
-      }
-    }
-    if (failed) break;
-    if (!wait_mma((ze - 1) & 1)) {
-      failed = true;
-      break;
-    }
-    epilogue(x0, y0, ze - 1, (ze - 1) & 1);
-    __syncthreads();  // the next column's first copies reuse slots the last epilogue's MMAs read
-  }
-  // MMAs still in flight after a wait that ran out finish before the tensor memory is freed
-  for (int b = 0; b < 2; ++b)
-    if (outstanding[b]) (void)tc_wait(&mma_bar[b], phase[b]);
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(S::TMEM_COLS)
-                 : "memory");
-}
-
-// ---------------------------------------------------------------------------------------------
-// dz-stacked pipelined form, for the layers with 32 or more input channels whose 27 taps of
-// weights stay resident in shared memory (27 x CIN x COUT x 2 bytes <= 64 KB).  The three dz
-// taps are stacked along N: the weights sit as [t9][chunk][rb * COUT + o][8] with
-// row block rb = 2 - dz, so one group of MMAs per INPUT plane z' (9 taps x CIN/16 slices, N =
-// 3 COUT) adds W(dz=2) In(z') to out(z'-1), W(1) In(z') to out(z') and W(0) In(z') to out(z'+1)
-// at once: a third of the MMAs of one group per output plane over the three input planes, and
-// each input patch is read by one group only.  The accumulators of a column of ZC output planes
-// and of the planes on either side lie side by side in tensor memory (COUT columns each, zeroed
-// when the column starts); the input planes just outside the column add their one relevant
-// third (N = COUT).
-// A block walks columns of ZC output planes along z at one (x, y) tile with a ring of three
-// input patches; per input plane z' of the column (zb-1 .. ze):
-//   wait for plane z' (copied two planes ahead), barrier; issue MMAs(z'), commit;
-//   wait MMAs(z'-1), the last reader of plane z'-1's slot: copy plane z'+2 into it, then the
-//   epilogue of out(z'-2), complete with MMAs(z'-1), while MMAs(z') run.
-// The MMA issue is unrolled over the taps and channel slices with the descriptors advanced by
-// constant offsets.
-template <int CIN, int COUT>
-struct TcZShape {
-  static_assert(CIN % 16 == 0 && COUT % 16 == 0, "channel counts");
-  static constexpr int CH = CIN / 8;
-  static constexpr int N3 = 3 * COUT;                  // the stacked N
-  static constexpr int PLANE = kTcHP * 16;
-  static constexpr int SLOT = CH * PLANE;              // one input plane's patch
-  static constexpr int WTS = 9 * CH * N3 * 16;         // all taps, [t9][chunk][rb COUT + o][8]
-  static constexpr int SMEM = WTS + 3 * SLOT + 128;
-  static constexpr int TMEM_COLS = 256;
-  static constexpr int ZC = TMEM_COLS / COUT - 2;      // output planes per z column
-  static constexpr bool FITS = WTS <= 64 * 1024 && N3 <= 256;
-};
-
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv3_tcz(const __nv_bfloat16* __restrict__ in,
-                                                   int in_stride, int in_off,
-                                                   const __nv_bfloat16* __restrict__ W,
-                                                   const float* __restrict__ bias,
-                                                   __nv_bfloat16* __restrict__ out,
-                                                   int out_stride, int out_off, int nx, int ny,
-                                                   int nz, int relu, int* err) {
-  using S = TcZShape<CIN, COUT>;
-  extern __shared__ __align__(128) unsigned char tcz_dyn[];
-  unsigned char* wts = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(tcz_dyn) + 127) & ~static_cast<uintptr_t>(127));
-  unsigned char* ring = wts + S::WTS;
-  __shared__ __align__(8) uint64_t mma_bar[2];
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_smem(&tmem_slot)),
-                 "r"(S::TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&mma_bar[0])) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&mma_bar[1])) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
+  if (tid < NB) bias_s[tid] = bias ? bias[o0 + tid] : 0.f;
   // all 27 taps of the weights, once per block, the dz taps stacked along N
-  for (int q = tid; q < 9 * S::CH * S::N3; q += 128) {
-    const int orow = q % S::N3, c = (q / S::N3) % S::CH, t9 = q / (S::N3 * S::CH);
-    const int rb = orow / COUT, o = orow % COUT, tap = (2 - rb) * 9 + t9;
-    tc_cp16(wts + ((t9 * S::CH + c) * S::N3 + orow) * 16,
-            W + ((size_t)tap * COUT + o) * CIN + 8 * c, 16);
+  for (int q = tid; q < 9 * 2 * S::KC * S::N3; q += kTcThreads) {
+    const int c = q % (2 * S::KC), orow = (q / (2 * S::KC)) % S::N3, t9 = q / (S::N3 * 2 * S::KC);
+    const int rb = orow / NB, o = orow % NB, tap = (2 - rb) * 9 + t9;
+    tc_cp16(wts + ((t9 * 2 * S::KC + c) * S::N3 + orow) * 16,
+            W + ((size_t)tap * COUT + o0 + o) * CIN + 8 * c, 16);
   }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  // the copies are generic-proxy writes the tensor cores read through the async proxy
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-  const uint32_t wts_s = tc_smem(wts), ring_s = tc_smem(ring);
-  constexpr uint32_t idesc3 = tc_idesc(S::N3), idesc1 = tc_idesc(COUT);
-  uint32_t phase[2] = {0u, 0u};
-  int outstanding[2] = {0, 0};  // MMAs committed to mma_bar[b] and not yet waited for
-  bool failed = false;
-
-  // copies of input plane zz's patch into ring slot (zz + 3) % 3, zero outside the grid; a
-  // commit group every call (empty past the column), so each wait leaves exactly one pending
-  auto load_plane = [&](int x0, int y0, int zz, bool copy) {
-    if (copy)
-      tc_load_patch<S::CH>(ring + ((zz + 3) % 3) * S::SLOT, in, in_stride, in_off, x0, y0, zz,
-                           nx, ny, nz, tid);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // bias + ReLU + BF16 store of tile (x0, y0, z) from its accumulator (column col)
-  auto epilogue = [&](int x0, int y0, int z, uint32_t col) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int r = warp * 32 + lane, px = x0 + (r & 7), py = y0 + (r >> 3);
-    __nv_bfloat16* dst =
-        out + ((size_t)px + (size_t)nx * ((size_t)py + (size_t)ny * z)) * out_stride + out_off;
-#pragma unroll
-    for (int cb = 0; cb < COUT; cb += 16) {
-      uint32_t v[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-            "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-            "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(lane_base + col + (uint32_t)cb));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      uint32_t packed[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float v0 = __uint_as_float(v[2 * q]) + (bias ? bias[cb + 2 * q] : 0.f);
-        float v1 = __uint_as_float(v[2 * q + 1]) + (bias ? bias[cb + 2 * q + 1] : 0.f);
-        if (relu) {
-          v0 = fmaxf(v0, 0.f);
-          v1 = fmaxf(v1, 0.f);
-        }
-        __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-        packed[q] = *reinterpret_cast<uint32_t*>(&h);
-      }
-      if (px < nx && py < ny) {
-        uint4* d4 = reinterpret_cast<uint4*>(dst + cb);
-        d4[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        d4[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      }
+  volatile int* abort_flag = &abort_word;
+  // a bounded wait; where it runs out (or another role's has) the block stops issuing work
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+    const int r = tc_wait(bar, parity, abort_flag);
+    if (r == 0) {
+      *abort_flag = 1;
+      atomicExch(err, 1);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  };
-  // block-uniform bounded wait for the MMAs committed to mma_bar[b]
-  auto wait_mma = [&](int b) -> bool {
-    const bool late = __syncthreads_or(!tc_wait(&mma_bar[b], phase[b]));
-    if (late) {
-      if (tid == 0) atomicExch(err, 2);
-      return false;
-    }
-    phase[b] ^= 1u;
-    outstanding[b] = 0;
-    return true;
+    return r == 1;
   };
 
   const int xt = tc_tiles_x(nx), yt = tc_tiles_y(ny);
-  const int zcols = (nz + S::ZC - 1) / S::ZC;
+  const int zcols = (nz + zc - 1) / zc;
   const long items = (long)xt * yt * zcols;
-  for (long item = blockIdx.x; item < items && !failed; item += gridDim.x) {
-    const int x0 = (int)(item % xt) * kTcTX;
-    const long rest = item / xt;
-    const int y0 = (int)(rest % yt) * kTcTY;
-    const int zb = (int)(rest / yt) * S::ZC, ze = min(nz, zb + S::ZC);
-    // accumulator of output plane z (zb-1 .. ze) at column (z - zb + 1) COUT
-    auto col = [&](int z) { return (uint32_t)((z - zb + 1) * COUT); };
-    // zero the column's accumulators (the previous column's epilogues have read theirs)
-    {
-      const uint32_t zero[16] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-      for (int c0 = 0; c0 < (ze - zb + 2) * COUT; c0 += 16)
-        asm volatile(
-            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
-            "%13,%14,%15,%16};" ::"r"(lane_base + (uint32_t)c0),
-            "r"(zero[0]), "r"(zero[1]), "r"(zero[2]), "r"(zero[3]), "r"(zero[4]), "r"(zero[5]),
-            "r"(zero[6]), "r"(zero[7]), "r"(zero[8]), "r"(zero[9]), "r"(zero[10]),
-            "r"(zero[11]), "r"(zero[12]), "r"(zero[13]), "r"(zero[14]), "r"(zero[15])
-            : "memory");
+  const long first = blockIdx.x / PARTS, step = gridDim.x / PARTS;
+  // the input planes of the whole block are counted: plane p's MMAs complete done[p % kTcDone]
+  auto wait_done = [&](uint32_t p) {
+    return wait(&done[p % kTcDone], (p / kTcDone) & 1u);
+  };
+
+  if (warp < kTcCopy0) {
+    // ---- epilogue: warp w reads lanes 32 (w % 4) .. (its 32 pixels) of each finished accumulator
+    const int wr = warp & 3;
+    const uint32_t lane_base = tmem + ((uint32_t)(wr * 32) << 16);
+    if (warp < 4) {
+      for (int c0 = 0; c0 < S::R * NB; c0 += 16) tc_zero16(lane_base + (uint32_t)c0);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        for (int q = 0; q < S::R; ++q) tc_arrive(&acc_empty[q]);
     }
-    load_plane(x0, y0, zb - 1, true);
-    load_plane(x0, y0, zb, true);
-    for (int zp = zb - 1; zp <= ze; ++zp) {
-      const int b = (zp + 1) & 1;
-      // plane zp (and, the first time, the weights) has landed; plane zp+1 may be in flight
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tid == 0) {
-        if (zp >= 0 && zp < nz) {  // zero padding outside the grid adds nothing
-          // the stacked row blocks this plane adds: rb = 2 - dz adds to out(zp - 1 + rb)
-          const int rb0 = zp < zb ? 2 : 0, rbn = (zp < zb || zp >= ze) ? 1 : 3;
-          const uint64_t a0 =
-              tc_desc(ring_s + (uint32_t)(((zp + 3) % 3) * S::SLOT), S::PLANE, kTcHX * 16);
-          const uint64_t b0 = tc_desc(wts_s + (uint32_t)(rb0 * COUT * 16), S::N3 * 16, 128);
-          const uint32_t d_tmem = tmem + col(zp - 1 + rb0);
-          const uint32_t idesc = rbn == 3 ? idesc3 : idesc1;
+    const int px0 = (wr * 32 + lane) & 7, py0 = (wr * 32 + lane) >> 3;
+    uint32_t v = 0, pb = 0;  // accumulators and input planes of the columns before
+    bool ok = true;
+    for (long item = first; item < items && ok; item += step) {
+      const int px = (int)(item % xt) * kTcTX + px0;
+      const long rest = item / xt;
+      const int py = (int)(rest % yt) * kTcTY + py0;
+      const int zb = (int)(rest / yt) * zc, ze = min(nz, zb + zc);
+      const int z0 = max(zb - 1, 0), z1 = min(ze, nz - 1);
+      __nv_bfloat16* dst = out + ((size_t)px + (size_t)nx * ((size_t)py + (size_t)ny * zb)) *
+                                     out_stride + out_off + o0;
+      for (int z = zb; z < ze; ++z, ++v, dst += (size_t)nx * ny * out_stride) {
+        if ((int)(v & 1u) != warp >> 2) continue;
+        const uint32_t slot = v % S::R;
+        // complete with the input plane below it (the last plane of the grid with its own)
+        ok = wait_done(pb + (uint32_t)(min(z + 1, z1) - z0));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t r[NB];
 #pragma unroll
-          for (int t9 = 0; t9 < 9; ++t9) {
-            const int dy = t9 / 3, dx = t9 % 3;
+        for (int cb = 0; cb < NB; cb += 16) {
+          uint32_t* q = r + cb;
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+              "%13,%14,%15}, [%16];"
+              : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]),
+                "=r"(q[6]), "=r"(q[7]), "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]),
+                "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+              : "r"(lane_base + slot * NB + (uint32_t)cb));
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int kc = 0; kc < CIN / 16; ++kc) {
-              const uint64_t a = tc_desc_at(a0, tc_tap_offset<S::CH>(dx, dy, kc));
-              const uint64_t bd = tc_desc_at(b0, (t9 * S::CH + 2 * kc) * S::N3 * 16);
-              asm volatile(
-                  "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-                  "l"(a), "l"(bd), "r"(idesc), "r"(1u)
-                  : "memory");
+        for (int cb = 0; cb < NB; cb += 16) tc_zero16(lane_base + slot * NB + (uint32_t)cb);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tc_arrive(&acc_empty[slot]);
+        if (px < nx && py < ny) {
+#pragma unroll
+          for (int cb = 0; cb < NB; cb += 8) {
+            uint32_t packed[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float v0 = __uint_as_float(r[cb + 2 * q]) + bias_s[cb + 2 * q];
+              float v1 = __uint_as_float(r[cb + 2 * q + 1]) + bias_s[cb + 2 * q + 1];
+              if (relu) {
+                v0 = fmaxf(v0, 0.f);
+                v1 = fmaxf(v1, 0.f);
+              }
+              __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+              packed[q] = *reinterpret_cast<uint32_t*>(&h);
             }
+            *reinterpret_cast<uint4*>(dst + cb) =
+                make_uint4(packed[0], packed[1], packed[2], packed[3]);
           }
         }
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                tc_smem(&mma_bar[b]))
-            : "memory");
       }
-      outstanding[b] = 1;
-      if (zp > zb - 1) {  // MMAs(zp-1) were the last readers of plane zp-1's slot
-        if (!wait_mma(b ^ 1)) {
-          failed = true;
-          break;
+      pb += (uint32_t)(z1 - z0 + 1);
+    }
+  } else if (warp < kTcMma) {
+    // ---- copies: a plane's 16-byte pieces in memory order (a pixel's channels, then the next
+    // pixel's) over the lanes of a group of copy warps, so that an instruction's pieces share lines;
+    // the groups take the planes in turn (about six pieces per lane and plane).  The
+    // copies signal the plane's barrier themselves when they have landed, so that all free slots of
+    // the ring are being filled at any time; the warp that sees the barrier complete fences them
+    // against the tensor cores' reads (a fence here would wait for the warp's copies in flight).
+    constexpr int CH = 2 * S::KC, N = kTcHP * CH, LANES = 32 * S::COPY_WARPS;
+    constexpr uint32_t GROUPS = kTcCopyWarps / S::COPY_WARPS;
+    constexpr int PIECES = (N + LANES - 1) / LANES;
+    const int t = (tid - 32 * kTcCopy0) % LANES;
+    const uint32_t group = (uint32_t)(warp - kTcCopy0) / S::COPY_WARPS;
+    uint32_t p = 0;
+    bool ok = true;
+    for (long item = first; item < items && ok; item += step) {
+      const int x0 = (int)(item % xt) * kTcTX - 1;
+      const long rest = item / xt;
+      const int y0 = (int)(rest % yt) * kTcTY - 1;
+      const int zb = (int)(rest / yt) * zc, ze = min(nz, zb + zc);
+      const int z0 = max(zb - 1, 0), z1 = min(ze, nz - 1);
+      // the lane's pixels in the plane, -1 outside the grid
+      int pix[PIECES];
+#pragma unroll
+      for (int q = 0; q < PIECES; ++q) {
+        const int h = (t + q * LANES) / CH, xx = x0 + h % kTcHX, yy = y0 + h / kTcHX;
+        const bool in_grid = h < kTcHP && xx >= 0 && xx < nx && yy >= 0 && yy < ny;
+        pix[q] = in_grid ? xx + nx * yy : -1;
+      }
+      for (int z = z0; z <= z1; ++z, ++p) {
+        if (p % GROUPS != group) continue;
+        const uint32_t slot = p % S::PLANES;
+        if (p >= S::PLANES) {
+          ok = wait_done(p - S::PLANES);  // the slot's last readers
+          if (!ok) break;
         }
-        load_plane(x0, y0, zp + 2, zp + 2 <= ze);
-        if (zp - 2 >= zb) epilogue(x0, y0, zp - 2, col(zp - 2));
-      } else {
-        load_plane(x0, y0, zp + 2, zp + 2 <= ze);
+        const __nv_bfloat16* src = in + (size_t)nx * ny * z * in_stride + in_off;
+        unsigned char* d = ring + slot * (uint32_t)(S::KC * S::SLOT);
+#pragma unroll
+        for (int q = 0; q < PIECES; ++q) {
+          const int e = t + q * LANES, h = e / CH, c = e % CH;
+          if (e < N)
+            tc_cp16(d + c * S::PLANE + h * 16,
+                    pix[q] >= 0 ? src + (size_t)pix[q] * in_stride + 8 * c : in,
+                    pix[q] >= 0 ? 16 : 0);
+        }
+        tc_arrive_copies(&full[slot]);
       }
     }
-    if (failed) break;
-    if (!wait_mma((ze + 1) & 1)) {  // MMAs(ze)
-      failed = true;
-      break;
-    }
-    epilogue(x0, y0, ze - 1, col(ze - 1));
-    // the next column zeroes accumulators and overwrites slots this column's last reads used
     asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
+  } else if (warp == kTcMma) {
+    // ---- MMAs: the whole warp runs the loop, so that the descriptors are warp-uniform values
+    // (the instruction's operands are uniform registers); an elected lane issues
+    const uint32_t wts_s = tc_smem(wts), ring_s = tc_smem(ring);
+    const bool leader = tc_elect();
+    const uint64_t a_ring = tc_desc(ring_s, S::PLANE, kTcHX * 16);
+    const uint64_t b_all = tc_desc(wts_s, S::N3 * 16, 128);
+    constexpr uint32_t i3 = tc_idesc(S::N3);
+    uint32_t ready = 0, p = 0;        // input planes known to be ready, and done
+    uint32_t slot = 0, bar = 0;       // p % PLANES, p % kTcDone
+    uint32_t s0 = 0;                  // accumulator of the plane's first output plane
+    for (long item = first; item < items && ready != kTcStop; item += step) {
+      const int zb = (int)(item / ((long)xt * yt)) * zc, ze = min(nz, zb + zc);
+      const int z0 = max(zb - 1, 0), z1 = min(ze, nz - 1);
+      for (int zp = z0; zp <= z1; ++zp) {
+        const uint64_t a0 = tc_desc_at(a_ring, slot * (uint32_t)(S::KC * S::SLOT));
+        const uint32_t d0 = tmem + s0 * NB;
+        // one or two MMAs for each tap and slice
+        auto taps = [&](uint64_t b1, uint32_t i1, auto split, uint64_t b2, uint32_t i2) {
+          if (leader) {
+#pragma unroll
+            for (int t9 = 0; t9 < 9; ++t9) {
+#pragma unroll
+              for (int kc = 0; kc < S::KC; ++kc) {
+                const uint64_t a = tc_desc_at(a0, kc * S::SLOT + (t9 / 3 * kTcHX + t9 % 3) * 16);
+                const uint32_t bo = (uint32_t)((t9 * S::KC + kc) * 2 * S::N3 * 16);
+                tc_mma(d0, a, tc_desc_at(b1, bo), i1);
+                if (split) tc_mma(tmem, a, tc_desc_at(b2, bo), i2);
+              }
+            }
+            tc_commit(&done[bar]);
+          }
+        };
+        if (ready <= p) ready = __shfl_sync(0xffffffffu, tc_ready(&ready_word, p), 0);
+        if (ready == kTcStop) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (zp > zb && zp < ze - 1 && s0 + 3 <= S::R) {
+          taps(b_all, i3, std::false_type{}, b_all, i3);
+          s0 = s0 + 1 == S::R ? 0 : s0 + 1;
+        } else {
+          // output planes lo .. hi, which this input plane adds to; their accumulators are adjacent
+          // but where the ring of accumulators starts again
+          const int lo = max(zb, zp - 1), hi = min(ze - 1, zp + 1), count = hi - lo + 1;
+          const int c1 = min(count, (int)(S::R - s0)), c2 = count - c1;
+          const uint64_t b1 = tc_desc_at(b_all, (uint32_t)((lo - (zp - 1)) * NB * 16));
+          if (c2)
+            taps(b1, tc_idesc(NB * c1), std::true_type{},
+                 tc_desc_at(b1, (uint32_t)(c1 * NB * 16)), tc_idesc(NB * c2));
+          else
+            taps(b1, tc_idesc(NB * c1), std::false_type{}, b1, i3);
+          // the next plane's first output plane; after a column, the next column's
+          const int next = zp == z1 ? ze : max(zb, zp);
+          s0 = (s0 + (uint32_t)(next - lo)) % S::R;
+        }
+        ++p;
+        slot = slot + 1 == S::PLANES ? 0 : slot + 1;
+        bar = (bar + 1) % kTcDone;
+      }
+    }
+    // every MMA has finished before the tensor memory is freed, also after a wait that ran out
+    if (leader) {
+      tc_commit(&done[kTcDone]);
+      (void)tc_wait(&done[kTcDone], 0u, nullptr);
+    }
+    __syncwarp();
+  } else {
+    // ---- the MMAs' waits: a wait's latency (about 350 clocks, ready or not) in the issuing warp
+    // would leave the tensor cores idle between planes.  Here half the lanes test the next 16 planes
+    // and half the next 16 accumulators at once (a barrier's next phase only: the one before is
+    // known to be complete), and the issuing warp reads one counter when the planes it knows of
+    // are used up.
+    constexpr int NF = S::PLANES < 16 ? S::PLANES : 16, NA = S::R < 16 ? S::R : 16;
+    uint32_t p = 0, vb = 0;          // planes published; accumulators of the columns before
+    uint32_t landed = 0, accs = 0;   // that are known to be ready
+    bool ok = true;
+    for (long item = first; item < items && ok; item += step) {
+      const int zb = (int)(item / ((long)xt * yt)) * zc, ze = min(nz, zb + zc);
+      const int z0 = max(zb - 1, 0), z1 = min(ze, nz - 1);
+      for (int zp = z0; zp <= z1 && ok; ++zp, ++p) {
+        const uint32_t need_acc = vb + (uint32_t)(min(ze - 1, zp + 1) - zb + 1);
+        for (long q = 0; landed <= p || accs < need_acc; ++q) {
+          const uint32_t n = lane < 16 ? landed + lane : accs + (uint32_t)(lane - 16);
+          const bool t = lane < 16 ? lane < NF && tc_test(&full[n % S::PLANES], (n / S::PLANES) & 1u)
+                                   : lane - 16 < NA &&
+                                         tc_test(&acc_empty[n % S::R], (n / S::R) & 1u);
+          const uint32_t m = ~__ballot_sync(0xffffffffu, t);
+          landed += (uint32_t)__ffs(m & 0xffffu | 0x10000u) - 1;
+          accs += (uint32_t)__ffs(m >> 16 | 0x10000u) - 1;
+          if (__any_sync(0xffffffffu, *abort_flag || q >= kTcSpin)) {
+            ok = false;
+            break;
+          }
+        }
+        // the copies are generic-proxy writes the tensor cores read through the async proxy
+        __syncwarp();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(tc_smem(&ready_word)),
+                       "r"(ok ? p + 1 : kTcStop)
+                       : "memory");
+      }
+      vb += (uint32_t)(ze - zb);
+    }
+    if (!ok && lane == 0 && !*abort_flag) {
+      *abort_flag = 1;
+      atomicExch(err, 1);
+    }
   }
-  // MMAs still in flight after a wait that ran out finish before the tensor memory is freed
-  for (int b = 0; b < 2; ++b)
-    if (outstanding[b]) (void)tc_wait(&mma_bar[b], phase[b]);
-  asm volatile("cp.async.wait_all;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(S::TMEM_COLS)
+  if (warp == kTcMma)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512)
                  : "memory");
 }
 
