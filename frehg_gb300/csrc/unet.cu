@@ -225,25 +225,6 @@ __global__ void k_pool(const bf16* __restrict__ in, int in_stride, int in_off, b
   }
 }
 
-// nearest 2x upsampling of a coarse field (stride c) into a channel slice of a fine buffer
-__global__ void k_up(const bf16* __restrict__ in, bf16* __restrict__ out, int out_stride,
-                     int out_off, int c, int nx, int ny, int nz) {
-  // one thread per fine cell and group of 8 channels (16-byte copies); c, out_stride and
-  // out_off are multiples of 8.  Cell counts of the network's grids stay below 2^32.
-  const uint32_t n = (uint32_t)nx * ny * nz;
-  const uint32_t g = (uint32_t)c / 8;
-  const uint32_t cx = nx / 2, cy = ny / 2;
-  const uint64_t tot = (uint64_t)n * g;
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < tot;
-       e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t p = (uint32_t)(e / g), cg = (uint32_t)(e - (uint64_t)p * g);
-    const uint32_t x = p % nx, yz = p / nx, y = yz % ny, z = yz / ny;
-    const uint32_t q = (x >> 1) + cx * ((y >> 1) + cy * (z >> 1));
-    const uint4 v = *reinterpret_cast<const uint4*>(in + (size_t)q * c + 8 * cg);
-    *reinterpret_cast<uint4*>(out + (size_t)p * out_stride + out_off + 8 * cg) = v;
-  }
-}
-
 // gradient of upsampling: gin[q] = sum of the 8 children of a fine gradient slice; one thread per
 // coarse cell and group of 8 channels (16-byte accesses)
 __global__ void k_up_bwd(const bf16* __restrict__ gout, int g_stride, int g_off,
@@ -278,37 +259,53 @@ __global__ void k_up_bwd(const bf16* __restrict__ gout, int g_stride, int g_off,
 }
 
 // network input: [r * rscale, (lnK - mean) * kscale, cap * cscale, 0 ...] in 16 channels
+// Two lanes per cell, the odd one writing the zero half: a warp's stores are contiguous (58 us
+// at 256 x 256 x 128, 94 with one lane's two stores per cell).
 __global__ void k_pack_input(const float* __restrict__ r, const float* __restrict__ lnk,
                              const float* __restrict__ cap, const float* __restrict__ rscale,
                              float kmean, float kscale, float cscale, bf16* __restrict__ x,
                              size_t n) {
   const float rs = *rscale;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n;
-       p += (size_t)gridDim.x * blockDim.x) {
-    uint4* o = reinterpret_cast<uint4*>(x + p * 16);  // two 16-byte stores per cell
-    o[0] = make_uint4(pack2(r[p] * rs, (lnk[p] - kmean) * kscale), pack2(cap[p] * cscale, 0.f),
-                      0u, 0u);
-    o[1] = make_uint4(0u, 0u, 0u, 0u);
+  const bool zero = threadIdx.x & 1;
+#pragma unroll 4
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < 2 * n;
+       e += (size_t)gridDim.x * blockDim.x) {
+    const size_t p = e >> 1;
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    if (!zero) {
+      o.x = pack2(r[p] * rs, (lnk[p] - kmean) * kscale);
+      o.y = pack2(cap[p] * cscale, 0.f);
+    }
+    reinterpret_cast<uint4*>(x)[e] = o;
   }
 }
 
 // 1 / rms of r (zero -> 1) in two deterministic passes: per-block partial sums of r^2, then one
 // block adds the partials in a fixed order.
 constexpr int kRmsBlocks = 1024;
-__global__ void k_rms_partial(const float* __restrict__ r, size_t n, double* __restrict__ part) {
-  double s = 0.0;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n;
-       p += (size_t)gridDim.x * blockDim.x)
-    s += (double)r[p] * r[p];
-  __shared__ double sh[32];
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sh[q];
-    part[blockIdx.x] = t;
+// Eight elements in flight per thread, in four FP64 sums, converted by integer operations (the
+// conversion instruction would share the FP64 unit): 42 -> 20 us at 256 x 256 x 128, bound by
+// one FP64 instruction per element.
+__global__ void __launch_bounds__(256) k_rms_partial(const float* __restrict__ r, size_t n,
+                                                     double* __restrict__ part) {
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  for (; p + 7 * step < n; p += 8 * step) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = r[p + q * step];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double d = f2d_scaled(v[q], 0);
+      s[q & 3] = fma(d, d, s[q & 3]);
+    }
   }
+  for (; p < n; p += step) s[0] = fma((double)r[p], (double)r[p], s[0]);
+  double t[1] = {(s[0] + s[1]) + (s[2] + s[3])};
+  __shared__ double sh[256];
+  block_sum<1>(t, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = t[0];
 }
 
 __global__ void k_rms_scale(const double* __restrict__ part, int nparts, size_t n,
@@ -509,23 +506,23 @@ static int conv_column(long tiles, int nz, long blocks) {
 // of three of N = 48 (44 each).  Two parts for 32 to 96 (N at most 256), 64 to 64 (221 KB of weights)
 // and 96 to 32, whose 166 KB of weights would leave less than two planes of patches (270 us in one
 // part with eleven of the twelve slices resident, 200 in two).
-template <int CIN, int COUT>
+template <int CIN, int COUT, int UP = 0>
 static void conv(const bf16* in, int in_stride, int in_off, const bf16* W, const float* bias,
                  bf16* out, int out_stride, int out_off, int nx, int ny, int nz, bool relu,
-                 cudaStream_t st) {
+                 cudaStream_t st, const bf16* coarse = nullptr) {
   constexpr int NB = COUT == 96 ? 48 : (27 * CIN * COUT * 2 > 150 * 1024 ? COUT / 2 : COUT);
   constexpr int PARTS = COUT / NB;
   using S = TcShape<CIN, NB>;
   // set on every launch: the attribute belongs to the current device, and the call is cheap
-  cudaFuncSetAttribute(k_conv3_tc<CIN, COUT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaFuncSetAttribute(k_conv3_tc<CIN, COUT, NB, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        S::SMEM);
   const long tiles = (long)tc_tiles_x(nx) * tc_tiles_y(ny), blocks = kNumSMs / PARTS;
   const int zc = conv_column(tiles, nz, blocks);
   const long items = tiles * ((nz + zc - 1) / zc);
   const int grid = (int)std::min(items, blocks) * PARTS;
-  k_conv3_tc<CIN, COUT, NB><<<grid, kTcThreads, S::SMEM, st>>>(
-      in, in_stride, in_off, W, bias, out, out_stride, out_off, nx, ny, nz, zc, relu ? 1 : 0,
-      tc_error_word());
+  k_conv3_tc<CIN, COUT, NB, UP><<<grid, kTcThreads, S::SMEM, st>>>(
+      in, in_stride, in_off, coarse, W, bias, out, out_stride, out_off, nx, ny, nz, zc,
+      relu ? 1 : 0, tc_error_word());
 }
 
 // the same convolution on the mma.sync kernel (the self-check's comparison)
@@ -541,19 +538,20 @@ static void conv_sync(const bf16* in, int in_stride, int in_off, const bf16* W,
 // Weight gradient: as many blocks as the device holds at once, dealt to the groups of 16 input
 // channels; z columns of 16 planes (two extra input planes each), shorter on small grids until
 // there are items enough for every block.
-template <int CIN, int COUT>
+template <int CIN, int COUT, int UP = 0>
 static void conv_dw(const bf16* in, int in_stride, int in_off, const bf16* g, int g_stride,
-                    int g_off, float* dW, int nx, int ny, int nz, cudaStream_t st) {
+                    int g_off, float* dW, int nx, int ny, int nz, cudaStream_t st,
+                    const bf16* coarse = nullptr) {
   using S = DwShape<COUT>;
   // set on every launch: the attribute belongs to the current device, and the call is cheap
-  cudaFuncSetAttribute(k_conv3_dw<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+  cudaFuncSetAttribute(k_conv3_dw<CIN, COUT, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
   const long tiles = (long)((nx + kDwT - 1) / kDwT) * ((ny + kDwT - 1) / kDwT);
   const long want = std::max<long>(1, (long)kNumSMs * S::BLOCKS / (CIN / 16));
   int zc = 16;
   while (zc > 4 && tiles * ((nz + zc - 1) / zc) < want) zc /= 2;
   const long items = tiles * ((nz + zc - 1) / zc);
   const dim3 grid((unsigned)std::min(items, want), CIN / 16);
-  k_conv3_dw<CIN, COUT><<<grid, kDwThreads, S::SMEM, st>>>(in, in_stride, in_off, g, g_stride,
+  k_conv3_dw<CIN, COUT, UP><<<grid, kDwThreads, S::SMEM, st>>>(in, in_stride, in_off, coarse, g, g_stride,
                                                            g_off, dW, nx, ny, nz, zc);
 }
 
@@ -580,8 +578,8 @@ struct frehg_unet {
   // activations
   int nx = 0, ny = 0, nz = 0;
   size_t cap1 = 0;
-  bf16 *x0 = nullptr, *a1 = nullptr, *cat1 = nullptr, *d1a = nullptr, *d1 = nullptr;
-  bf16 *p1 = nullptr, *a2 = nullptr, *cat2 = nullptr, *d2a = nullptr, *d2 = nullptr;
+  bf16 *x0 = nullptr, *a1 = nullptr, *e1 = nullptr, *d1a = nullptr, *d1 = nullptr;
+  bf16 *p1 = nullptr, *a2 = nullptr, *e2 = nullptr, *d2a = nullptr, *d2 = nullptr;
   bf16 *p2 = nullptr, *a3 = nullptr, *e3 = nullptr;
   bf16 *g_d1 = nullptr, *g_d1a = nullptr, *g_cat1 = nullptr, *g_a1 = nullptr;
   bf16 *g_d2 = nullptr, *g_d2a = nullptr, *g_cat2 = nullptr, *g_p1 = nullptr, *g_a2 = nullptr;
@@ -651,12 +649,12 @@ int ensure_acts(frehg_unet* net, int nx, int ny, int nz) {
   };
   FG_TRY(A(&net->x0, n1 * 16));
   FG_TRY(A(&net->a1, n1 * 16));
-  FG_TRY(A(&net->cat1, n1 * 48));
+  FG_TRY(A(&net->e1, n1 * 16));
   FG_TRY(A(&net->d1a, n1 * 16));
   FG_TRY(A(&net->d1, n1 * 16));
   FG_TRY(A(&net->p1, n2 * 16));
   FG_TRY(A(&net->a2, n2 * 32));
-  FG_TRY(A(&net->cat2, n2 * 96));
+  FG_TRY(A(&net->e2, n2 * 32));
   FG_TRY(A(&net->d2a, n2 * 32));
   FG_TRY(A(&net->d2, n2 * 32));
   FG_TRY(A(&net->p2, n3 * 32));
@@ -696,18 +694,16 @@ int forward(frehg_unet* net, const float* r, const float* lnk, const float* cap,
   k_pack_input<<<blocks_for(n1), 256, 0, st>>>(r, lnk, cap, net->scal, net->kmean, net->kscale,
                                                net->cscale, net->x0, n1);
   conv<16, 16>(net->x0, 16, 0, W + net->wboff[0], M + net->boff[0], net->a1, 16, 0, nx, ny, nz, true, st);
-  conv<16, 16>(net->a1, 16, 0, W + net->wboff[1], M + net->boff[1], net->cat1, 48, 32, nx, ny, nz, true, st);
-  k_pool<<<blocks_for(n2 * 2), 256, 0, st>>>(net->cat1, 48, 32, net->p1, 16, nx, ny, nz);
+  conv<16, 16>(net->a1, 16, 0, W + net->wboff[1], M + net->boff[1], net->e1, 16, 0, nx, ny, nz, true, st);
+  k_pool<<<blocks_for(n2 * 2), 256, 0, st>>>(net->e1, 16, 0, net->p1, 16, nx, ny, nz);
   conv<16, 32>(net->p1, 16, 0, W + net->wboff[2], M + net->boff[2], net->a2, 32, 0, x2, y2, z2, true, st);
-  conv<32, 32>(net->a2, 32, 0, W + net->wboff[3], M + net->boff[3], net->cat2, 96, 64, x2, y2, z2, true, st);
-  k_pool<<<blocks_for(n3 * 4), 256, 0, st>>>(net->cat2, 96, 64, net->p2, 32, x2, y2, z2);
+  conv<32, 32>(net->a2, 32, 0, W + net->wboff[3], M + net->boff[3], net->e2, 32, 0, x2, y2, z2, true, st);
+  k_pool<<<blocks_for(n3 * 4), 256, 0, st>>>(net->e2, 32, 0, net->p2, 32, x2, y2, z2);
   conv<32, 64>(net->p2, 32, 0, W + net->wboff[4], M + net->boff[4], net->a3, 64, 0, x3, y3, z3, true, st);
   conv<64, 64>(net->a3, 64, 0, W + net->wboff[5], M + net->boff[5], net->e3, 64, 0, x3, y3, z3, true, st);
-  k_up<<<blocks_for(n2 * 64), 256, 0, st>>>(net->e3, net->cat2, 96, 0, 64, x2, y2, z2);
-  conv<96, 32>(net->cat2, 96, 0, W + net->wboff[6], M + net->boff[6], net->d2a, 32, 0, x2, y2, z2, true, st);
+  conv<96, 32, 64>(net->e2, 32, 0, W + net->wboff[6], M + net->boff[6], net->d2a, 32, 0, x2, y2, z2, true, st, net->e3);
   conv<32, 32>(net->d2a, 32, 0, W + net->wboff[7], M + net->boff[7], net->d2, 32, 0, x2, y2, z2, true, st);
-  k_up<<<blocks_for(n1 * 32), 256, 0, st>>>(net->d2, net->cat1, 48, 0, 32, nx, ny, nz);
-  conv<48, 16>(net->cat1, 48, 0, W + net->wboff[8], M + net->boff[8], net->d1a, 16, 0, nx, ny, nz, true, st);
+  conv<48, 16, 32>(net->e1, 16, 0, W + net->wboff[8], M + net->boff[8], net->d1a, 16, 0, nx, ny, nz, true, st, net->d2);
   conv<16, 16>(net->d1a, 16, 0, W + net->wboff[9], M + net->boff[9], net->d1, 16, 0, nx, ny, nz, true, st);
   k_out<<<blocks_for(n1), 256, 0, st>>>(net->d1, M + net->ooff, scaled_out ? net->scal + 1 : nullptr,
                                         y, n1);
@@ -744,7 +740,7 @@ int backward(frehg_unet* net, const float* target, cudaStream_t st) {
   conv_dw<16, 16>(net->d1a, 16, 0, net->g_d1, 16, 0, G + net->woff[9], nx, ny, nz, st);
   conv<16, 16>(net->g_d1, 16, 0, T + net->wboff[9], nullptr, net->g_d1a, 16, 0, nx, ny, nz, false, st);
   mask(c16, net->g_d1a, 16, 0, net->d1a, 16, 0, n1, 8);
-  conv_dw<48, 16>(net->cat1, 48, 0, net->g_d1a, 16, 0, G + net->woff[8], nx, ny, nz, st);
+  conv_dw<48, 16, 32>(net->e1, 16, 0, net->g_d1a, 16, 0, G + net->woff[8], nx, ny, nz, st, net->d2);
   conv<16, 48>(net->g_d1a, 16, 0, T + net->wboff[8], nullptr, net->g_cat1, 48, 0, nx, ny, nz, false, st);
   // level 2 decoder
   k_up_bwd<<<blocks_for(n2 * 4), 256, 0, st>>>(net->g_cat1, 48, 0, net->g_d2, 32, nx, ny, nz);
@@ -752,7 +748,7 @@ int backward(frehg_unet* net, const float* target, cudaStream_t st) {
   conv_dw<32, 32>(net->d2a, 32, 0, net->g_d2, 32, 0, G + net->woff[7], x2, y2, z2, st);
   conv<32, 32>(net->g_d2, 32, 0, T + net->wboff[7], nullptr, net->g_d2a, 32, 0, x2, y2, z2, false, st);
   mask(c32, net->g_d2a, 32, 0, net->d2a, 32, 0, n2, 6);
-  conv_dw<96, 32>(net->cat2, 96, 0, net->g_d2a, 32, 0, G + net->woff[6], x2, y2, z2, st);
+  conv_dw<96, 32, 64>(net->e2, 32, 0, net->g_d2a, 32, 0, G + net->woff[6], x2, y2, z2, st, net->e3);
   conv<32, 96>(net->g_d2a, 32, 0, T + net->wboff[6], nullptr, net->g_cat2, 96, 0, x2, y2, z2, false, st);
   // level 3
   k_up_bwd<<<blocks_for(n3 * 8), 256, 0, st>>>(net->g_cat2, 96, 0, net->g_e3, 64, x2, y2, z2);
@@ -764,7 +760,7 @@ int backward(frehg_unet* net, const float* target, cudaStream_t st) {
   conv<64, 32>(net->g_a3, 64, 0, T + net->wboff[4], nullptr, net->g_p2, 32, 0, x3, y3, z3, false, st);
   // level 2 encoder: e2 gradient = skip part + pooling part
   k_grad_mask<32, true><<<red_blocks(n2 * 4), 256, 0, st>>>(
-      net->g_cat2, 96, 64, net->cat2, 96, 64, net->g_p2, x2, y2, n2, G + net->boff[3]);
+      net->g_cat2, 96, 64, net->e2, 32, 0, net->g_p2, x2, y2, n2, G + net->boff[3]);
   conv_dw<32, 32>(net->a2, 32, 0, net->g_cat2, 96, 64, G + net->woff[3], x2, y2, z2, st);
   conv<32, 32>(net->g_cat2, 96, 64, T + net->wboff[3], nullptr, net->g_a2, 32, 0, x2, y2, z2, false, st);
   mask(c32, net->g_a2, 32, 0, net->a2, 32, 0, n2, 2);
@@ -772,7 +768,7 @@ int backward(frehg_unet* net, const float* target, cudaStream_t st) {
   conv<32, 16>(net->g_a2, 32, 0, T + net->wboff[2], nullptr, net->g_p1, 16, 0, x2, y2, z2, false, st);
   // level 1 encoder: e1 gradient = skip part + pooling part
   k_grad_mask<16, true><<<red_blocks(n1 * 2), 256, 0, st>>>(
-      net->g_cat1, 48, 32, net->cat1, 48, 32, net->g_p1, nx, ny, n1, G + net->boff[1]);
+      net->g_cat1, 48, 32, net->e1, 16, 0, net->g_p1, nx, ny, n1, G + net->boff[1]);
   conv_dw<16, 16>(net->a1, 16, 0, net->g_cat1, 48, 32, G + net->woff[1], nx, ny, nz, st);
   conv<16, 16>(net->g_cat1, 48, 32, T + net->wboff[1], nullptr, net->g_a1, 16, 0, nx, ny, nz, false, st);
   mask(c16, net->g_a1, 16, 0, net->a1, 16, 0, n1, 0);

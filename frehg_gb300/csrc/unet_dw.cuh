@@ -67,11 +67,12 @@ __device__ __forceinline__ void dw_mma(float (&d)[4], const uint32_t (&a)[4], ui
 
 // blockIdx.y: the group of 16 input channels; blocks of one group stride over the work items
 // (an x/y tile times a z column of zc planes).  dW is added to (FP32 atomics, one per
-// accumulator and block).
-template <int CIN, int COUT>
+// accumulator and block).  UP > 0: the first UP input channels are the nearest 2x upsampling of
+// `coarse` (UP channels); `in` holds the others.
+template <int CIN, int COUT, int UP>
 __global__ void __launch_bounds__(kDwThreads, DwShape<COUT>::BLOCKS) k_conv3_dw(
     const __nv_bfloat16* __restrict__ in, int in_stride, int in_off,
-    const __nv_bfloat16* __restrict__ gout, int g_stride, int g_off, float* __restrict__ dW, int nx,
+    const __nv_bfloat16* __restrict__ coarse, const __nv_bfloat16* __restrict__ gout, int g_stride, int g_off, float* __restrict__ dW, int nx,
     int ny, int nz, int zc) {
   using S = DwShape<COUT>;
   extern __shared__ __align__(128) unsigned char dw_smem[];
@@ -112,10 +113,14 @@ __global__ void __launch_bounds__(kDwThreads, DwShape<COUT>::BLOCKS) k_conv3_dw(
       for (int p = tid; p < kDwHPix; p += kDwThreads) {
         const int xx = x0 + p % kDwH - 1, yy = y0 + p / kDwH - 1;
         const bool ok = zok && xx >= 0 && xx < nx && yy >= 0 && yy < ny;
-        const __nv_bfloat16* src =
-            ok ? in + ((size_t)xx + (size_t)nx * ((size_t)yy + (size_t)ny * zz)) * in_stride +
-                     in_off + ic
-               : in;
+        const __nv_bfloat16* src = in;
+        if (ok && UP > 0 && ic < UP)
+          src = coarse + ((size_t)(xx >> 1) +
+                          (size_t)(nx >> 1) * ((size_t)(yy >> 1) + (size_t)(ny >> 1) * (zz >> 1))) *
+                             UP + ic;
+        else if (ok)
+          src = in + ((size_t)xx + (size_t)nx * ((size_t)yy + (size_t)ny * zz)) * in_stride + in_off +
+                ic - UP;
         tc_cp16(dst + p * 16, src, ok ? 16 : 0);
         tc_cp16(dst + (kDwHPix + p) * 16, ok ? src + 8 : in, ok ? 16 : 0);
       }

@@ -5,9 +5,9 @@
 // row r = 8 py + px) = sum over the 27 taps and the input channels of A[128 x 16] . B[16 x COUT],
 // tcgen05.mma.cta_group::1.kind::f16 (BF16 operands, FP32 accumulation, M = 128, K = 16).
 // An MMA of M = 128 takes 32 + N / 4 clocks up to N = 96 (shared-memory reads: 4 KB of A, 32 N bytes
-// of B) and N / 2 above (measured, whatever the alignment of A), so the three dz taps are stacked along N: the weights sit as [t9][chunk][rb COUT + o][8] with
-// row block rb = 2 - dz, and one group of MMAs per INPUT plane z' (9 taps x CIN/16 slices, N =
-// 3 COUT) adds W(dz=2) In(z') to out(z'-1), W(1) In(z') to out(z') and W(0) In(z') to out(z'+1):
+// of B) and N / 2 above (measured, whatever the alignment of A), so the three dz taps are stacked
+// along N: the weights sit as [t9][chunk][rb COUT + o][8] with row block rb = 2 - dz, and one group
+// of MMAs per INPUT plane z' (9 taps x CIN/16 slices, N = 3 COUT) adds W(dz=2) In(z') to out(z'-1), W(1) In(z') to out(z') and W(0) In(z') to out(z'+1):
 // a third of the MMAs of one group per output plane over three input planes, and each input plane
 // is read once per tile.
 // Operands sit in shared memory in the no-swizzle K-major core-matrix layout, which the
@@ -27,8 +27,11 @@
 // A block walks z columns of zc output planes (which cost zc + 2 input planes; conv_column chooses
 // zc so that the last blocks do not work alone).  The order of the sums is (dz, t9, channel slice)
 // for every output, whatever the columns.
-// Bound by the MMAs' shared-memory reads for 16 input channels, by the copies' 32-byte sectors for
-// 48 and 96.  256 x 256 x 128, against one MMA group per output plane and per-plane barriers of one
+// Bound by shared memory: the MMAs' reads (44 clocks of the 61 that an MMA of 48 -> 16 takes) and
+// the copies, which pass through L1.  (Copies past L1 are slower but for 96 channels, 16 copy warps
+// no faster.)  The decoder convolutions read the upsampled half of their input from the coarse
+// field, as the stored concatenation took 170 us more in all at 256 x 256 x 128.
+//  256 x 256 x 128, against one MMA group per output plane and per-plane barriers of one
 // warpgroup: 16 -> 16 305 -> 153 us, 48 -> 16 617 -> 372; 128 x 128 x 64: 96 -> 32 628 -> 200, 32 ->
 // 32 96 -> 61; 64 x 64 x 32: 64 -> 64 112 -> 33.
 //
@@ -202,9 +205,12 @@ constexpr int kTcCopyWarps = 8, kTcCopy0 = 8, kTcMma = kTcCopy0 + kTcCopyWarps;
 constexpr int kTcThreads = 32 * (kTcMma + 2);
 constexpr int kTcDone = 64;  // barriers of finished input planes, more than the roles can be apart
 
-template <int CIN, int COUT, int NB>
+// UP > 0: the first UP input channels are the nearest 2x upsampling of the coarse field `coarse` (UP
+// channels), read where it lies; `in` holds the others.
+template <int CIN, int COUT, int NB, int UP>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_conv3_tc(const __nv_bfloat16* __restrict__ in, int in_stride, int in_off,
+               const __nv_bfloat16* __restrict__ coarse,
                const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                __nv_bfloat16* __restrict__ out, int out_stride, int out_off, int nx, int ny, int nz,
                int zc, int relu, int* err) {
@@ -366,13 +372,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const int y0 = (int)(rest % yt) * kTcTY - 1;
       const int zb = (int)(rest / yt) * zc, ze = min(nz, zb + zc);
       const int z0 = max(zb - 1, 0), z1 = min(ze, nz - 1);
-      // the lane's pixels in the plane, -1 outside the grid
+      // the lane's pixels in the plane (of the coarse field for its channels), -1 outside the grid
       int pix[PIECES];
 #pragma unroll
       for (int q = 0; q < PIECES; ++q) {
         const int h = (t + q * LANES) / CH, xx = x0 + h % kTcHX, yy = y0 + h / kTcHX;
         const bool in_grid = h < kTcHP && xx >= 0 && xx < nx && yy >= 0 && yy < ny;
-        pix[q] = in_grid ? xx + nx * yy : -1;
+        const bool up = UP > 0 && (t + q * LANES) % CH < UP / 8;
+        pix[q] = !in_grid ? -1 : up ? (xx >> 1) + (nx >> 1) * (yy >> 1) : xx + nx * yy;
       }
       for (int z = z0; z <= z1; ++z, ++p) {
         if (p % GROUPS != group) continue;
@@ -381,15 +388,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           ok = wait_done(p - S::PLANES);  // the slot's last readers
           if (!ok) break;
         }
-        const __nv_bfloat16* src = in + (size_t)nx * ny * z * in_stride + in_off;
+        const __nv_bfloat16* src = in + (size_t)nx * ny * z * in_stride + in_off - UP;
+        const __nv_bfloat16* csrc =
+            UP > 0 ? coarse + (size_t)(nx >> 1) * (ny >> 1) * (z >> 1) * UP : nullptr;
         unsigned char* d = ring + slot * (uint32_t)(S::KC * S::SLOT);
 #pragma unroll
         for (int q = 0; q < PIECES; ++q) {
           const int e = t + q * LANES, h = e / CH, c = e % CH;
+          const bool up = UP > 0 && c < UP / 8;
           if (e < N)
             tc_cp16(d + c * S::PLANE + h * 16,
-                    pix[q] >= 0 ? src + (size_t)pix[q] * in_stride + 8 * c : in,
-                    pix[q] >= 0 ? 16 : 0);
+                    pix[q] < 0 ? in
+                               : (up ? csrc + (size_t)pix[q] * UP
+                                     : src + (size_t)pix[q] * in_stride) + 8 * c,
+                    pix[q] < 0 ? 0 : 16);
         }
         tc_arrive_copies(&full[slot]);
       }
