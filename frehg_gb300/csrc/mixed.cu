@@ -3,8 +3,9 @@
 //
 // The operator is the same unit-diagonal scaled stencil as the FP64 path (A~ = D^-1/2 A D^-1/2,
 // b~ = D^-1/2 b); its couplings are rounded once to FP32.  Each refinement sweep
-//   1. forms the true residual r~ = b~ - A~ x~ in FP64 (FP64 couplings) and its unscaled norm
-//      ||b - A x|| = ||r~ / s||; stops when ||b - A x|| <= ir_rtol * ||b||;
+//   1. forms the true residual r~ = b~ - A~ x~ in FP64 (FP64 couplings; the float-float operator's
+//      from exact FP32 products) and its unscaled norm ||b - A x|| = ||r~ / s||; stops when
+//      ||b - A x|| <= ir_rtol * ||b||;
 //   2. solves A~32 e = fp32(r~ 2^-k) with FP32 CG to a relative reduction inner_rtol (dot
 //      products in FP32 with Kahan compensation per thread, combined in FP64 across
 //      threads/blocks; 2^-k, a power of two near 1/||r~||, keeps FP32 away from underflow);
@@ -26,6 +27,38 @@
 
 namespace fg {
 
+// A complete sweep: the refinement test on the new true residual and the next inner system, by the
+// last block.  sum_rhs: the squares of the right-hand side r~ / 2^k' just written (2^k' next above
+// the previous ||r~||), sum_true: of (r~ / s) / unscale.
+template <bool LOOSE>
+__device__ __forceinline__ void sweep_tail(CgDevState* ir, CgDevState* in, double sum_rhs,
+                                           double sum_true, double unscale, double ir_rtol,
+                                           double inner_rtol) {
+  const double rn = sqrt(sum_true) * unscale;
+  ir->ir_its += 1;
+  ir->its += in->its;
+  ir->ir_rnorm = rn;
+  ir->dp = rn;
+  const double rs0 = pow2d(pow2_above(ir->a));
+  ir->a = sqrt(sum_rhs) * rs0;
+  if (isnan(rn) || isinf(rn)) {
+    ir->status = kDivergedNanOrInf;
+  } else if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol) || sum_rhs == 0.0) {
+    ir->status = rn < ir->atol ? kConvergedAtol : kConvergedRtol;
+  }
+  if (ir->status == 0) {
+    // the inner CG state, as k_ir_scale sets it, for the right-hand side r~ / rs0
+    ir->rscale = rs0;
+    in->beta = sum_rhs;
+    in->rnorm0 = sqrt(sum_rhs);
+    set_inner_tolerance<LOOSE>(in, inner_rtol, rn, fmax(ir_rtol * ir->ir_bnorm, ir->atol));
+    in->iter = 0;
+    in->its = 0;
+    in->dpi = 0.0;
+    in->status = 0;
+  }
+}
+
 // r~ = s b - A~ x~ (FP64); sums of r~^2 (scale of the inner system),
 // (r~/s)^2 = (sq r~)^2 for the true residual (sq = 1/s) and b^2 for ||b||.  The last block
 // runs the refinement test.  The inner solution e needs no zeroing: the inner solve's first
@@ -39,7 +72,7 @@ namespace fg {
 // ill-conditioned systems).
 // The inner iterations and k_ir_update are launched ahead of the host's knowledge of the inner
 // solve's state: as long as it runs (in->status == 0) this kernel returns at once.
-template <bool FIRST, bool INV_S = false>
+template <bool FIRST>
 __global__ void __launch_bounds__(256) k_ir_residual(
     const double* __restrict__ a0, const double* __restrict__ a1, const double* __restrict__ a2,
     const double* __restrict__ s, const double* __restrict__ sq, const double* __restrict__ b,
@@ -92,8 +125,7 @@ __global__ void __launch_bounds__(256) k_ir_residual(
         if (k + 1 < n2) ax = fma(a2[c], x[c + s01], ax);
         const double r = fma(s[c], b[c], -ax);
         const float rf = ff_hi_of(r);
-        // sq r~ = r~ / s (INV_S: s holds floats and sq is not stored)
-        const float sqc = INV_S ? __frcp_rn(ff_hi_of(s[c])) : ff_hi_of(sq[c]);
+        const float sqc = ff_hi_of(sq[c]);  // sq r~ = r~ / s
         const float q0 = rf * sig0, q1 = rf * sqc * sig1;
         rfo[c] = q0;  // the next inner solve's right-hand side, r~ / rs0 (rs0 = 2^k)
         k0.add(q0 * q0);
@@ -107,34 +139,19 @@ __global__ void __launch_bounds__(256) k_ir_residual(
   double tot[FIRST ? 3 : 2];
   if (!grid_sum<FIRST ? 3 : 2>(v, partials, &ir->arrive[0], tot)) return;
   if (flat_tid() == 0) {
-    const double rn = FIRST ? sqrt(tot[1]) : sqrt(tot[1]) * unscale;
     if constexpr (FIRST) {
+      const double rn = sqrt(tot[1]);
       ir->ir_bnorm = sqrt(tot[2]);
+      ir->ir_rnorm = rn;
+      ir->dp = rn;
+      ir->a = sqrt(tot[0]);
+      ir->first_a = ir->a;
+      if (isnan(rn) || isinf(rn))
+        ir->status = kDivergedNanOrInf;
+      else if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol) || tot[0] == 0.0)
+        ir->status = rn < ir->atol ? kConvergedAtol : kConvergedRtol;
     } else {
-      ir->ir_its += 1;  // a sweep is complete
-      ir->its += in->its;
-    }
-    ir->ir_rnorm = rn;
-    ir->dp = rn;
-    // ||r~||; later sweeps summed (r~ / rs0)^2, the FP32 right-hand side they wrote
-    const double rs0 = FIRST ? 1.0 : pow2d(pow2_above(ir->a));
-    ir->a = sqrt(tot[0]) * rs0;
-    if (FIRST) ir->first_a = ir->a;
-    if (isnan(rn) || isinf(rn)) {
-      ir->status = kDivergedNanOrInf;
-    } else if (rn <= fmax(ir_rtol * ir->ir_bnorm, ir->atol) || tot[0] == 0.0) {
-      ir->status = rn < ir->atol ? kConvergedAtol : kConvergedRtol;
-    }
-    if (!FIRST && ir->status == 0) {
-      // the inner CG state, as k_ir_scale sets it, for the right-hand side r~ / rs0
-      ir->rscale = rs0;
-      in->beta = tot[0];
-      in->rnorm0 = sqrt(tot[0]);
-      set_inner_tolerance<INV_S>(in, inner_rtol, rn, fmax(ir_rtol * ir->ir_bnorm, ir->atol));
-      in->iter = 0;
-      in->its = 0;
-      in->dpi = 0.0;
-      in->status = 0;
+      sweep_tail<false>(ir, in, tot[0], tot[1], unscale, ir_rtol, inner_rtol);
     }
   }
 }
@@ -675,6 +692,203 @@ __global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e,
     ir_update_cells<false>(x, e, n, rs, scale);
 }
 
+// x~ += 2^k e for the sweeps whose residual is updated (k_ir_sweep), not recomputed: e becomes the
+// change that x~ really made, fl(x~ + 2^k e) - x~, so that the updated residual is that of the
+// stored x~.  That change is a float: a multiple of ulp(x~) no longer than e's own 24 bits.  The
+// first sweep's x~ = 2^k e is exact and written by k_ir_sweep.
+__global__ void k_ir_update_exact(double* __restrict__ x, float* __restrict__ e, size_t n,
+                                  const CgDevState* ir, const CgDevState* in) {
+  if (ir->status || in->status == 0 || ir->ir_its == 0 || in->iter == 0) return;
+  const int scale = pow2_above(ir->rscale) - 1;  // rscale = 2^scale
+  const float back = pow2f_of(-scale);
+  const size_t gid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  auto step = [&](float& ev, double& xv) {
+    const double y = xv + f2d_scaled(ev, scale);
+    ev = ff_hi_of(y - xv) * back;
+    xv = y;
+  };
+  float4* e4 = reinterpret_cast<float4*>(e);
+  double2* x2 = reinterpret_cast<double2*>(x);
+  for (size_t q = gid; q < n / 4; q += stride) {
+    float4 ev = e4[q];
+    double2 lo = x2[2 * q], hi = x2[2 * q + 1];
+    step(ev.x, lo.x);
+    step(ev.y, lo.y);
+    step(ev.z, hi.x);
+    step(ev.w, hi.y);
+    e4[q] = ev;
+    x2[2 * q] = lo;
+    x2[2 * q + 1] = hi;
+  }
+  for (size_t c = (n & ~(size_t)3) + gid; c < n; c += stride) step(e[c], x[c]);
+}
+
+__device__ __forceinline__ float scale_of(float d) { return rsqrtf(d == 0.0f ? 1.0f : d); }
+
+// x 2^k as three floats h + m + l (24 + 24 + 5 bits of the significand, truncated in turn), by
+// integer operations.  Below 2^-126: zero; beyond the float range, inf and NaN: NaN.
+struct Float3 {
+  float h, m, l;
+};
+__device__ __forceinline__ Float3 split3(double x, int k) {
+  const int hx = __double2hiint(x), lx = __double2loint(x);
+  const int fe = ((hx >> 20) & 0x7ff) - (1023 - 127) + k;  // the float's biased exponent
+  const int sign = hx & (int)0x80000000;
+  Float3 r;
+  r.h = __int_as_float(sign | (fe << 23) | ((hx & 0x000fffff) << 3) | (int)((unsigned)lx >> 29));
+  const float p2 = __int_as_float(sign | ((fe & 0xff) << 23));
+  const unsigned low = (unsigned)lx & 0x1fffffffu;
+  r.m = __fmul_rn(__fmul_rn(__uint2float_rn(low & ~31u), 0x1p-52f), p2);
+  r.l = __fmul_rn(__fmul_rn(__uint2float_rn(low & 31u), 0x1p-52f), p2);
+  if (fe < 1) r.h = r.m = r.l = 0.0f;
+  if (fe > 254) r.h = __int_as_float(0x7fc00000);
+  return r;
+}
+
+// An exact sum of floats in three levels (the extraction of S. M. Rump, T. Ogita, S. Oishi, "Accurate
+// floating-point summation part I", SIAM J. Sci. Comput. 31(1), 2008): with 2^m above every term,
+// s0 collects the terms' bits down to 2^(m-20), s1 (which the products' low parts enter) those
+// down to 2^(m-39), both without rounding for up to 16 and 32 terms, s2 the rest: the sum is within
+// about 2^(m-57), where FP64's partial sums round at 2^(m-54).
+struct ExactSum {
+  float g0, g1, s0, s1, s2;
+  // m: the largest magnitude of the terms
+  __device__ __forceinline__ explicit ExactSum(float m) {
+    const int e = max(__float_as_int(m), 0x12000000) & 0x7f800000;  // 2^-91 at least
+    g0 = __int_as_float(e + (5 << 23));
+    g1 = __int_as_float(e - (14 << 23));
+    s0 = s1 = s2 = 0.0f;
+  }
+  __device__ __forceinline__ void low(float x) {
+    const float h = __fsub_rn(__fadd_rn(g1, x), g1);
+    s1 = __fadd_rn(s1, h);
+    s2 = __fadd_rn(s2, __fsub_rn(x, h));
+  }
+  __device__ __forceinline__ void add(float x) {
+    const float h = __fsub_rn(__fadd_rn(g0, x), g0);
+    s0 = __fadd_rn(s0, h);
+    low(__fsub_rn(x, h));
+  }
+  __device__ __forceinline__ ff value() const {
+    const ff t = two_sum(s0, s1);
+    return fast_two_sum(t.h, __fadd_rn(t.l, s2));
+  }
+};
+
+// The refinement residual of the float-float operator (a = hi + lo exactly), updated instead of
+// recomputed: r~ - A~ (2^k e), or s b - A~ (2^k e) in the first sweep, from exact FP32 products summed
+// in ExactSum, so that it stays the true residual of x~ to 2^-48 of itself and 2^-57 of its terms
+// (the FP64 stencil product rounds at 2^-53 of them) while the FP64 pipe, which bound that product
+// at 690 us for 56.6M cells, has nothing to do.  With the x~ update: 690 + 155 -> 607 + 132 us there,
+// 62 + 14 -> 54 + 12 for 2.9M cells, bound by its 380 instructions per warp and cell.  r~ is kept as float pairs in units of
+// the inner system's scale; the leading floats are the next right-hand side.  The first sweep also
+// writes x~ = 2^k e.
+struct SweepArgs {
+  const float *h0, *h1, *h2, *l0, *l1, *l2;  // A~
+  const float *dg, *e;                       // the diagonal (scale factors), the correction
+  const double* b;
+  double* x;
+  float2* r;
+  float* rf;
+};
+
+template <bool FIRST>
+__device__ __forceinline__ void sweep_cells(const SweepArgs& a, int n0, int n1, int n2, int planes,
+                                            int tiles, int scale, bool moved, float to_next,
+                                            float to_true, Kahan32& k0, Kahan32& k1) {
+  const int t0 = (n0 + 31) / 32;
+  const size_t s01 = (size_t)n0 * n1;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int i0 = (tile % t0) * 32 + threadIdx.x;
+    const int i1 = (tile / t0) * 8 + threadIdx.y;
+    if (i0 >= n0 || i1 >= n1) continue;
+    const bool xm = i0 > 0, xp = i0 + 1 < n0, ym = i1 > 0, yp = i1 + 1 < n1;
+    const int kb = blockIdx.y * planes, ke = min(n2, kb + planes);
+    size_t c = (size_t)i0 + (size_t)n0 * i1 + s01 * kb;
+    auto ev = [&](bool in, size_t at) { return in && moved ? a.e[at] : 0.0f; };
+    float eu = ev(kb > 0 && kb < ke, c - s01), ec = ev(kb < ke, c);
+    float hu = kb > 0 && kb < ke ? a.h2[c - s01] : 0.0f;
+    float lu = kb > 0 && kb < ke ? a.l2[c - s01] : 0.0f;
+    for (int k = kb; k < ke; ++k, c += s01) {
+      const bool zp = k + 1 < n2;
+      const float ed = ev(zp, c + s01);
+      const float en[6] = {ev(xm, c - 1), ev(xp, c + 1), ev(ym, c - n0), ev(yp, c + n0), eu, ed};
+      const float h2 = a.h2[c], l2 = a.l2[c];
+      const float ah[6] = {xm ? a.h0[c - 1] : 0.0f, a.h0[c], ym ? a.h1[c - n0] : 0.0f, a.h1[c],
+                           hu, h2};
+      const float al[6] = {xm ? a.l0[c - 1] : 0.0f, a.l0[c], ym ? a.l1[c - n0] : 0.0f, a.l1[c],
+                           lu, l2};
+      const float sc = scale_of(a.dg[c]);
+      Float3 bs;
+      float2 r;
+      if (FIRST) {
+        bs = split3(a.b[c], -scale);
+        r.x = __fmul_rn(sc, bs.h);
+        r.y = __fmaf_rn(sc, bs.h, -r.x);
+      } else {
+        r = a.r[c];
+      }
+      float p[6], m = fmaxf(fabsf(r.x), fabsf(ec));
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        p[q] = __fmul_rn(-ah[q], en[q]);
+        m = fmaxf(m, fabsf(p[q]));
+      }
+      ExactSum sum(m);
+      sum.add(r.x);
+      sum.low(r.y);
+      if (FIRST) {
+        const float pm = __fmul_rn(sc, bs.m);
+        sum.low(pm);
+        sum.s2 = __fadd_rn(sum.s2, __fmaf_rn(sc, bs.l, __fmaf_rn(sc, bs.m, -pm)));
+      }
+      sum.add(-ec);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        sum.add(p[q]);
+        sum.low(__fmaf_rn(-ah[q], en[q], -p[q]));
+        sum.low(__fmul_rn(-al[q], en[q]));
+      }
+      const ff v = sum.value();
+      const float q0 = v.h * to_next;
+      a.rf[c] = q0;
+      a.r[c] = make_float2(q0, v.l * to_next);
+      const float q1 = v.h * __frcp_rn(sc) * to_true;  // r~ / s
+      k0.add(q0 * q0);
+      k1.add(q1 * q1);
+      if (FIRST) a.x[c] = f2d_scaled(ec, scale);
+      eu = ec;
+      ec = ed;
+      hu = h2;
+      lu = l2;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256, 4) k_ir_sweep(SweepArgs a, int n0, int n1, int n2,
+                                                     int planes, int tiles, CgDevState* ir,
+                                                     CgDevState* in, double* partials,
+                                                     double ir_rtol, double inner_rtol) {
+  if (ir->status || in->status == 0) return;
+  const int scale = pow2_above(ir->rscale) - 1;  // rscale = 2^scale
+  const int next = pow2_above(ir->a);            // the next inner system's
+  const int tru = pow2_above(ir->ir_rnorm);
+  const bool moved = in->iter > 0;  // else e was not written: no correction
+  const float to_next = pow2f_of(min(max(scale - next, -120), 120));
+  const float to_true = pow2f_of(min(max(scale - tru, -120), 120));
+  Kahan32 k0, k1;
+  if (ir->ir_its == 0)
+    sweep_cells<true>(a, n0, n1, n2, planes, tiles, scale, moved, to_next, to_true, k0, k1);
+  else
+    sweep_cells<false>(a, n0, n1, n2, planes, tiles, scale, moved, to_next, to_true, k0, k1);
+  double v[2] = {k0.value(), k1.value()};
+  double tot[2];
+  if (!grid_sum<2>(v, partials, &ir->arrive[0], tot)) return;
+  if (flat_tid() == 0)
+    sweep_tail<true>(ir, in, tot[0], tot[1], pow2d(tru), ir_rtol, inner_rtol);
+}
+
 __global__ void k_to_f32(const double* __restrict__ a0, const double* __restrict__ a1,
                          const double* __restrict__ a2, float* __restrict__ f0,
                          float* __restrict__ f1, float* __restrict__ f2, size_t n) {
@@ -792,12 +1006,9 @@ __device__ __forceinline__ ff scaled_coupling64(double* a, size_t c, double sc, 
 
 // the float-float path's scale factors are floats, and so are the couplings the float-float
 // Picard assembly writes: a s_c s_n = a (p_h + p_l) with p = s_c s_n exact, one float-float by
-// float product, stored in FP64 for the refinement residual
-__device__ __forceinline__ ff scaled_coupling_f(float af, double* a, size_t c, float sc,
-                                                float sn) {
-  const ff v = ff_mul_f(two_prod(sc, sn), af);
-  a[c] = ff_to_double(v);
-  return v;
+// float product; the pair is the operator that k_ir_sweep's residual uses
+__device__ __forceinline__ ff scaled_coupling_f(float af, float sc, float sn) {
+  return ff_mul_f(two_prod(sc, sn), af);
 }
 
 __global__ void __launch_bounds__(128) k_scale_mixed(double* __restrict__ a0,
@@ -867,14 +1078,12 @@ __global__ void __launch_bounds__(128) k_scale_mixed(double* __restrict__ a0,
 // diagonal, the couplings and b are read once.  The assembly wrote
 // the diagonal (dg) and the unscaled couplings (f0-f2) as floats; f0-f2 are overwritten in
 // place by the scaled FP32 copies, and the FP64 scaled couplings go to a0-a2.
-__device__ __forceinline__ float scale_of(float d) { return rsqrtf(d == 0.0f ? 1.0f : d); }
-
 // One cell of the preparation: scale factors sc (its own), sx, sy, sz (the +1 neighbours'), the
 // unscaled couplings e0-e2 (0 towards absent neighbours); writes the scaled operator, s and the
 // first right-hand side and returns the scaled axis-2 coupling.
 struct PrepOut {
-  double *a0, *a1, *a2, *s;
-  float *f0, *f1, *f2, *rf;
+  double* s;
+  float *f0, *f1, *f2, *l0, *l1, *l2, *rf;  // the couplings' leading and low floats
 };
 __device__ __forceinline__ ff prep_cell(const PrepOut& o, size_t c, float e0, float e1, float e2,
                                         float sc, float sx, float sy, float sz, bool hx, bool hy,
@@ -882,15 +1091,15 @@ __device__ __forceinline__ ff prep_cell(const PrepOut& o, size_t c, float e0, fl
   const ff zero = ff_make(0.0f);
   o.s[c] = f2d_scaled(sc, 0);
   ff v0 = zero, v1 = zero, v2 = zero;
-  if (hx) v0 = scaled_coupling_f(e0, o.a0, c, sc, sx);
-  else o.a0[c] = 0.0;
-  if (hy) v1 = scaled_coupling_f(e1, o.a1, c, sc, sy);
-  else o.a1[c] = 0.0;
-  if (hz) v2 = scaled_coupling_f(e2, o.a2, c, sc, sz);
-  else o.a2[c] = 0.0;
+  if (hx) v0 = scaled_coupling_f(e0, sc, sx);
+  if (hy) v1 = scaled_coupling_f(e1, sc, sy);
+  if (hz) v2 = scaled_coupling_f(e2, sc, sz);
   o.f0[c] = v0.h;
   o.f1[c] = v1.h;
   o.f2[c] = v2.h;
+  o.l0[c] = v0.l;
+  o.l1[c] = v1.l;
+  o.l2[c] = v2.l;
   // first sweep: x~ = 0 (the first k_ir_update writes x~ without reading it), r~ = s b,
   // kept only as its FP32 form r~ 2^-e (the inner right-hand side), with the sums of
   // squares of r~ 2^-e and b 2^-e (with x~ = 0 the true residual is b) compensated in FP32
@@ -1066,6 +1275,9 @@ __global__ void k_inv64(const double* __restrict__ s, double* __restrict__ sq, s
     sq[c] = 1.0 / s[c];
 }
 
+// the float-float operator's low floats lie where the FP64 couplings do otherwise
+static float* low32(double* a) { return reinterpret_cast<float*>(a); }
+
 int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
                              const frehg_solver_config& cfg) {
   const size_t n = A.n;
@@ -1105,9 +1317,10 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
         FG_CUDA(cudaFuncSetAttribute(k_prep_ff_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)split_sh));
       FG_LAUNCH(prof, st, "k_prep_ff",
-                (4.0 + 12.0 + 8.0 + 24.0 + 12.0 + 8.0 + 4.0 + (line ? 8.0 : 0.0)) * dn,
+                (4.0 + 12.0 + 8.0 + 12.0 + 12.0 + 8.0 + 4.0 + (line ? 8.0 : 0.0)) * dn,
                 {
-                  const PrepOut o = {A.a0, A.a1, A.a2, r, op32.a0, op32.a1, op32.a2, rf};
+                  const PrepOut o = {r, op32.a0, op32.a1, op32.a2, low32(A.a0), low32(A.a1),
+                                     low32(A.a2), rf};
                   const float* dg = reinterpret_cast<const float*>(A.s);
                   if (split)
                     k_prep_ff_split<<<std::min(groups, 6 * kNumSMs), 32 * kPrepWarps, split_sh,
@@ -1136,11 +1349,13 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
     A.scaled = true;
     return FREHG_OK;
   }
-  // an operator scaled by an earlier solve: derive sq (unless r holds s), the FP32 copy and
-  // the factors from it
-  if (!A.s_in_r) FG_LAUNCH(prof, st, "k_inv64", 16.0 * dn, k_inv64<<<nb, 256, 0, st>>>(A.s, r, n));
-  FG_LAUNCH(prof, st, "k_to_f32", 36.0 * dn,
-            k_to_f32<<<nb, 256, 0, st>>>(A.a0, A.a1, A.a2, op32.a0, op32.a1, op32.a2, n));
+  // an operator scaled by an earlier solve: derive sq, the FP32 copy and the factors from it (the
+  // float-float preparation's are all still in place, the line factors if it made them)
+  if (!A.s_in_r) {
+    FG_LAUNCH(prof, st, "k_inv64", 16.0 * dn, k_inv64<<<nb, 256, 0, st>>>(A.s, r, n));
+    FG_LAUNCH(prof, st, "k_to_f32", 36.0 * dn,
+              k_to_f32<<<nb, 256, 0, st>>>(A.a0, A.a1, A.a2, op32.a0, op32.a1, op32.a2, n));
+  }
   if (line)
     FG_LAUNCH(prof, st, "k_line_factor", 16.0 * dn,
               k_line_factor<<<lb, 128, 0, st>>>(A.a2, lkf, dinvf, ncol, A.n2));
@@ -1283,18 +1498,24 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
   // x~ += 2^k e and the next true residual with the next inner system (both return at once on the
   // device while the inner solve still runs)
   auto sweep_end = [&]() {
-    FG_LAUNCH(prof, st, "k_ir_update", 20.0 * dn,
-              k_ir_update<<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
-    FG_LAUNCH(prof, st, "k_ir_residual", 52.0 * dn, {
-      if (A.s_in_r)
-        k_ir_residual<false, true><<<L.grid, L.block, 0, st>>>(
-            A.a0, A.a1, A.a2, sv, sv, A.b, x, rres, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
-            partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol);
-      else
-        k_ir_residual<false><<<L.grid, L.block, 0, st>>>(
-            A.a0, A.a1, A.a2, A.s, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
-            partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol);
-    });
+    if (A.s_in_r) {
+      const SweepArgs sa = {op32.a0, op32.a1, op32.a2, low32(A.a0), low32(A.a1), low32(A.a2),
+                            reinterpret_cast<const float*>(A.s), xf, A.b, x,
+                            reinterpret_cast<float2*>(rres), rf};
+      FG_LAUNCH(prof, st, "k_ir_update", 24.0 * dn,
+                k_ir_update_exact<<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
+      FG_LAUNCH(prof, st, "k_ir_sweep", 56.0 * dn,
+                k_ir_sweep<<<L.grid, L.block, 0, st>>>(sa, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
+                                                       dst32, partials, cfg.ir_rtol,
+                                                       cfg.inner_rtol));
+    } else {
+      FG_LAUNCH(prof, st, "k_ir_update", 20.0 * dn,
+                k_ir_update<<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
+      FG_LAUNCH(prof, st, "k_ir_residual", 52.0 * dn,
+                k_ir_residual<false><<<L.grid, L.block, 0, st>>>(
+                    A.a0, A.a1, A.a2, A.s, r, A.b, x, rres, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
+                    partials, cfg.ir_rtol, rf, dst32, cfg.inner_rtol));
+    }
   };
 
   // Rounds of: the inner solve's start (on a new sweep), some inner iterations, the sweep's end,
@@ -1385,7 +1606,7 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
       }
       if (hst->ir_its == sweeps) {
         prof->idle("k_ir_update", 1);
-        prof->idle("k_ir_residual", 1);
+        prof->idle(A.s_in_r ? "k_ir_sweep" : "k_ir_residual", 1);
       }
     }
     if (dbg)
