@@ -405,61 +405,101 @@ __global__ void __launch_bounds__(128) k32_spmv_v4(const float* __restrict__ a0,
 // instead of one for each cell beside the tile's own, from L1 and L2).  28 B/cell, against 36
 // for a direction pass and a product: 260 us at 768 x 768 x 96, 0.90 of the copy peak (the product
 // alone was 210, the direction's pass 160).
-__global__ void __launch_bounds__(256) k32_dir_spmv(
+// This form is for row lengths that are no multiple of 4: a thread owns four rows of a column and
+// marches through its planes, so that loads stay coalesced along axis 0, a row's couplings and
+// directions serve the rows on either side, and a level's loads are in flight together (203 x 149 x
+// 96: 40 us an iteration with one row per thread, 32 so).
+constexpr int kDirRows = 4;
+template <bool FIRST>
+__device__ __forceinline__ void dir_spmv_rows(
+    const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
+    const float* __restrict__ z, const float* __restrict__ po, float* __restrict__ pn,
+    float* __restrict__ w, float bc, int n0, int n1, int n2, int planes, int tiles, Kahan32& acc) {
+  constexpr int R = kDirRows;
+  auto dir = [&](size_t c) { return FIRST ? z[c] : fmaf(bc, po[c], z[c]); };
+  const int t0 = (n0 + 31) / 32, lane = threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const size_t s01 = (size_t)n0 * n1;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int i0 = (tile % t0) * 32 + lane;
+    const int j0 = ((tile / t0) * blockDim.y + threadIdx.y) * R;
+    const int nr = min(R, n1 - j0);  // the warp's rows
+    if (nr <= 0) continue;
+    const int kb = blockIdx.y * planes, ke = min(n2, kb + planes);
+    // lanes past the row's end and rows past the last repeat the last ones (nothing is stored, and
+    // the couplings towards them are zero)
+    size_t c = (size_t)min(i0, n0 - 1) + (size_t)n0 * j0 + s01 * kb;
+    int off[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) off[r] = n0 * min(r, nr - 1);
+    const bool south = j0 > 0, north = j0 + nr < n1;
+    const bool left = lane == 0 && i0 > 0, edge = left || (lane == 31 && i0 + 1 < n0);
+    float pm[R], am[R], pc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      pm[r] = kb > 0 ? dir(c - s01 + off[r]) : 0.0f;
+      am[r] = kb > 0 ? a2[c - s01 + off[r]] : 0.0f;
+      pc[r] = dir(c + off[r]);
+    }
+    for (int k = kb; k < ke; ++k, c += s01) {
+      float pp[R], A0[R], A1[R], A2[R], pe[R], ae[R];
+      const size_t ce = left ? c - 1 : c + 1;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        pp[r] = k + 1 < n2 ? dir(c + s01 + off[r]) : 0.0f;
+        A0[r] = a0[c + off[r]];
+        A1[r] = a1[c + off[r]];
+        A2[r] = a2[c + off[r]];
+        pe[r] = edge ? dir(ce + off[r]) : 0.0f;
+        ae[r] = left ? a0[c - 1 + off[r]] : 0.0f;
+      }
+      const float pS = south ? dir(c - n0) : 0.0f, AS = south ? a1[c - n0] : 0.0f;
+      const float pN = north ? dir(c + (size_t)n0 * nr) : 0.0f;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float pl = __shfl_up_sync(full, pc[r], 1), al = __shfl_up_sync(full, A0[r], 1);
+        float pr = __shfl_down_sync(full, pc[r], 1);
+        if (lane == 0) {
+          pl = pe[r];
+          al = ae[r];
+        }
+        if (lane == 31) pr = pe[r];
+        float v = fmaf(al, pl, pc[r]);
+        v = fmaf(A0[r], pr, v);
+        v = r == 0 ? fmaf(AS, pS, v) : fmaf(A1[r - 1], pc[r - 1], v);
+        v = fmaf(A1[r], r + 1 < R && r + 1 < nr ? pc[r + 1] : pN, v);
+        v = fmaf(am[r], pm[r], v);
+        v = fmaf(A2[r], pp[r], v);
+        if (r < nr && i0 < n0) {
+          pn[c + off[r]] = pc[r];
+          w[c + off[r]] = v;
+          acc.add(pc[r] * v);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        pm[r] = pc[r];
+        pc[r] = pp[r];
+        am[r] = A2[r];
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128) k32_dir_spmv(
     const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
     const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
     float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
     double* partials) {
   if (st->status) return;
-  const bool first = st->iter == 0, odd = st->iter & 1;
-  const float bc = first ? 0.0f : (float)st->bcoef;
-  const float* __restrict__ po = odd ? p1 : p0;
-  float* __restrict__ pn = odd ? p0 : p1;
-  auto dir = [&](size_t c) { return first ? z[c] : fmaf(bc, po[c], z[c]); };
-  const int t0 = (n0 + 31) / 32, lane = threadIdx.x;
-  const unsigned full = 0xffffffffu;
-  const size_t s01 = (size_t)n0 * n1;
+  const bool odd = st->iter & 1;
+  const float* po = odd ? p1 : p0;
+  float* pn = odd ? p0 : p1;
   Kahan32 acc;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int i0 = (tile % t0) * 32 + lane;
-    const int i1 = (tile / t0) * 8 + threadIdx.y;
-    const bool act = i0 < n0 && i1 < n1;
-    const int kb = blockIdx.y * planes, ke = min(n2, kb + planes);
-    size_t c = act ? (size_t)i0 + (size_t)n0 * i1 + s01 * kb : 0;
-    float pm = 0.0f, am = 0.0f;
-    if (act && kb > 0) {
-      pm = dir(c - s01);
-      am = a2[c - s01];
-    }
-    float pc = act ? dir(c) : 0.0f;
-    for (int k = kb; k < ke; ++k) {
-      const float pp = act && k + 1 < n2 ? dir(c + s01) : 0.0f;
-      const float ac = act ? a2[c] : 0.0f, ax = act ? a0[c] : 0.0f;
-      float pl = __shfl_up_sync(full, pc, 1), al = __shfl_up_sync(full, ax, 1);
-      float pr = __shfl_down_sync(full, pc, 1);
-      if (act) {
-        if (lane == 0 && i0 > 0) {
-          pl = dir(c - 1);
-          al = a0[c - 1];
-        }
-        if (lane == 31 && i0 + 1 < n0) pr = dir(c + 1);
-        float v = pc;
-        if (i0 > 0) v = fmaf(al, pl, v);
-        if (i0 + 1 < n0) v = fmaf(ax, pr, v);
-        if (i1 > 0) v = fmaf(a1[c - n0], dir(c - n0), v);
-        if (i1 + 1 < n1) v = fmaf(a1[c], dir(c + n0), v);
-        v = fmaf(am, pm, v);
-        v = fmaf(ac, pp, v);
-        pn[c] = pc;
-        w[c] = v;
-        acc.add(pc * v);
-      }
-      pm = pc;
-      pc = pp;
-      am = ac;
-      c += s01;
-    }
-  }
+  if (st->iter == 0)
+    dir_spmv_rows<true>(a0, a1, a2, z, po, pn, w, 0.0f, n0, n1, n2, planes, tiles, acc);
+  else
+    dir_spmv_rows<false>(a0, a1, a2, z, po, pn, w, (float)st->bcoef, n0, n1, n2, planes, tiles, acc);
   double loc[1] = {acc.value()};
   double tot[1];
   if (!grid_sum<1>(loc, partials, &st->arrive[1], tot)) return;
@@ -547,11 +587,13 @@ __global__ void __launch_bounds__(128) k32_dir_spmv_v4(
   if (flat_tid() == 0) spmv32_tail(st, tot[0]);
 }
 
-// launch geometry of k32_spmv_v4: (32 x 4) threads cover 128 x 4 cells of a plane
-static StencilLaunch launch_v4(int n0, int n1, int n2) {
+// launch geometry of k32_spmv_v4 and of the row form: (32 x 4) threads cover 128 x 4 cells of a
+// plane, or 32 x 16
+static StencilLaunch launch_v4(int n0, int n1, int n2, bool rows = false) {
   StencilLaunch L;
   L.block = dim3(32, 4, 1);
-  const long tiles = (long)((n0 + 127) / 128) * ((n1 + 3) / 4);
+  const long tiles = rows ? (long)((n0 + 31) / 32) * ((n1 + 4 * kDirRows - 1) / (4 * kDirRows))
+                          : (long)((n0 + 127) / 128) * ((n1 + 3) / 4);
   // one wave of eight 128-thread blocks per SM: each z chunk reads two more planes and each block
   // ends with a reduction on the FP64 pipe (line-PCG product at 256 x 256 x 128: 56 us, 65 with
   // four times the blocks; the same at 768 x 768 x 96)
@@ -1387,6 +1429,7 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
   const StencilLaunch L = stencil_launch(A.n0, A.n1, A.n2);
   const bool vec4 = (A.n0 % 4) == 0 && getenv("FREHG_NO_VEC4") == nullptr;
   const StencilLaunch L4 = launch_v4(A.n0, A.n1, A.n2);
+  const StencilLaunch LR = launch_v4(A.n0, A.n1, A.n2, true);
   FG_CUDA(cudaGetLastError());
   // inner preconditioner: Jacobi (unit diagonal, z = r) or vertical lines
   const bool line = !strcmp(cfg.pc_type, "line");
@@ -1425,9 +1468,9 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
                                                        A.n0, A.n1, A.n2, L4.planes, L4.tiles,
                                                        dst32, partials);
         else
-          k32_dir_spmv<<<L.grid, L.block, 0, s>>>(op32.a0, op32.a1, op32.a2, uf, pf, pf2, wf,
-                                                  A.n0, A.n1, A.n2, L.planes, L.tiles, dst32,
-                                                  partials);
+          k32_dir_spmv<<<LR.grid, LR.block, 0, s>>>(op32.a0, op32.a1, op32.a2, uf, pf, pf2, wf,
+                                                    A.n0, A.n1, A.n2, LR.planes, LR.tiles, dst32,
+                                                    partials);
       });
       FG_LAUNCH(pr, s, "k32_line_step", 36.0 * dn,
                 launch_line_step<false>(xf, rf, pf, pf2, wf, lkf, dinvf, uf, ncol, nzl, dst32,
