@@ -83,6 +83,27 @@ class Profiler {
     if (prof) (prof)->end(slot_, st, name, bytes);      \
   } while (0)
 
+// A launch whose blocks may be placed while the stream's previous kernel drains: the kernel calls
+// grid_begin() (reduce.cuh) before it touches memory, which waits for that kernel's end and lets the
+// next such launch be placed in turn.  The steps of small grids are chains of kernels of 5 to 15 us,
+// of which the launches took a tenth (Picard steps of 40 x 40 x 100 12.1 -> 10.6 ms).  Only for
+// kernels that begin so.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Upper bound of the blocks any reduction kernel launches (partials buffers are sized to it).
 constexpr int kMaxRedBlocks = 32768;
 // largest system the FP64 Jacobi-PCG runs as one launch per iteration by default: on GB300 the
@@ -306,6 +327,9 @@ int fetch_small(void* host_mapped, const void* dev, size_t bytes, cudaStream_t s
 // two of them by one launch, of the same size
 int fetch_small2(void* host_mapped, const void* dev, void* host_mapped2, const void* dev2,
                  size_t bytes, cudaStream_t st);
+// *a = va (and *b = vb) by one small launch: a copy from the host stalls the stream's kernels longer
+int set_states(CgDevState* a, const CgDevState& va, CgDevState* b, const CgDevState& vb,
+               cudaStream_t st);
 int alloc_mapped(void** host, size_t bytes);
 
 }  // namespace fg

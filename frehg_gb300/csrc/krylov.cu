@@ -75,6 +75,7 @@ StencilLaunch stencil_launch(int n0, int n1, int n2) {
 namespace {
 __global__ void k_fetch_words(const unsigned* __restrict__ src, unsigned* __restrict__ dst,
                               int words) {
+  grid_begin();
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
 }
 }  // namespace
@@ -87,8 +88,8 @@ int alloc_mapped(void** host, size_t bytes) {
 int fetch_small(void* host_mapped, const void* dev, size_t bytes, cudaStream_t st) {
   void* d = nullptr;
   FG_CUDA(cudaHostGetDevicePointer(&d, host_mapped, 0));
-  k_fetch_words<<<1, 32, 0, st>>>(static_cast<const unsigned*>(dev), static_cast<unsigned*>(d),
-                                  (int)(bytes / 4));
+  launch_chained(k_fetch_words, 1, 32, 0, st, static_cast<const unsigned*>(dev),
+                 static_cast<unsigned*>(d), (int)(bytes / 4));
   FG_CUDA(cudaGetLastError());
   return FREHG_OK;
 }
@@ -97,6 +98,7 @@ namespace {
 __global__ void k_fetch_words2(const unsigned* __restrict__ src, unsigned* __restrict__ dst,
                                const unsigned* __restrict__ src2, unsigned* __restrict__ dst2,
                                int words) {
+  grid_begin();
   for (int i = threadIdx.x; i < words; i += blockDim.x) {
     dst[i] = src[i];
     dst2[i] = src2[i];
@@ -109,10 +111,24 @@ int fetch_small2(void* host_mapped, const void* dev, void* host_mapped2, const v
   void *d = nullptr, *d2 = nullptr;
   FG_CUDA(cudaHostGetDevicePointer(&d, host_mapped, 0));
   FG_CUDA(cudaHostGetDevicePointer(&d2, host_mapped2, 0));
-  k_fetch_words2<<<1, 32, 0, st>>>(static_cast<const unsigned*>(dev), static_cast<unsigned*>(d),
-                                   static_cast<const unsigned*>(dev2), static_cast<unsigned*>(d2),
-                                   (int)(bytes / 4));
+  launch_chained(k_fetch_words2, 1, 32, 0, st, static_cast<const unsigned*>(dev),
+                 static_cast<unsigned*>(d), static_cast<const unsigned*>(dev2),
+                 static_cast<unsigned*>(d2), (int)(bytes / 4));
   FG_CUDA(cudaGetLastError());
+  return FREHG_OK;
+}
+
+namespace {
+__global__ void k_set_states(CgDevState* a, CgDevState va, CgDevState* b, CgDevState vb) {
+  grid_begin();
+  *a = va;
+  if (b) *b = vb;
+}
+}  // namespace
+
+int set_states(CgDevState* a, const CgDevState& va, CgDevState* b, const CgDevState& vb,
+               cudaStream_t st) {
+  FG_CUDA(launch_chained(k_set_states, 1, 1, 0, st, a, va, b, vb));
   return FREHG_OK;
 }
 
@@ -127,6 +143,7 @@ int reduction_blocks(size_t n, int threads, int per_thread) {
 // operator scaling
 
 __global__ void k_diag_rsqrt(double* __restrict__ s, size_t n) {
+  grid_begin();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
     double d = s[c];
@@ -138,6 +155,7 @@ __global__ void k_diag_rsqrt(double* __restrict__ s, size_t n) {
 __global__ void k_scale_offdiag(double* __restrict__ a0, double* __restrict__ a1,
                                 double* __restrict__ a2, const double* __restrict__ s, int n0,
                                 int n1, int n2, int planes, int tiles) {
+  grid_begin();
   const int t0 = (n0 + 31) / 32;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int i0 = (tile % t0) * 32 + threadIdx.x;
@@ -163,6 +181,7 @@ __global__ void k_scale_offdiag(double* __restrict__ a0, double* __restrict__ a1
 __global__ void k_cg_init(const double* __restrict__ s, const double* __restrict__ b,
                           double* __restrict__ x, double* __restrict__ r, size_t n,
                           CgDevState* st, double* partials) {
+  grid_begin();
   double v[2] = {0.0, 0.0};
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
@@ -815,6 +834,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
 
 __global__ void k_unscale(const double* __restrict__ s, const double* __restrict__ xs,
                           double* __restrict__ x, size_t n) {
+  grid_begin();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x)
     x[c] = s[c] * xs[c];
@@ -935,12 +955,13 @@ int KrylovSolver::scale(Stencil64& A, cudaStream_t st) {
   }
   const int nb = reduction_blocks(A.n, 256, 4);
   const double n = (double)A.n;
-  FG_LAUNCH(prof, st, "k_diag_rsqrt", 16.0 * n, k_diag_rsqrt<<<nb, 256, 0, st>>>(A.s, A.n));
+  FG_LAUNCH(prof, st, "k_diag_rsqrt", 16.0 * n, launch_chained(k_diag_rsqrt, nb, 256, 0, st, A.s,
+                                                               A.n));
   FG_CUDA(cudaGetLastError());
   const StencilLaunch L = stencil_launch(A.n0, A.n1, A.n2);
   FG_LAUNCH(prof, st, "k_scale_offdiag", 56.0 * n,
-            k_scale_offdiag<<<L.grid, L.block, 0, st>>>(A.a0, A.a1, A.a2, A.s, A.n0, A.n1, A.n2,
-                                                        L.planes, L.tiles));
+            launch_chained(k_scale_offdiag, L.grid, L.block, 0, st, A.a0, A.a1, A.a2, A.s, A.n0,
+                           A.n1, A.n2, L.planes, L.tiles));
   FG_CUDA(cudaGetLastError());
   A.scaled = true;
   return FREHG_OK;
@@ -1134,11 +1155,11 @@ int KrylovSolver::solve64(Stencil64& A, double* x_out, const frehg_solver_config
   init.atol = cfg.atol;
   init.divtol = 1.0e4;
   init.max_it = cfg.max_it;
-  FG_CUDA(cudaMemcpyAsync(dst, &init, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
+  FG_TRY(set_states(dst, init, nullptr, init, st));
   const int nb = reduction_blocks(n, 256, 4);
   const double dn = (double)n;
   FG_LAUNCH(prof, st, "k_cg_init", 32.0 * dn,
-            k_cg_init<<<nb, 256, 0, st>>>(A.s, A.b, x, r, n, dst, partials));
+            launch_chained(k_cg_init, nb, 256, 0, st, A.s, A.b, x, r, n, dst, partials));
   FG_CUDA(cudaGetLastError());
 
   // by default the whole loop in one launch, where the system fits (and no per-kernel times are
@@ -1245,7 +1266,7 @@ int KrylovSolver::solve64(Stencil64& A, double* x_out, const frehg_solver_config
 int KrylovSolver::finish64(Stencil64& A, double* x_out, cudaStream_t st, CgResult* res, int nb) {
   if (!keep_scaled) {
     FG_LAUNCH(prof, st, "k_unscale", 24.0 * (double)A.n,
-              k_unscale<<<nb, 256, 0, st>>>(scale_vector(A), x, x_out, A.n));
+              launch_chained(k_unscale, nb, 256, 0, st, scale_vector(A), x, x_out, A.n));
     FG_CUDA(cudaGetLastError());
   }
   res->its = hst->its;

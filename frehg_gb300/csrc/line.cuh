@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(32 * W, L > 8 ? 1 : 2) k32_line_step(
     const float* __restrict__ p1, const float* __restrict__ w, const float* __restrict__ lk,
     const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
     double* partials) {
+  grid_begin();
   if (st->status) return;
   __shared__ float2 fwd[W][32], bwd[W][32];
   __shared__ float lfirst[W + 1][32];
@@ -270,6 +271,7 @@ __global__ void __launch_bounds__(128) k32_line_step_long(
     const float* __restrict__ p1, const float* __restrict__ w, const float* __restrict__ lk,
     const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
     double* partials) {
+  grid_begin();
   if (st->status) return;
   const float a = FIRST ? 0.0f : (float)st->a;
   const float* p = (st->iter & 1) ? p0 : p1;
@@ -319,8 +321,8 @@ inline void launch_line_step(float* x, float* r, const float* p0, const float* p
   // pipe (about 3,000 clocks of it per block; one block per group took 0.5 ms instead of 0.2 on
   // 768 x 768 columns), and a third block per SM would wait for a second wave
 #define FG_LINE_STEP(W, LEV)                                                              \
-  k32_line_step<FIRST, W, LEV><<<std::min(groups, (LEV > 8 ? 1 : 2) * kNumSMs), 32 * W, 0, s>>>(x, r, p0, p1, w, lk, dinv, z, ncol, nz, \
-                                                         dst, partials)
+  launch_chained(k32_line_step<FIRST, W, LEV>, std::min(groups, (LEV > 8 ? 1 : 2) * kNumSMs), \
+                 32 * W, 0, s, x, r, p0, p1, w, lk, dinv, z, ncol, nz, dst, partials)
   if (nz <= 32) FG_LINE_STEP(16, 2);
   else if (nz <= 64) FG_LINE_STEP(16, 4);
   else if (nz <= 96) FG_LINE_STEP(16, 6);
@@ -328,8 +330,8 @@ inline void launch_line_step(float* x, float* r, const float* p0, const float* p
   else if (nz <= 256) FG_LINE_STEP(16, 16);
   else {
     const int lb = (ncol + 127) / 128;
-    k32_line_step_long<FIRST><<<lb < kMaxRedBlocks ? lb : kMaxRedBlocks, 128, 0, s>>>(
-        x, r, p0, p1, w, lk, dinv, z, ncol, nz, dst, partials);
+    launch_chained(k32_line_step_long<FIRST>, lb < kMaxRedBlocks ? lb : kMaxRedBlocks, 128, 0, s, x,
+                   r, p0, p1, w, lk, dinv, z, ncol, nz, dst, partials);
   }
 #undef FG_LINE_STEP
 }

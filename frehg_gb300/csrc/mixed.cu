@@ -491,6 +491,7 @@ __global__ void __launch_bounds__(128) k32_dir_spmv(
     const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
     float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
     double* partials) {
+  grid_begin();
   if (st->status) return;
   const bool odd = st->iter & 1;
   const float* po = odd ? p1 : p0;
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(128) k32_dir_spmv_v4(
     const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
     float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
     double* partials) {
+  grid_begin();
   if (st->status) return;
   const bool first = st->iter == 0, odd = st->iter & 1;
   const float bc = first ? 0.0f : (float)st->bcoef;
@@ -740,6 +742,7 @@ __global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e,
 // first sweep's x~ = 2^k e is exact and written by k_ir_sweep.
 __global__ void k_ir_update_exact(double* __restrict__ x, float* __restrict__ e, size_t n,
                                   const CgDevState* ir, const CgDevState* in) {
+  grid_begin();
   if (ir->status || in->status == 0 || ir->ir_its == 0 || in->iter == 0) return;
   const int scale = pow2_above(ir->rscale) - 1;  // rscale = 2^scale
   const float back = pow2f_of(-scale);
@@ -912,6 +915,7 @@ __global__ void __launch_bounds__(256, 4) k_ir_sweep(SweepArgs a, int n0, int n1
                                                      int planes, int tiles, CgDevState* ir,
                                                      CgDevState* in, double* partials,
                                                      double ir_rtol, double inner_rtol) {
+  grid_begin();
   if (ir->status || in->status == 0) return;
   const int scale = pow2_above(ir->rscale) - 1;  // rscale = 2^scale
   const int next = pow2_above(ir->a);            // the next inner system's
@@ -1200,6 +1204,7 @@ __global__ void __launch_bounds__(128) k_prep_ff(
     float* __restrict__ lk, float* __restrict__ dinv, int n0, int n1, int n2, int line,
     CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
     double inner_rtol) {
+  grid_begin();
   const int ncol = n0 * n1;
   const size_t sk = (size_t)ncol;
   const float sig = pow2f_of(-sig_exp);
@@ -1263,6 +1268,7 @@ __global__ void __launch_bounds__(32 * kPrepWarps) k_prep_ff_split(
     float* __restrict__ lk, float* __restrict__ dinv, int n0, int n1, int n2, int line,
     CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
     double inner_rtol) {
+  grid_begin();
   extern __shared__ float2 prep_sh[];  // [n2][32]
   const int ncol = n0 * n1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t sk = (size_t)ncol;
@@ -1347,8 +1353,7 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
       memset(&in0, 0, sizeof(in0));
       ir0.atol = cfg.atol;
       in0.max_it = cfg.max_it;
-      FG_CUDA(cudaMemcpyAsync(dst, &ir0, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
-      FG_CUDA(cudaMemcpyAsync(dst32, &in0, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
+      FG_TRY(set_states(dst, ir0, dst32, in0, st));
       // the first inner right-hand side's scale: 2^-e with 2^(e-1) <= the previous solve's
       // first residual norm < 2^e
       const int sig_exp = pow2_above(first_rnorm[rnorm_slot & 1]);
@@ -1365,14 +1370,14 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
                                      low32(A.a2), rf};
                   const float* dg = reinterpret_cast<const float*>(A.s);
                   if (split)
-                    k_prep_ff_split<<<std::min(groups, 6 * kNumSMs), 32 * kPrepWarps, split_sh,
-                                      st>>>(
-                        o, dg, A.b, lkf, dinvf, A.n0, A.n1, A.n2, line ? 1 : 0, dst, partials,
-                        cfg.ir_rtol, dst32, sig_exp, cfg.inner_rtol);
+                    launch_chained(k_prep_ff_split, std::min(groups, 6 * kNumSMs), 32 * kPrepWarps,
+                                   split_sh, st, o, dg, A.b, lkf, dinvf, A.n0, A.n1, A.n2,
+                                   line ? 1 : 0, dst, partials, cfg.ir_rtol, dst32, sig_exp,
+                                   cfg.inner_rtol);
                   else
-                    k_prep_ff<<<lb, 128, 0, st>>>(o, dg, A.b, lkf, dinvf, A.n0, A.n1, A.n2,
-                                                  line ? 1 : 0, dst, partials, cfg.ir_rtol,
-                                                  dst32, sig_exp, cfg.inner_rtol);
+                    launch_chained(k_prep_ff, lb, 128, 0, st, o, dg, A.b, lkf, dinvf, A.n0, A.n1,
+                                   A.n2, line ? 1 : 0, dst, partials, cfg.ir_rtol, dst32, sig_exp,
+                                   cfg.inner_rtol);
                 });
       FG_CUDA(cudaGetLastError());
       A.scaled = true;
@@ -1443,8 +1448,7 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
     memset(&in0, 0, sizeof(in0));
     ir0.atol = cfg.atol;
     in0.max_it = cfg.max_it;
-    FG_CUDA(cudaMemcpyAsync(dst, &ir0, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(dst32, &in0, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
+    FG_TRY(set_states(dst, ir0, dst32, in0, st));
   }
   // where the scale factors are: A.s, or r (as floats) after the float-float preparation
   const double* sv = A.s_in_r ? r : A.s;
@@ -1464,13 +1468,11 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
     if (line) {
       FG_LAUNCH(pr, s, dir_name, 28.0 * dn, {
         if (vec4)
-          k32_dir_spmv_v4<<<L4.grid, L4.block, 0, s>>>(op32.a0, op32.a1, op32.a2, uf, pf, pf2, wf,
-                                                       A.n0, A.n1, A.n2, L4.planes, L4.tiles,
-                                                       dst32, partials);
+          launch_chained(k32_dir_spmv_v4, L4.grid, L4.block, 0, s, op32.a0, op32.a1, op32.a2, uf,
+                         pf, pf2, wf, A.n0, A.n1, A.n2, L4.planes, L4.tiles, dst32, partials);
         else
-          k32_dir_spmv<<<LR.grid, LR.block, 0, s>>>(op32.a0, op32.a1, op32.a2, uf, pf, pf2, wf,
-                                                    A.n0, A.n1, A.n2, LR.planes, LR.tiles, dst32,
-                                                    partials);
+          launch_chained(k32_dir_spmv, LR.grid, LR.block, 0, s, op32.a0, op32.a1, op32.a2, uf, pf,
+                         pf2, wf, A.n0, A.n1, A.n2, LR.planes, LR.tiles, dst32, partials);
       });
       FG_LAUNCH(pr, s, "k32_line_step", 36.0 * dn,
                 launch_line_step<false>(xf, rf, pf, pf2, wf, lkf, dinvf, uf, ncol, nzl, dst32,
@@ -1546,11 +1548,10 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
                             reinterpret_cast<const float*>(A.s), xf, A.b, x,
                             reinterpret_cast<float2*>(rres), rf};
       FG_LAUNCH(prof, st, "k_ir_update", 24.0 * dn,
-                k_ir_update_exact<<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));
+                launch_chained(k_ir_update_exact, nb, 256, 0, st, x, xf, n, dst, dst32));
       FG_LAUNCH(prof, st, "k_ir_sweep", 56.0 * dn,
-                k_ir_sweep<<<L.grid, L.block, 0, st>>>(sa, A.n0, A.n1, A.n2, L.planes, L.tiles, dst,
-                                                       dst32, partials, cfg.ir_rtol,
-                                                       cfg.inner_rtol));
+                launch_chained(k_ir_sweep, L.grid, L.block, 0, st, sa, A.n0, A.n1, A.n2, L.planes,
+                               L.tiles, dst, dst32, partials, cfg.ir_rtol, cfg.inner_rtol));
     } else {
       FG_LAUNCH(prof, st, "k_ir_update", 20.0 * dn,
                 k_ir_update<<<nb, 256, 0, st>>>(x, xf, n, dst, dst32));

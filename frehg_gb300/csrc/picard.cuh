@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(256) k_pic_assemble(ReArgs a, double* __restri
                                                       double* __restrict__ a2,
                                                       double* __restrict__ bvec, int planes,
                                                       int tiles) {
+  grid_begin();
   const double dt = a.sc->dt_used;
   const double V = a.dx * a.dy * a.dz;
   const double Az = a.dx * a.dy;
@@ -284,6 +285,7 @@ __device__ __forceinline__ double pic_limited(double dc, long long lim_bits, lon
 template <bool SCALED = false>
 __global__ void k_pic_update(ReArgs a, const double* __restrict__ d,
                              const double* __restrict__ s = nullptr) {
+  grid_begin();
   const long long kAbs = 0x7fffffffffffffffll;
   long long m = 0;
   const double lim = a.picard_dh_max;
@@ -318,6 +320,7 @@ __global__ void k_pic_update(ReArgs a, const double* __restrict__ d,
 
 // conservative water-content update + boundary / elastic volumes + time
 __global__ void __launch_bounds__(256) k_pic_final(ReArgs a, int planes, int tiles) {
+  grid_begin();
   const double dt = a.sc->dt_used;
   const double V = a.dx * a.dy * a.dz;
   const double inv_V = 1.0 / V;

@@ -187,6 +187,7 @@ template <bool ALL_FF>
 __global__ void __launch_bounds__(256, 4) k_pic_update_constit_ff(
     ReArgs a, const double* __restrict__ d, const double* __restrict__ s,
     double* __restrict__ kr, double* __restrict__ th, double* __restrict__ cap) {
+  grid_begin();
   const long long kAbs = 0x7fffffffffffffffll;
   long long m = 0;
   const double lim = a.picard_dh_max;
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(256, 4) k_pic_assemble_ff(ReArgs a, T* __restr
                                                            T* __restrict__ a2,
                                                            double* __restrict__ bvec, int planes,
                                                            int tiles) {
+  grid_begin();
   __shared__ FfYPlane ys[2];
   // the launch's constants in shared memory rather than in 20 registers per thread
   __shared__ FfConst K;

@@ -594,19 +594,19 @@ static int pca_step(frehg_re* re) {
   const int nb = nblocks(re->n);
   Profiler* prof = &re->prof;
   const double n = (double)re->n, sb = soil_bytes(re);
-  FG_LAUNCH(prof, st, "k_step_begin", 0.0, k_step_begin<<<1, 1, 0, st>>>(re->sc));
+  FG_LAUNCH(prof, st, "k_step_begin", 0.0, launch_chained(k_step_begin, 1, 1, 0, st, re->sc));
   // computeKFace inputs at h^n
   FG_LAUNCH(prof, st, "k_kr", (24.0 + sb) * n,
-            (k_constit<false, true><<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(
-                a, a.h_old, re->kr, nullptr, re->cap)));
+            (launch_chained(k_constit<false, true>, spread_blocks(re->n), kSpreadThreads, 0, st, a,
+                            a.h_old, re->kr, nullptr, re->cap)));
   // groundwaterMatCoeff + groundwaterRhs + assembly
   const StencilLaunch L = stencil_launch(re->nx, re->ny, re->nz);
   re->A.scaled = false;
   re->A.s_in_r = false;
   re->A.f32_entries = false;
   FG_LAUNCH(prof, st, "k_assemble", (72.0 + sb) * n,
-            k_assemble<<<L.grid, L.block, 0, st>>>(a, re->A.s, re->A.a0, re->A.a1, re->A.a2,
-                                                   re->A.b, L.planes, L.tiles));
+            launch_chained(k_assemble, L.grid, L.block, 0, st, a,
+                           re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, L.planes, L.tiles));
   FG_CUDA(cudaGetLastError());
   // LinearSolver::solve
   CgResult res;
@@ -618,11 +618,11 @@ static int pca_step(frehg_re* re) {
   if (rc != FREHG_OK) return rc;
   // enforceHeadBc + computeKFace + updateDiagnostics at h^{n+1} (the solve wrote h^{n+1})
   FG_LAUNCH(prof, st, "k_post", (24.0 + sb) * n,
-            k_post<<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(a));
+            launch_chained(k_post, spread_blocks(re->n), kSpreadThreads, 0, st, a));
   FG_CUDA(cudaGetLastError());
   // groundwaterFlux + updateWaterContent (+ dq of adaptiveTimeStep, boundary budgets)
   FG_LAUNCH(prof, st, "k_correct", (73.0 + sb) * n,
-            k_correct<<<L.grid, L.block, 0, st>>>(a, L.planes, L.tiles));
+            launch_chained(k_correct, L.grid, L.block, 0, st, a, L.planes, L.tiles));
   FG_CUDA(cudaGetLastError());
   // reallocateWaterContent: relax to the sequential sweep's fixed point
   const int top_sat = (re->p.bc_type[5] == 1 && re->p.htop >= 0.0) ? 1 : 0;
@@ -632,7 +632,7 @@ static int pca_step(frehg_re* re) {
   for (;;) {
     FG_CUDA(cudaMemsetAsync(&re->sc->changed, 0, sizeof(int), st));
     FG_LAUNCH(prof, st, "k_realloc_sweep", 2.0 * n,
-              k_realloc_sweep<<<cb, 128, 0, st>>>(a, top_sat));
+              launch_chained(k_realloc_sweep, cb, 128, 0, st, a, top_sat));
     FG_CUDA(cudaGetLastError());
     ++sweeps;
     int changed = 0;
@@ -649,7 +649,7 @@ static int pca_step(frehg_re* re) {
   re->cnt.realloc_sweeps += sweeps;
   // apply reallocation, clampWaterContent, adaptiveTimeStep
   FG_LAUNCH(prof, st, "k_finalize", (25.0 + sb) * n,
-            k_finalize<<<L.grid, L.block, 0, st>>>(a, top_sat, L.planes, L.tiles));
+            launch_chained(k_finalize, L.grid, L.block, 0, st, a, top_sat, L.planes, L.tiles));
   FG_CUDA(cudaGetLastError());
   if (prof->on) {
     FG_CUDA(cudaStreamSynchronize(st));
@@ -778,7 +778,7 @@ static int picard_step(frehg_re* re) {
   bool last_fused = false;
   for (;;) {
     FG_CUDA(cudaMemcpyAsync(&re->sc->dt, &dt, sizeof(double), cudaMemcpyHostToDevice, st));
-    FG_LAUNCH(prof, st, "k_step_begin", 0.0, k_step_begin<<<1, 1, 0, st>>>(re->sc));
+    FG_LAUNCH(prof, st, "k_step_begin", 0.0, launch_chained(k_step_begin, 1, 1, 0, st, re->sc));
     FG_LAUNCH(prof, st, "k_copy64", 16.0 * n,
               k_copy64<<<nb, 256, 0, st>>>(a.h_new, a.h_old, re->n));
     bool converged = false;
@@ -791,25 +791,26 @@ static int picard_step(frehg_re* re) {
     for (its = 0; its < re->p.picard_max_it; ++its) {
       if (!picard_ff(re))
         FG_LAUNCH(prof, st, "k_kr", (32.0 + sb) * n,
-                  (k_constit<true, true><<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(
-                      a, a.h_new, re->kr, re->wch, re->cap)));
+                  (launch_chained(k_constit<true, true>,
+                                  spread_blocks(re->n), kSpreadThreads, 0, st, a, a.h_new,
+                                  re->kr, re->wch, re->cap)));
       else if (constit_ready) {
       } else if (all_ff)
         FG_LAUNCH(prof, st, "k_kr_ff", (32.0 + sb) * n,
-                  (k_constit_ff<true, true, true><<<nb, 256, 0, st>>>(a, a.h_new, re->kr,
-                                                                      re->wch, re->cap)));
+                  (launch_chained(k_constit_ff<true, true, true>, nb, 256, 0, st, a, a.h_new,
+                                  re->kr, re->wch, re->cap)));
       else
         FG_LAUNCH(prof, st, "k_kr_ff", (32.0 + sb) * n,
-                  (k_constit_ff<true, true, false><<<nb, 256, 0, st>>>(a, a.h_new, re->kr,
-                                                                       re->wch, re->cap)));
+                  (launch_chained(k_constit_ff<true, true, false>, nb, 256, 0, st, a, a.h_new,
+                                  re->kr, re->wch, re->cap)));
       re->A.scaled = false;
       re->A.s_in_r = false;
       re->A.f32_entries = f32;
       if (!picard_ff(re))
         FG_LAUNCH(prof, st, "k_pic_assemble", (88.0 + sb) * n,
-                  k_pic_assemble<<<PL.grid, PL.block, 0, st>>>(a, re->A.s, re->A.a0, re->A.a1,
-                                                               re->A.a2, re->A.b, PL.planes,
-                                                               PL.tiles));
+                  launch_chained(k_pic_assemble, PL.grid, PL.block, 0, st, a,
+                                 re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, PL.planes,
+                                 PL.tiles));
       else if (f32) {
         // diagonal and couplings as floats (the float-float preparation's input)
         float* dgf = reinterpret_cast<float*>(re->A.s);
@@ -819,20 +820,22 @@ static int picard_step(frehg_re* re) {
         if (staged) {
         } else if (iso)
           FG_LAUNCH(prof, st, "k_pic_assemble_ff", (72.0 + sb) * n,
-                    (k_pic_assemble_ff<true, false, float><<<PL.grid, PL.block, 0, st>>>(
-                        a, dgf, o.a0, o.a1, o.a2, re->A.b, PL.planes, PL.tiles)));
+                    (launch_chained(k_pic_assemble_ff<true, false, float>, PL.grid, PL.block, 0, st,
+                                    a, dgf, o.a0, o.a1, o.a2, re->A.b, PL.planes, PL.tiles)));
         else
           FG_LAUNCH(prof, st, "k_pic_assemble_ff", (72.0 + sb) * n,
-                    (k_pic_assemble_ff<false, false, float><<<PL.grid, PL.block, 0, st>>>(
-                        a, dgf, o.a0, o.a1, o.a2, re->A.b, PL.planes, PL.tiles)));
+                    (launch_chained(k_pic_assemble_ff<false, false, float>, PL.grid, PL.block, 0,
+                                    st, a, dgf, o.a0, o.a1, o.a2, re->A.b, PL.planes, PL.tiles)));
       } else if (iso)
         FG_LAUNCH(prof, st, "k_pic_assemble_ff", (88.0 + sb) * n,
-                  k_pic_assemble_ff<true><<<PL.grid, PL.block, 0, st>>>(
-                      a, re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, PL.planes, PL.tiles));
+                  launch_chained(k_pic_assemble_ff<true>, PL.grid, PL.block, 0, st, a,
+                                 re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, PL.planes,
+                                 PL.tiles));
       else
         FG_LAUNCH(prof, st, "k_pic_assemble_ff", (88.0 + sb) * n,
-                  k_pic_assemble_ff<false><<<PL.grid, PL.block, 0, st>>>(
-                      a, re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, PL.planes, PL.tiles));
+                  launch_chained(k_pic_assemble_ff<false>, PL.grid, PL.block, 0, st, a,
+                                 re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, PL.planes,
+                                 PL.tiles));
       FG_CUDA(cudaGetLastError());
       CgResult res;
       // the update below applies x = s x~ (PCSOR solves the unscaled system into scratch)
@@ -862,19 +865,21 @@ static int picard_step(frehg_re* re) {
       }
       if (sor)
         FG_LAUNCH(prof, st, "k_pic_update", 24.0 * n,
-                  k_pic_update<false><<<nb, 256, 0, st>>>(a, re->scratch));
+                  launch_chained(k_pic_update<false>, nb, 256, 0, st, a, re->scratch, nullptr));
       else if (fused_update && all_ff)
         FG_LAUNCH(prof, st, "k_pic_update_kr_ff", (56.0 + sb) * n,
-                  k_pic_update_constit_ff<true><<<nb, 256, 0, st>>>(
-                      a, re->ksp.x, re->ksp.scale_vector(re->A), re->kr2, re->wch2, re->cap2));
+                  launch_chained(k_pic_update_constit_ff<true>, nb, 256, 0, st, a,
+                                 re->ksp.x, re->ksp.scale_vector(re->A), re->kr2, re->wch2,
+                                 re->cap2));
       else if (fused_update)
         FG_LAUNCH(prof, st, "k_pic_update_kr_ff", (56.0 + sb) * n,
-                  k_pic_update_constit_ff<false><<<nb, 256, 0, st>>>(
-                      a, re->ksp.x, re->ksp.scale_vector(re->A), re->kr2, re->wch2, re->cap2));
+                  launch_chained(k_pic_update_constit_ff<false>, nb, 256, 0, st, a,
+                                 re->ksp.x, re->ksp.scale_vector(re->A), re->kr2, re->wch2,
+                                 re->cap2));
       else
         FG_LAUNCH(prof, st, "k_pic_update", 32.0 * n,
-                  k_pic_update<true><<<nb, 256, 0, st>>>(a, re->ksp.x,
-                                                         re->ksp.scale_vector(re->A)));
+                  launch_chained(k_pic_update<true>, nb, 256, 0, st, a,
+                                 re->ksp.x, re->ksp.scale_vector(re->A)));
       FG_CUDA(cudaGetLastError());
       FG_TRY(fetch_small(re->sc_host, re->sc, sizeof(ReScalars), st));
       FG_CUDA(cudaStreamSynchronize(st));
@@ -917,15 +922,15 @@ static int picard_step(frehg_re* re) {
   }
   if (!picard_ff(re))
     FG_LAUNCH(prof, st, "k_pic_final", (40.0 + sb) * n,
-              k_pic_final<<<PL.grid, PL.block, 0, st>>>(a, PL.planes, PL.tiles));
+              launch_chained(k_pic_final, PL.grid, PL.block, 0, st, a, PL.planes, PL.tiles));
   else if (iso)
     FG_LAUNCH(prof, st, "k_pic_final_ff", (40.0 + sb) * n,
-              (k_pic_assemble_ff<true, true, double><<<PL.grid, PL.block, 0, st>>>(
-                  a, nullptr, nullptr, nullptr, nullptr, nullptr, PL.planes, PL.tiles)));
+              (launch_chained(k_pic_assemble_ff<true, true, double>, PL.grid, PL.block, 0, st, a,
+                              nullptr, nullptr, nullptr, nullptr, nullptr, PL.planes, PL.tiles)));
   else
     FG_LAUNCH(prof, st, "k_pic_final_ff", (40.0 + sb) * n,
-              (k_pic_assemble_ff<false, true, double><<<PL.grid, PL.block, 0, st>>>(
-                  a, nullptr, nullptr, nullptr, nullptr, nullptr, PL.planes, PL.tiles)));
+              (launch_chained(k_pic_assemble_ff<false, true, double>, PL.grid, PL.block, 0, st, a,
+                              nullptr, nullptr, nullptr, nullptr, nullptr, PL.planes, PL.tiles)));
   FG_CUDA(cudaGetLastError());
   if (last_fused) {
     // the last update formed the values at the step's final head (the final update above,
@@ -1661,8 +1666,8 @@ int frehg_re_check_staged_assembly(frehg_re* re, int64_t* mismatches) {
       rc = FREHG_ERR_UNSUPPORTED;
     }
     if (rc == FREHG_OK) {
-      k_pic_assemble_ff<true, false, float><<<PL.grid, PL.block, 0, st>>>(
-          a, f[1][0], f[1][1], f[1][2], f[1][3], b[1], PL.planes, PL.tiles);
+      launch_chained(k_pic_assemble_ff<true, false, float>, PL.grid, PL.block, 0, st, a, f[1][0],
+                     f[1][1], f[1][2], f[1][3], b[1], PL.planes, PL.tiles);
       if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
         set_error("assembly self-check launch failed");
         rc = FREHG_ERR_CUDA;
@@ -1784,15 +1789,15 @@ int frehg_re_training_pairs(frehg_re* re, int npairs, const int* iters, int targ
   const int nb = nblocks(re->n);
   const size_t n = re->n;
   // the next step's system at the current state (nothing advances)
-  k_step_begin<<<1, 1, 0, st>>>(re->sc);
-  k_constit<false, true><<<spread_blocks(re->n), kSpreadThreads, 0, st>>>(a, a.h_old, re->kr,
-                                                                          nullptr, re->cap);
+  launch_chained(k_step_begin, 1, 1, 0, st, re->sc);
+  launch_chained(k_constit<false, true>, spread_blocks(re->n), kSpreadThreads, 0, st, a, a.h_old,
+                 re->kr, nullptr, re->cap);
   const StencilLaunch L = stencil_launch(re->nx, re->ny, re->nz);
   re->A.scaled = false;
   re->A.s_in_r = false;
   re->A.f32_entries = false;
-  k_assemble<<<L.grid, L.block, 0, st>>>(a, re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b,
-                                         L.planes, L.tiles);
+  launch_chained(k_assemble, L.grid, L.block, 0, st, a,
+                 re->A.s, re->A.a0, re->A.a1, re->A.a2, re->A.b, L.planes, L.tiles);
   k_net_fields<<<nb, 256, 0, st>>>(a, lnk_out, cap_out);
   FG_CUDA(cudaGetLastError());
   // x~* of the scaled system, FP64 Jacobi-PCG to the handle's rtol

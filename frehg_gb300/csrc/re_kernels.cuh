@@ -145,12 +145,16 @@ __device__ __forceinline__ bool cell_sat(const ReArgs& a, size_t c, size_t col, 
 // ---- kernels ---------------------------------------------------------------------------------
 
 // savePreviousStepFields' scalar part: the dt this step applies (ReSolver.cpp:932)
-__global__ void k_step_begin(ReScalars* sc) { sc->dt_used = sc->dt; }
+__global__ void k_step_begin(ReScalars* sc) {
+  grid_begin();
+  sc->dt_used = sc->dt;
+}
 
 // kr (and optionally theta and C) at the given head, from one set of transcendentals
 template <bool THETA, bool CAP>
 __global__ void k_constit(ReArgs a, const double* __restrict__ h, double* __restrict__ kr,
                           double* __restrict__ th, double* __restrict__ cap) {
+  grid_begin();
   // the column index is only needed for a per-column class map; 32-bit when it fits
   const bool col_map = a.soil.cid && !a.soil.cid3d;
   const bool small = a.n <= 0xffffffffull;
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(256, 4) k_constit_ff(ReArgs a, const double* _
                                                        double* __restrict__ kr,
                                                        double* __restrict__ th,
                                                        double* __restrict__ cap) {
+  grid_begin();
   const bool col_map = a.soil.cid && !a.soil.cid3d;
   const bool small = a.n <= 0xffffffffull;
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < a.n;
@@ -206,6 +211,7 @@ __global__ void __launch_bounds__(256) k_assemble(ReArgs a, double* __restrict__
                                                   double* __restrict__ a2,
                                                   double* __restrict__ bvec, int planes,
                                                   int tiles) {
+  grid_begin();
   const int t0 = (a.nx + 31) / 32;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
   const int i = (tile % t0) * 32 + threadIdx.x;
@@ -330,6 +336,7 @@ __global__ void __launch_bounds__(256) k_assemble(ReArgs a, double* __restrict__
 
 // kr(h^{n+1}) and theta(h^{n+1}) once the solve has written h^{n+1} (re_solve_unpack).
 __global__ void k_post(ReArgs a) {
+  grid_begin();
   const bool col_map = a.soil.cid && !a.soil.cid3d;
   const bool small = a.n <= 0xffffffffull;
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < a.n;
@@ -354,6 +361,7 @@ __device__ __forceinline__ double flux_z_inner(const ReArgs& a, double Kc, doubl
 
 // groundwaterFlux + updateWaterContent + adaptiveTimeStep's dq (ReSolver.cpp:671-786, 891-905)
 __global__ void __launch_bounds__(256) k_correct(ReArgs a, int planes, int tiles) {
+  grid_begin();
   const double dtg = a.sc->dt_used;
   const double dtq = a.sc->dtn;  // adaptiveTimeStep resets params_.dt = dtn_ before dq
   const int t0 = (a.nx + 31) / 32;
@@ -511,6 +519,7 @@ __device__ __forceinline__ bool ghost_sat(const ReArgs& a, size_t c, size_t col)
 // the least fixed point is the sequential result; one thread walks a column (k order) and
 // re-reads lateral predecessors, so each sweep extends every chain by at least one lateral hop.
 __global__ void k_realloc_sweep(ReArgs a, int top_sat) {
+  grid_begin();
   const size_t col = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (col >= a.ncol) return;
   const int i = (int)(col % a.nx), j = (int)(col / a.nx);
@@ -555,6 +564,7 @@ __global__ void k_realloc_sweep(ReArgs a, int top_sat) {
 // adaptiveTimeStep Courant bound (:906-910); the last block updates dt (:921-928) and time.
 // Launched on (32 x 8)-column tiles marching through `planes` levels (no index divisions).
 __global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int planes, int tiles) {
+  grid_begin();
   double dtco = INFINITY;
   const int t0 = (a.nx + 31) / 32;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {

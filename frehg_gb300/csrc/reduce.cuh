@@ -32,6 +32,13 @@ __device__ __forceinline__ int flat_nthreads() { return blockDim.x * blockDim.y;
 __device__ __forceinline__ int flat_bid() { return blockIdx.x + blockIdx.y * gridDim.x; }
 __device__ __forceinline__ int flat_nblocks() { return gridDim.x * gridDim.y; }
 
+// The first statement of a kernel that launch_chained() starts: the next launch may be placed, and
+// everything the stream did before is complete and visible.
+__device__ __forceinline__ void grid_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Sum NV values over the block; the result is valid in every thread.  Uses sh[NV * CAP]; a
 // __syncthreads has to come between this and the next use of sh.
 // The threads' values (folded by shuffles to CAP at most) go through shared memory to one warp

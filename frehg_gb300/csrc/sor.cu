@@ -392,6 +392,7 @@ __device__ __forceinline__ double sor_wait_value() {
 __global__ void k_sor_prep(const double* __restrict__ d, const double* __restrict__ b,
                            double* __restrict__ invd, double* __restrict__ x,
                            double* __restrict__ r, double* __restrict__ z, size_t n) {
+  grid_begin();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
     const double dc = d[c];
@@ -407,6 +408,7 @@ __global__ void k_sor_prep(const double* __restrict__ d, const double* __restric
 __global__ void k_sor_slots(SorGeom g, SorSlots S, const double* __restrict__ a0,
                             const double* __restrict__ a1, const double* __restrict__ a2,
                             const double* __restrict__ invd, size_t slots) {
+  grid_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < slots;
        e += (size_t)gridDim.x * blockDim.x) {
     const int lane = (int)(e & 31);
@@ -584,6 +586,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     const double* __restrict__ a1, const double* __restrict__ a2, const double* __restrict__ b,
     double* __restrict__ x, double* __restrict__ x_out, int n0, int n1, int n2, double rtol,
     double atol, double divtol, int max_it, CgDevState* dst) {
+  grid_begin();
   extern __shared__ double sor_sh[];
   __shared__ CgDevState st;
   __shared__ double red[128];  // (the vectors of 3,600 cells leave 2 KB)
@@ -769,9 +772,9 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  8 * kSorSolveCells * (int)sizeof(double)));
     FG_LAUNCH(prof, st, "k_sor_solve", 48.0 * dn,
-              kernel<<<1, kSorSolveThreads, smem, st>>>(
-                  g, A.s, A.a0, A.a1, A.a2, A.b, x, x_out ? x_out : x, A.n0, A.n1, A.n2, cfg.rtol,
-                  cfg.atol, 1.0e4, cfg.max_it, dst));
+              launch_chained(kernel, 1, kSorSolveThreads, smem, st, g, A.s, A.a0, A.a1, A.a2, A.b, x,
+                             x_out ? x_out : x, A.n0, A.n1, A.n2, cfg.rtol, cfg.atol, 1.0e4,
+                             cfg.max_it, dst));
     FG_CUDA(cudaGetLastError());
     FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
     FG_CUDA(cudaStreamSynchronize(st));
@@ -796,7 +799,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   init.atol = cfg.atol;
   init.divtol = 1.0e4;
   init.max_it = cfg.max_it;
-  FG_CUDA(cudaMemcpyAsync(dst, &init, sizeof(CgDevState), cudaMemcpyHostToDevice, st));
+  FG_TRY(set_states(dst, init, nullptr, init, st));
   const int nb = reduction_blocks(n, 256, 4);
   double* xs = x;  // the graph keeps fixed pointers; x_out receives a copy
   auto sweeps = [&](cudaStream_t s) -> cudaError_t {
@@ -812,11 +815,11 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     return cudaLaunchKernelEx(&lc, kernel, g, S, (const double*)r, zs, dst);
   };
   FG_LAUNCH(prof, st, "k_sor_prep", 48.0 * dn,
-            k_sor_prep<<<nb, 256, 0, st>>>(A.s, A.b, invd, xs, r, zs, n));
+            launch_chained(k_sor_prep, nb, 256, 0, st, A.s, A.b, invd, xs, r, zs, n));
   const double* ax[3] = {A.a0, A.a1, A.a2};
   FG_LAUNCH(prof, st, "k_sor_slots", 32.0 * dn + 64.0 * (double)slots,
-            k_sor_slots<<<reduction_blocks(slots, 256, 1), 256, 0, st>>>(
-                g, S, ax[g.ax[0]], ax[g.ax[1]], ax[g.ax[2]], invd, slots));
+            launch_chained(k_sor_slots, reduction_blocks(slots, 256, 1), 256, 0, st, g, S,
+                           ax[g.ax[0]], ax[g.ax[1]], ax[g.ax[2]], invd, slots));
   cudaError_t le = cudaSuccess;
   FG_LAUNCH(prof, st, "k_sor_sweeps", 16.0 * dn + 72.0 * (double)slots, le = sweeps(st));
   if (le != cudaSuccess && sweep_blocks > 1) {
