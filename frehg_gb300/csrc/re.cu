@@ -594,11 +594,10 @@ static int pca_step(frehg_re* re) {
   const int nb = nblocks(re->n);
   Profiler* prof = &re->prof;
   const double n = (double)re->n, sb = soil_bytes(re);
-  FG_LAUNCH(prof, st, "k_step_begin", 0.0, launch_chained(k_step_begin, 1, 1, 0, st, re->sc));
   // computeKFace inputs at h^n
   FG_LAUNCH(prof, st, "k_kr", (24.0 + sb) * n,
             (launch_chained(k_constit<false, true>, spread_blocks(re->n), kSpreadThreads, 0, st, a,
-                            a.h_old, re->kr, nullptr, re->cap)));
+                            a.h_old, re->kr, nullptr, re->cap, re->sc)));
   // groundwaterMatCoeff + groundwaterRhs + assembly
   const StencilLaunch L = stencil_launch(re->nx, re->ny, re->nz);
   re->A.scaled = false;
@@ -629,7 +628,16 @@ static int pca_step(frehg_re* re) {
   const int cb = (int)((re->ncol + 127) / 128);
   const int max_sweeps = (int)re->n + 2;
   int sweeps = 0;
-  for (;;) {
+  if (re->ncol <= kReallocCols && re->n <= kReallocCells) {
+    const size_t flags = (re->n + 15) & ~(size_t)15;
+    // on every step: the attribute belongs to the current device, and the call is cheap
+    if (flags > 40 * 1024)
+      FG_CUDA(cudaFuncSetAttribute(k_realloc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kReallocCells));
+    FG_LAUNCH(prof, st, "k_realloc", 2.0 * n,
+              launch_chained(k_realloc, 1, kReallocThreads, flags, st, a, top_sat));
+    FG_CUDA(cudaGetLastError());
+  } else for (;;) {
     FG_CUDA(cudaMemsetAsync(&re->sc->changed, 0, sizeof(int), st));
     FG_LAUNCH(prof, st, "k_realloc_sweep", 2.0 * n,
               launch_chained(k_realloc_sweep, cb, 128, 0, st, a, top_sat));
@@ -793,7 +801,7 @@ static int picard_step(frehg_re* re) {
         FG_LAUNCH(prof, st, "k_kr", (32.0 + sb) * n,
                   (launch_chained(k_constit<true, true>,
                                   spread_blocks(re->n), kSpreadThreads, 0, st, a, a.h_new,
-                                  re->kr, re->wch, re->cap)));
+                                  re->kr, re->wch, re->cap, nullptr)));
       else if (constit_ready) {
       } else if (all_ff)
         FG_LAUNCH(prof, st, "k_kr_ff", (32.0 + sb) * n,
@@ -1717,6 +1725,7 @@ int frehg_re_get_counters(const frehg_re* re, frehg_re_counters* c) {
   c->kernel_launches = re->prof.launches;
   FG_TRY(read_scalars(re));
   c->elastic_volume = re->sc_host->vol_elastic;
+  c->realloc_sweeps += (int64_t)re->sc_host->sweeps;
   return FREHG_OK;
 }
 
@@ -1791,7 +1800,7 @@ int frehg_re_training_pairs(frehg_re* re, int npairs, const int* iters, int targ
   // the next step's system at the current state (nothing advances)
   launch_chained(k_step_begin, 1, 1, 0, st, re->sc);
   launch_chained(k_constit<false, true>, spread_blocks(re->n), kSpreadThreads, 0, st, a, a.h_old,
-                 re->kr, nullptr, re->cap);
+                 re->kr, nullptr, re->cap, nullptr);
   const StencilLaunch L = stencil_launch(re->nx, re->ny, re->nz);
   re->A.scaled = false;
   re->A.s_in_r = false;

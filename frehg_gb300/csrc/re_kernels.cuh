@@ -47,6 +47,7 @@ struct ReScalars {
   double vol_bot;   // cumulative bottom-face inflow volume
   double vol_elastic;
   int changed;      // reallocation sweep changed a flag
+  unsigned long long sweeps;  // sweeps that k_realloc did (host counters read it)
   int stage_err;    // staged (TMA) assembly: nonzero when one of its bounded waits ran out
   unsigned int arrive[8];
 };
@@ -144,7 +145,8 @@ __device__ __forceinline__ bool cell_sat(const ReArgs& a, size_t c, size_t col, 
 
 // ---- kernels ---------------------------------------------------------------------------------
 
-// savePreviousStepFields' scalar part: the dt this step applies (ReSolver.cpp:932)
+// savePreviousStepFields' scalar part: the dt this step applies (ReSolver.cpp:932); a PCA step's first
+// k_constit does it
 __global__ void k_step_begin(ReScalars* sc) {
   grid_begin();
   sc->dt_used = sc->dt;
@@ -153,8 +155,10 @@ __global__ void k_step_begin(ReScalars* sc) {
 // kr (and optionally theta and C) at the given head, from one set of transcendentals
 template <bool THETA, bool CAP>
 __global__ void k_constit(ReArgs a, const double* __restrict__ h, double* __restrict__ kr,
-                          double* __restrict__ th, double* __restrict__ cap) {
+                          double* __restrict__ th, double* __restrict__ cap,
+                          ReScalars* begin = nullptr) {
   grid_begin();
+  if (begin && blockIdx.x == 0 && threadIdx.x == 0) begin->dt_used = begin->dt;
   // the column index is only needed for a per-column class map; 32-bit when it fits
   const bool col_map = a.soil.cid && !a.soil.cid3d;
   const bool small = a.n <= 0xffffffffull;
@@ -518,46 +522,92 @@ __device__ __forceinline__ bool ghost_sat(const ReArgs& a, size_t c, size_t col)
 // faces), succ = sat_old of the unvisited ones (k+1 or the bottom ghost, i+1, j+1).  On this DAG
 // the least fixed point is the sequential result; one thread walks a column (k order) and
 // re-reads lateral predecessors, so each sweep extends every chain by at least one lateral hop.
-__global__ void k_realloc_sweep(ReArgs a, int top_sat) {
-  grid_begin();
-  const size_t col = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (col >= a.ncol) return;
+// flags: a.flags or a copy of it, where the sweeps read (set flags go to both).  The own column's
+// flags, which only its thread changes, are read 16 levels at a time, and only the levels that may
+// become saturated are looked at in turn: a load per level took 28 us for 100 levels, now 9.
+constexpr int kReallocLevels = 16;
+__device__ __forceinline__ int realloc_column(const ReArgs& a, uint8_t* flags, size_t col,
+                                              int top_sat) {
   const int i = (int)(col % a.nx), j = (int)(col / a.nx);
   bool prev = top_sat != 0;  // top rule for k = 0
   int changed = 0;
-  for (int k = 0; k < a.nz; ++k) {
-    const size_t c = col + a.ncol * k;
-    const uint8_t f = a.flags[c];
-    bool sat = (f & (F_SAT_OLD | F_SAT_NEW)) != 0;
-    if (!sat && (f & F_WCH_SAT)) {
-      bool adj = prev;
+  for (int k0 = 0; k0 < a.nz; k0 += kReallocLevels) {
+    // of the group's levels: saturated ones, and those that may become so
+    unsigned sat = 0, may = 0;
+    uint8_t own[kReallocLevels];
+#pragma unroll
+    for (int u = 0; u < kReallocLevels; ++u)
+      own[u] = k0 + u < a.nz ? flags[col + a.ncol * (k0 + u)] : 0;
+#pragma unroll
+    for (int u = 0; u < kReallocLevels; ++u) {
+      if (own[u] & (F_SAT_OLD | F_SAT_NEW)) sat |= 1u << u;
+      else if (own[u] & F_WCH_SAT) may |= 1u << u;
+    }
+    for (; may; may &= may - 1) {
+      const int u = __ffs(may) - 1, k = k0 + u;
+      const size_t c = col + a.ncol * k;
+      const uint8_t f = flags[c];
+      bool adj = u ? (sat >> (u - 1)) & 1u : prev;
       if (i > 0) {
-        const uint8_t g = ((volatile uint8_t*)a.flags)[c - 1];
+        const uint8_t g = ((volatile uint8_t*)flags)[c - 1];
         adj |= (g & F_OPEN_XP) && (g & F_SAT_NEW);
       }
       if (j > 0) {
-        const uint8_t g = ((volatile uint8_t*)a.flags)[c - a.nx];
+        const uint8_t g = ((volatile uint8_t*)flags)[c - a.nx];
         adj |= (g & F_OPEN_YP) && (g & F_SAT_NEW);
       }
       if (!adj) {
         if (k + 1 < a.nz)
-          adj = (a.flags[c + a.ncol] & F_SAT_OLD) != 0;
+          adj = (flags[c + a.ncol] & F_SAT_OLD) != 0;
         else
           adj = ghost_sat(a, c, col);
       }
       if (!adj && (f & F_OPEN_XP))
-        adj = (i + 1 < a.nx) ? (a.flags[c + 1] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
+        adj = (i + 1 < a.nx) ? (flags[c + 1] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
       if (!adj && (f & F_OPEN_YP))
-        adj = (j + 1 < a.ny) ? (a.flags[c + a.nx] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
+        adj = (j + 1 < a.ny) ? (flags[c + a.nx] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
       if (adj) {
-        sat = true;
-        a.flags[c] = f | F_SAT_NEW;
+        sat |= 1u << u;
+        flags[c] = f | F_SAT_NEW;
+        if (flags != a.flags) a.flags[c] = f | F_SAT_NEW;
         changed = 1;
       }
     }
-    prev = sat;
+    prev = (sat >> (kReallocLevels - 1)) & 1u;
   }
-  if (changed) a.sc->changed = 1;
+  return changed;
+}
+
+__global__ void k_realloc_sweep(ReArgs a, int top_sat) {
+  grid_begin();
+  const size_t col = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (col < a.ncol && realloc_column(a, a.flags, col, top_sat)) a.sc->changed = 1;
+}
+
+// The whole relaxation in one block on a copy of the flags in shared memory, for grids of few columns:
+// no read-back between the sweeps, so the step's host waits for its solve only (two sweeps and their read-backs
+// took 70 us of a step of 40 x 40 x 100, now 37).
+// Every sweep but the last sets a flag, so there are at most n + 1.
+constexpr int kReallocThreads = 1024;
+constexpr size_t kReallocCols = 2048, kReallocCells = 200 * 1024;
+__global__ void __launch_bounds__(kReallocThreads) k_realloc(ReArgs a, int top_sat) {
+  extern __shared__ __align__(16) uint8_t realloc_flags[];
+  grid_begin();
+  const uint4* src = reinterpret_cast<const uint4*>(a.flags);
+  uint4* dst = reinterpret_cast<uint4*>(realloc_flags);
+  for (size_t q = threadIdx.x; q < a.n / 16; q += blockDim.x) dst[q] = src[q];
+  for (size_t c = (a.n & ~(size_t)15) + threadIdx.x; c < a.n; c += blockDim.x)
+    realloc_flags[c] = a.flags[c];
+  __syncthreads();
+  unsigned long long sweeps = 0;
+  int changed;
+  do {
+    changed = 0;
+    for (size_t col = threadIdx.x; col < a.ncol; col += blockDim.x)
+      changed |= realloc_column(a, realloc_flags, col, top_sat);
+    ++sweeps;
+  } while (__syncthreads_or(changed) && sweeps <= a.n + 1);
+  if (threadIdx.x == 0) a.sc->sweeps += sweeps;
 }
 
 // Apply the reallocation (ReSolver.cpp:825-833), clampWaterContent (:839-853) and the
