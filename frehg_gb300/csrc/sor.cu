@@ -576,6 +576,81 @@ __global__ void k_sor_update(double* __restrict__ x, double* __restrict__ r,
     v[c] = sor_wait_value();
 }
 
+// The sweeps of a system that is one line of cells (a soil column), by one warp: first-order linear
+// recurrences, solved as a scan.  A lane takes a chunk of consecutive cells; per sweep it solves the
+// chunk from zero, the chunks' ends are combined over the lanes in five steps, and every cell gets its
+// share of what enters its chunk.  The recurrence's factors do not change during a solve, so their
+// products (within chunks: `pf`, `pb`; over lanes: registers) are formed once.  2 n / 32 + 5
+// dependent FP64 instructions a sweep (64 to 85 clocks each) instead of n: the solve of a column of
+// 100 cells takes 30 us, 58 in order.
+struct LineScan {
+  int lo, hi;  // the lane's cells
+  double f[5], b[5];
+  double *pf, *pb;
+  const double* e;  // coupling c to c + 1 over the diagonal of c
+  int n;
+
+  // products of the chunk's factors before step s over lanes, then combined with the neighbour's
+  __device__ __forceinline__ static void steps(double (&out)[5], double a, bool up, int lane) {
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      out[q] = a;
+      const double t = up ? __shfl_up_sync(0xffffffffu, a, 1 << q)
+                          : __shfl_down_sync(0xffffffffu, a, 1 << q);
+      if (up ? lane >= (1 << q) : lane + (1 << q) < 32) a *= t;
+    }
+  }
+
+  __device__ __forceinline__ LineScan(const double* e_, double* pf_, double* pb_, int n_)
+      : pf(pf_), pb(pb_), e(e_), n(n_) {
+    const int lane = threadIdx.x & 31, m = (n + 31) / 32;
+    lo = min(n, lane * m);
+    hi = min(n, lo + m);
+    double a = 1.0;
+    for (int c = lo; c < hi; ++c) pf[c] = a = c ? a * -e[c - 1] : 0.0;
+    steps(f, a, true, lane);
+    a = 1.0;
+    for (int c = hi - 1; c >= lo; --c) pb[c] = a = c + 1 < n ? a * -e[c] : 0.0;
+    steps(b, a, false, lane);
+  }
+
+  // v_c = r_c - e_{c-1} v_{c-1}
+  __device__ __forceinline__ void forward(const double* r, double* v) const {
+    const int lane = threadIdx.x & 31;
+    double y = 0.0;
+    for (int c = lo; c < hi; ++c) {
+      y = c > lo ? fma(-e[c - 1], y, r[c]) : r[c];
+      v[c] = y;
+    }
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const double t = __shfl_up_sync(0xffffffffu, y, 1 << q);
+      if (lane >= (1 << q)) y = fma(f[q], t, y);
+    }
+    const double in = __shfl_up_sync(0xffffffffu, y, 1);
+    if (lane)
+      for (int c = lo; c < hi; ++c) v[c] = fma(pf[c], in, v[c]);
+  }
+
+  // z_c = v_c - e_c z_{c+1}
+  __device__ __forceinline__ void backward(const double* v, double* z) const {
+    const int lane = threadIdx.x & 31;
+    double y = 0.0;
+    for (int c = hi - 1; c >= lo; --c) {
+      y = c + 1 < hi ? fma(-e[c], y, v[c]) : v[c];
+      z[c] = y;
+    }
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const double t = __shfl_down_sync(0xffffffffu, y, 1 << q);
+      if (lane + (1 << q) < 32) y = fma(b[q], t, y);
+    }
+    const double in = __shfl_down_sync(0xffffffffu, y, 1);
+    if (lane < 31)
+      for (int c = lo; c < hi; ++c) z[c] = fma(pb[c], in, z[c]);
+  }
+};
+
 // The whole solve of a small system in one block: the same iteration with every vector that the
 // sweeps or the neighbours read in shared memory (e, 1/d, r, v, z, p), the operator and x in
 // global memory (each thread its own cells).  w = A p lives where v does (v is written by the next
@@ -618,10 +693,13 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     z[c] = sor_wait_value();
   }
   __syncthreads();
-  const int tiles = g.nb1 * g.nb2;
+  const int tiles = AXES == 0 ? 0 : g.nb1 * g.nb2;
+  // one line: its sweeps by warp 0, the products in the arrays of the axes without couplings
+  LineScan line(g0, sor_sh + g.ax[1] * n, sor_sh + g.ax[2] * n, AXES == 0 && warp == 0 ? n : 0);
   // z = M r and (z.z, z.r) into the scalar steps; block-uniform
   auto apply = [&](bool init) {
     bool ok = true;
+    if (AXES == 0 && warp == 0) line.forward(r, v);
     for (int t = warp; t < tiles && ok; t += kWarps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
       ok = sor_tile<true, AXES>(g, L, SorShared(true, g, L, r, g0, g1, g2, v), &st.bar_timeout);
@@ -631,6 +709,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     // v / d by all threads: in the sweep it would be one more FP64 instruction per step
     for (int c = tid; c < n; c += kSorSolveThreads) v[c] *= invd[c];
     __syncthreads();
+    if (AXES == 0 && warp == 0) line.backward(v, z);
     for (int t = warp + (tiles - 1 - warp) / kWarps * kWarps; warp < tiles && t >= 0 && ok;
          t -= kWarps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
