@@ -161,7 +161,7 @@ struct CgDevState {
   double ir_bnorm, ir_rnorm;  // refinement loop norms (mixed precision)
   double rscale;              // the inner right-hand side is r~ / rscale (mixed precision)
   int ir_its;       // complete refinement sweeps (its: their inner iterations)
-  int pad_;
+  int fresh;        // inner system just set up: its first preconditioner application is due
   double first_a;   // ||r~|| of the first sweep
   // grid barrier of the one-launch CG iteration (k_cg_iter): arrival count, generation, and
   // the flag a block sets when its bounded wait ran out
@@ -170,6 +170,7 @@ struct CgDevState {
   // inner FP32 solve: below ttol_soft (0: unused) it runs kSoftIterations more at most towards ttol
   int soft_its;
   double ttol_soft;
+  int sweep_its[4];  // inner iterations of refinement sweeps 0, 1, 2 and of the last one
 };
 
 // KSPConvergedReason values
@@ -277,6 +278,7 @@ class KrylovSolver {
   int rnorm_slot = 1;
   // inner iterations launched at once: what recent first and later sweeps took
   int spec32[2] = {1, 1};
+  bool two_sweeps = false;  // the last solve took more than one sweep
   size_t cap_line = 0;
   float *lkf = nullptr, *dinvf = nullptr, *uf = nullptr, *pf2 = nullptr;
   // PCSOR (pc_type "sor", precision 0): 1/d, the preconditioned residual, the sweeps' operands in

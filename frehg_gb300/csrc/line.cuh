@@ -94,6 +94,7 @@ __device__ __forceinline__ void line_step_tail(CgDevState* st, double rzn, doubl
   if (FIRST) {
     st->beta = rzn;
     st->bcoef = 0.0;
+    st->fresh = 0;
     if (!(rzn > 0.0)) st->status = rzn == 0.0 ? kConvergedAtol : kDivergedIndefinitePc;
     return;
   }
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(32 * W, L > 8 ? 1 : 2) k32_line_step(
     const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
     double* partials) {
   grid_begin();
-  if (st->status) return;
+  if (st->status || (FIRST && !st->fresh)) return;
   __shared__ float2 fwd[W][32], bwd[W][32];
   __shared__ float lfirst[W + 1][32];
   const float a = FIRST ? 0.0f : (float)st->a;
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(128) k32_line_step_long(
     const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
     double* partials) {
   grid_begin();
-  if (st->status) return;
+  if (st->status || (FIRST && !st->fresh)) return;
   const float a = FIRST ? 0.0f : (float)st->a;
   const float* p = (st->iter & 1) ? p0 : p1;
   const bool xfirst = st->iter == 0;

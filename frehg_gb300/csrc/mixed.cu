@@ -35,6 +35,7 @@ __device__ __forceinline__ void sweep_tail(CgDevState* ir, CgDevState* in, doubl
                                            double sum_true, double unscale, double ir_rtol,
                                            double inner_rtol) {
   const double rn = sqrt(sum_true) * unscale;
+  ir->sweep_its[min(ir->ir_its, 3)] = in->its;
   ir->ir_its += 1;
   ir->its += in->its;
   ir->ir_rnorm = rn;
@@ -55,6 +56,7 @@ __device__ __forceinline__ void sweep_tail(CgDevState* ir, CgDevState* in, doubl
     in->iter = 0;
     in->its = 0;
     in->dpi = 0.0;
+    in->fresh = 1;
     in->status = 0;
   }
 }
@@ -203,6 +205,7 @@ __global__ void k_ir_scale(const double* __restrict__ rres, float* __restrict__ 
     in->iter = 0;
     in->its = 0;
     in->dpi = 0.0;
+    in->fresh = 1;
     in->status = tot[0] == 0.0 ? kConvergedAtol : 0;
   }
 }
@@ -1193,6 +1196,7 @@ __device__ __forceinline__ void prep_tail(CgDevState* ir, CgDevState* in, const 
     in->iter = 0;
     in->its = 0;
     in->dpi = 0.0;
+    in->fresh = 1;
     in->status = 0;
   } else {
     in->status = kConvergedAtol;
@@ -1574,9 +1578,22 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
   if (net.net != nullptr) FG_TRY(fetch());  // the network's loop is host-driven
   int sweeps = 0;     // complete sweeps
   int round = 0;      // rounds of the current sweep
-  int total = 0, sweep_its = 0;
+  int total = 0;      // inner iterations
+  // a sweep's start (on its first round) and some inner iterations; the number launched
+  auto launch_sweep = [&](int sweep, int rnd) {
+    if (rnd == 0) line_first();
+    const int spec = spec32[sweep > 0];
+    if (graphs && (rnd > 0 || spec > 8)) {
+      cudaGraphLaunch(g32, st);
+      if (prof) prof->launches += 3 * chunk;
+      return chunk;
+    }
+    const int its = rnd == 0 ? std::max(1, std::min(spec, 8)) : 4 << std::min(rnd - 1, 3);
+    for (int q = 0; q < its; ++q) iteration(st, prof);
+    return its;
+  };
   for (;;) {
-    int launched = 0;
+    int launched = 0, ends = 1;
     // a sweep that starts with the network's budget (twice the reference solve's inner
     // iterations) spent runs without it, as do the later ones
     if (net.net != nullptr && !fcg_fallback && net.max_inner > 0 && total >= net.max_inner)
@@ -1613,15 +1630,13 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
         FG_CUDA(cudaMemcpyAsync(&dst32->status, &stop, sizeof(int), cudaMemcpyHostToDevice, st));
       }
     } else {
-      if (round == 0) line_first();
-      const int spec = spec32[sweeps > 0];
-      if (graphs && (round > 0 || spec > 8)) {
-        FG_CUDA(cudaGraphLaunch(g32, st));
-        if (prof) prof->launches += 3 * chunk;
-        launched = chunk;
-      } else {
-        launched = round == 0 ? std::max(1, std::min(spec, 8)) : 4 << std::min(round - 1, 3);
-        for (int q = 0; q < launched; ++q) iteration(st, prof);
+      launched = launch_sweep(sweeps, round);
+      // where the last solve took a second sweep, it is launched behind the first without a
+      // read-back between them (7 us of a sweep's 70 at 40 x 40 x 100)
+      if (line && net.net == nullptr && sweeps == 0 && round == 0 && two_sweeps) {
+        sweep_end();
+        launched += launch_sweep(1, 0);
+        ends = 2;
       }
     }
     sweep_end();
@@ -1636,8 +1651,7 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
     }
     if (hst->first_a > 0.0 && std::isfinite(hst->first_a))
       first_rnorm[rnorm_slot & 1] = hst->first_a;
-    const bool ended = hst->ir_its > sweeps || hst->status != 0;
-    const int done = hst->its + (ended ? 0 : hst32->its) - total;
+    const int done = hst->its + (hst->status == 0 ? hst32->its : 0) - total;
     if (prof && prof->on && launched > 0) {
       const int64_t idle = std::max(0, launched - std::max(0, done));
       if (line) {
@@ -1648,24 +1662,23 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
         prof->idle(spmv_name, idle);
         prof->idle("k32_update", idle);
       }
-      if (hst->ir_its == sweeps) {
-        prof->idle("k_ir_update", 1);
-        prof->idle(A.s_in_r ? "k_ir_sweep" : "k_ir_residual", 1);
+      if (const int idle_ends = ends - (hst->ir_its - sweeps); idle_ends > 0) {
+        prof->idle("k_ir_update", idle_ends);
+        prof->idle(A.s_in_r ? "k_ir_sweep" : "k_ir_residual", idle_ends);
       }
     }
     if (dbg)
       fprintf(stderr, "ir sweep %d round %d: launched %d done %d; true |r| %.3e / |b| %.3e status %d\n",
               sweeps, round, launched, done, hst->ir_rnorm, hst->ir_bnorm, hst->status);
     total += done;
-    sweep_its += done;
     ++round;
-    if (ended) {
-      if (launched > 0) spec32[sweeps > 0] = std::max(sweep_its, spec32[sweeps > 0] - 1);
-      sweeps = hst->ir_its;
-      round = sweep_its = 0;
-    }
+    for (; sweeps < hst->ir_its; ++sweeps, round = hst32->its > 0 ? 1 : 0)
+      if (launched > 0)
+        spec32[sweeps > 0] =
+            std::max(hst->sweep_its[std::min(sweeps, 3)], spec32[sweeps > 0] - 1);
     if (hst->status != 0 || sweeps >= max_sweeps) break;
   }
+  two_sweeps = sweeps > 1;
   // stopped before the first update: x~ = 0
   if (sweeps == 0)
     FG_LAUNCH(prof, st, "k_zero64", 8.0 * dn, k_zero64<<<nb, 256, 0, st>>>(x, n));
