@@ -190,41 +190,6 @@ __global__ void __launch_bounds__(256) k_grad_mask(bf16* __restrict__ g, int g_s
   }
 }
 
-// 2x2x2 average pooling: out (coarse, stride C) from a channel slice of in (fine)
-// 2x2x2 mean pooling of a channel slice: one thread per coarse cell and group of 8 channels
-// (16-byte loads of the eight children, one 16-byte store); c, in_stride and in_off are
-// multiples of 8, and the network's cell counts stay below 2^32
-__global__ void k_pool(const bf16* __restrict__ in, int in_stride, int in_off, bf16* __restrict__ out,
-                       int c, int nx, int ny, int nz) {
-  const uint32_t cx = nx / 2, cy = ny / 2, cz = nz / 2;
-  const uint32_t g = (uint32_t)c / 8;
-  const uint64_t tot = (uint64_t)cx * cy * cz * g;
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < tot;
-       e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t q = (uint32_t)(e / g), cg = (uint32_t)(e - (uint64_t)q * g);
-    const uint32_t x = q % cx, yz = q / cx, y = yz % cy, z = yz / cy;
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t p = (2 * x + (k & 1)) + (uint32_t)nx * ((2 * y + ((k >> 1) & 1)) +
-                                                             (uint32_t)ny * (2 * z + (k >> 2)));
-      const uint4 v = *reinterpret_cast<const uint4*>(in + (size_t)p * in_stride + in_off + 8 * cg);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float2 f = __bfloat1622float2(h[u]);
-        s[2 * u] += f.x;
-        s[2 * u + 1] += f.y;
-      }
-    }
-    uint4 o;
-    uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) ow[u] = pack2(0.125f * s[2 * u], 0.125f * s[2 * u + 1]);
-    *reinterpret_cast<uint4*>(out + (size_t)q * c + 8 * cg) = o;
-  }
-}
-
 // gradient of upsampling: gin[q] = sum of the 8 children of a fine gradient slice; one thread per
 // coarse cell and group of 8 channels (16-byte accesses)
 __global__ void k_up_bwd(const bf16* __restrict__ gout, int g_stride, int g_off,
@@ -322,29 +287,6 @@ __global__ void k_rms_scale(const double* __restrict__ part, int nparts, size_t 
     const double rms = sqrt(t / (double)n);
     *scale = rms > 0.0 ? (float)(1.0 / rms) : 1.0f;
     *inv = rms > 0.0 ? (float)rms : 1.0f;
-  }
-}
-
-// y[p] = (w_o . d1[p] + b_o) * outscale
-__global__ void k_out(const bf16* __restrict__ d1, const float* __restrict__ wo,
-                      const float* __restrict__ outscale, float* __restrict__ y, size_t n) {
-  const float s = outscale ? *outscale : 1.0f;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n;
-       p += (size_t)gridDim.x * blockDim.x) {
-    float v = wo[16];
-    const uint4* dv = reinterpret_cast<const uint4*>(d1 + p * 16);  // two 16-byte loads
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const uint4 w = dv[half];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float2 f = __bfloat1622float2(h[u]);
-        v = fmaf(wo[8 * half + 2 * u], f.x, v);
-        v = fmaf(wo[8 * half + 2 * u + 1], f.y, v);
-      }
-    }
-    y[p] = v * s;
   }
 }
 
@@ -485,11 +427,12 @@ int* tc_error_word() {
 
 // Output planes per z column: the smallest time of the busiest block, in input planes, over the
 // columns it walks (a column of zc output planes reads zc + 2 input planes).
-static int conv_column(long tiles, int nz, long blocks) {
+static int conv_column(long tiles, int nz, long blocks, bool even) {
   int best = nz;
   long best_cost = LONG_MAX;
   for (int cols = 1; cols <= nz; ++cols) {
-    const int zc = (nz + cols - 1) / cols;
+    int zc = (nz + cols - 1) / cols;
+    if (even) zc += zc & 1;
     const long items = tiles * ((nz + zc - 1) / zc);
     const long cost = (items + blocks - 1) / blocks * (zc + 2);
     if (cost < best_cost) {
@@ -506,23 +449,23 @@ static int conv_column(long tiles, int nz, long blocks) {
 // of three of N = 48 (44 each).  Two parts for 32 to 96 (N at most 256), 64 to 64 (221 KB of weights)
 // and 96 to 32, whose 166 KB of weights would leave less than two planes of patches (270 us in one
 // part with eleven of the twelve slices resident, 200 in two).
-template <int CIN, int COUT, int UP = 0>
+template <int CIN, int COUT, int UP = 0, int EPI = kTcPlain>
 static void conv(const bf16* in, int in_stride, int in_off, const bf16* W, const float* bias,
                  bf16* out, int out_stride, int out_off, int nx, int ny, int nz, bool relu,
-                 cudaStream_t st, const bf16* coarse = nullptr) {
+                 cudaStream_t st, const bf16* coarse = nullptr, const TcExtra& extra = TcExtra()) {
   constexpr int NB = COUT == 96 ? 48 : (27 * CIN * COUT * 2 > 150 * 1024 ? COUT / 2 : COUT);
   constexpr int PARTS = COUT / NB;
   using S = TcShape<CIN, NB>;
   // set on every launch: the attribute belongs to the current device, and the call is cheap
-  cudaFuncSetAttribute(k_conv3_tc<CIN, COUT, NB, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       S::SMEM);
+  cudaFuncSetAttribute(k_conv3_tc<CIN, COUT, NB, UP, EPI>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
   const long tiles = (long)tc_tiles_x(nx) * tc_tiles_y(ny), blocks = kNumSMs / PARTS;
-  const int zc = conv_column(tiles, nz, blocks);
+  const int zc = conv_column(tiles, nz, blocks, EPI == kTcPool);
   const long items = tiles * ((nz + zc - 1) / zc);
   const int grid = (int)std::min(items, blocks) * PARTS;
-  k_conv3_tc<CIN, COUT, NB, UP><<<grid, kTcThreads, S::SMEM, st>>>(
+  k_conv3_tc<CIN, COUT, NB, UP, EPI><<<grid, kTcThreads, S::SMEM, st>>>(
       in, in_stride, in_off, coarse, W, bias, out, out_stride, out_off, nx, ny, nz, zc,
-      relu ? 1 : 0, tc_error_word());
+      relu ? 1 : 0, extra, tc_error_word());
 }
 
 // the same convolution on the mma.sync kernel (the self-check's comparison)
@@ -678,12 +621,13 @@ int ensure_acts(frehg_unet* net, int nx, int ny, int nz) {
   return FREHG_OK;
 }
 
-// forward pass; y = network output times `outscale` (rms of r) when scaled_out
+// forward pass; y = network output times `outscale` (rms of r) when scaled_out; keep: the last layer's
+// activations are stored (a backward pass follows)
 int forward(frehg_unet* net, const float* r, const float* lnk, const float* cap, float* y,
-            bool scaled_out, cudaStream_t st) {
+            bool scaled_out, bool keep, cudaStream_t st) {
   const int nx = net->nx, ny = net->ny, nz = net->nz;
   const int x2 = nx / 2, y2 = ny / 2, z2 = nz / 2, x3 = nx / 4, y3 = ny / 4, z3 = nz / 4;
-  const size_t n1 = (size_t)nx * ny * nz, n2 = n1 / 8, n3 = n1 / 64;
+  const size_t n1 = (size_t)nx * ny * nz;
   const float* M = net->master;
   const bf16* W = net->wb;
   {
@@ -694,20 +638,24 @@ int forward(frehg_unet* net, const float* r, const float* lnk, const float* cap,
   k_pack_input<<<blocks_for(n1), 256, 0, st>>>(r, lnk, cap, net->scal, net->kmean, net->kscale,
                                                net->cscale, net->x0, n1);
   conv<16, 16>(net->x0, 16, 0, W + net->wboff[0], M + net->boff[0], net->a1, 16, 0, nx, ny, nz, true, st);
-  conv<16, 16>(net->a1, 16, 0, W + net->wboff[1], M + net->boff[1], net->e1, 16, 0, nx, ny, nz, true, st);
-  k_pool<<<blocks_for(n2 * 2), 256, 0, st>>>(net->e1, 16, 0, net->p1, 16, nx, ny, nz);
+  TcExtra pool1, pool2, last;
+  pool1.pooled = net->p1;
+  pool2.pooled = net->p2;
+  last.wo = M + net->ooff;
+  last.scale = scaled_out ? net->scal + 1 : nullptr;
+  last.y = y;
+  conv<16, 16, 0, kTcPool>(net->a1, 16, 0, W + net->wboff[1], M + net->boff[1], net->e1, 16, 0, nx,
+                           ny, nz, true, st, nullptr, pool1);
   conv<16, 32>(net->p1, 16, 0, W + net->wboff[2], M + net->boff[2], net->a2, 32, 0, x2, y2, z2, true, st);
-  conv<32, 32>(net->a2, 32, 0, W + net->wboff[3], M + net->boff[3], net->e2, 32, 0, x2, y2, z2, true, st);
-  k_pool<<<blocks_for(n3 * 4), 256, 0, st>>>(net->e2, 32, 0, net->p2, 32, x2, y2, z2);
+  conv<32, 32, 0, kTcPool>(net->a2, 32, 0, W + net->wboff[3], M + net->boff[3], net->e2, 32, 0, x2,
+                           y2, z2, true, st, nullptr, pool2);
   conv<32, 64>(net->p2, 32, 0, W + net->wboff[4], M + net->boff[4], net->a3, 64, 0, x3, y3, z3, true, st);
   conv<64, 64>(net->a3, 64, 0, W + net->wboff[5], M + net->boff[5], net->e3, 64, 0, x3, y3, z3, true, st);
   conv<96, 32, 64>(net->e2, 32, 0, W + net->wboff[6], M + net->boff[6], net->d2a, 32, 0, x2, y2, z2, true, st, net->e3);
   conv<32, 32>(net->d2a, 32, 0, W + net->wboff[7], M + net->boff[7], net->d2, 32, 0, x2, y2, z2, true, st);
   conv<48, 16, 32>(net->e1, 16, 0, W + net->wboff[8], M + net->boff[8], net->d1a, 16, 0, nx, ny, nz, true, st, net->d2);
-  conv<16, 16>(net->d1a, 16, 0, W + net->wboff[9], M + net->boff[9], net->d1, 16, 0, nx, ny, nz, true, st);
-  k_out<<<blocks_for(n1), 256, 0, st>>>(net->d1, M + net->ooff, scaled_out ? net->scal + 1 : nullptr,
-                                        y, n1);
-  (void)n3;
+  conv<16, 16, 0, kTcOut>(net->d1a, 16, 0, W + net->wboff[9], M + net->boff[9],
+                          keep ? net->d1 : nullptr, 16, 0, nx, ny, nz, true, st, nullptr, last);
   FG_CUDA(cudaGetLastError());
   return FREHG_OK;
 }
@@ -784,7 +732,7 @@ namespace fg {
 int unet_apply(frehg_unet* net, int nx, int ny, int nz, const float* r, const float* lnk,
                const float* cap, float* z, cudaStream_t st) {
   FG_TRY(ensure_acts(net, nx, ny, nz));
-  return forward(net, r, lnk, cap, z, true, st);
+  return forward(net, r, lnk, cap, z, true, false, st);
 }
 }  // namespace fg
 
@@ -999,7 +947,7 @@ int frehg_unet_forward(frehg_unet* net, int nx, int ny, int nz, const float* r, 
   FG_ARG(net && r && lnk && cap && y, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   FG_TRY(ensure_acts(net, nx, ny, nz));
-  FG_TRY(forward(net, r, lnk, cap, y, true, st));
+  FG_TRY(forward(net, r, lnk, cap, y, true, false, st));
   FG_CUDA(cudaStreamSynchronize(st));
   return check_tc_error();
 }
@@ -1011,7 +959,7 @@ int frehg_unet_loss_grad(frehg_unet* net, int nx, int ny, int nz, const float* r
   FG_ARG(net && r && lnk && cap && target, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   FG_TRY(ensure_acts(net, nx, ny, nz));
-  FG_TRY(forward(net, r, lnk, cap, net->y, false, st));
+  FG_TRY(forward(net, r, lnk, cap, net->y, false, true, st));
   FG_TRY(backward(net, target, st));
   if (loss) FG_CUDA(cudaMemcpyAsync(loss, net->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
   if (grad_host)

@@ -30,9 +30,8 @@
 // Bound by shared memory: the MMAs' reads (44 clocks of the 61 that an MMA of 48 -> 16 takes) and
 // the copies, which pass through L1.  (Copies past L1 are slower but for 96 channels, 16 copy warps
 // no faster.)  The decoder convolutions read the upsampled half of their input from the coarse
-// field, as the stored concatenation took 170 us more in all at 256 x 256 x 128.
-//  256 x 256 x 128, against one MMA group per output plane and per-plane barriers of one
-// warpgroup: 16 -> 16 305 -> 153 us, 48 -> 16 617 -> 372; 128 x 128 x 64: 96 -> 32 628 -> 200, 32 ->
+// field, as the stored concatenation took 170 us more in all at 256 x 256 x 128.  There, against one
+// MMA group per output plane and per-plane barriers of one warpgroup: 16 -> 16 305 -> 153 us, 48 -> 16 617 -> 372; 128 x 128 x 64: 96 -> 32 628 -> 200, 32 ->
 // 32 96 -> 61; 64 x 64 x 32: 64 -> 64 112 -> 33.
 //
 // Every wait is bounded: a wait that runs out records an error word, the block's other waits see
@@ -129,6 +128,10 @@ __device__ __forceinline__ int tc_wait(uint64_t* bar, uint32_t parity, const vol
   return 0;
 }
 
+__device__ __forceinline__ float2 tc_bf16x2(uint32_t v) {
+  return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v));
+}
+
 // the published count of ready planes once it exceeds p (kTcStop: the block stops)
 __device__ __forceinline__ uint32_t tc_ready(const uint32_t* word, uint32_t p) {
   for (long q = 0; q < 16 * kTcSpin; ++q) {
@@ -205,15 +208,25 @@ constexpr int kTcCopyWarps = 8, kTcCopy0 = 8, kTcMma = kTcCopy0 + kTcCopyWarps;
 constexpr int kTcThreads = 32 * (kTcMma + 2);
 constexpr int kTcDone = 64;  // barriers of finished input planes, more than the roles can be apart
 
+// What else the epilogue does with a layer's output (at 256 x 256 x 128 the pooling in a pass of its own
+// took 53 us, here 36; the output layer 50, here 2).
+enum TcEpilogue { kTcPlain, kTcPool, kTcOut };
+struct TcExtra {
+  __nv_bfloat16* pooled = nullptr;  // kTcPool: the 2x2x2 means (COUT channels), zc and nz even
+  const float* wo = nullptr;        // kTcOut: y = (w_o . out + b_o) scale, COUT = 16
+  const float* scale = nullptr;     // (1 where null)
+  float* y = nullptr;
+};
+
 // UP > 0: the first UP input channels are the nearest 2x upsampling of the coarse field `coarse` (UP
 // channels), read where it lies; `in` holds the others.
-template <int CIN, int COUT, int NB, int UP>
+template <int CIN, int COUT, int NB, int UP, int EPI>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_conv3_tc(const __nv_bfloat16* __restrict__ in, int in_stride, int in_off,
                const __nv_bfloat16* __restrict__ coarse,
                const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                __nv_bfloat16* __restrict__ out, int out_stride, int out_off, int nx, int ny, int nz,
-               int zc, int relu, int* err) {
+               int zc, int relu, TcExtra extra, int* err) {
   using S = TcShape<CIN, NB>;
   constexpr int PARTS = COUT / NB;
   extern __shared__ __align__(128) unsigned char tc_dyn[];
@@ -226,7 +239,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   __shared__ uint32_t ready_word;  // input planes whose slices and accumulators are ready
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
-  __shared__ float bias_s[NB];
+  __shared__ float bias_s[NB], wo_s[EPI == kTcOut ? NB + 1 : 1];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform to the compiler, too
   const int part = blockIdx.x % PARTS, o0 = part * NB;
@@ -247,6 +260,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     abort_word = 0;
   }
   if (tid < NB) bias_s[tid] = bias ? bias[o0 + tid] : 0.f;
+  if (EPI == kTcOut && tid <= NB) wo_s[tid] = extra.wo[tid];
   // all 27 taps of the weights, once per block, the dz taps stacked along N
   for (int q = tid; q < 9 * 2 * S::KC * S::N3; q += kTcThreads) {
     const int c = q % (2 * S::KC), orow = (q / (2 * S::KC)) % S::N3, t9 = q / (S::N3 * 2 * S::KC);
@@ -295,6 +309,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     const int px0 = (wr * 32 + lane) & 7, py0 = (wr * 32 + lane) >> 3;
     uint32_t v = 0, pb = 0;  // accumulators and input planes of the columns before
+    const float yscale = EPI == kTcOut && extra.scale ? *extra.scale : 1.f;
     bool ok = true;
     for (long item = first; item < items && ok; item += step) {
       const int px = (int)(item % xt) * kTcTX + px0;
@@ -304,8 +319,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const int z0 = max(zb - 1, 0), z1 = min(ze, nz - 1);
       __nv_bfloat16* dst = out + ((size_t)px + (size_t)nx * ((size_t)py + (size_t)ny * zb)) *
                                      out_stride + out_off + o0;
+      float pool[EPI == kTcPool ? NB : 1];  // of the plane pair that this warp's group takes
       for (int z = zb; z < ze; ++z, ++v, dst += (size_t)nx * ny * out_stride) {
-        if ((int)(v & 1u) != warp >> 2) continue;
+        if ((int)((EPI == kTcPool ? v >> 1 : v) & 1u) != warp >> 2) continue;
         const uint32_t slot = v % S::R;
         // complete with the input plane below it (the last plane of the grid with its own)
         ok = wait_done(pb + (uint32_t)(min(z + 1, z1) - z0));
@@ -330,23 +346,66 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) tc_arrive(&acc_empty[slot]);
-        if (px < nx && py < ny) {
+        const bool in_grid = px < nx && py < ny;
+        uint32_t packed[NB / 2];
 #pragma unroll
-          for (int cb = 0; cb < NB; cb += 8) {
-            uint32_t packed[4];
+        for (int q = 0; q < NB / 2; ++q) {
+          float v0 = __uint_as_float(r[2 * q]) + bias_s[2 * q];
+          float v1 = __uint_as_float(r[2 * q + 1]) + bias_s[2 * q + 1];
+          if (relu) {
+            v0 = fmaxf(v0, 0.f);
+            v1 = fmaxf(v1, 0.f);
+          }
+          __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+          packed[q] = *reinterpret_cast<uint32_t*>(&h);
+        }
+        if (in_grid && (EPI != kTcOut || out != nullptr)) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float v0 = __uint_as_float(r[cb + 2 * q]) + bias_s[cb + 2 * q];
-              float v1 = __uint_as_float(r[cb + 2 * q + 1]) + bias_s[cb + 2 * q + 1];
-              if (relu) {
-                v0 = fmaxf(v0, 0.f);
-                v1 = fmaxf(v1, 0.f);
-              }
-              __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-              packed[q] = *reinterpret_cast<uint32_t*>(&h);
+          for (int q = 0; q < NB / 8; ++q)
+            reinterpret_cast<uint4*>(dst)[q] = make_uint4(packed[4 * q], packed[4 * q + 1],
+                                                          packed[4 * q + 2], packed[4 * q + 3]);
+        }
+        if constexpr (EPI == kTcOut) {
+          float t = wo_s[NB];
+#pragma unroll
+          for (int q = 0; q < NB / 2; ++q) {
+            const float2 f = tc_bf16x2(packed[q]);
+            t = fmaf(wo_s[2 * q], f.x, t);
+            t = fmaf(wo_s[2 * q + 1], f.y, t);
+          }
+          if (in_grid) extra.y[(size_t)px + (size_t)nx * ((size_t)py + (size_t)ny * z)] = t * yscale;
+        }
+        if constexpr (EPI == kTcPool) {
+          // the pixels right, below and below right are lanes + 1, + 8, + 9 (four rows of eight)
+#pragma unroll
+          for (int q = 0; q < NB / 2; ++q) {
+            float2 t = z & 1 ? make_float2(pool[2 * q], pool[2 * q + 1]) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int off = u == 0 ? 0 : u == 1 ? 1 : u == 2 ? 8 : 9;
+              const float2 f =
+                  tc_bf16x2(off ? __shfl_down_sync(0xffffffffu, packed[q], off) : packed[q]);
+              t.x += f.x;
+              t.y += f.y;
             }
-            *reinterpret_cast<uint4*>(dst + cb) =
-                make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            pool[2 * q] = t.x;
+            pool[2 * q + 1] = t.y;
+          }
+          if ((z & 1) && in_grid && !(px & 1) && !(py & 1)) {
+            const size_t c = (size_t)(px >> 1) +
+                             (size_t)(nx >> 1) * ((size_t)(py >> 1) + (size_t)(ny >> 1) * (z >> 1));
+            uint4* pd = reinterpret_cast<uint4*>(extra.pooled + c * COUT + o0);
+#pragma unroll
+            for (int q = 0; q < NB / 8; ++q) {
+              uint32_t w4[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                __nv_bfloat162 h = __floats2bfloat162_rn(0.125f * pool[8 * q + 2 * u],
+                                                         0.125f * pool[8 * q + 2 * u + 1]);
+                w4[u] = *reinterpret_cast<uint32_t*>(&h);
+              }
+              pd[q] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+            }
           }
         }
       }
