@@ -655,9 +655,13 @@ static int pca_step(frehg_re* re) {
     }
   }
   re->cnt.realloc_sweeps += sweeps;
-  // apply reallocation, clampWaterContent, adaptiveTimeStep
+  // apply reallocation, clampWaterContent, adaptiveTimeStep: in two halves where a block or two per
+  // SM and plane leave the FP64 unit waiting for a chain (100 cells: 18.4 -> 14.3 us)
+  const bool split = (size_t)L.grid.x * L.grid.y * L.planes <= 2 * (size_t)kNumSMs;
   FG_LAUNCH(prof, st, "k_finalize", (25.0 + sb) * n,
-            launch_chained(k_finalize, L.grid, L.block, 0, st, a, top_sat, L.planes, L.tiles));
+            launch_chained(split ? k_finalize<true> : k_finalize<false>,
+                           dim3(L.grid.x, L.grid.y * (split ? 2 : 1)), L.block, 0, st, a, top_sat,
+                           L.planes, L.tiles));
   FG_CUDA(cudaGetLastError());
   if (prof->on) {
     FG_CUDA(cudaStreamSynchronize(st));

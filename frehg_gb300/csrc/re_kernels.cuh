@@ -613,8 +613,14 @@ __global__ void __launch_bounds__(kReallocThreads) k_realloc(ReArgs a, int top_s
 // Apply the reallocation (ReSolver.cpp:825-833), clampWaterContent (:839-853) and the
 // adaptiveTimeStep Courant bound (:906-910); the last block updates dt (:921-928) and time.
 // Launched on (32 x 8)-column tiles marching through `planes` levels (no index divisions).
+// SPLIT: blocks of even y do the update and those of odd y the Courant bound, whose chains of about 100
+// dependent FP64 instructions each would otherwise follow one another.  Both read what the other does not
+// change: the bound sees the water content before or after the update's clamp, with the same result.
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int planes, int tiles) {
   grid_begin();
+  const bool update = !SPLIT || !(blockIdx.y & 1), bound = !SPLIT || (blockIdx.y & 1);
+  const int slab = SPLIT ? blockIdx.y >> 1 : blockIdx.y;
   double dtco = INFINITY;
   const int t0 = (a.nx + 31) / 32;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -622,7 +628,7 @@ __global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int pla
   const int j = (tile / t0) * 8 + threadIdx.y;
   if (i >= a.nx || j >= a.ny) continue;
   const size_t col = (size_t)i + (size_t)a.nx * j;
-  const int kb = blockIdx.y * planes, ke = min(a.nz, kb + planes);
+  const int kb = slab * planes, ke = min(a.nz, kb + planes);
   for (int k = kb; k < ke; ++k) {
     const size_t c = col + a.ncol * k;
     const CellSoil s = soil_of(a.soil, c, col);
@@ -647,7 +653,7 @@ __global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int pla
       if (!adj && (f & F_OPEN_YP))
         adj = (j + 1 < a.ny) ? (a.flags[c + a.nx] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
       if (!adj) {
-        if (wc < 0.9999 * s.ths) a.h_new[c] = vg_head(s, wc);
+        if (update && wc < 0.9999 * s.ths) a.h_new[c] = vg_head(s, wc);
       } else {
         wc = a.wch[c];
       }
@@ -656,8 +662,8 @@ __global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int pla
       wc = s.ths;
     else if (wc < s.thr)
       wc = s.thr;
-    a.w_new[c] = wc;
-    if (a.adaptive && k > 0 && wc < s.ths) {
+    if (update) a.w_new[c] = wc;
+    if (bound && a.adaptive && k > 0 && wc < s.ths) {
       const double dk = vg_dKdwc(s, wc, s.Ksz);
       const double dt_co = a.co_max * a.dz / dk;
       if (dt_co < dtco) dtco = dt_co;  // std::min(dt_Comin, dt_Co): NaN is skipped

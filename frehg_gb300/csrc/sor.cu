@@ -447,7 +447,8 @@ __device__ __forceinline__ int sor_converged(CgDevState* s, double rnorm) {
 
 // KSPSolve_CG's scalar steps after a preconditioner application (||z||^2 = zz, z.r = zr): the
 // stopping test and the next direction's coefficient; INIT: before the first iteration.
-template <bool INIT>
+// QUOTIENT false: the caller forms bcoef = beta / betaold itself
+template <bool INIT, bool QUOTIENT = true>
 __device__ __forceinline__ void sor_scalars(CgDevState* st, double zz, double zr) {
   const double dp = sqrt(zz);
   st->dp = dp;
@@ -481,6 +482,7 @@ __device__ __forceinline__ void sor_scalars(CgDevState* st, double zz, double zr
     st->status = kConvergedAtol;
     return;
   }
+  if (!QUOTIENT) return;
   st->bcoef = st->beta / st->betaold;
   if (st->bcoef < 0.0) st->status = kDivergedIndefinitePc;
 }
@@ -664,9 +666,11 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
   grid_begin();
   extern __shared__ double sor_sh[];
   __shared__ CgDevState st;
+  __shared__ double quot;  // beta / the last beta, by warp 1 while thread 0 tests the norm
+  double beta = 0.0;       // (thread 32's)
   __shared__ double red[128];  // (the vectors of 3,600 cells leave 2 KB)
   const int n = n0 * n1 * n2, tid = threadIdx.x, warp = tid >> 5;
-  constexpr int kWarps = kSorSolveThreads / 32;
+  const int nt = blockDim.x, warps = nt >> 5;
   double *e0 = sor_sh, *e1 = e0 + n, *e2 = e1 + n, *invd = e2 + n, *r = invd + n, *v = r + n,
          *z = v + n, *p = z + n;
   // the couplings in the order of the geometry's axes
@@ -680,7 +684,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     st.bar_timeout = 0;
     st.bcoef = st.beta = st.betaold = st.dp = st.dpiold = 0.0;
   }
-  for (int c = tid; c < n; c += kSorSolveThreads) {
+  for (int c = tid; c < n; c += nt) {
     const double dc = d[c];
     const double id = 1.0 / (dc == 0.0 ? 1.0 : dc);
     invd[c] = id;
@@ -700,25 +704,25 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
   auto apply = [&](bool init) {
     bool ok = true;
     if (AXES == 0 && warp == 0) line.forward(r, v);
-    for (int t = warp; t < tiles && ok; t += kWarps) {
+    for (int t = warp; t < tiles && ok; t += warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
       ok = sor_tile<true, AXES>(g, L, SorShared(true, g, L, r, g0, g1, g2, v), &st.bar_timeout);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
     // v / d by all threads: in the sweep it would be one more FP64 instruction per step
-    for (int c = tid; c < n; c += kSorSolveThreads) v[c] *= invd[c];
+    for (int c = tid; c < n; c += nt) v[c] *= invd[c];
     __syncthreads();
     if (AXES == 0 && warp == 0) line.backward(v, z);
-    for (int t = warp + (tiles - 1 - warp) / kWarps * kWarps; warp < tiles && t >= 0 && ok;
-         t -= kWarps) {
+    for (int t = warp + (tiles - 1 - warp) / warps * warps; warp < tiles && t >= 0 && ok;
+         t -= warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
       ok = sor_tile<false, AXES>(g, L, SorShared(false, g, L, v, g0, g1, g2, z), &st.bar_timeout);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
     double s[2] = {0.0, 0.0};
-    for (int c = tid; c < n; c += kSorSolveThreads) {
+    for (int c = tid; c < n; c += nt) {
       s[0] = fma(z[c], z[c], s[0]);
       s[1] = fma(z[c], r[c], s[1]);
     }
@@ -727,22 +731,31 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
       if (st.bar_timeout)
         st.status = kGridBarrierTimeout;
       else if (init)
-        sor_scalars<true>(&st, s[0], s[1]);
+        sor_scalars<true, false>(&st, s[0], s[1]);
       else
-        sor_scalars<false>(&st, s[0], s[1]);
+        sor_scalars<false, false>(&st, s[0], s[1]);
+    }
+    if (tid == 32) {
+      quot = init ? 0.0 : s[1] / beta;
+      beta = s[1];
     }
     __syncthreads();
+    if (st.status == 0 && quot < 0.0) {
+      __syncthreads();
+      if (tid == 0) st.status = kDivergedIndefinitePc;
+      __syncthreads();
+    }
   };
   apply(true);
   const int s1 = n0, s2 = n0 * n1;
   while (st.status == 0) {
-    const double bc = st.bcoef;
+    const double bc = quot;
     const bool first = st.iter == 0;
-    for (int c = tid; c < n; c += kSorSolveThreads) p[c] = first ? z[c] : fma(bc, p[c], z[c]);
+    for (int c = tid; c < n; c += nt) p[c] = first ? z[c] : fma(bc, p[c], z[c]);
     __syncthreads();
     double acc[1] = {0.0};
     double* w = v;
-    for (int c = tid; c < n; c += kSorSolveThreads) {
+    for (int c = tid; c < n; c += nt) {
       const int i0 = c % n0, q = c / n0, i1 = q % n1, i2 = q / n1;
       const double pc = p[c];
       double y = d[c] * pc;
@@ -760,7 +773,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     __syncthreads();
     if (st.status) break;
     const double a = st.a;
-    for (int c = tid; c < n; c += kSorSolveThreads) {
+    for (int c = tid; c < n; c += nt) {
       x[c] = fma(a, p[c], x[c]);
       r[c] = fma(-a, w[c], r[c]);
       v[c] = sor_wait_value();
@@ -770,7 +783,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     apply(false);
   }
   if (st.status > 0 && x_out != x)
-    for (int c = tid; c < n; c += kSorSolveThreads) x_out[c] = x[c];
+    for (int c = tid; c < n; c += nt) x_out[c] = x[c];
   if (tid == 0) {
     dst->its = st.its;
     dst->iter = st.iter;
@@ -846,12 +859,14 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   };
   if (n <= (size_t)kSorSolveCells) {
     const int smem = 8 * (int)n * (int)sizeof(double);
+    // no more warps than cells need: each takes part in every sum on the FP64 unit
+    const int threads = std::min(kSorSolveThreads, std::max(64, ((int)n + 31) / 32 * 32));
     // on every solve: the attribute belongs to the current device, and the call is cheap
     auto kernel = g.axes == 2 ? k_sor_solve<2> : (g.axes == 1 ? k_sor_solve<1> : k_sor_solve<0>);
     FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  8 * kSorSolveCells * (int)sizeof(double)));
     FG_LAUNCH(prof, st, "k_sor_solve", 48.0 * dn,
-              launch_chained(kernel, 1, kSorSolveThreads, smem, st, g, A.s, A.a0, A.a1, A.a2, A.b, x,
+              launch_chained(kernel, 1, threads, smem, st, g, A.s, A.a0, A.a1, A.a2, A.b, x,
                              x_out ? x_out : x, A.n0, A.n1, A.n2, cfg.rtol, cfg.atol, 1.0e4,
                              cfg.max_it, dst));
     FG_CUDA(cudaGetLastError());
