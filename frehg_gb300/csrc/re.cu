@@ -265,11 +265,12 @@ static ReArgs make_args(frehg_re* re) {
 // simple device helpers for the C API
 
 namespace {
+template <bool SMALL>
 __global__ void k_theta_of_h(ReArgs a, const double* __restrict__ h, double* __restrict__ w) {
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < a.n;
        c += (size_t)gridDim.x * blockDim.x) {
     const CellSoil s = soil_of(a.soil, c, c % a.ncol);
-    w[c] = vg_theta_initial(s, h[c]);
+    w[c] = SMALL ? vg_theta(s, h[c]) : vg_theta_initial(s, h[c]);
   }
 }
 __global__ void k_h_of_theta(ReArgs a, const double* __restrict__ w, double* __restrict__ h) {
@@ -346,6 +347,11 @@ static int nblocks(size_t n) { return reduction_blocks(n, 256, 4); }
 // with four cells each, 1,500 cells ran on two SMs (k_kr 30 us, now 11) and 160,000 on one
 // block per SM (75 us, now 46).
 constexpr int kSpreadThreads = 64;
+// Up to this many cells the initial water content and the Courant bound take the CUDA library's
+// pow() in the reference's form: the kernels' time is the latency of one chain, which pow() makes
+// 4 us longer, and the results are the reference form's to the bit (vg_dKdwc_lanes says why that is
+// worth it).  Above, the FP64 units' rate counts, and the table-driven powers take a third of it.
+constexpr size_t kPowCells = 8192;
 static int spread_blocks(size_t n) {
   return (int)std::min<size_t>((n + kSpreadThreads - 1) / kSpreadThreads, (size_t)kNumSMs * 32);
 }
@@ -656,12 +662,16 @@ static int pca_step(frehg_re* re) {
   }
   re->cnt.realloc_sweeps += sweeps;
   // apply reallocation, clampWaterContent, adaptiveTimeStep: in two halves where a block or two per
-  // SM and plane leave the FP64 unit waiting for a chain (100 cells: 18.4 -> 14.3 us)
-  const bool split = (size_t)L.grid.x * L.grid.y * L.planes <= 2 * (size_t)kNumSMs;
+  // SM and plane leave the FP64 unit waiting for a chain (100 cells: 18.4 -> 14.3 us, in the
+  // reference's powers 18.4), and in those powers up to kPowCells
+  const size_t blocks = (size_t)L.grid.x * L.grid.y;
+  const bool split = blocks * L.planes <= 2 * (size_t)kNumSMs;
+  const bool lanes = split && n <= kPowCells;
+  const int shares = lanes ? std::max(1, (int)((4 * re->n + 256 * blocks - 1) / (256 * blocks))) : 1;
   FG_LAUNCH(prof, st, "k_finalize", (25.0 + sb) * n,
-            launch_chained(split ? k_finalize<true> : k_finalize<false>,
-                           dim3(L.grid.x, L.grid.y * (split ? 2 : 1)), L.block, 0, st, a, top_sat,
-                           L.planes, L.tiles));
+            launch_chained(lanes ? k_finalize<2> : (split ? k_finalize<1> : k_finalize<0>),
+                           dim3(L.grid.x, L.grid.y * (split ? 1 + shares : 1)), L.block, 0, st, a,
+                           top_sat, L.planes, L.tiles, shares));
   FG_CUDA(cudaGetLastError());
   if (prof->on) {
     FG_CUDA(cudaStreamSynchronize(st));
@@ -1204,7 +1214,8 @@ int frehg_re_set_initial_head(frehg_re* re, const double* h) {
   FG_CUDA(cudaStreamSynchronize(re->stream));
   FG_CUDA(cudaMemcpy(re->H[re->cur], h, re->n * sizeof(double), cudaMemcpyHostToDevice));
   ReArgs a = make_args(re);
-  k_theta_of_h<<<spread_blocks(re->n), kSpreadThreads, 0, re->stream>>>(a, re->H[re->cur], re->W[re->cur]);
+  auto theta = re->n <= kPowCells ? k_theta_of_h<true> : k_theta_of_h<false>;
+  theta<<<spread_blocks(re->n), kSpreadThreads, 0, re->stream>>>(a, re->H[re->cur], re->W[re->cur]);
   FG_CUDA(cudaGetLastError());
   FG_CUDA(cudaStreamSynchronize(re->stream));
   re->have_state = true;

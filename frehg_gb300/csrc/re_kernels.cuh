@@ -610,65 +610,102 @@ __global__ void __launch_bounds__(kReallocThreads) k_realloc(ReArgs a, int top_s
   if (threadIdx.x == 0) a.sc->sweeps += sweeps;
 }
 
-// Apply the reallocation (ReSolver.cpp:825-833), clampWaterContent (:839-853) and the
-// adaptiveTimeStep Courant bound (:906-910); the last block updates dt (:921-928) and time.
-// Launched on (32 x 8)-column tiles marching through `planes` levels (no index divisions).
-// SPLIT: blocks of even y do the update and those of odd y the Courant bound, whose chains of about 100
-// dependent FP64 instructions each would otherwise follow one another.  Both read what the other does not
-// change: the bound sees the water content before or after the update's clamp, with the same result.
-template <bool SPLIT>
-__global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int planes, int tiles) {
-  grid_begin();
-  const bool update = !SPLIT || !(blockIdx.y & 1), bound = !SPLIT || (blockIdx.y & 1);
-  const int slab = SPLIT ? blockIdx.y >> 1 : blockIdx.y;
-  double dtco = INFINITY;
-  const int t0 = (a.nx + 31) / 32;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-  const int i = (tile % t0) * 32 + threadIdx.x;
-  const int j = (tile / t0) * 8 + threadIdx.y;
-  if (i >= a.nx || j >= a.ny) continue;
-  const size_t col = (size_t)i + (size_t)a.nx * j;
-  const int kb = slab * planes, ke = min(a.nz, kb + planes);
-  for (int k = kb; k < ke; ++k) {
-    const size_t c = col + a.ncol * k;
-    const CellSoil s = soil_of(a.soil, c, col);
-    const uint8_t f = a.flags[c];
-    double wc = a.w_new[c];
-    if (f & F_SAT_OLD) {
-      wc = s.ths;
-    } else {
-      // adjacentToSat with the sequential sweep's view
-      bool adj = (k == 0) ? (top_sat != 0) : (a.flags[c - a.ncol] & F_SAT_NEW) != 0;
-      if (!adj && i > 0) {
-        const uint8_t g = a.flags[c - 1];
-        adj = (g & F_OPEN_XP) && (g & F_SAT_NEW);
-      }
-      if (!adj && j > 0) {
-        const uint8_t g = a.flags[c - a.nx];
-        adj = (g & F_OPEN_YP) && (g & F_SAT_NEW);
-      }
-      if (!adj) adj = (k + 1 < a.nz) ? (a.flags[c + a.ncol] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
-      if (!adj && (f & F_OPEN_XP))
-        adj = (i + 1 < a.nx) ? (a.flags[c + 1] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
-      if (!adj && (f & F_OPEN_YP))
-        adj = (j + 1 < a.ny) ? (a.flags[c + a.nx] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
-      if (!adj) {
-        if (update && wc < 0.9999 * s.ths) a.h_new[c] = vg_head(s, wc);
-      } else {
-        wc = a.wch[c];
-      }
+// The reallocation's result for the water content of one cell (ReSolver.cpp:825-833) and the clamp
+// (clampWaterContent, :839-853); HEAD: a drained cell's head from it.
+template <bool HEAD>
+__device__ __forceinline__ double final_content(const ReArgs& a, const CellSoil& s, int top_sat,
+                                                size_t c, size_t col, int i, int j, int k) {
+  const uint8_t f = a.flags[c];
+  double wc = a.w_new[c];
+  if (f & F_SAT_OLD) {
+    wc = s.ths;
+  } else {
+    // adjacentToSat with the sequential sweep's view
+    bool adj = (k == 0) ? (top_sat != 0) : (a.flags[c - a.ncol] & F_SAT_NEW) != 0;
+    if (!adj && i > 0) {
+      const uint8_t g = a.flags[c - 1];
+      adj = (g & F_OPEN_XP) && (g & F_SAT_NEW);
     }
-    if (wc > s.ths)
-      wc = s.ths;
-    else if (wc < s.thr)
-      wc = s.thr;
-    if (update) a.w_new[c] = wc;
-    if (bound && a.adaptive && k > 0 && wc < s.ths) {
-      const double dk = vg_dKdwc(s, wc, s.Ksz);
-      const double dt_co = a.co_max * a.dz / dk;
-      if (dt_co < dtco) dtco = dt_co;  // std::min(dt_Comin, dt_Co): NaN is skipped
+    if (!adj && j > 0) {
+      const uint8_t g = a.flags[c - a.nx];
+      adj = (g & F_OPEN_YP) && (g & F_SAT_NEW);
+    }
+    if (!adj) adj = (k + 1 < a.nz) ? (a.flags[c + a.ncol] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
+    if (!adj && (f & F_OPEN_XP))
+      adj = (i + 1 < a.nx) ? (a.flags[c + 1] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
+    if (!adj && (f & F_OPEN_YP))
+      adj = (j + 1 < a.ny) ? (a.flags[c + a.nx] & F_SAT_OLD) != 0 : ghost_sat(a, c, col);
+    if (!adj) {
+      if (HEAD && wc < 0.9999 * s.ths) a.h_new[c] = vg_head(s, wc);
+    } else {
+      wc = a.wch[c];
     }
   }
+  if (wc > s.ths)
+    wc = s.ths;
+  else if (wc < s.thr)
+    wc = s.thr;
+  return wc;
+}
+
+// Apply the reallocation and the clamp, and the adaptiveTimeStep Courant bound (:906-910); the last
+// block updates dt (:921-928) and time.  Launched on (32 x 8)-column tiles marching through `planes`
+// levels (no index divisions).
+// FORM 1 and 2: blocks of one y in 1 + `shares` do the update and the others the bound, whose chains of
+// about 100 (FORM 2: 200) dependent FP64 instructions each would otherwise follow one another.  Both
+// read what the other does not change: the bound sees the water content before or after the update's
+// clamp, with the same result.  FORM 2: the bound in the reference's own powers, four lanes per cell
+// (vg_dKdwc_lanes), the cells in order over the bound's warps.
+template <int FORM>
+__global__ void __launch_bounds__(256) k_finalize(ReArgs a, int top_sat, int planes, int tiles,
+                                                  int shares) {
+  grid_begin();
+  const int slab = FORM ? blockIdx.y / (1 + shares) : blockIdx.y;
+  const int share = FORM ? blockIdx.y % (1 + shares) : 0;
+  const bool update = share == 0, bound = !FORM || share > 0;
+  double dtco = INFINITY;
+  auto take = [&](double dk) {
+    const double dt_co = a.co_max * a.dz / dk;
+    if (dt_co < dtco) dtco = dt_co;  // std::min(dt_Comin, dt_Co): NaN is skipped
+  };
+  if (FORM == 2 && bound) {
+    // (a small grid: 32-bit indices)
+    const unsigned n = (unsigned)a.n, ncol = (unsigned)a.ncol, nx = (unsigned)a.nx;
+    const unsigned slabs = gridDim.y / (1 + shares), warps = flat_nthreads() >> 5;
+    const unsigned block = blockIdx.x + gridDim.x * (slab + slabs * (share - 1));
+    const unsigned warp = flat_tid() >> 5, cell = (flat_tid() & 31) >> 2;
+    const unsigned step = gridDim.x * slabs * shares * warps * 8;
+    // (consecutive groups on different blocks: on one SM they share an FP64 unit)
+    for (unsigned c0 = (warp * gridDim.x * slabs * shares + block) * 8; a.adaptive && c0 < n; c0 += step) {
+      const unsigned c = min(c0 + cell, n - 1), col = c % ncol;
+      const int k = (int)(c / ncol), j = (int)(col / nx), i = (int)(col - j * nx);
+      const CellSoil s = soil_of(a.soil, c, col);
+      const double wc = final_content<false>(a, s, top_sat, c, col, i, j, k);
+      const bool need = k > 0 && wc < s.ths;
+      if (!__any_sync(0xffffffffu, need)) continue;
+      const double dk = vg_dKdwc_lanes(s, wc, s.Ksz);
+      if (need) take(dk);
+    }
+  }
+  const int t0 = (a.nx + 31) / 32;
+  for (int tile = blockIdx.x; tile < tiles && (FORM < 2 || update); tile += gridDim.x) {
+    const int i = (tile % t0) * 32 + threadIdx.x;
+    const int j = (tile / t0) * 8 + threadIdx.y;
+    if (i >= a.nx || j >= a.ny) continue;
+    const size_t col = (size_t)i + (size_t)a.nx * j;
+    const int kb = slab * planes, ke = min(a.nz, kb + planes);
+    for (int k = kb; k < ke; ++k) {
+      const size_t c = col + a.ncol * k;
+      const CellSoil s = soil_of(a.soil, c, col);
+      double wc;
+      if (update) {
+        wc = final_content<true>(a, s, top_sat, c, col, i, j, k);
+        a.w_new[c] = wc;
+      } else {
+        wc = final_content<false>(a, s, top_sat, c, col, i, j, k);
+      }
+      if (FORM < 2 && bound && a.adaptive && k > 0 && wc < s.ths) take(vg_dKdwc(s, wc, s.Ksz));
+    }
   }
   // -max(-x) gives the NaN-skipping min
   double m;

@@ -10,14 +10,21 @@
 // with 1/d formed once as PETSc's MatSOR does (a zero diagonal entry taken as 1), the product
 // d y formed as y / (1/d), and the neighbour terms in the reference's column order.
 //
-// Evaluation.  With v = D y the two sweeps need one fused multiply-add per neighbour and cell:
+// Evaluation, larger systems.  With v = D y the two sweeps need one fused multiply-add per
+// neighbour and cell:
 //   v_c = r_c - sum e_m v_m        (m the lower neighbours, e_m = a_m / d_m at the neighbour)
 //   z_c = v_c / d_c - sum e_c z_u  (u the upper neighbours, e_c = a_c / d_c at the cell)
 // with the same e = a / d for both, formed once per solve (a zero diagonal entry taken as 1, as
 // MatSOR does).  This is the same preconditioner as the product / difference / scaling sequence
 // of MatSOR to rounding; on GB300 a warp issues one FP64 instruction per 64 clocks however few of
 // its lanes are active, so the dependent FP64 instructions per cell are what the sweeps cost
-// (three instead of seven, and no division).
+// (three instead of seven, and no division).  A line of cells (a soil column) takes the same form.
+// Evaluation, small systems of several lines.  MatSOR's products, differences and scalings, each
+// rounded and in its order, and the sums in the order of sor_sum: the results are those of the
+// sequential form (a launch per hyperplane) to the bit.  Such a solve ends after tens of iterations
+// within its own rounding noise (3 % of the residual) of the tolerance: with another rounding one
+// solve in four of a 50 x 30 section stopped an iteration earlier or later, 1e-9 in the head.  It
+// costs 5 FP64 instructions a step instead of 2 (50 us an application of that section, 29 before).
 //
 // Schedule.  A cell depends only on its lower (backward: upper) neighbours, so the sequential
 // order is a wavefront.  One warp owns a tile of 32 lines (lines run along the longest axis, the
@@ -33,11 +40,11 @@
 //   larger: one cooperative launch (all tiles' blocks resident) per preconditioner application
 //   and the CG kernels around it, captured as graphs.
 // Measured on GB300, one application (both sweeps): 405,000 cells (90 x 75 x 60) 244 us against
-// 1.1 ms for a launch per hyperplane; 4,096 cells 45 us; a whole solve of a 100-cell column
-// (four applications, three iterations) 59 us, of a 50 x 30 section 93 us, where one block with a
-// barrier and an L2 round trip per hyperplane took 168 and 228 us for each application.  A step
-// costs about 85 clocks per dependent FP64 instruction, a handover to the next tile about 10,000
-// clocks (the tile's skew, a group of steps and the trip through the L2).
+// 1.1 ms for a launch per hyperplane; 4,096 cells 45 us; a whole solve of a 100-cell column (four
+// applications, three iterations) 28 us, of a 50 x 30 section 161 us for 3.2 applications, where
+// one block with a barrier and an L2 round trip per hyperplane took 168 and 228 us for each
+// application.  A step costs about 85 clocks per dependent FP64 instruction, a handover to the next
+// tile about 10,000 clocks (the tile's skew, a group of steps and the trip through the L2).
 #include "internal.h"
 #include "reduce.cuh"
 
@@ -65,6 +72,7 @@ struct SorGeom {
   int nb1, nb2;  // tiles along them
   int steps;     // steps of a full tile
   int axes;      // tile axes of more than one cell (one: the first)
+  int ord[3];    // this geometry's axes in the column order of the reference's rows (forward)
 };
 
 SorGeom sor_geom(const Stencil64& A) {
@@ -85,6 +93,9 @@ SorGeom sor_geom(const Stencil64& A) {
   // 8 x 4 lines; along an axis with fewer than that, as many as it has (rounded up to a power of
   // two), and the others along its partner
   g.axes = (g.n[1] > 1) + (g.n[2] > 1);
+  for (int q = 0; q < 3; ++q)
+    for (int m = 0; m < 3; ++m)
+      if (A.ref_order[q] == ord[m]) g.ord[q] = m;
   g.t2 = 4;
   while (g.t2 > 1 && g.t2 / 2 >= g.n[2]) g.t2 /= 2;
   g.t1 = 32 / g.t2;
@@ -129,9 +140,9 @@ struct SorLane {
   }
 };
 
-// The operands of N consecutive steps of one lane: start value, couplings over d with the
-// neighbours one step back along the line and the two tile axes, the scale of the start value
-// (global form), and the values of neighbouring tiles.
+// The operands of N consecutive steps of one lane: start value, couplings (global form: over d)
+// with the neighbours one step back along the line and the two tile axes, 1 / d, and the values
+// of neighbouring tiles.
 template <int N>
 struct SorSet {
   double a[N], c0[N], c1[N], c2[N], w[N], f1[N], f2[N];
@@ -224,14 +235,33 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
       const int i0 = at(q0 + u);
       double x = P::kGlobal && !FWD ? S.w[u] * S.a[u] : S.a[u];
       // the line's first cell has no coupling back: v is still 0 there
-      x = fma(-S.c0[u], v, x);
-      if (AXES > 0) {
-        const double y = __shfl_sync(0xffffffffu, v, from1);
-        x = fma(-S.c1[u], edge1 ? S.f1[u] : y, x);
-      }
-      if (AXES > 1) {
-        const double y = __shfl_sync(0xffffffffu, v, from2);
-        x = fma(-S.c2[u], edge2 ? S.f2[u] : y, x);
+      if (!P::kGlobal) {
+        // every operation rounded, the neighbours in the column order of the reference's rows
+        const double y1 = AXES > 0 ? __shfl_sync(0xffffffffu, v, from1) : 0.0;
+        const double y2 = AXES > 1 ? __shfl_sync(0xffffffffu, v, from2) : 0.0;
+        const double p0 = __dmul_rn(S.c0[u], v);
+        const double p1 = AXES > 0 ? __dmul_rn(S.c1[u], edge1 ? S.f1[u] : y1) : 0.0;
+        const double p2 = AXES > 1 ? __dmul_rn(S.c2[u], edge2 ? S.f2[u] : y2) : 0.0;
+        if (AXES < 2) {
+          const bool line_first = (g.ord[0] == 0 || (g.ord[1] == 0 && g.ord[0] == 2)) == FWD;
+          x = __dsub_rn(__dsub_rn(x, line_first ? p0 : p1), line_first ? p1 : p0);
+        } else {
+          const int first = FWD ? g.ord[0] : g.ord[2], last = FWD ? g.ord[2] : g.ord[0];
+          x = __dsub_rn(x, first == 0 ? p0 : (first == 1 ? p1 : p2));
+          x = __dsub_rn(x, g.ord[1] == 0 ? p0 : (g.ord[1] == 1 ? p1 : p2));
+          x = __dsub_rn(x, last == 0 ? p0 : (last == 1 ? p1 : p2));
+        }
+        x = __dmul_rn(x, S.w[u]);
+      } else {
+        x = fma(-S.c0[u], v, x);
+        if (AXES > 0) {
+          const double y = __shfl_sync(0xffffffffu, v, from1);
+          x = fma(-S.c1[u], edge1 ? S.f1[u] : y, x);
+        }
+        if (AXES > 1) {
+          const double y = __shfl_sync(0xffffffffu, v, from2);
+          x = fma(-S.c2[u], edge2 ? S.f2[u] : y, x);
+        }
       }
       const bool on = (unsigned)i0 < len_on;
       v = on ? x : v;
@@ -251,18 +281,17 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
   return ok;
 }
 
-// the vectors in shared memory in cell order: src r (forward) or v / d, out v or z, e the couplings
-// over d
+// the vectors in shared memory in cell order: src r (forward) or d y, out y or z, e the couplings
 struct SorShared {
   static constexpr bool kGlobal = false;
   static constexpr int kGroup = 2;  // 8 % faster than 4 on a 100-cell column
-  const double *src, *e0, *e1, *e2;  // e shifted to the neighbour's (forward)
+  const double *src, *invd, *e0, *e1, *e2;  // e shifted to the neighbour's (forward)
   double* out;
   int first, s0, o1, o2;
   __device__ __forceinline__ SorShared(bool fwd, const SorGeom& g, const SorLane& L,
-                                       const double* src_, const double* e0_, const double* e1_,
-                                       const double* e2_, double* out_)
-      : src(src_), e0(e0_), e1(e1_), e2(e2_), out(out_) {
+                                       const double* src_, const double* invd_, const double* e0_,
+                                       const double* e1_, const double* e2_, double* out_)
+      : src(src_), invd(invd_), e0(e0_), e1(e1_), e2(e2_), out(out_) {
     s0 = (int)g.s[0];
     o1 = fwd ? -(int)g.s[1] : (int)g.s[1];
     o2 = fwd ? -(int)g.s[2] : (int)g.s[2];
@@ -272,9 +301,10 @@ struct SorShared {
   }
   template <bool FWD, int AXES>
   __device__ __forceinline__ void load(int, int, int ic, double& a, double& c0, double& c1,
-                                       double& c2, double&) const {
+                                       double& c2, double& w) const {
     const int c = first + s0 * ic;
     a = src[c];
+    w = invd[c];
     c0 = e0[FWD ? c - (ic > 0 ? s0 : 0) : c];
     if (AXES > 0) c1 = e1[c];
     if (AXES > 1) c2 = e2[c];
@@ -653,10 +683,68 @@ struct LineScan {
   }
 };
 
+// y / (1/d), rounded as a division: the product with d and one correction by its exact remainder
+// (Markstein's theorem, IBM J. Res. Dev. 34, 1990).  A division here is a tenth of an application.
+__device__ __forceinline__ double sor_undo(double y, double invd, double d) {
+  const double dc = d == 0.0 ? 1.0 : d, q = y * dc;
+  return fma(fma(-q, invd, y), dc, q);
+}
+
+// Sums of NV values over a block of at most 256 threads, in the order of `nb` such blocks with four
+// cells a thread whose warps add by butterflies: acc[q][b] are thread t's cells t + 256 b +
+// 256 nb k, k = 0, 1, ...  Within a warp the sums of different (q, b) share the butterfly's steps
+// (each step halves the lanes of a sum and the sums of a lane: 9 FP64 instructions for eight sums,
+// not 40); the warps' sums are added by one warp per value.  Valid in every thread; sh[NV * 32].
+constexpr int kSorParts = (kSorSolveCells + 1023) / 1024;
+template <int NV>
+__device__ __forceinline__ void sor_sum(double (&acc)[NV * kSorParts], double (&tot)[NV],
+                                        double* sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = blockDim.x >> 5;
+  constexpr int M = NV * kSorParts;  // 4 or 8
+  int have = M;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+    if (have > 1) {
+      have >>= 1;
+#pragma unroll
+      for (int i = 0; i < M / 2; ++i)
+        if (i < have) {
+          const double mine = up ? acc[i + have] : acc[i], theirs = up ? acc[i] : acc[i + have];
+          acc[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+        }
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    }
+  }
+  // the sum a lane holds: the halves taken, from the highest lane bit
+  constexpr int kShare = 32 / M;
+  const int which = lane / kShare;
+  if (lane % kShare == 0) sh[which * 8 + warp] = acc[0];
+  if (warp == 0)
+    for (int w = warps; w < 8; ++w)
+      if (lane % kShare == 0) sh[which * 8 + w] = 0.0;
+  __syncthreads();
+  if (warp < NV) {
+    double t = sh[warp * 32 + lane];
+    t += __shfl_xor_sync(0xffffffffu, t, 4);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 16);
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+    __syncwarp();
+    if (lane == 0) sh[warp * 32] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) tot[q] = sh[q * 32];
+}
+
 // The whole solve of a small system in one block: the same iteration with every vector that the
-// sweeps or the neighbours read in shared memory (e, 1/d, r, v, z, p), the operator and x in
-// global memory (each thread its own cells).  w = A p lives where v does (v is written by the next
-// sweep).  x_out receives the solution of a converged solve.
+// sweeps or the neighbours read in shared memory (the couplings, of a line over d; 1/d, r, v, z, p),
+// the operator and x in global memory (each thread its own cells).  w = A p lives where v does (v is
+// written by the next sweep).  x_out receives the solution of a converged solve.
 template <int AXES>
 __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     SorGeom g, const double* __restrict__ d, const double* __restrict__ a0,
@@ -668,9 +756,10 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
   __shared__ CgDevState st;
   __shared__ double quot;  // beta / the last beta, by warp 1 while thread 0 tests the norm
   double beta = 0.0;       // (thread 32's)
-  __shared__ double red[128];  // (the vectors of 3,600 cells leave 2 KB)
+  __shared__ double red[64];
   const int n = n0 * n1 * n2, tid = threadIdx.x, warp = tid >> 5;
   const int nt = blockDim.x, warps = nt >> 5;
+  const int parts = (n + 1023) / 1024;  // (one where the block has fewer than 256 threads)
   double *e0 = sor_sh, *e1 = e0 + n, *e2 = e1 + n, *invd = e2 + n, *r = invd + n, *v = r + n,
          *z = v + n, *p = z + n;
   // the couplings in the order of the geometry's axes
@@ -688,9 +777,9 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     const double dc = d[c];
     const double id = 1.0 / (dc == 0.0 ? 1.0 : dc);
     invd[c] = id;
-    e0[c] = a0[c] * id;
-    e1[c] = a1[c] * id;
-    e2[c] = a2[c] * id;
+    e0[c] = AXES ? a0[c] : a0[c] * id;
+    e1[c] = AXES ? a1[c] : a1[c] * id;
+    e2[c] = AXES ? a2[c] : a2[c] * id;
     x[c] = 0.0;
     r[c] = b[c];
     v[c] = sor_wait_value();
@@ -706,27 +795,30 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     if (AXES == 0 && warp == 0) line.forward(r, v);
     for (int t = warp; t < tiles && ok; t += warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
-      ok = sor_tile<true, AXES>(g, L, SorShared(true, g, L, r, g0, g1, g2, v), &st.bar_timeout);
+      ok = sor_tile<true, AXES>(g, L, SorShared(true, g, L, r, invd, g0, g1, g2, v), &st.bar_timeout);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
-    // v / d by all threads: in the sweep it would be one more FP64 instruction per step
-    for (int c = tid; c < n; c += nt) v[c] *= invd[c];
+    // d y (a line: v / d) by all threads: in the sweep it would lengthen the chain
+    for (int c = tid; c < n; c += nt)
+      v[c] = AXES ? sor_undo(v[c], invd[c], d[c]) : v[c] * invd[c];
     __syncthreads();
     if (AXES == 0 && warp == 0) line.backward(v, z);
     for (int t = warp + (tiles - 1 - warp) / warps * warps; warp < tiles && t >= 0 && ok;
          t -= warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
-      ok = sor_tile<false, AXES>(g, L, SorShared(false, g, L, v, g0, g1, g2, z), &st.bar_timeout);
+      ok = sor_tile<false, AXES>(g, L, SorShared(false, g, L, v, invd, g0, g1, g2, z), &st.bar_timeout);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
-    double s[2] = {0.0, 0.0};
-    for (int c = tid; c < n; c += nt) {
-      s[0] = fma(z[c], z[c], s[0]);
-      s[1] = fma(z[c], r[c], s[1]);
-    }
-    block_sum<2, 64>(s, red);
+    double part[2 * kSorParts] = {}, s[2];
+#pragma unroll
+    for (int q = 0; q < kSorParts; ++q)
+      for (int c = tid + q * nt; q < parts && c < n; c += nt * parts) {
+        part[q] = fma(z[c], z[c], part[q]);
+        part[kSorParts + q] = fma(z[c], r[c], part[kSorParts + q]);
+      }
+    sor_sum<2>(part, s, red);
     if (tid == 0) {
       if (st.bar_timeout)
         st.status = kGridBarrierTimeout;
@@ -753,23 +845,25 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     const bool first = st.iter == 0;
     for (int c = tid; c < n; c += nt) p[c] = first ? z[c] : fma(bc, p[c], z[c]);
     __syncthreads();
-    double acc[1] = {0.0};
+    double acc[kSorParts] = {}, pw[1];
     double* w = v;
-    for (int c = tid; c < n; c += nt) {
-      const int i0 = c % n0, q = c / n0, i1 = q % n1, i2 = q / n1;
-      const double pc = p[c];
-      double y = d[c] * pc;
-      if (i0 > 0) y = fma(a0[c - 1], p[c - 1], y);
-      if (i0 + 1 < n0) y = fma(a0[c], p[c + 1], y);
-      if (i1 > 0) y = fma(a1[c - s1], p[c - s1], y);
-      if (i1 + 1 < n1) y = fma(a1[c], p[c + s1], y);
-      if (i2 > 0) y = fma(a2[c - s2], p[c - s2], y);
-      if (i2 + 1 < n2) y = fma(a2[c], p[c + s2], y);
-      w[c] = y;
-      acc[0] = fma(pc, y, acc[0]);
-    }
-    block_sum<1, 64>(acc, red);
-    if (tid == 0) sor_alpha(&st, acc[0]);
+#pragma unroll
+    for (int k = 0; k < kSorParts; ++k)
+      for (int c = tid + k * nt; k < parts && c < n; c += nt * parts) {
+        const int i0 = c % n0, q = c / n0, i1 = q % n1, i2 = q / n1;
+        const double pc = p[c];
+        double y = d[c] * pc;
+        if (i0 > 0) y = fma(a0[c - 1], p[c - 1], y);
+        if (i0 + 1 < n0) y = fma(a0[c], p[c + 1], y);
+        if (i1 > 0) y = fma(a1[c - s1], p[c - s1], y);
+        if (i1 + 1 < n1) y = fma(a1[c], p[c + s1], y);
+        if (i2 > 0) y = fma(a2[c - s2], p[c - s2], y);
+        if (i2 + 1 < n2) y = fma(a2[c], p[c + s2], y);
+        w[c] = y;
+        acc[k] = fma(pc, y, acc[k]);
+      }
+    sor_sum<1>(acc, pw, red);
+    if (tid == 0) sor_alpha(&st, pw[0]);
     __syncthreads();
     if (st.status) break;
     const double a = st.a;

@@ -160,7 +160,7 @@ __device__ __forceinline__ double vg_head(const CellSoil& s, double wc) {
   return log((wc - s.thr) / (s.ths - s.thr)) / 0.1634;
 }
 
-// waterContentFromHead of an initial state: vg_theta with the table-driven powers for the van
+// waterContentFromHead of a large initial state: vg_theta with the table-driven powers for the van
 // Genuchten branch (theta at heads of -1e-4 to -1e3 m: 3.7e-16 of the exact value at most,
 // 6e-17 rms, as with pow(), which took 19.5 ms of FP64 pipe for 56.6M cells; now 8.5).
 __device__ __forceinline__ double vg_theta_initial(const CellSoil& s, double h) {
@@ -349,14 +349,37 @@ __device__ __forceinline__ double vg_dKdwc(const CellSoil& s, double wc, double 
     return (term1 + term2) / (s.ths - s.thr);
   }
   // with q = se^{1/m}, a = 1 - q and term0 = a^m: a^{m-1} = term0 / a and
-  // se^{(2-m)/(2m)} = q se^{-1/2}: two powers instead of five (a chain of about 600 FP64
-  // instructions, which held k_finalize at 31 us on 100 cells; now 18)
+  // se^{(2-m)/(2m)} = q se^{-1/2}: two powers instead of five
   const double q = fpow(se, s.inv_m);
   const double a = 1.0 - q;
   const double term0 = fpow(a, mm);
   const double rs = rsqrt(se);
   const double term1 = 0.5 * Ks * rs * (1.0 - term0) * (1.0 - term0);
   const double term2 = 2.0 * Ks * (q * rs) * (1.0 - term0) * (term0 / a);
+  return (term1 + term2) / (s.ths - s.thr);
+}
+
+// dKdwc of one cell by four lanes, in the reference's own powers: their chain of about 400 FP64
+// instructions is two powers long instead of four (every lane of the warp takes part).  For small
+// grids, where a chain's latency is the kernel's time and the values are worth keeping to the bit: the
+// Courant bound's last bit reaches the system through dt, and a solve whose residual ends near its
+// tolerance (a 50 x 30 section at 24 iterations) then stops one iteration earlier or later, 1e-9 in
+// the head.
+__device__ __forceinline__ double vg_dKdwc_lanes(const CellSoil& s, double wc, double Ks) {
+  if (__any_sync(0xffffffffu, s.use_mvg)) return vg_dKdwc(s, wc, Ks);
+  const int part = threadIdx.x & 3, base = threadIdx.x & 28;
+  double theta = wc;
+  if (theta > 0.9999 * s.ths && theta < s.ths) theta = 0.9999 * s.ths;
+  const double mm = s.m;
+  const double se = (theta - s.thr) / (s.ths - s.thr);
+  const double p = pow(se, part == 1 ? -0.5 : (part == 2 ? (2.0 - mm) / (2.0 * mm) : s.inv_m));
+  const double a = 1.0 - __shfl_sync(0xffffffffu, p, base);
+  const double r = pow(a, part == 1 ? mm - 1.0 : mm);
+  const double term0 = __shfl_sync(0xffffffffu, r, base);
+  const double term1 =
+      0.5 * Ks * __shfl_sync(0xffffffffu, p, base + 1) * (1.0 - term0) * (1.0 - term0);
+  const double term2 = 2.0 * Ks * __shfl_sync(0xffffffffu, p, base + 2) * (1.0 - term0) *
+                       __shfl_sync(0xffffffffu, r, base + 1);
   return (term1 + term2) / (s.ths - s.thr);
 }
 
