@@ -1588,7 +1588,11 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
       if (prof) prof->launches += 3 * chunk;
       return chunk;
     }
-    const int its = rnd == 0 ? std::max(1, std::min(spec, 8)) : 4 << std::min(rnd - 1, 3);
+    // An idle iteration costs 5 to 8 us, another round about 25 (two idle launches, the read-back).
+    // Sweeps that run over their prediction do so by one iteration mostly (2, then more); the few
+    // long ones vary between 1 and 27 from solve to solve, so they go on in eights.
+    const int its = rnd == 0 ? std::max(1, std::min(spec, 8))
+                             : (spec > 8 ? 8 : 2 << std::min(rnd - 1, 2));
     for (int q = 0; q < its; ++q) iteration(st, prof);
     return its;
   };
