@@ -265,7 +265,7 @@ def network_roofline(net, w, stream):
     tf = flops / (ms / 1000.0) / 1e12
     del r, lnk, cap, y
     torch.cuda.empty_cache()
-    return {"bound": "tensor", "kernel": "U-Net forward (k_conv3_tcz / k_conv3_tc: tcgen05.mma "
+    return {"bound": "tensor", "kernel": "U-Net forward (k_conv3_tc: tcgen05.mma "
                                           "BF16, FP32 accumulators in TMEM)",
             "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak,
             "peak_source": kind, "ms_per_application": ms, "flop_per_application": flops}

@@ -106,7 +106,8 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
 
 // Upper bound of the blocks any reduction kernel launches (partials buffers are sized to it).
 constexpr int kMaxRedBlocks = 32768;
-// largest system the FP64 Jacobi-PCG runs as one launch per iteration by default: on GB300 the
+// largest system the FP64 Jacobi-PCG runs as one launch per iteration by default where the whole solve is
+// not one launch (k_cg_solve: larger systems, profiling, a refused cooperative launch): on GB300 the
 // one-launch form is up to 8 % faster up to about 32k unknowns; beyond, its two grid barriers
 // and half occupancy weigh about as much as the three kernels' launch gaps (25 % slower at
 // 262k, 5 % faster at 1M, 6 % slower at 2M and 8.4M unknowns)

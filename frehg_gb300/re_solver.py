@@ -330,7 +330,8 @@ class ReSolver:
 
     def set_fused_iteration(self, on):
         """FP64 Jacobi-PCG solves as one cooperative launch per iteration (True), three kernels
-        (False) or, None (the default), one launch up to 65,536 unknowns (not in reference)."""
+        (False) or, None (the default), one launch for the whole solve up to 622,592 unknowns (not
+        in reference)."""
         v = -1 if on is None else int(bool(on))
         check(self._lib.frehg_re_set_fused_iteration(self._h, v), "setFusedIteration")
 

@@ -120,7 +120,8 @@ typedef struct frehg_solver_config {
   int32_t max_it;         /* default 10000                                                   */
   int32_t precision;      /* 0 = fp64 throughout, 1 = fp32 Krylov under fp64 refinement      */
   double ir_rtol;         /* refinement stop: true relative residual, default 1e-10          */
-  double inner_rtol;      /* fp32 inner solve relative tolerance, default 1e-4               */
+  double inner_rtol;      /* fp32 inner solve relative tolerance, default 1e-4; a sweep aims
+                             lower where that reaches the refinement's own tolerance         */
 } frehg_solver_config;
 
 void frehg_soil_params_default(frehg_soil_params* s);
@@ -283,13 +284,14 @@ int frehg_cg_solve(frehg_cg* cg, frehg_system* sys, const double* b, double* x, 
 int frehg_cg_iteration_count(const frehg_cg* cg, int* its);   /* getIterationCount */
 int frehg_cg_residual_norm(const frehg_cg* cg, double* rnorm); /* getResidualNorm   */
 int frehg_cg_converged_reason(const frehg_cg* cg, int* reason); /* KSPConvergedReason */
-/* Not in reference: the FP64 Jacobi-PCG iteration (precision 0, pc_type "jacobi") as one
- * cooperative launch (direction, stencil product with p.w and update with the norms, separated
- * by grid barriers whose waits are bounded) or as three kernels.  on = 1: one launch wherever
- * the device has cooperative launches; 0: three kernels; -1 (default): one launch for systems
- * of at most 65,536 unknowns, where it is the faster form on GB300, three kernels above.  The
- * two forms sum the dot products over different block partitions, so their last bits (and, in
- * a borderline case, an iteration count) may differ. */
+/* Not in reference: the form of the FP64 Jacobi-PCG (precision 0, pc_type "jacobi").  on = 1: each
+ * iteration one cooperative launch (direction, stencil product with p.w and update with the norms,
+ * separated by grid barriers whose waits are bounded) wherever the device has cooperative
+ * launches; 0: three kernels per iteration; -1 (default): the whole solve one cooperative launch
+ * with its vectors in registers for systems of at most 622,592 unknowns, three kernels above; while
+ * kernels are profiled one by one, one launch per iteration up to 65,536 unknowns and three
+ * kernels above.  The forms sum the dot products over different block partitions, so their last
+ * bits (and, in a borderline case, an iteration count) may differ. */
 int frehg_cg_set_fused_iteration(frehg_cg* cg, int on);
 /* Self-check of the one-launch iteration's grid barrier (not in reference): two cooperative
  * blocks meet at one barrier whose wait is bounded by `polls` polls; skip_block = 0 or 1 makes
