@@ -24,7 +24,7 @@
 // sequential form (a launch per hyperplane) to the bit.  Such a solve ends after tens of iterations
 // within its own rounding noise (3 % of the residual) of the tolerance: with another rounding one
 // solve in four of a 50 x 30 section stopped an iteration earlier or later, 1e-9 in the head.  It
-// costs 5 FP64 instructions a step instead of 2 (50 us an application of that section, 29 before).
+// costs 5 FP64 instructions a step instead of 2 (47 us an application of that section, 29 before).
 //
 // Schedule.  A cell depends only on its lower (backward: upper) neighbours, so the sequential
 // order is a wavefront.  One warp owns a tile of 32 lines (lines run along the longest axis, the
@@ -41,7 +41,7 @@
 //   and the CG kernels around it, captured as graphs.
 // Measured on GB300, one application (both sweeps): 405,000 cells (90 x 75 x 60) 244 us against
 // 1.1 ms for a launch per hyperplane; 4,096 cells 45 us; a whole solve of a 100-cell column (four
-// applications, three iterations) 28 us, of a 50 x 30 section 161 us for 3.2 applications, where
+// applications, three iterations) 28 us, of a 50 x 30 section 150 us for 3.2 applications, where
 // one block with a barrier and an L2 round trip per hyperplane took 168 and 228 us for each
 // application.  A step costs about 85 clocks per dependent FP64 instruction, a handover to the next
 // tile about 10,000 clocks (the tile's skew, a group of steps and the trip through the L2).
@@ -243,8 +243,8 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
         const double p1 = AXES > 0 ? __dmul_rn(S.c1[u], edge1 ? S.f1[u] : y1) : 0.0;
         const double p2 = AXES > 1 ? __dmul_rn(S.c2[u], edge2 ? S.f2[u] : y2) : 0.0;
         if (AXES < 2) {
-          const bool line_first = (g.ord[0] == 0 || (g.ord[1] == 0 && g.ord[0] == 2)) == FWD;
-          x = __dsub_rn(__dsub_rn(x, line_first ? p0 : p1), line_first ? p1 : p0);
+          constexpr bool kLineFirst = P::kLineFirst == FWD;
+          x = __dsub_rn(__dsub_rn(x, kLineFirst ? p0 : p1), kLineFirst ? p1 : p0);
         } else {
           const int first = FWD ? g.ord[0] : g.ord[2], last = FWD ? g.ord[2] : g.ord[0];
           x = __dsub_rn(x, first == 0 ? p0 : (first == 1 ? p1 : p2));
@@ -282,8 +282,9 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
 }
 
 // the vectors in shared memory in cell order: src r (forward) or d y, out y or z, e the couplings
+template <bool LINE_FIRST>
 struct SorShared {
-  static constexpr bool kGlobal = false;
+  static constexpr bool kGlobal = false, kLineFirst = LINE_FIRST;
   static constexpr int kGroup = 2;  // 8 % faster than 4 on a 100-cell column
   const double *src, *invd, *e0, *e1, *e2;  // e shifted to the neighbour's (forward)
   double* out;
@@ -332,7 +333,7 @@ struct SorSlots {
 // The far neighbours' values: forward in the slot array (the last lane of the tile before took
 // the same position t1 - 1 or t2 - 1 steps later), backward in z.
 struct SorGlobal {
-  static constexpr bool kGlobal = true;
+  static constexpr bool kGlobal = true, kLineFirst = true;
   static constexpr int kGroup = 4;  // 2: 20 % slower, the loads' latency shows
   const SorSlots& S;
   const double* r;
@@ -745,7 +746,7 @@ __device__ __forceinline__ void sor_sum(double (&acc)[NV * kSorParts], double (&
 // sweeps or the neighbours read in shared memory (the couplings, of a line over d; 1/d, r, v, z, p),
 // the operator and x in global memory (each thread its own cells).  w = A p lives where v does (v is
 // written by the next sweep).  x_out receives the solution of a converged solve.
-template <int AXES>
+template <int AXES, bool LINE_FIRST = true>
 __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     SorGeom g, const double* __restrict__ d, const double* __restrict__ a0,
     const double* __restrict__ a1, const double* __restrict__ a2, const double* __restrict__ b,
@@ -795,7 +796,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     if (AXES == 0 && warp == 0) line.forward(r, v);
     for (int t = warp; t < tiles && ok; t += warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
-      ok = sor_tile<true, AXES>(g, L, SorShared(true, g, L, r, invd, g0, g1, g2, v), &st.bar_timeout);
+      ok = sor_tile<true, AXES>(g, L, SorShared<LINE_FIRST>(true, g, L, r, invd, g0, g1, g2, v), &st.bar_timeout);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
@@ -807,7 +808,7 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     for (int t = warp + (tiles - 1 - warp) / warps * warps; warp < tiles && t >= 0 && ok;
          t -= warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
-      ok = sor_tile<false, AXES>(g, L, SorShared(false, g, L, v, invd, g0, g1, g2, z), &st.bar_timeout);
+      ok = sor_tile<false, AXES>(g, L, SorShared<LINE_FIRST>(false, g, L, v, invd, g0, g1, g2, z), &st.bar_timeout);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
@@ -956,7 +957,12 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     // no more warps than cells need: each takes part in every sum on the FP64 unit
     const int threads = std::min(kSorSolveThreads, std::max(64, ((int)n + 31) / 32 * 32));
     // on every solve: the attribute belongs to the current device, and the call is cheap
-    auto kernel = g.axes == 2 ? k_sor_solve<2> : (g.axes == 1 ? k_sor_solve<1> : k_sor_solve<0>);
+    // two axes: the order of their terms known to the compiler (161 -> 150 us on a 50 x 30 section:
+    // a selection per term is as long as half an FP64 instruction in the chain)
+    const bool line_first = g.ord[0] == 0 || (g.ord[1] == 0 && g.ord[0] == 2);
+    auto kernel = g.axes == 2   ? k_sor_solve<2>
+                  : g.axes == 1 ? (line_first ? k_sor_solve<1, true> : k_sor_solve<1, false>)
+                                : k_sor_solve<0>;
     FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  8 * kSorSolveCells * (int)sizeof(double)));
     FG_LAUNCH(prof, st, "k_sor_solve", 48.0 * dn,
