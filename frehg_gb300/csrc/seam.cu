@@ -9,6 +9,7 @@
 // arrays use the owned order directly, with axis 0 = k, axis 1 = i, axis 2 = j.
 #include "internal.h"
 
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstring>
@@ -216,7 +217,7 @@ class Placer {
   int place(long row, long col, double v) {
     if (row != at) {
       FG_ARG(row >= 0 && row < n, "row %ld outside [0,%zu)", row, (size_t)n);
-      if (at >= 0 && row == at + 1) {
+      if (row == at + 1) {
         if (++k == n0) {
           k = 0;
           if (++i == n1) {
@@ -250,7 +251,7 @@ class Placer {
  private:
   double *diag, *up0, *dn0, *up1, *dn1, *up2, *dn2;
   long n, n0, n1, n2, s2;
-  long at = -1, k = 0, i = 0, j = 0;
+  long at = LONG_MIN, k = 0, i = 0, j = 0;  // at: the last row, within the system (none: no row's value)
 };
 }  // namespace
 
