@@ -284,7 +284,7 @@ class KrylovSolver {
   float *lkf = nullptr, *dinvf = nullptr, *uf = nullptr, *pf2 = nullptr;
   // PCSOR (pc_type "sor", precision 0): 1/d, the preconditioned residual, the sweeps' operands in
   // the order its warps take them, iteration graph
-  int ensure_sor(size_t n, size_t slots);
+  int ensure_sor(size_t n, size_t slot_doubles);
   size_t cap_sor = 0, cap_slots = 0;
   double *invd = nullptr, *zs = nullptr, *sor_slots = nullptr;
   cudaGraphExec_t gsor = nullptr;

@@ -72,15 +72,35 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
   for (int q = 0; q < NV; ++q) v[q] = sh[q * CAP];
 }
 
+// The same by butterflies in every warp and one over the warps' sums; valid in thread 0.
+template <int NV, int CAP = 256>
+__device__ __forceinline__ void block_sum_butterfly(double (&v)[NV], double* sh) {
+  const int tid = flat_tid(), lane = tid & 31, wid = tid >> 5, nw = flat_nthreads() >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    v[q] = warp_sum(v[q]);
+    if (lane == 0) sh[q * CAP + wid] = v[q];
+  }
+  __syncthreads();
+  if (wid == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = warp_sum(lane < nw ? sh[q * CAP + lane] : 0.0);
+  }
+}
+
 // Grid-wide sum through per-block partials; returns true in every thread of the last block
 // to arrive, where tot[] (valid in thread 0) holds the deterministic grid total.
-template <int NV>
+// BUTTERFLY: the blocks' sums in the order of butterflies.
+template <int NV, bool BUTTERFLY = false>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* partials, unsigned int* arrive,
                          double (&tot)[NV]) {
   __shared__ double sh[NV * 256];
   __shared__ unsigned int ticket;
   const int tid = flat_tid(), bid = flat_bid(), nb = flat_nblocks();
-  block_sum<NV>(v, sh);
+  if (BUTTERFLY)
+    block_sum_butterfly<NV>(v, sh);
+  else
+    block_sum<NV>(v, sh);
   if (tid == 0) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) partials[q * kMaxRedBlocks + bid] = v[q];
@@ -96,7 +116,10 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* partials, unsi
     acc[q] = 0.0;
     for (int b = tid; b < nb; b += flat_nthreads()) acc[q] += __ldcg(&partials[q * kMaxRedBlocks + b]);
   }
-  block_sum<NV>(acc, sh);
+  if (BUTTERFLY)
+    block_sum_butterfly<NV>(acc, sh);
+  else
+    block_sum<NV>(acc, sh);
 #pragma unroll
   for (int q = 0; q < NV; ++q) tot[q] = acc[q];
   if (tid == 0) *arrive = 0u;

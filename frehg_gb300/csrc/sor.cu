@@ -62,6 +62,8 @@ constexpr long kSorPolls = 1L << 22;  // polls of one value before a sweep gives
 // largest system solved in one block: eight shared arrays of FP64 (64 bytes a cell, 227 KB)
 constexpr int kSorSolveCells = 3600;
 constexpr int kSorSolveThreads = 256;
+// threads of a sweeping block
+__host__ __device__ constexpr int sor_sweep_threads(bool rounded) { return rounded ? 128 : 32; }
 
 struct SorGeom {
   // line axis, then the two tile axes: extents and strides
@@ -209,6 +211,7 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
 #pragma unroll
     for (int u = 0; P::kGlobal && u < N; ++u) {
       t ^= __double2loint(S.a[u]) ^ __double2loint(S.c0[u]);
+      if (P::kRounded) t ^= __double2loint(S.w[u]);
       if (AXES > 0) t ^= __double2loint(S.c1[u]);
       if (AXES > 1) t ^= __double2loint(S.c2[u]);
     }
@@ -233,9 +236,9 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
 #pragma unroll
     for (int u = 0; u < N; ++u) {
       const int i0 = at(q0 + u);
-      double x = P::kGlobal && !FWD ? S.w[u] * S.a[u] : S.a[u];
+      double x = !P::kRounded && !FWD ? S.w[u] * S.a[u] : S.a[u];
       // the line's first cell has no coupling back: v is still 0 there
-      if (!P::kGlobal) {
+      if (P::kRounded) {
         // every operation rounded, the neighbours in the column order of the reference's rows
         const double y1 = AXES > 0 ? __shfl_sync(0xffffffffu, v, from1) : 0.0;
         const double y2 = AXES > 1 ? __shfl_sync(0xffffffffu, v, from2) : 0.0;
@@ -284,7 +287,7 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
 // the vectors in shared memory in cell order: src r (forward) or d y, out y or z, e the couplings
 template <bool LINE_FIRST>
 struct SorShared {
-  static constexpr bool kGlobal = false, kLineFirst = LINE_FIRST;
+  static constexpr bool kGlobal = false, kRounded = true, kLineFirst = LINE_FIRST;
   static constexpr int kGroup = 2;  // 8 % faster than 4 on a 100-cell column
   const double *src, *invd, *e0, *e1, *e2;  // e shifted to the neighbour's (forward)
   double* out;
@@ -322,18 +325,21 @@ struct SorShared {
 
 // Larger systems keep the sweeps' operands in the order the warps take them ("slots"):
 // slot = (tile * steps + t) * 32 + lane, so a step's loads are consecutive.
+// ROUNDED: the couplings as they are, not over d.
 struct SorSlots {
   double2* f01;  // forward: couplings over d with the line's previous cell and along tile axis 1
   double* f2;    // and along tile axis 2 (0 where there is no neighbour)
   double2* e01;  // backward, the same
   double2* e2d;  // backward: along tile axis 2, and 1 / d
   double* v;     // forward values
+  double* u;     // ROUNDED: those times d, the backward sweep's right-hand side
 };
 
 // The far neighbours' values: forward in the slot array (the last lane of the tile before took
 // the same position t1 - 1 or t2 - 1 steps later), backward in z.
+template <bool ROUNDED, bool LINE_FIRST>
 struct SorGlobal {
-  static constexpr bool kGlobal = true, kLineFirst = true;
+  static constexpr bool kGlobal = true, kRounded = ROUNDED, kLineFirst = LINE_FIRST;
   static constexpr int kGroup = 4;  // 2: 20 % slower, the loads' latency shows
   const SorSlots& S;
   const double* r;
@@ -363,8 +369,9 @@ struct SorGlobal {
       c0 = f.x;
       c1 = f.y;
       if (AXES > 1) c2 = __ldg(S.f2 + slot);
+      if (ROUNDED) w = __ldg(&S.e2d[slot].y);
     } else {
-      a = S.v[slot];
+      a = ROUNDED ? S.u[slot] : S.v[slot];
       const double2 e = __ldg(S.e01 + slot), d = __ldg(S.e2d + slot);
       c0 = e.x;
       c1 = e.y;
@@ -387,26 +394,51 @@ struct SorGlobal {
   }
 };
 
+// y / (1/d), rounded as a division: the product with d and one correction by its exact remainder
+// (Markstein's theorem, IBM J. Res. Dev. 34, 1990).  A division here is a tenth of an application.
+__device__ __forceinline__ double sor_undo(double y, double invd, double d) {
+  const double dc = d == 0.0 ? 1.0 : d, q = y * dc;
+  return fma(fma(-q, invd, y), dc, q);
+}
+
 // Both sweeps over all tiles, one warp per block, every block resident (cooperative launch).  A
 // block's tiles are in row order forward and in the reverse order backward, so each tile comes
 // after the tiles it reads from wherever they run.
-template <int AXES>
-__global__ void __launch_bounds__(32) k_sor_sweeps(SorGeom g, SorSlots S,
-                                                   const double* __restrict__ r, double* z,
-                                                   CgDevState* st) {
+// ROUNDED: three more warps wait while the first one sweeps; between the sweeps all four form d y
+// of the block's tiles, which in the sweep would lengthen the one warp's instruction stream by half.
+template <int AXES, bool ROUNDED, bool LINE_FIRST>
+__global__ void __launch_bounds__(sor_sweep_threads(ROUNDED))
+    k_sor_sweeps(SorGeom g, SorSlots S, const double* __restrict__ r, const double* __restrict__ d,
+                 const double* __restrict__ invd, double* z, CgDevState* st) {
   if (st->status) return;
+  using Ops = SorGlobal<ROUNDED, LINE_FIRST>;
   const int tiles = g.nb1 * g.nb2;
+  const bool sweeps = threadIdx.x < 32;
   bool ok = true;
   int last = -1;
   for (int b = blockIdx.x; b < tiles && ok; b += gridDim.x) {
     const SorLane L(g, b % g.nb1, b / g.nb1);
-    ok = sor_tile<true, AXES>(g, L, SorGlobal(S, g, L, b, r, z), &st->bar_timeout);
+    if (sweeps) ok = sor_tile<true, AXES>(g, L, Ops(S, g, L, b, r, z), &st->bar_timeout);
     last = b;
   }
+  if (ROUNDED) {
+    __syncthreads();
+    for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
+      const SorLane L(g, b % g.nb1, b / g.nb1);
+      for (int t = threadIdx.x >> 5; t < g.steps; t += sor_sweep_threads(ROUNDED) / 32) {
+        const size_t slot = ((size_t)b * g.steps + t) * 32 + (threadIdx.x & 31);
+        const int i0 = t - L.l1 - L.l2;
+        if (!L.line || i0 < 0 || i0 >= g.n[0]) continue;
+        const size_t c = (size_t)i0 * g.s[0] + (size_t)L.i1 * g.s[1] + (size_t)L.i2 * g.s[2];
+        S.u[slot] = sor_undo(S.v[slot], invd[c], d[c]);
+      }
+    }
+    __syncthreads();
+  }
   __syncwarp();
-  for (int b = last; b >= 0 && ok; b -= gridDim.x) {
+  for (int b = last; sweeps && b >= 0 && ok; b -= gridDim.x) {
     const SorLane L(g, b % g.nb1, b / g.nb1);
-    ok = sor_tile<false, AXES>(g, L, SorGlobal(S, g, L, b, r, z), &st->bar_timeout);
+    ok = sor_tile<false, AXES>(g, L, Ops(S, g, L, b, r, z), &st->bar_timeout);
   }
   if (!ok && threadIdx.x == 0) {
     atomicExch(&st->bar_timeout, 1);
@@ -436,6 +468,7 @@ __global__ void k_sor_prep(const double* __restrict__ d, const double* __restric
 
 // the sweeps' operands in slot order, and v set to "not there yet"; a0, a1, a2 in the order of the
 // geometry's axes
+template <bool ROUNDED>
 __global__ void k_sor_slots(SorGeom g, SorSlots S, const double* __restrict__ a0,
                             const double* __restrict__ a1, const double* __restrict__ a2,
                             const double* __restrict__ invd, size_t slots) {
@@ -453,12 +486,13 @@ __global__ void k_sor_slots(SorGeom g, SorSlots S, const double* __restrict__ a0
     if (i0 >= 0 && i0 < g.n[0] && i1 < g.n[1] && i2 < g.n[2]) {
       const size_t c = (size_t)i0 * g.s[0] + (size_t)i1 * g.s[1] + (size_t)i2 * g.s[2];
       const double id = invd[c];
-      if (i0 > 0) f.x = a0[c - g.s[0]] * invd[c - g.s[0]];
-      if (i1 > 0) f.y = a1[c - g.s[1]] * invd[c - g.s[1]];
-      if (i2 > 0) f2 = a2[c - g.s[2]] * invd[c - g.s[2]];
-      if (i0 + 1 < g.n[0]) h.x = a0[c] * id;
-      if (i1 + 1 < g.n[1]) h.y = a1[c] * id;
-      if (i2 + 1 < g.n[2]) w.x = a2[c] * id;
+      auto over_d = [&](const double* a, size_t m) { return ROUNDED ? a[m] : a[m] * invd[m]; };
+      if (i0 > 0) f.x = over_d(a0, c - g.s[0]);
+      if (i1 > 0) f.y = over_d(a1, c - g.s[1]);
+      if (i2 > 0) f2 = over_d(a2, c - g.s[2]);
+      if (i0 + 1 < g.n[0]) h.x = over_d(a0, c);
+      if (i1 + 1 < g.n[1]) h.y = over_d(a1, c);
+      if (i2 + 1 < g.n[2]) w.x = over_d(a2, c);
       w.y = id;
     }
     S.f01[e] = f;
@@ -532,7 +566,7 @@ __device__ __forceinline__ void sor_alpha(CgDevState* st, double dpi) {
 
 // ||z|| and beta = z.r after a preconditioner application; the last block runs
 // KSPSolve_CG's scalar steps (stopping test, beta ratio) as in the Jacobi path.
-template <bool INIT>
+template <bool INIT, bool ROUNDED>
 __global__ void k_sor_dots(const double* __restrict__ z, const double* __restrict__ r, size_t n,
                            CgDevState* st, double* partials) {
   if (st->status) return;
@@ -544,7 +578,7 @@ __global__ void k_sor_dots(const double* __restrict__ z, const double* __restric
     v[1] = fma(zc, r[c], v[1]);
   }
   double tot[2];
-  if (!grid_sum<2>(v, partials, &st->arrive[3], tot)) return;
+  if (!grid_sum<2, ROUNDED>(v, partials, &st->arrive[3], tot)) return;
   if (flat_tid() == 0) sor_scalars<INIT>(st, tot[0], tot[1]);
 }
 
@@ -560,6 +594,7 @@ __global__ void k_sor_p(const double* __restrict__ z, double* __restrict__ p, si
 }
 
 // w = A p with the diagonal, p.w, alpha = beta / p.w
+template <bool ROUNDED>
 __global__ void __launch_bounds__(256) k_sor_spmv(const double* __restrict__ d,
                                                   const double* __restrict__ a0,
                                                   const double* __restrict__ a1,
@@ -587,7 +622,7 @@ __global__ void __launch_bounds__(256) k_sor_spmv(const double* __restrict__ d,
     acc[0] = fma(pc, v, acc[0]);
   }
   double tot[1];
-  if (!grid_sum<1>(acc, partials, &st->arrive[1], tot)) return;
+  if (!grid_sum<1, ROUNDED>(acc, partials, &st->arrive[1], tot)) return;
   if (flat_tid() == 0) sor_alpha(st, tot[0]);
 }
 
@@ -683,13 +718,6 @@ struct LineScan {
       for (int c = lo; c < hi; ++c) z[c] = fma(pb[c], in, z[c]);
   }
 };
-
-// y / (1/d), rounded as a division: the product with d and one correction by its exact remainder
-// (Markstein's theorem, IBM J. Res. Dev. 34, 1990).  A division here is a tenth of an application.
-__device__ __forceinline__ double sor_undo(double y, double invd, double d) {
-  const double dc = d == 0.0 ? 1.0 : d, q = y * dc;
-  return fma(fma(-q, invd, y), dc, q);
-}
 
 // Sums of NV values over a block of at most 256 threads, in the order of `nb` such blocks with four
 // cells a thread whose warps add by butterflies: acc[q][b] are thread t's cells t + 256 b +
@@ -890,12 +918,12 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
 
 // blocks of a cooperative k_sor_sweeps launch: one per tile, at most what the device holds at once
 // (0: no cooperative launch)
-int sor_sweep_blocks(const SorGeom& g, const void* kernel) {
+int sor_sweep_blocks(const SorGeom& g, const void* kernel, int threads) {
   int dev = 0, coop = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32, 0) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -905,7 +933,7 @@ int sor_sweep_blocks(const SorGeom& g, const void* kernel) {
 
 }  // namespace
 
-int KrylovSolver::ensure_sor(size_t n, size_t slots) {
+int KrylovSolver::ensure_sor(size_t n, size_t slot_doubles) {
   if (n > cap_sor || !invd) {
     cudaFree(invd);
     cudaFree(zs);
@@ -915,12 +943,12 @@ int KrylovSolver::ensure_sor(size_t n, size_t slots) {
     FG_CUDA(cudaMalloc(&zs, n * sizeof(double)));
     cap_sor = n;
   }
-  if (slots > cap_slots || !sor_slots) {
+  if (slot_doubles > cap_slots || !sor_slots) {
     cudaFree(sor_slots);
     sor_slots = nullptr;
     cap_slots = 0;
-    FG_CUDA(cudaMalloc(&sor_slots, slots * 8 * sizeof(double)));
-    cap_slots = slots;
+    FG_CUDA(cudaMalloc(&sor_slots, slot_doubles * sizeof(double)));
+    cap_slots = slot_doubles;
   }
   return FREHG_OK;
 }
@@ -934,6 +962,9 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   const size_t n = A.n;
   const SorGeom g = sor_geom(A);
   const double dn = (double)n;
+  // two axes: the order of their terms known to the compiler (161 -> 150 us on a 50 x 30 section: a
+  // selection per term is as long as half an FP64 instruction in the chain)
+  const bool line_first = g.ord[0] == 0 || (g.ord[1] == 0 && g.ord[0] == 2);
   auto finish = [&]() -> int {
     res->its = hst->its;
     res->reason = hst->status;
@@ -957,9 +988,6 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     // no more warps than cells need: each takes part in every sum on the FP64 unit
     const int threads = std::min(kSorSolveThreads, std::max(64, ((int)n + 31) / 32 * 32));
     // on every solve: the attribute belongs to the current device, and the call is cheap
-    // two axes: the order of their terms known to the compiler (161 -> 150 us on a 50 x 30 section:
-    // a selection per term is as long as half an FP64 instruction in the chain)
-    const bool line_first = g.ord[0] == 0 || (g.ord[1] == 0 && g.ord[0] == 2);
     auto kernel = g.axes == 2   ? k_sor_solve<2>
                   : g.axes == 1 ? (line_first ? k_sor_solve<1, true> : k_sor_solve<1, false>)
                                 : k_sor_solve<0>;
@@ -976,17 +1004,24 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     return finish();
   }
   const size_t slots = (size_t)g.nb1 * g.nb2 * g.steps * 32;
-  FG_TRY(ensure_sor(n, slots));
+  const bool rounded = g.axes == 1;
+  FG_TRY(ensure_sor(n, slots * (rounded ? 9 : 8)));
   SorSlots S;
   S.f01 = reinterpret_cast<double2*>(sor_slots);
   S.e01 = S.f01 + slots;
   S.e2d = S.e01 + slots;
   S.f2 = reinterpret_cast<double*>(S.e2d + slots);
   S.v = S.f2 + slots;
+  S.u = rounded ? S.v + slots : nullptr;
   // one block (all tiles in order, nothing to wait for) where the device refuses cooperative
   // launches
-  auto kernel = g.axes == 2 ? k_sor_sweeps<2> : (g.axes == 1 ? k_sor_sweeps<1> : k_sor_sweeps<0>);
-  const int sweep_blocks = coop_failed ? 1 : std::max(1, sor_sweep_blocks(g, (const void*)kernel));
+  auto kernel = g.axes == 2   ? k_sor_sweeps<2, false, true>
+                : g.axes == 1 ? (line_first ? k_sor_sweeps<1, true, true>
+                                            : k_sor_sweeps<1, true, false>)
+                              : k_sor_sweeps<0, false, true>;
+  const int sweep_threads = sor_sweep_threads(rounded);
+  const int sweep_blocks =
+      coop_failed ? 1 : std::max(1, sor_sweep_blocks(g, (const void*)kernel, sweep_threads));
   CgDevState init;
   memset(&init, 0, sizeof(init));
   init.rtol = cfg.rtol;
@@ -996,26 +1031,31 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   FG_TRY(set_states(dst, init, nullptr, init, st));
   const int nb = reduction_blocks(n, 256, 4);
   double* xs = x;  // the graph keeps fixed pointers; x_out receives a copy
+  auto dots_first = rounded ? k_sor_dots<true, true> : k_sor_dots<true, false>;
+  auto dots = rounded ? k_sor_dots<false, true> : k_sor_dots<false, false>;
+  auto spmv = rounded ? k_sor_spmv<true> : k_sor_spmv<false>;
   auto sweeps = [&](cudaStream_t s) -> cudaError_t {
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)sweep_blocks);
-    lc.blockDim = dim3(32);
+    lc.blockDim = dim3((unsigned)sweep_threads);
     lc.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     lc.attrs = at;
     lc.numAttrs = sweep_blocks > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&lc, kernel, g, S, (const double*)r, zs, dst);
+    return cudaLaunchKernelEx(&lc, kernel, g, S, (const double*)r, (const double*)A.s,
+                              (const double*)invd, zs, dst);
   };
   FG_LAUNCH(prof, st, "k_sor_prep", 48.0 * dn,
             launch_chained(k_sor_prep, nb, 256, 0, st, A.s, A.b, invd, xs, r, zs, n));
   const double* ax[3] = {A.a0, A.a1, A.a2};
   FG_LAUNCH(prof, st, "k_sor_slots", 32.0 * dn + 64.0 * (double)slots,
-            launch_chained(k_sor_slots, reduction_blocks(slots, 256, 1), 256, 0, st, g, S,
-                           ax[g.ax[0]], ax[g.ax[1]], ax[g.ax[2]], invd, slots));
+            launch_chained(rounded ? k_sor_slots<true> : k_sor_slots<false>,
+                           reduction_blocks(slots, 256, 1), 256, 0, st, g, S, ax[g.ax[0]], ax[g.ax[1]],
+                           ax[g.ax[2]], invd, slots));
   cudaError_t le = cudaSuccess;
-  FG_LAUNCH(prof, st, "k_sor_sweeps", 16.0 * dn + 72.0 * (double)slots, le = sweeps(st));
+  FG_LAUNCH(prof, st, "k_sor_sweeps", 16.0 * dn + (rounded ? 96.0 : 72.0) * (double)slots, le = sweeps(st));
   if (le != cudaSuccess && sweep_blocks > 1) {
     cudaGetLastError();
     coop_failed = true;
@@ -1023,20 +1063,20 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   }
   FG_CUDA(le);
   FG_LAUNCH(prof, st, "k_sor_dots", 16.0 * dn,
-            k_sor_dots<true><<<nb, 256, 0, st>>>(zs, r, n, dst, partials));
+            dots_first<<<nb, 256, 0, st>>>(zs, r, n, dst, partials));
   FG_CUDA(cudaGetLastError());
 
   // one iteration: p, w = A p (alpha), x/r update, z = M r, norms and beta
   auto iteration = [&](cudaStream_t s, Profiler* pr) -> int {
     FG_LAUNCH(pr, s, "k_sor_p", 24.0 * dn, k_sor_p<<<nb, 256, 0, s>>>(zs, p, n, dst));
     FG_LAUNCH(pr, s, "k_sor_spmv", 48.0 * dn,
-              k_sor_spmv<<<nb, 256, 0, s>>>(A.s, A.a0, A.a1, A.a2, p, w, A.n0, A.n1, A.n2, dst,
+              spmv<<<nb, 256, 0, s>>>(A.s, A.a0, A.a1, A.a2, p, w, A.n0, A.n1, A.n2, dst,
                                             partials));
     FG_LAUNCH(pr, s, "k_sor_update", 56.0 * dn + 8.0 * (double)slots,
               k_sor_update<<<nb, 256, 0, s>>>(xs, r, p, w, S.v, slots, zs, n, dst));
-    FG_LAUNCH(pr, s, "k_sor_sweeps", 16.0 * dn + 72.0 * (double)slots, FG_CUDA(sweeps(s)));
+    FG_LAUNCH(pr, s, "k_sor_sweeps", 16.0 * dn + (rounded ? 96.0 : 72.0) * (double)slots, FG_CUDA(sweeps(s)));
     FG_LAUNCH(pr, s, "k_sor_dots", 16.0 * dn,
-              k_sor_dots<false><<<nb, 256, 0, s>>>(zs, r, n, dst, partials));
+              dots<<<nb, 256, 0, s>>>(zs, r, n, dst, partials));
     return FREHG_OK;
   };
   // iterations between two reads of the status: few, as a solve takes from 1 to a few tens of
