@@ -87,7 +87,9 @@ class Profiler {
 // grid_begin() (reduce.cuh) before it touches memory, which waits for that kernel's end and lets the
 // next such launch be placed in turn.  The steps of small grids are chains of kernels of 5 to 15 us,
 // of which the launches took a tenth (Picard steps of 40 x 40 x 100 12.1 -> 10.6 ms).  Only for
-// kernels that begin so.
+// kernels that begin so, and whose pointer parameters are plain: such a kernel's life overlaps that of
+// the kernels that write what it reads, so that __restrict__, which would let the compiler read
+// through the non-coherent path or ahead of the wait, would promise what is not so.
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                                   cudaStream_t st, A... args) {

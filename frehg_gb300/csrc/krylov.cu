@@ -73,8 +73,7 @@ StencilLaunch stencil_launch(int n0, int n1, int n2) {
 }
 
 namespace {
-__global__ void k_fetch_words(const unsigned* __restrict__ src, unsigned* __restrict__ dst,
-                              int words) {
+__global__ void k_fetch_words(const unsigned* src, unsigned* dst, int words) {
   grid_begin();
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
 }
@@ -95,9 +94,8 @@ int fetch_small(void* host_mapped, const void* dev, size_t bytes, cudaStream_t s
 }
 
 namespace {
-__global__ void k_fetch_words2(const unsigned* __restrict__ src, unsigned* __restrict__ dst,
-                               const unsigned* __restrict__ src2, unsigned* __restrict__ dst2,
-                               int words) {
+__global__ void k_fetch_words2(const unsigned* src, unsigned* dst, const unsigned* src2,
+                               unsigned* dst2, int words) {
   grid_begin();
   for (int i = threadIdx.x; i < words; i += blockDim.x) {
     dst[i] = src[i];
@@ -142,7 +140,7 @@ int reduction_blocks(size_t n, int threads, int per_thread) {
 // ------------------------------------------------------------------------------------------
 // operator scaling
 
-__global__ void k_diag_rsqrt(double* __restrict__ s, size_t n) {
+__global__ void k_diag_rsqrt(double* s, size_t n) {
   grid_begin();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
@@ -152,9 +150,8 @@ __global__ void k_diag_rsqrt(double* __restrict__ s, size_t n) {
   }
 }
 
-__global__ void k_scale_offdiag(double* __restrict__ a0, double* __restrict__ a1,
-                                double* __restrict__ a2, const double* __restrict__ s, int n0,
-                                int n1, int n2, int planes, int tiles) {
+__global__ void k_scale_offdiag(double* a0, double* a1, double* a2, const double* s, int n0, int n1,
+                                int n2, int planes, int tiles) {
   grid_begin();
   const int t0 = (n0 + 31) / 32;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -178,8 +175,7 @@ __global__ void k_scale_offdiag(double* __restrict__ a0, double* __restrict__ a1
 // FP64 CG kernels
 
 // r~ = s b, x~ = 0; ||B b|| and beta = r~.r~; iteration-0 stopping test.
-__global__ void k_cg_init(const double* __restrict__ s, const double* __restrict__ b,
-                          double* __restrict__ x, double* __restrict__ r, size_t n,
+__global__ void k_cg_init(const double* s, const double* b, double* x, double* r, size_t n,
                           CgDevState* st, double* partials) {
   grid_begin();
   double v[2] = {0.0, 0.0};
@@ -854,8 +850,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
   }
 }
 
-__global__ void k_unscale(const double* __restrict__ s, const double* __restrict__ xs,
-                          double* __restrict__ x, size_t n) {
+__global__ void k_unscale(const double* s, const double* xs, double* x, size_t n) {
   grid_begin();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x)

@@ -129,10 +129,8 @@ __device__ __forceinline__ void line_step_tail(CgDevState* st, double rzn, doubl
 // warps: 8 with twice the levels fit fewer blocks (573 us), 32 lengthen the carry's chain (610).
 template <bool FIRST, int W, int L>
 __global__ void __launch_bounds__(32 * W, L > 8 ? 1 : 2) k32_line_step(
-    float* __restrict__ x, float* __restrict__ r, const float* __restrict__ p0,
-    const float* __restrict__ p1, const float* __restrict__ w, const float* __restrict__ lk,
-    const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
-    double* partials) {
+    float* x, float* r, const float* p0, const float* p1, const float* w, const float* lk,
+    const float* dinv, float* z, int ncol, int nz, CgDevState* st, double* partials) {
   grid_begin();
   if (st->status || (FIRST && !st->fresh)) return;
   __shared__ float2 fwd[W][32], bwd[W][32];
@@ -268,10 +266,8 @@ __global__ void __launch_bounds__(32 * W, L > 8 ? 1 : 2) k32_line_step(
 // hold (256 levels): the forward sweep leaves u in z, the backward sweep overwrites it.
 template <bool FIRST>
 __global__ void __launch_bounds__(128) k32_line_step_long(
-    float* __restrict__ x, float* __restrict__ r, const float* __restrict__ p0,
-    const float* __restrict__ p1, const float* __restrict__ w, const float* __restrict__ lk,
-    const float* __restrict__ dinv, float* __restrict__ z, int ncol, int nz, CgDevState* st,
-    double* partials) {
+    float* x, float* r, const float* p0, const float* p1, const float* w, const float* lk,
+    const float* dinv, float* z, int ncol, int nz, CgDevState* st, double* partials) {
   grid_begin();
   if (st->status || (FIRST && !st->fresh)) return;
   const float a = FIRST ? 0.0f : (float)st->a;

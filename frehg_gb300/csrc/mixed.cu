@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256) k32_spmv(const float* __restrict__ a0,
 // Vectorised variant for n0 % 4 == 0: a thread owns 4 consecutive cells along axis 0 (16-byte
 // loads of p and the couplings); the axis-0 neighbours across threads come from warp shuffles,
 // the axis-2 neighbours roll in registers while the thread marches through its planes.
-__device__ __forceinline__ float4 ld4(const float* __restrict__ a, size_t c) {
+__device__ __forceinline__ float4 ld4(const float* a, size_t c) {
   return *reinterpret_cast<const float4*>(a + c);
 }
 
@@ -415,9 +415,9 @@ __global__ void __launch_bounds__(128) k32_spmv_v4(const float* __restrict__ a0,
 constexpr int kDirRows = 4;
 template <bool FIRST>
 __device__ __forceinline__ void dir_spmv_rows(
-    const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
-    const float* __restrict__ z, const float* __restrict__ po, float* __restrict__ pn,
-    float* __restrict__ w, float bc, int n0, int n1, int n2, int planes, int tiles, Kahan32& acc) {
+    const float* a0, const float* a1, const float* a2, const float* z, const float* po,
+    float* __restrict__ pn, float* __restrict__ w, float bc, int n0, int n1, int n2, int planes,
+    int tiles, Kahan32& acc) {
   constexpr int R = kDirRows;
   auto dir = [&](size_t c) { return FIRST ? z[c] : fmaf(bc, po[c], z[c]); };
   const int t0 = (n0 + 31) / 32, lane = threadIdx.x;
@@ -490,10 +490,8 @@ __device__ __forceinline__ void dir_spmv_rows(
 }
 
 __global__ void __launch_bounds__(128) k32_dir_spmv(
-    const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
-    const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
-    float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
-    double* partials) {
+    const float* a0, const float* a1, const float* a2, const float* z, float* p0, float* p1,
+    float* w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st, double* partials) {
   grid_begin();
   if (st->status) return;
   const bool odd = st->iter & 1;
@@ -512,16 +510,14 @@ __global__ void __launch_bounds__(128) k32_dir_spmv(
 
 // n0 a multiple of 4: four cells per thread, 16-byte accesses
 __global__ void __launch_bounds__(128) k32_dir_spmv_v4(
-    const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,
-    const float* __restrict__ z, float* __restrict__ p0, float* __restrict__ p1,
-    float* __restrict__ w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st,
-    double* partials) {
+    const float* a0, const float* a1, const float* a2, const float* z, float* p0, float* p1,
+    float* w, int n0, int n1, int n2, int planes, int tiles, CgDevState* st, double* partials) {
   grid_begin();
   if (st->status) return;
   const bool first = st->iter == 0, odd = st->iter & 1;
   const float bc = first ? 0.0f : (float)st->bcoef;
-  const float* __restrict__ po = odd ? p1 : p0;
-  float* __restrict__ pn = odd ? p0 : p1;
+  const float* po = odd ? p1 : p0;
+  float* pn = odd ? p0 : p1;
   auto dir4 = [&](size_t c) {
     float4 v = ld4(z, c);
     if (!first) {
@@ -743,8 +739,8 @@ __global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e,
 // change that x~ really made, fl(x~ + 2^k e) - x~, so that the updated residual is that of the
 // stored x~.  That change is a float: a multiple of ulp(x~) no longer than e's own 24 bits.  The
 // first sweep's x~ = 2^k e is exact and written by k_ir_sweep.
-__global__ void k_ir_update_exact(double* __restrict__ x, float* __restrict__ e, size_t n,
-                                  const CgDevState* ir, const CgDevState* in) {
+__global__ void k_ir_update_exact(double* x, float* e, size_t n, const CgDevState* ir,
+                                  const CgDevState* in) {
   grid_begin();
   if (ir->status || in->status == 0 || ir->ir_its == 0 || in->iter == 0) return;
   const int scale = pow2_above(ir->rscale) - 1;  // rscale = 2^scale
@@ -1204,9 +1200,8 @@ __device__ __forceinline__ void prep_tail(CgDevState* ir, CgDevState* in, const 
 }
 
 __global__ void __launch_bounds__(128) k_prep_ff(
-    PrepOut o, const float* __restrict__ dg, const double* __restrict__ b,
-    float* __restrict__ lk, float* __restrict__ dinv, int n0, int n1, int n2, int line,
-    CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
+    PrepOut o, const float* dg, const double* b, float* lk, float* dinv, int n0, int n1, int n2,
+    int line, CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
     double inner_rtol) {
   grid_begin();
   const int ncol = n0 * n1;
@@ -1268,9 +1263,8 @@ constexpr int kPrepWarps = 8;
 constexpr int kPrepLevels = 190;         // 48 KB of scaled couplings beside the sums' 4 KB
 constexpr int kPrepSplitGroups = 2048;   // 65,536 columns: above, the march is the faster
 __global__ void __launch_bounds__(32 * kPrepWarps) k_prep_ff_split(
-    PrepOut o, const float* __restrict__ dg, const double* __restrict__ b,
-    float* __restrict__ lk, float* __restrict__ dinv, int n0, int n1, int n2, int line,
-    CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
+    PrepOut o, const float* dg, const double* b, float* lk, float* dinv, int n0, int n1, int n2,
+    int line, CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
     double inner_rtol) {
   grid_begin();
   extern __shared__ float2 prep_sh[];  // [n2][32]

@@ -128,11 +128,8 @@ __device__ __forceinline__ PicRow pic_row(const ReArgs& a, const CellSoil& s, si
 // its column and carries the face below a level to the next level as that level's face above,
 // and takes a cell's -x face from the lane to its left (warp shuffle; lane 0 evaluates its own).
 // Launched on (32 x 8)-column tiles marching through `planes` levels: a warp is one tile row.
-__global__ void __launch_bounds__(256) k_pic_assemble(ReArgs a, double* __restrict__ dg,
-                                                      double* __restrict__ a0,
-                                                      double* __restrict__ a1,
-                                                      double* __restrict__ a2,
-                                                      double* __restrict__ bvec, int planes,
+__global__ void __launch_bounds__(256) k_pic_assemble(ReArgs a, double* dg, double* a0, double* a1,
+                                                      double* a2, double* bvec, int planes,
                                                       int tiles) {
   grid_begin();
   const double dt = a.sc->dt_used;
@@ -283,8 +280,7 @@ __device__ __forceinline__ double pic_limited(double dc, long long lim_bits, lon
 }
 
 template <bool SCALED = false>
-__global__ void k_pic_update(ReArgs a, const double* __restrict__ d,
-                             const double* __restrict__ s = nullptr) {
+__global__ void k_pic_update(ReArgs a, const double* d, const double* s = nullptr) {
   grid_begin();
   const long long kAbs = 0x7fffffffffffffffll;
   long long m = 0;

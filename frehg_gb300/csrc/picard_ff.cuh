@@ -184,9 +184,9 @@ __device__ __forceinline__ void ff_bottom_face(const ReArgs& a, const FfConst& K
 // the current ones still hold the values at the previous head, which the final update of a
 // converged step uses).  Same bits as the two kernels; one read of the head instead of two.
 template <bool ALL_FF>
-__global__ void __launch_bounds__(256, 4) k_pic_update_constit_ff(
-    ReArgs a, const double* __restrict__ d, const double* __restrict__ s,
-    double* __restrict__ kr, double* __restrict__ th, double* __restrict__ cap) {
+__global__ void __launch_bounds__(256, 4) k_pic_update_constit_ff(ReArgs a, const double* d,
+                                                                  const double* s, double* kr,
+                                                                  double* th, double* cap) {
   grid_begin();
   const long long kAbs = 0x7fffffffffffffffll;
   long long m = 0;
@@ -258,12 +258,8 @@ struct FfYPlane {
 // T: the type of the diagonal and couplings written (FP32 values either way; float when the
 // mixed-precision solve's preparation reads them, which halves their traffic).
 template <bool ISO, bool FINAL = false, typename T = double>
-__global__ void __launch_bounds__(256, 4) k_pic_assemble_ff(ReArgs a, T* __restrict__ dg,
-                                                           T* __restrict__ a0,
-                                                           T* __restrict__ a1,
-                                                           T* __restrict__ a2,
-                                                           double* __restrict__ bvec, int planes,
-                                                           int tiles) {
+__global__ void __launch_bounds__(256, 4) k_pic_assemble_ff(ReArgs a, T* dg, T* a0, T* a1, T* a2,
+                                                            double* bvec, int planes, int tiles) {
   grid_begin();
   __shared__ FfYPlane ys[2];
   // the launch's constants in shared memory rather than in 20 registers per thread

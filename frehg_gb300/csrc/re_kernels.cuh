@@ -154,8 +154,7 @@ __global__ void k_step_begin(ReScalars* sc) {
 
 // kr (and optionally theta and C) at the given head, from one set of transcendentals
 template <bool THETA, bool CAP>
-__global__ void k_constit(ReArgs a, const double* __restrict__ h, double* __restrict__ kr,
-                          double* __restrict__ th, double* __restrict__ cap,
+__global__ void k_constit(ReArgs a, const double* h, double* kr, double* th, double* cap,
                           ReScalars* begin = nullptr) {
   grid_begin();
   if (begin && blockIdx.x == 0 && threadIdx.x == 0) begin->dt_used = begin->dt;
@@ -179,10 +178,8 @@ __global__ void k_constit(ReArgs a, const double* __restrict__ h, double* __rest
 // (vg_constit_ff); MVG and exponential classes take the FP64 forms.  ALL_FF: every class is
 // van Genuchten (not MVG), and the FP64 forms are not compiled in.
 template <bool THETA, bool CAP, bool ALL_FF>
-__global__ void __launch_bounds__(256, 4) k_constit_ff(ReArgs a, const double* __restrict__ h,
-                                                       double* __restrict__ kr,
-                                                       double* __restrict__ th,
-                                                       double* __restrict__ cap) {
+__global__ void __launch_bounds__(256, 4) k_constit_ff(ReArgs a, const double* h, double* kr,
+                                                       double* th, double* cap) {
   grid_begin();
   const bool col_map = a.soil.cid && !a.soil.cid3d;
   const bool small = a.n <= 0xffffffffull;
@@ -210,11 +207,8 @@ __global__ void __launch_bounds__(256, 4) k_constit_ff(ReArgs a, const double* _
 
 // groundwaterMatCoeff + groundwaterRhs + the COO rows of assembleAndSolve, written as the
 // diagonal (into A.s), the +x/+y/+z couplings and b.
-__global__ void __launch_bounds__(256) k_assemble(ReArgs a, double* __restrict__ dg,
-                                                  double* __restrict__ a0, double* __restrict__ a1,
-                                                  double* __restrict__ a2,
-                                                  double* __restrict__ bvec, int planes,
-                                                  int tiles) {
+__global__ void __launch_bounds__(256) k_assemble(ReArgs a, double* dg, double* a0, double* a1,
+                                                  double* a2, double* bvec, int planes, int tiles) {
   grid_begin();
   const int t0 = (a.nx + 31) / 32;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {

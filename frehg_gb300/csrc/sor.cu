@@ -452,9 +452,8 @@ __device__ __forceinline__ double sor_wait_value() {
 
 // 1/d (a zero diagonal entry replaced by 1, MatSOR / PCJacobi), x = 0, r = b, and z set to "not
 // there yet"
-__global__ void k_sor_prep(const double* __restrict__ d, const double* __restrict__ b,
-                           double* __restrict__ invd, double* __restrict__ x,
-                           double* __restrict__ r, double* __restrict__ z, size_t n) {
+__global__ void k_sor_prep(const double* d, const double* b, double* invd, double* x, double* r,
+                           double* z, size_t n) {
   grid_begin();
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
@@ -469,9 +468,8 @@ __global__ void k_sor_prep(const double* __restrict__ d, const double* __restric
 // the sweeps' operands in slot order, and v set to "not there yet"; a0, a1, a2 in the order of the
 // geometry's axes
 template <bool ROUNDED>
-__global__ void k_sor_slots(SorGeom g, SorSlots S, const double* __restrict__ a0,
-                            const double* __restrict__ a1, const double* __restrict__ a2,
-                            const double* __restrict__ invd, size_t slots) {
+__global__ void k_sor_slots(SorGeom g, SorSlots S, const double* a0, const double* a1,
+                            const double* a2, const double* invd, size_t slots) {
   grid_begin();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < slots;
        e += (size_t)gridDim.x * blockDim.x) {
@@ -776,10 +774,9 @@ __device__ __forceinline__ void sor_sum(double (&acc)[NV * kSorParts], double (&
 // written by the next sweep).  x_out receives the solution of a converged solve.
 template <int AXES, bool LINE_FIRST = true>
 __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
-    SorGeom g, const double* __restrict__ d, const double* __restrict__ a0,
-    const double* __restrict__ a1, const double* __restrict__ a2, const double* __restrict__ b,
-    double* __restrict__ x, double* __restrict__ x_out, int n0, int n1, int n2, double rtol,
-    double atol, double divtol, int max_it, CgDevState* dst) {
+    SorGeom g, const double* d, const double* a0, const double* a1, const double* a2,
+    const double* b, double* x, double* x_out, int n0, int n1, int n2, double rtol, double atol,
+    double divtol, int max_it, CgDevState* dst) {
   grid_begin();
   extern __shared__ double sor_sh[];
   __shared__ CgDevState st;
@@ -809,11 +806,11 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     e0[c] = AXES ? a0[c] : a0[c] * id;
     e1[c] = AXES ? a1[c] : a1[c] * id;
     e2[c] = AXES ? a2[c] : a2[c] * id;
-    x[c] = 0.0;
     r[c] = b[c];
     v[c] = sor_wait_value();
     z[c] = sor_wait_value();
   }
+  for (int c = tid; c < n; c += nt) x[c] = 0.0;
   __syncthreads();
   const int tiles = AXES == 0 ? 0 : g.nb1 * g.nb2;
   // one line: its sweeps by warp 0, the products in the arrays of the axes without couplings
