@@ -61,6 +61,8 @@ struct frehg_re {
   bool constit_fresh = false;
   ReScalars* sc = nullptr;
   ReScalars* sc_host = nullptr;
+  int* unsettled = nullptr;    // (mapped) sweeps after which k_realloc gave up, 0: it did not
+  long realloc_limit = -1;     // sweeps of a reallocation before it gives up; -1: more than can be
   double* partials = nullptr;
   double* xch = nullptr;  // surface-exchange staging (eta, bottom, q, total), on first use
   double* gh_top = nullptr;    // top-layer ghost copies (h then wc) from before an exchange
@@ -118,6 +120,7 @@ frehg_re::~frehg_re() {
   cudaFree(scratch);
   cudaFree(sc);
   cudaFreeHost(sc_host);
+  cudaFreeHost(unsettled);
   cudaFree(partials);
   cudaFree(cls);
   cudaFree(cid);
@@ -590,6 +593,16 @@ static double soil_bytes(const frehg_re* re) {
   return (re->fKs ? 8.0 : 0.0) + (re->falpha ? 8.0 : 0.0) + (re->cid && re->cid3d ? 1.0 : 0.0);
 }
 
+// Behind a synchronisation of the handle's stream: the error of a one-block reallocation that did not
+// settle (whose step has returned).
+static int realloc_settled(const frehg_re* re) {
+  const int sweeps = *static_cast<volatile int*>(re->unsettled);
+  if (sweeps == 0) return FREHG_OK;
+  *re->unsettled = 0;
+  set_error("reallocation relaxation did not settle after %d sweeps", sweeps);
+  return FREHG_ERR_STATE;
+}
+
 // ------------------------------------------------------------------------------------------
 // PCA step (ReSolver::advanceStep, ReSolver.cpp:931-969)
 
@@ -621,6 +634,7 @@ static int pca_step(frehg_re* re) {
   re->cnt.ksp_iterations += res.its;
   re->cnt.ir_sweeps += res.ir_its;
   if (rc != FREHG_OK) return rc;
+  FG_TRY(realloc_settled(re));  // of the step before (the solve has synchronised)
   // enforceHeadBc + computeKFace + updateDiagnostics at h^{n+1} (the solve wrote h^{n+1})
   FG_LAUNCH(prof, st, "k_post", (24.0 + sb) * n,
             launch_chained(k_post, spread_blocks(re->n), kSpreadThreads, 0, st, a));
@@ -632,7 +646,7 @@ static int pca_step(frehg_re* re) {
   // reallocateWaterContent: relax to the sequential sweep's fixed point
   const int top_sat = (re->p.bc_type[5] == 1 && re->p.htop >= 0.0) ? 1 : 0;
   const int cb = (int)((re->ncol + 127) / 128);
-  const int max_sweeps = (int)re->n + 2;
+  const long max_sweeps = re->realloc_limit >= 0 ? re->realloc_limit : (long)re->n + 2;
   int sweeps = 0;
   if (re->ncol <= kReallocCols && re->n <= kReallocCells) {
     const size_t flags = (re->n + 15) & ~(size_t)15;
@@ -640,8 +654,11 @@ static int pca_step(frehg_re* re) {
     if (flags > 40 * 1024)
       FG_CUDA(cudaFuncSetAttribute(k_realloc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kReallocCells));
+    void* unsettled = nullptr;
+    FG_CUDA(cudaHostGetDevicePointer(&unsettled, re->unsettled, 0));
     FG_LAUNCH(prof, st, "k_realloc", 2.0 * n,
-              launch_chained(k_realloc, 1, kReallocThreads, flags, st, a, top_sat));
+              launch_chained(k_realloc, 1, kReallocThreads, flags, st, a, top_sat, max_sweeps,
+                             static_cast<int*>(unsettled)));
     FG_CUDA(cudaGetLastError());
   } else for (;;) {
     FG_CUDA(cudaMemsetAsync(&re->sc->changed, 0, sizeof(int), st));
@@ -765,7 +782,7 @@ static int launch_staged_assembly(frehg_re* re, const ReArgs& a, const StencilLa
 static int read_scalars(const frehg_re* re) {
   FG_TRY(fetch_small(re->sc_host, re->sc, sizeof(ReScalars), re->stream));
   FG_CUDA(cudaStreamSynchronize(re->stream));
-  return FREHG_OK;
+  return realloc_settled(re);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1059,8 +1076,10 @@ int frehg_re_create(int nx, int ny, int nz, const frehg_re_params* p, frehg_re**
   ALLOC(re->sc, sizeof(ReScalars));
   ALLOC(re->partials, 4 * kMaxRedBlocks * sizeof(double));
 #undef ALLOC
-  if (alloc_mapped(reinterpret_cast<void**>(&re->sc_host), sizeof(ReScalars)) != FREHG_OK)
+  if (alloc_mapped(reinterpret_cast<void**>(&re->sc_host), sizeof(ReScalars)) != FREHG_OK ||
+      alloc_mapped(reinterpret_cast<void**>(&re->unsettled), sizeof(int)) != FREHG_OK)
     return fail(FREHG_ERR_CUDA);
+  *re->unsettled = 0;
   if (re->A.alloc(nx, ny, nz) != FREHG_OK) return fail(FREHG_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&re->own_stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(FREHG_ERR_CUDA);
@@ -1300,6 +1319,18 @@ int frehg_re_advance_steps(frehg_re* re, int nsteps) {
 }
 
 
+int frehg_re_check_realloc_limit(frehg_re* re, int max_sweeps, int* status) {
+  clear_error();
+  FG_ARG(re && status && max_sweeps >= 0, "bad argument");
+  FG_ARG(re->p.scheme == 0, "the reallocation is part of the PCA step");
+  re->realloc_limit = max_sweeps;
+  const int step = advance_one(re);
+  re->realloc_limit = -1;
+  const int end = frehg_re_sync(re);
+  *status = step != FREHG_OK ? step : end;
+  return FREHG_OK;
+}
+
 int frehg_re_dt(const frehg_re* re, double* dt) {
   clear_error();
   FG_ARG(re && dt, "null argument");
@@ -1490,7 +1521,7 @@ int frehg_re_get_interior(frehg_re* re, const char* name, double* out, int devic
                           device_out ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                           re->stream));
   FG_CUDA(cudaStreamSynchronize(re->stream));
-  return FREHG_OK;
+  return realloc_settled(re);
 }
 
 int frehg_re_get_interior_async(frehg_re* re, const char* name, double* out) {
@@ -1944,7 +1975,7 @@ int frehg_re_sync(frehg_re* re) {
   FG_ARG(re, "null handle");
   FG_CUDA(cudaStreamSynchronize(re->stream));
   FG_TRY(wait_copies(re, -1, true));
-  return FREHG_OK;
+  return realloc_settled(re);
 }
 
 }  // extern "C"

@@ -581,10 +581,13 @@ __global__ void k_realloc_sweep(ReArgs a, int top_sat) {
 // The whole relaxation in one block on a copy of the flags in shared memory, for grids of few columns:
 // no read-back between the sweeps, so the step's host waits for its solve only (two sweeps and their read-backs
 // took 70 us of a step of 40 x 40 x 100, now 37).
-// Every sweep but the last sets a flag, so there are at most n + 1.
+// Every sweep but the last sets a flag, so there are at most n + 1; a block still at it after `limit` more
+// than that many tells the host through `unsettled` (mapped host memory, read behind the stream's next
+// synchronisation).
 constexpr int kReallocThreads = 1024;
 constexpr size_t kReallocCols = 2048, kReallocCells = 200 * 1024;
-__global__ void __launch_bounds__(kReallocThreads) k_realloc(ReArgs a, int top_sat) {
+__global__ void __launch_bounds__(kReallocThreads) k_realloc(ReArgs a, int top_sat, long limit,
+                                                             int* unsettled) {
   extern __shared__ __align__(16) uint8_t realloc_flags[];
   grid_begin();
   const uint4* src = reinterpret_cast<const uint4*>(a.flags);
@@ -593,15 +596,19 @@ __global__ void __launch_bounds__(kReallocThreads) k_realloc(ReArgs a, int top_s
   for (size_t c = (a.n & ~(size_t)15) + threadIdx.x; c < a.n; c += blockDim.x)
     realloc_flags[c] = a.flags[c];
   __syncthreads();
-  unsigned long long sweeps = 0;
+  long sweeps = 0;
   int changed;
   do {
     changed = 0;
     for (size_t col = threadIdx.x; col < a.ncol; col += blockDim.x)
       changed |= realloc_column(a, realloc_flags, col, top_sat);
     ++sweeps;
-  } while (__syncthreads_or(changed) && sweeps <= a.n + 1);
-  if (threadIdx.x == 0) a.sc->sweeps += sweeps;
+    changed = __syncthreads_or(changed);
+  } while (changed && sweeps <= limit);
+  if (threadIdx.x == 0) {
+    a.sc->sweeps += (unsigned long long)sweeps;
+    if (changed) *unsettled = (int)min(sweeps, (long)INT_MAX);
+  }
 }
 
 // The reallocation's result for the water content of one cell (ReSolver.cpp:825-833) and the clamp

@@ -457,6 +457,12 @@ int frehg_re_check_staged_assembly(frehg_re* re, int64_t* mismatches);
  * error word (2: a consumer's wait ran out) and the handle's word is cleared, so the handle
  * steps normally afterwards.  Same handles as frehg_re_check_staged_assembly. */
 int frehg_re_check_staged_wait(frehg_re* re, int* err_word);
+/* Self-check of the PCA step's reallocation limit (not in reference): one step whose reallocation
+ * gives up when it has not settled after max_sweeps + 1 sweeps (a step's own limit is above what
+ * any state can need), then a synchronisation; *status receives what they report: FREHG_OK, or
+ * FREHG_ERR_STATE.  On grids whose reallocation runs in one block a step that gave up has returned
+ * FREHG_OK and advanced, and the handle's next call that synchronises reports it, once. */
+int frehg_re_check_realloc_limit(frehg_re* re, int max_sweeps, int* status);
 
 #ifdef __cplusplus
 }
