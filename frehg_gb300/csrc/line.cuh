@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(32 * W, L > 8 ? 1 : 2) k32_line_step(
 }
 
 // The same step with one thread per column, for columns longer than k32_line_step's registers
-// hold (256 levels): the forward sweep leaves u in z, the backward sweep overwrites it.
+// hold (256 levels): the forward sweep leaves u in z, the backward sweep overwrites it.  Levels in
+// groups, whose loads all come before the group's stores (the compiler may not move them across).
 template <bool FIRST>
 __global__ void __launch_bounds__(128) k32_line_step_long(
     float* x, float* r, const float* p0, const float* p1, const float* w, const float* lk,
@@ -274,32 +275,56 @@ __global__ void __launch_bounds__(128) k32_line_step_long(
   const float* p = (st->iter & 1) ? p0 : p1;
   const bool xfirst = st->iter == 0;
   const size_t sk = (size_t)ncol;
+  constexpr int U = 4;
   Kahan32 rz, rr;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
        col += gridDim.x * blockDim.x) {
     float y = 0.0f;
     size_t c = (size_t)col;
-#pragma unroll 4
-    for (int k = 0; k < nz; ++k, c += sk) {
-      float rk = r[c];
-      if (!FIRST) {
-        x[c] = fmaf(a, p[c], xfirst ? 0.0f : x[c]);
-        rk = fmaf(-a, w[c], rk);
-        r[c] = rk;
+    for (int k = 0; k < nz; k += U) {
+      float rv[U], lv[U], dv[U], pv[U], wv[U], xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t cu = c + sk * min(u, nz - 1 - k);
+        rv[u] = r[cu];
+        lv[u] = lk[cu];
+        dv[u] = dinv[cu];
+        pv[u] = FIRST ? 0.0f : p[cu];
+        wv[u] = FIRST ? 0.0f : w[cu];
+        xv[u] = FIRST || xfirst ? 0.0f : x[cu];
       }
-      y = fmaf(-lk[c], y, rk);
-      const float uk = y * dinv[c];
-      z[c] = uk;
-      rz.add(y * uk);
-      rr.add(rk * rk);
+#pragma unroll
+      for (int u = 0; u < U; ++u, c += sk) {
+        if (k + u >= nz) break;
+        if (!FIRST) {
+          x[c] = fmaf(a, pv[u], xv[u]);
+          rv[u] = fmaf(-a, wv[u], rv[u]);
+          r[c] = rv[u];
+        }
+        y = fmaf(-lv[u], y, rv[u]);
+        const float uk = y * dv[u];
+        z[c] = uk;
+        rz.add(y * uk);
+        rr.add(rv[u] * rv[u]);
+      }
     }
     float zz = 0.0f, lnext = 0.0f;
-#pragma unroll 4
-    for (int k = nz - 1; k >= 0; --k) {
-      c -= sk;
-      zz = fmaf(-lnext, zz, z[c]);
-      lnext = lk[c];
-      z[c] = zz;
+    c = (size_t)col + sk * (nz - 1);
+    for (int k = nz - 1; k >= 0; k -= U) {
+      float uv[U], lv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t cu = c - sk * min(u, k);
+        uv[u] = z[cu];
+        lv[u] = lk[cu];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u, c -= sk) {
+        if (k - u < 0) break;
+        zz = fmaf(-lnext, zz, uv[u]);
+        lnext = lv[u];
+        z[c] = zz;
+      }
     }
   }
   double loc[2] = {rz.value(), rr.value()};
