@@ -279,6 +279,7 @@ SIGNATURES = {
     "frehg_re_check_staged_assembly": (C.c_int, [_VP, C.POINTER(C.c_int64)]),
     "frehg_re_check_staged_wait": (C.c_int, [_VP, _PI]),
     "frehg_re_check_realloc_limit": (C.c_int, [_VP, C.c_int, _PI]),
+    "frehg_re_check_refinement": (C.c_int, [_VP, _PD, C.c_int, _PD]),
     "frehg_unet_conv_check": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
                                         C.c_int, C.c_int, C.c_int, C.c_int, C.c_uint64,
                                         C.POINTER(C.c_double), C.POINTER(C.c_double)]),

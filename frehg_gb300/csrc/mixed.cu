@@ -737,8 +737,10 @@ __global__ void k_ir_update(double* __restrict__ x, const float* __restrict__ e,
 
 // x~ += 2^k e for the sweeps whose residual is updated (k_ir_sweep), not recomputed: e becomes the
 // change that x~ really made, fl(x~ + 2^k e) - x~, so that the updated residual is that of the
-// stored x~.  That change is a float: a multiple of ulp(x~) no longer than e's own 24 bits.  The
-// first sweep's x~ = 2^k e is exact and written by k_ir_sweep.
+// stored x~.  That change is a float, a multiple of ulp(x~) no longer than e's own 24 bits, but where
+// the sum has a larger exponent than x~ and e: there one ulp of x~ is dropped (in few cells; half an
+// ulp of the sum, as a recomputed residual's rounding is).  The first sweep's x~ = 2^k e is exact and
+// written by k_ir_sweep.
 __global__ void k_ir_update_exact(double* x, float* e, size_t n, const CgDevState* ir,
                                   const CgDevState* in) {
   grid_begin();
@@ -824,10 +826,11 @@ struct ExactSum {
 // recomputed: r~ - A~ (2^k e), or s b - A~ (2^k e) in the first sweep, from exact FP32 products summed
 // in ExactSum, so that it stays the true residual of x~ to 2^-48 of itself and 2^-57 of its terms
 // (the FP64 stencil product rounds at 2^-53 of them) while the FP64 pipe, which bound that product
-// at 690 us for 56.6M cells, has nothing to do.  With the x~ update: 690 + 155 -> 607 + 132 us there,
-// 62 + 14 -> 54 + 12 for 2.9M cells, bound by its 380 instructions per warp and cell.  r~ is kept as float pairs in units of
-// the inner system's scale; the leading floats are the next right-hand side.  The first sweep also
-// writes x~ = 2^k e.
+// at 690 us for 56.6M cells, has nothing to do.  The low couplings' products enter with their own
+// rounding errors: without those it was off by 1.7e-16 of its terms at 40 x 40 x 100, 5e-19 so.
+// With the x~ update: 690 + 155 -> 613 + 132 us for 56.6M cells, 62 + 14 -> 55 + 12 for 2.9M, bound by
+// its 392 instructions per warp and cell.  r~ is kept as float pairs in units of the inner system's
+// scale; the leading floats are the next right-hand side.  The first sweep also writes x~ = 2^k e.
 struct SweepArgs {
   const float *h0, *h1, *h2, *l0, *l1, *l2;  // A~
   const float *dg, *e;                       // the diagonal (scale factors), the correction
@@ -892,7 +895,9 @@ __device__ __forceinline__ void sweep_cells(const SweepArgs& a, int n0, int n1, 
       for (int q = 0; q < 6; ++q) {
         sum.add(p[q]);
         sum.low(__fmaf_rn(-ah[q], en[q], -p[q]));
-        sum.low(__fmul_rn(-al[q], en[q]));
+        const float pl = __fmul_rn(-al[q], en[q]);
+        sum.low(pl);
+        sum.s2 = __fadd_rn(sum.s2, __fmaf_rn(-al[q], en[q], -pl));
       }
       const ff v = sum.value();
       const float q0 = v.h * to_next;

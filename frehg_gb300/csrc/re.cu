@@ -1684,6 +1684,97 @@ int frehg_re_check_staged_wait(frehg_re* re, int* err_word) {
   return rc;
 }
 
+int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, double out[6]) {
+  clear_error();
+  FG_ARG(re && out && solves > 0, "bad argument");
+  FG_ARG(re->finalized, "check before a finalized state");
+  if (re->p.scheme != 1 || !picard_ff(re) || !mixed_solve(re)) {
+    set_error("the float-float refinement serves Picard handles in mixed precision");
+    return FREHG_ERR_UNSUPPORTED;
+  }
+  const size_t n = re->n;
+  cudaStream_t st = re->stream;
+  re->constit_fresh = false;
+  FG_TRY(wait_copies(re, 1 - re->cur, false));
+  FG_TRY(re->ksp.ensure32(n));
+  const ReArgs a = make_args(re);
+  const StencilLaunch PL = stencil_launch(re->nx, re->ny, re->nz);
+  const Stencil32& o = re->ksp.op32;
+  // the first Picard system of the next step (classes that are not van Genuchten too)
+  launch_chained(k_step_begin, 1, 1, 0, st, re->sc);
+  k_copy64<<<nblocks(n), 256, 0, st>>>(a.h_new, a.h_old, n);
+  launch_chained(k_constit_ff<true, true, false>, nblocks(n), 256, 0, st, a, a.h_new, re->kr,
+                 re->wch, re->cap);
+  launch_chained(k_pic_assemble_ff<false, false, float>, PL.grid, PL.block, 0, st, a,
+                 reinterpret_cast<float*>(re->A.s), o.a0, o.a1, o.a2, re->A.b, PL.planes, PL.tiles);
+  FG_CUDA(cudaGetLastError());
+  if (rhs)
+    FG_CUDA(cudaMemcpyAsync(re->A.b, rhs, n * sizeof(double), cudaMemcpyHostToDevice, st));
+  re->A.scaled = false;
+  re->A.s_in_r = false;
+  re->A.f32_entries = true;
+  re->ksp.keep_scaled = true;
+  CgResult res;
+  int rc = FREHG_OK;
+  for (int q = 0; q < solves && rc == FREHG_OK; ++q) rc = solve_system(re, re->scratch, &res);
+  re->ksp.keep_scaled = false;
+  FG_TRY(rc);
+  // A~ = hi + lo with a unit diagonal, s b and x~ on the host
+  const KrylovSolver& k = re->ksp;
+  std::vector<float> hi[3], lo[3], kept(2 * n);
+  std::vector<double> s(n), b(n), x(n);
+  const float* hp[3] = {o.a0, o.a1, o.a2};
+  const double* lp[3] = {re->A.a0, re->A.a1, re->A.a2};
+  for (int q = 0; q < 3; ++q) {
+    hi[q].resize(n);
+    lo[q].resize(n);
+    FG_CUDA(cudaMemcpy(hi[q].data(), hp[q], n * sizeof(float), cudaMemcpyDeviceToHost));
+    FG_CUDA(cudaMemcpy(lo[q].data(), lp[q], n * sizeof(float), cudaMemcpyDeviceToHost));
+  }
+  FG_CUDA(cudaMemcpy(s.data(), k.r, n * sizeof(double), cudaMemcpyDeviceToHost));
+  FG_CUDA(cudaMemcpy(b.data(), re->A.b, n * sizeof(double), cudaMemcpyDeviceToHost));
+  FG_CUDA(cudaMemcpy(x.data(), k.x, n * sizeof(double), cudaMemcpyDeviceToHost));
+  FG_CUDA(cudaMemcpy(kept.data(), k.rres, 2 * n * sizeof(float), cudaMemcpyDeviceToHost));
+  const size_t off[3] = {1, (size_t)re->nx, (size_t)re->nx * re->ny};
+  std::vector<long double> r(n);
+  long double rt = 0, rk = 0, nb = 0, nt = 0;
+  for (size_t c = 0; c < n; ++c) {
+    const int at[3] = {(int)(c % re->nx), (int)(c / re->nx % re->ny), (int)(c / off[2])};
+    const int len[3] = {re->nx, re->ny, re->nz};
+    long double ax = x[c], t = fabsl((long double)x[c]);
+    auto term = [&](int q, size_t m, size_t to) {
+      const long double p = ((long double)hi[q][m] + lo[q][m]) * x[to];
+      ax += p;
+      t += fabsl(p);
+    };
+    for (int q = 0; q < 3; ++q) {
+      if (at[q] > 0) term(q, c - off[q], c - off[q]);
+      if (at[q] + 1 < len[q]) term(q, c, c + off[q]);
+    }
+    r[c] = (long double)s[c] * b[c] - ax;
+    const long double kc = (long double)kept[2 * c] + kept[2 * c + 1];
+    rt += r[c] * r[c];
+    rk += kc * kc;
+    nb += (long double)b[c] * b[c];
+    nt += t / s[c] * (t / s[c]);
+  }
+  // the kept residual is in units of a power of two
+  const long double unit = rk > 0 ? exp2l(roundl(log2l(sqrtl(rt / rk)))) : 1.0L;
+  long double nr = 0, nd = 0;
+  for (size_t c = 0; c < n; ++c) {
+    const long double d = r[c] - unit * ((long double)kept[2 * c] + kept[2 * c + 1]);
+    nr += r[c] / s[c] * (r[c] / s[c]);
+    nd += d / s[c] * (d / s[c]);
+  }
+  out[0] = (double)sqrtl(nr);
+  out[1] = res.rnorm;
+  out[2] = (double)sqrtl(nb);
+  out[3] = (double)sqrtl(nt);
+  out[4] = (double)sqrtl(nd);
+  out[5] = res.ir_its;
+  return FREHG_OK;
+}
+
 int frehg_re_check_staged_assembly(frehg_re* re, int64_t* mismatches) {
   clear_error();
   FG_ARG(re && mismatches, "null argument");

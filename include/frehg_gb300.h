@@ -463,6 +463,14 @@ int frehg_re_check_staged_wait(frehg_re* re, int* err_word);
  * FREHG_ERR_STATE.  On grids whose reallocation runs in one block a step that gave up has returned
  * FREHG_OK and advanced, and the handle's next call that synchronises reports it, once. */
 int frehg_re_check_realloc_limit(frehg_re* re, int max_sweeps, int* status);
+/* Self-check of the refinement of a Picard handle in mixed precision with float-float kernels (not
+ * in reference): assembles the first Picard system A d = b of the next step (rhs: b, host, n values,
+ * or null for the system's own), solves it `solves` times in a row, and compares with the operator
+ * that the solve used, on the host in extended precision.  out: ||b - A d||, the norm the solve
+ * reported for it, ||b||, the norm of the sum of the residual's terms' magnitudes, the norm of the
+ * difference between the residual and the one that the solve kept, and the last solve's refinement
+ * sweeps.  The handle's state stays but for the step's start (hn, wcn), which is overwritten. */
+int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, double out[6]);
 
 #ifdef __cplusplus
 }
