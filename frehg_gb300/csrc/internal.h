@@ -274,6 +274,7 @@ class KrylovSolver {
   // scaling of the operator for the mixed path (sq = D^1/2 into r, FP32 copy, line factors)
   int prep_mixed(Stencil64& A, cudaStream_t st, bool line, const frehg_solver_config& cfg);
   bool first_done = false;  // prep_mixed formed the first refinement residual and its state
+  bool ff_line = false;     // the float-float preparation made the line factors
   // first residual norms of earlier solves, the scale of the next one's: slot 0 for the first
   // solve of a time step (its residual is orders of magnitude above the previous step's last
   // one), slot 1 for the later (Picard) solves; the caller picks the slot

@@ -1387,6 +1387,7 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
       A.s_in_r = true;
       A.f32_entries = false;
       first_done = true;
+      ff_line = line;
       return FREHG_OK;
     }
     FG_LAUNCH(prof, st, "k_diag_rsqrt_sq", 24.0 * dn,
@@ -1399,13 +1400,18 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
     A.scaled = true;
     return FREHG_OK;
   }
-  // an operator scaled by an earlier solve: derive sq, the FP32 copy and the factors from it (the
-  // float-float preparation's are all still in place, the line factors if it made them)
-  if (!A.s_in_r) {
-    FG_LAUNCH(prof, st, "k_inv64", 16.0 * dn, k_inv64<<<nb, 256, 0, st>>>(A.s, r, n));
-    FG_LAUNCH(prof, st, "k_to_f32", 36.0 * dn,
-              k_to_f32<<<nb, 256, 0, st>>>(A.a0, A.a1, A.a2, op32.a0, op32.a1, op32.a2, n));
+  // an operator scaled by an earlier solve.  The float-float preparation's scale factors, operator
+  // and line factors are still in place; factors it did not make cannot be made now (A.a2 holds the
+  // couplings' low floats)
+  if (A.s_in_r) {
+    if (!line || ff_line) return FREHG_OK;
+    set_error("operator prepared for another preconditioner of the float-float solve; reassemble it");
+    return FREHG_ERR_STATE;
   }
+  // else derive sq, the FP32 copy and the factors from it
+  FG_LAUNCH(prof, st, "k_inv64", 16.0 * dn, k_inv64<<<nb, 256, 0, st>>>(A.s, r, n));
+  FG_LAUNCH(prof, st, "k_to_f32", 36.0 * dn,
+            k_to_f32<<<nb, 256, 0, st>>>(A.a0, A.a1, A.a2, op32.a0, op32.a1, op32.a2, n));
   if (line)
     FG_LAUNCH(prof, st, "k_line_factor", 16.0 * dn,
               k_line_factor<<<lb, 128, 0, st>>>(A.a2, lkf, dinvf, ncol, A.n2));

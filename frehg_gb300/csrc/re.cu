@@ -1684,7 +1684,7 @@ int frehg_re_check_staged_wait(frehg_re* re, int* err_word) {
   return rc;
 }
 
-int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, double out[6]) {
+int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, double out[7]) {
   clear_error();
   FG_ARG(re && out && solves > 0, "bad argument");
   FG_ARG(re->finalized, "check before a finalized state");
@@ -1772,6 +1772,7 @@ int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, doubl
   out[3] = (double)sqrtl(nt);
   out[4] = (double)sqrtl(nd);
   out[5] = res.ir_its;
+  out[6] = res.inner_its;
   return FREHG_OK;
 }
 

@@ -469,8 +469,8 @@ int frehg_re_check_realloc_limit(frehg_re* re, int max_sweeps, int* status);
  * that the solve used, on the host in extended precision.  out: ||b - A d||, the norm the solve
  * reported for it, ||b||, the norm of the sum of the residual's terms' magnitudes, the norm of the
  * difference between the residual and the one that the solve kept, and the last solve's refinement
- * sweeps.  The handle's state stays but for the step's start (hn, wcn), which is overwritten. */
-int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, double out[6]);
+ * sweeps and inner iterations.  The handle's state stays but for the step's start (hn, wcn), which is overwritten. */
+int frehg_re_check_refinement(frehg_re* re, const double* rhs, int solves, double out[7]);
 
 #ifdef __cplusplus
 }
