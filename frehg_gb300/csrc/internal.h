@@ -216,6 +216,25 @@ struct NetPrecond {
 
 // Jacobi-preconditioned CG in FP64 (one cooperative launch or three kernels per iteration,
 // CUDA-graph chunks), with an optional FP32 inner solve under FP64 iterative refinement.
+// What a captured iteration holds besides the solver's own buffers (whose reallocation destroys the
+// graph): the operator, its shape, and the form of the launches.
+struct GraphKey {
+  const void* op[4] = {nullptr, nullptr, nullptr, nullptr};
+  int dims[3] = {0, 0, 0};
+  int form = 0;
+  cudaStream_t stream = nullptr;
+  GraphKey() = default;
+  GraphKey(const Stencil64& A, int form_, cudaStream_t st)
+      : op{A.s, A.a0, A.a1, A.a2}, dims{A.n0, A.n1, A.n2}, form(form_), stream(st) {}
+  bool operator==(const GraphKey& o) const {
+    for (int q = 0; q < 4; ++q)
+      if (op[q] != o.op[q]) return false;
+    for (int q = 0; q < 3; ++q)
+      if (dims[q] != o.dims[q]) return false;
+    return form == o.form && stream == o.stream;
+  }
+};
+
 class KrylovSolver {
  public:
   ~KrylovSolver();
@@ -245,14 +264,12 @@ class KrylovSolver {
   // graphs
   cudaGraphExec_t g64 = nullptr;
   cudaGraphExec_t g32 = nullptr;
-  const void* g64_key = nullptr;
-  const void* g64_key2 = nullptr;
+  GraphKey g64_key;
   // the FP64 Jacobi-PCG iteration as one cooperative launch (k_cg_iter) rather than three
   // kernels, where the device has cooperative launches: 1 always, 0 never, -1 (default) for
   // systems of at most kFusedAutoCells unknowns (larger ones run faster as three kernels);
-  // g64_form: the form g64 holds; coop_failed: a cooperative capture failed, use three kernels
+  // coop_failed: a cooperative capture failed, use three kernels
   int fused64 = -1;
-  int g64_form = -1;
   bool coop_failed = false;
   // the one-launch solve's exchange words and the number of solves that have used them
   void* solve_words = nullptr;
@@ -291,15 +308,8 @@ class KrylovSolver {
   size_t cap_sor = 0, cap_slots = 0;
   double *invd = nullptr, *zs = nullptr, *sor_slots = nullptr;
   cudaGraphExec_t gsor = nullptr;
-  const void* gsor_key = nullptr;
-  const void* gsor_key2 = nullptr;
-  const void* gsor_key3 = nullptr;
-  cudaStream_t gsor_stream = nullptr;
-  size_t gsor_n = 0;
-  int gsor_dims[3] = {0, 0, 0};
+  GraphKey gsor_key;
   const void* g32_key = nullptr;
-  cudaStream_t g_stream = nullptr;
-  size_t g_n = 0;
 
  private:
   int solve64(Stencil64& A, double* x_out, const frehg_solver_config& cfg, cudaStream_t st,

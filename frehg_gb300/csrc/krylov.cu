@@ -940,9 +940,9 @@ int KrylovSolver::ensure(size_t n) {
   cudaFree(p);
   cudaFree(w);
   x = r = p = w = nullptr;
-  if (g64) {
-    cudaGraphExecDestroy(g64);
-    g64 = nullptr;
+  for (cudaGraphExec_t* g : {&g64, &gsor}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
   }
   FG_CUDA(cudaMalloc(&x, n * sizeof(double)));
   FG_CUDA(cudaMalloc(&r, n * sizeof(double)));
@@ -1227,9 +1227,8 @@ int KrylovSolver::solve64(Stencil64& A, double* x_out, const frehg_solver_config
     }
     return finish64(A, x_out, st, res, nb);
   }
-  const bool rebuild = !g64 || g64_key != (const void*)A.a0 || g64_key2 != (const void*)A.s ||
-                       g_stream != st || g_n != n || g64_form != form;
-  if (rebuild) {
+  const GraphKey key(A, form, st);
+  if (!g64 || !(g64_key == key)) {
     if (g64) cudaGraphExecDestroy(g64);
     g64 = nullptr;
     cudaStream_t cap_st;
@@ -1267,11 +1266,7 @@ int KrylovSolver::solve64(Stencil64& A, double* x_out, const frehg_solver_config
       set_error("graph instantiate failed: %s", cudaGetErrorString(e));
       return FREHG_ERR_CUDA;
     }
-    g64_key = A.a0;
-    g64_key2 = A.s;
-    g_stream = st;
-    g_n = n;
-    g64_form = form;
+    g64_key = key;
   }
   // iteration 0 may already have converged
   FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));

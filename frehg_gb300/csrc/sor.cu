@@ -931,6 +931,10 @@ int sor_sweep_blocks(const SorGeom& g, const void* kernel, int threads) {
 }  // namespace
 
 int KrylovSolver::ensure_sor(size_t n, size_t slot_doubles) {
+  if (gsor && (n > cap_sor || slot_doubles > cap_slots)) {
+    cudaGraphExecDestroy(gsor);
+    gsor = nullptr;
+  }
   if (n > cap_sor || !invd) {
     cudaFree(invd);
     cudaFree(zs);
@@ -1092,10 +1096,8 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
       FG_TRY(prof->flush());
     }
   } else if (hst->status == 0) {
-    const int dims[3] = {A.n0, A.n1, A.n2};
-    const bool rebuild = !gsor || gsor_key != (const void*)A.a0 || gsor_key2 != (const void*)sor_slots || gsor_key3 != (const void*)invd ||
-                         gsor_stream != st || gsor_n != n || memcmp(gsor_dims, dims, sizeof(dims));
-    if (rebuild) {
+    const GraphKey key(A, sweep_blocks, st);
+    if (!gsor || !(gsor_key == key)) {
       if (gsor) cudaGraphExecDestroy(gsor);
       gsor = nullptr;
       cudaStream_t cap_st;
@@ -1118,12 +1120,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
         set_error("SOR graph instantiate failed: %s", cudaGetErrorString(e));
         return FREHG_ERR_CUDA;
       }
-      gsor_key = A.a0;
-      gsor_key2 = sor_slots;
-      gsor_key3 = invd;
-      gsor_stream = st;
-      gsor_n = n;
-      memcpy(gsor_dims, dims, sizeof(dims));
+      gsor_key = key;
     }
     const int max_launch = cfg.max_it / chunk + 2;
     int q = 0;
