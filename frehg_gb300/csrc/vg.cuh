@@ -161,8 +161,8 @@ __device__ __forceinline__ double vg_head(const CellSoil& s, double wc) {
 }
 
 // waterContentFromHead of a large initial state: vg_theta with the table-driven powers for the van
-// Genuchten branch (theta at heads of -1e-4 to -1e3 m: 3.7e-16 of the exact value at most,
-// 6e-17 rms, as with pow(), which took 19.5 ms of FP64 pipe for 56.6M cells; now 8.5).
+// Genuchten branch (no less accurate than pow(), which took 19.5 ms of FP64 pipe for 56.6M cells; now
+// 9.1).
 __device__ __forceinline__ double vg_theta_initial(const CellSoil& s, double h) {
   if (!s.use_vg || s.use_mvg) return vg_theta(s, h);
   if (h > s.aev) return s.ths;
