@@ -682,8 +682,8 @@ static int pca_step(frehg_re* re) {
   // SM and plane leave the FP64 unit waiting for a chain (100 cells: 18.4 -> 14.3 us, in the
   // reference's powers 18.4), and in those powers up to kPowCells
   const size_t blocks = (size_t)L.grid.x * L.grid.y;
-  const bool split = blocks * L.planes <= 2 * (size_t)kNumSMs;
-  const bool lanes = split && n <= kPowCells;
+  const bool lanes = re->n <= kPowCells;
+  const bool split = lanes || blocks * L.planes <= 2 * (size_t)kNumSMs;
   const int shares = lanes ? std::max(1, (int)((4 * re->n + 256 * blocks - 1) / (256 * blocks))) : 1;
   FG_LAUNCH(prof, st, "k_finalize", (25.0 + sb) * n,
             launch_chained(lanes ? k_finalize<2> : (split ? k_finalize<1> : k_finalize<0>),

@@ -366,7 +366,6 @@ __device__ __forceinline__ double vg_dKdwc(const CellSoil& s, double wc, double 
 // tolerance (a 50 x 30 section at 24 iterations) then stops one iteration earlier or later, 1e-9 in
 // the head.
 __device__ __forceinline__ double vg_dKdwc_lanes(const CellSoil& s, double wc, double Ks) {
-  if (__any_sync(0xffffffffu, s.use_mvg)) return vg_dKdwc(s, wc, Ks);
   const int part = threadIdx.x & 3, base = threadIdx.x & 28;
   double theta = wc;
   if (theta > 0.9999 * s.ths && theta < s.ths) theta = 0.9999 * s.ths;
@@ -380,7 +379,8 @@ __device__ __forceinline__ double vg_dKdwc_lanes(const CellSoil& s, double wc, d
       0.5 * Ks * __shfl_sync(0xffffffffu, p, base + 1) * (1.0 - term0) * (1.0 - term0);
   const double term2 = 2.0 * Ks * __shfl_sync(0xffffffffu, p, base + 2) * (1.0 - term0) *
                        __shfl_sync(0xffffffffu, r, base + 1);
-  return (term1 + term2) / (s.ths - s.thr);
+  // (a modified van Genuchten cell's four lanes take its own form, whatever the warp's other cells do)
+  return s.use_mvg ? vg_dKdwc(s, wc, Ks) : (term1 + term2) / (s.ths - s.thr);
 }
 
 }  // namespace fg
