@@ -271,6 +271,9 @@ class KrylovSolver {
   // coop_failed: a cooperative capture failed, use three kernels
   int fused64 = -1;
   bool coop_failed = false;
+  // self-check of the one-launch forms' waits: the last block (the sweeps': the first tile) stays away,
+  // and the others' waits run out after so many polls (0: none of this)
+  long check_polls = 0;
   // the one-launch solve's exchange words and the number of solves that have used them
   void* solve_words = nullptr;
   unsigned long long solve_count = 0;

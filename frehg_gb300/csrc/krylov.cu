@@ -528,12 +528,12 @@ constexpr int kSolveWordBlocks = 16;  // blocks that exchange without the counte
 constexpr long kSolvePolls = 1L << 22;
 
 // all blocks have arrived: a count that only grows within a launch (bar_count, zero before it)
-__device__ __forceinline__ bool solve_arrive_wait(CgDevState* st, unsigned target) {
+__device__ __forceinline__ bool solve_arrive_wait(CgDevState* st, unsigned target, long polls) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
   unsigned v = 0;
   for (long q = 0; v < target; ++q) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->bar_count) : "memory");
-    if (q >= kSolvePolls) {
+    if (q >= polls) {
       atomicExch(&st->bar_timeout, 1);
       return false;
     }
@@ -565,7 +565,8 @@ __device__ __forceinline__ bool word_get(const SolveWord* p, unsigned long long 
 // words w[b], b = first + lane + 32 j up to last, until all carry `epoch` (one warp); the sum of
 // this lane's, in order of b.  *ok false when the wait ran out.
 __device__ __forceinline__ double words_wait(const SolveWord* w, int first, int last,
-                                             unsigned long long epoch, bool* ok, CgDevState* st) {
+                                             unsigned long long epoch, bool* ok, CgDevState* st,
+                                             long polls) {
   const int lane = threadIdx.x & 31;
   double v[kSolveBlocks / 32];
   for (long q = 0;; ++q) {
@@ -577,7 +578,7 @@ __device__ __forceinline__ double words_wait(const SolveWord* w, int first, int 
       if (b <= last && !word_get(w + b, epoch, &v[j])) have = false;
     }
     if (__all_sync(0xffffffffu, have)) break;
-    if (q >= kSolvePolls) {
+    if (q >= polls) {
       *ok = false;
       if (lane == 0) atomicExch(&st->bar_timeout, 1);
       break;
@@ -605,7 +606,7 @@ struct SolveScalars {
 template <int NV, bool RELEASE>
 __device__ __forceinline__ bool solve_sum(double (&v)[NV], SolveWord* words, CgDevState* st,
                                           unsigned long long epoch, unsigned target, double* sh,
-                                          double* buf, int* ok_sh) {
+                                          double* buf, int* ok_sh, long polls) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   int parts = warps;
   if (warps >= 8) {
@@ -647,14 +648,15 @@ __device__ __forceinline__ bool solve_sum(double (&v)[NV], SolveWord* words, CgD
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
-      if (!solve_arrive_wait(st, target)) *ok_sh = 0;
+      if (!solve_arrive_wait(st, target, polls)) *ok_sh = 0;
     }
     __syncthreads();
   }
   if (warp < NV) {
     if (gridDim.x > 1) {
       bool ok = true;
-      t = warp_sum(words_wait(words + warp * kSolveBlocks, 0, (int)gridDim.x - 1, epoch, &ok, st));
+      t = warp_sum(words_wait(words + warp * kSolveBlocks, 0, (int)gridDim.x - 1, epoch, &ok, st,
+                              polls));
       if (RELEASE) __threadfence();
       if (!ok) *ok_sh = 0;
     }
@@ -725,7 +727,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
     const double* __restrict__ a0, const double* __restrict__ a1, const double* __restrict__ a2,
     const double* __restrict__ s, double* __restrict__ x_out, double* r_io, double* p0, double* p1,
     unsigned n, unsigned s1, unsigned s2, CgDevState* st, SolveWord* words,
-    unsigned long long epoch) {
+    unsigned long long epoch, int absent, long polls) {
+  if ((int)blockIdx.x == absent) return;  // (a self-check of the waits)
   __shared__ SolveScalars ss;
   __shared__ double sh[32], buf[2 * kSolveThreads];
   if (threadIdx.x == 0) {
@@ -782,7 +785,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
         }
         const int b = (int)blockIdx.x;
         words_wait(words + 3 * kSolveBlocks, max(0, b - reach), min((int)gridDim.x - 1, b + reach),
-                   epoch, &there, st);
+                   epoch, &there, st, polls);
         __threadfence();
         if (!there) ss.ok = 0;
       }
@@ -811,7 +814,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
       }
     }
     if (!(ok = solve_sum<1, false>(acc, words + 2 * kSolveBlocks, st, ++epoch, target += gridDim.x,
-                                   sh, buf, &ss.ok)))
+                                   sh, buf, &ss.ok, polls)))
       break;
     if (threadIdx.x == 0) solve_alpha(ss, sh[0]);
     __syncthreads();
@@ -830,8 +833,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_cg_solve(
         v[1] = fma(z, z, v[1]);
       }
     }
-    if (!(ok = solve_sum<2, REDIR>(v, words, st, ++epoch, target += gridDim.x, sh, buf,
-                                   &ss.ok)))
+    if (!(ok = solve_sum<2, REDIR>(v, words, st, ++epoch, target += gridDim.x, sh, buf, &ss.ok,
+                                   polls)))
       break;
     if (threadIdx.x == 0) solve_tail(ss, sh[0], sh[16]);
     __syncthreads();
@@ -955,6 +958,7 @@ int KrylovSolver::ensure(size_t n) {
     FG_TRY(alloc_mapped(reinterpret_cast<void**>(&hst), sizeof(CgDevState)));
     FG_CUDA(cudaMalloc(&solve_words, 4 * kSolveBlocks * sizeof(SolveWord)));
     FG_CUDA(cudaMemset(solve_words, 0, 4 * kSolveBlocks * sizeof(SolveWord)));
+    FG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // (the solves run on streams that do not wait)
   }
   cap = n;
   return FREHG_OK;
@@ -1119,13 +1123,13 @@ static bool solve_shape(size_t n, SolveShape* sh) {
   sh->blocks = (int)((n + per - 1) / per);
   // the wait for the neighbouring blocks costs about 1,500 clocks, forming their directions
   // 6 x 19 per warp and cell
-  sh->redir = sh->blocks > 1 && 6 * 19 * sh->cells * (sh->threads / 32) < 1500;
+  sh->redir = sh->blocks > 1 && sh->cells <= 3 && 6 * 19 * sh->cells * (sh->threads / 32) < 1500;
   return true;
 }
 
 static cudaError_t launch_cg_solve(const SolveShape& sh, cudaStream_t st, const Stencil64& A,
                                    double* x, double* r, double* p, double* p2, CgDevState* dst,
-                                   void* words, unsigned long long epoch) {
+                                   void* words, unsigned long long epoch, long check_polls) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)sh.blocks);
   cfg.blockDim = dim3((unsigned)sh.threads);
@@ -1139,21 +1143,20 @@ static cudaError_t launch_cg_solve(const SolveShape& sh, cudaStream_t st, const 
     return cudaLaunchKernelEx(&cfg, kernel, (const double*)A.a0, (const double*)A.a1,
                               (const double*)A.a2, (const double*)A.s, x, r, p, p2, (unsigned)A.n,
                               (unsigned)A.n0, (unsigned)(A.n0 * A.n1), dst,
-                              static_cast<SolveWord*>(words), epoch);
+                              static_cast<SolveWord*>(words), epoch,
+                              check_polls && sh.blocks > 1 ? sh.blocks - 1 : -1,
+                              check_polls ? check_polls : kSolvePolls);
   };
-#define FG_SOLVE_CASE(KK) \
-  case KK: return sh.redir ? go(k_cg_solve<KK, true>) : go(k_cg_solve<KK, false>);
-  switch (sh.cells) {
-    FG_SOLVE_CASE(1)
-    FG_SOLVE_CASE(2)
-    FG_SOLVE_CASE(3)
-    FG_SOLVE_CASE(4)
-    FG_SOLVE_CASE(5)
-    FG_SOLVE_CASE(6)
-    FG_SOLVE_CASE(7)
+  switch (sh.cells) {  // (redir: at most three, solve_shape)
+    case 1: return sh.redir ? go(k_cg_solve<1, true>) : go(k_cg_solve<1, false>);
+    case 2: return sh.redir ? go(k_cg_solve<2, true>) : go(k_cg_solve<2, false>);
+    case 3: return sh.redir ? go(k_cg_solve<3, true>) : go(k_cg_solve<3, false>);
+    case 4: return go(k_cg_solve<4, false>);
+    case 5: return go(k_cg_solve<5, false>);
+    case 6: return go(k_cg_solve<6, false>);
+    case 7: return go(k_cg_solve<7, false>);
     default: return go(k_cg_solve<8, false>);
   }
-#undef FG_SOLVE_CASE
 }
 
 static int chunk_for(size_t n) {
@@ -1185,7 +1188,7 @@ int KrylovSolver::solve64(Stencil64& A, double* x_out, const frehg_solver_config
     SolveShape sh;
     if (solve_shape(n, &sh)) {
       const cudaError_t e = launch_cg_solve(sh, st, A, x, r, p, w, dst, solve_words,
-                                            ++solve_count << 32);
+                                            ++solve_count << 32, check_polls);
       if (e == cudaSuccess) {
         if (prof) prof->launches += 1;
         FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));

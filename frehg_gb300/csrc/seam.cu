@@ -369,6 +369,16 @@ int frehg_cg_solve(frehg_cg* cg, frehg_system* s, const double* b, double* x, in
   return FREHG_OK;
 }
 
+int frehg_cg_check_waits(frehg_cg* cg, frehg_system* s, const double* b, long long polls,
+                         int* status) {
+  clear_error();
+  FG_ARG(cg && s && b && status && polls > 0, "bad argument");
+  cg->ksp.check_polls = (long)polls;
+  *status = frehg_cg_solve(cg, s, b, nullptr, 0);
+  cg->ksp.check_polls = 0;
+  return FREHG_OK;
+}
+
 int frehg_cg_iteration_count(const frehg_cg* cg, int* its) {
   clear_error();
   FG_ARG(cg && its, "null argument");

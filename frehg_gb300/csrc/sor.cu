@@ -159,7 +159,7 @@ struct SorSet {
 // others are left out.  Returns false when a wait ran out.
 template <bool FWD, int AXES, class P>
 __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, const P& ops,
-                                         int* abort_word) {
+                                         int* abort_word, long polls) {
   constexpr int N = P::kGroup;
   const int lane = threadIdx.x & 31;
   const int steps = g.n[0] + L.x1 + L.x2 - 2;
@@ -225,7 +225,7 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
           if (AXES > 1 && sor_missing(S.f2[u])) S.f2[u] = sor_peek(ops.template near2<FWD>(ic));
         }
         // (warp-uniform: every lane sees the same k, and the abort word is voted on)
-        if (k > kSorPolls ||
+        if (k > polls ||
             ((k & 1023) == 1023 &&
              __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(abort_word) != 0)))
           ok = false;
@@ -409,8 +409,9 @@ __device__ __forceinline__ double sor_undo(double y, double invd, double d) {
 template <int AXES, bool ROUNDED, bool LINE_FIRST>
 __global__ void __launch_bounds__(sor_sweep_threads(ROUNDED))
     k_sor_sweeps(SorGeom g, SorSlots S, const double* __restrict__ r, const double* __restrict__ d,
-                 const double* __restrict__ invd, double* z, CgDevState* st) {
-  if (st->status) return;
+                 const double* __restrict__ invd, double* z, CgDevState* st, int absent,
+                 long polls) {
+  if (st->status || (int)blockIdx.x == absent) return;  // (absent: a self-check of the waits)
   using Ops = SorGlobal<ROUNDED, LINE_FIRST>;
   const int tiles = g.nb1 * g.nb2;
   const bool sweeps = threadIdx.x < 32;
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(sor_sweep_threads(ROUNDED))
   int last = -1;
   for (int b = blockIdx.x; b < tiles && ok; b += gridDim.x) {
     const SorLane L(g, b % g.nb1, b / g.nb1);
-    if (sweeps) ok = sor_tile<true, AXES>(g, L, Ops(S, g, L, b, r, z), &st->bar_timeout);
+    if (sweeps) ok = sor_tile<true, AXES>(g, L, Ops(S, g, L, b, r, z), &st->bar_timeout, polls);
     last = b;
   }
   if (ROUNDED) {
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(sor_sweep_threads(ROUNDED))
   __syncwarp();
   for (int b = last; sweeps && b >= 0 && ok; b -= gridDim.x) {
     const SorLane L(g, b % g.nb1, b / g.nb1);
-    ok = sor_tile<false, AXES>(g, L, Ops(S, g, L, b, r, z), &st->bar_timeout);
+    ok = sor_tile<false, AXES>(g, L, Ops(S, g, L, b, r, z), &st->bar_timeout, polls);
   }
   if (!ok && threadIdx.x == 0) {
     atomicExch(&st->bar_timeout, 1);
@@ -776,7 +777,7 @@ template <int AXES, bool LINE_FIRST = true>
 __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     SorGeom g, const double* d, const double* a0, const double* a1, const double* a2,
     const double* b, double* x, double* x_out, int n0, int n1, int n2, double rtol, double atol,
-    double divtol, int max_it, CgDevState* dst) {
+    double divtol, int max_it, CgDevState* dst, int absent, long polls) {
   grid_begin();
   extern __shared__ double sor_sh[];
   __shared__ CgDevState st;
@@ -820,8 +821,10 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     bool ok = true;
     if (AXES == 0 && warp == 0) line.forward(r, v);
     for (int t = warp; t < tiles && ok; t += warps) {
+      if (t == absent) continue;  // (a self-check of the waits)
       const SorLane L(g, t % g.nb1, t / g.nb1);
-      ok = sor_tile<true, AXES>(g, L, SorShared<LINE_FIRST>(true, g, L, r, invd, g0, g1, g2, v), &st.bar_timeout);
+      const SorShared<LINE_FIRST> ops(true, g, L, r, invd, g0, g1, g2, v);
+      ok = sor_tile<true, AXES>(g, L, ops, &st.bar_timeout, polls);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
@@ -833,7 +836,8 @@ __global__ void __launch_bounds__(kSorSolveThreads) k_sor_solve(
     for (int t = warp + (tiles - 1 - warp) / warps * warps; warp < tiles && t >= 0 && ok;
          t -= warps) {
       const SorLane L(g, t % g.nb1, t / g.nb1);
-      ok = sor_tile<false, AXES>(g, L, SorShared<LINE_FIRST>(false, g, L, v, invd, g0, g1, g2, z), &st.bar_timeout);
+      const SorShared<LINE_FIRST> ops(false, g, L, v, invd, g0, g1, g2, z);
+      ok = sor_tile<false, AXES>(g, L, ops, &st.bar_timeout, polls);
     }
     if (!ok) atomicExch(&st.bar_timeout, 1);
     __syncthreads();
@@ -966,6 +970,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   // two axes: the order of their terms known to the compiler (161 -> 150 us on a 50 x 30 section: a
   // selection per term is as long as half an FP64 instruction in the chain)
   const bool line_first = g.ord[0] == 0 || (g.ord[1] == 0 && g.ord[0] == 2);
+  const long polls = check_polls ? check_polls : kSorPolls;
   auto finish = [&]() -> int {
     res->its = hst->its;
     res->reason = hst->status;
@@ -992,12 +997,13 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     auto kernel = g.axes == 2   ? k_sor_solve<2>
                   : g.axes == 1 ? (line_first ? k_sor_solve<1, true> : k_sor_solve<1, false>)
                                 : k_sor_solve<0>;
+    const int absent = check_polls && g.axes > 0 && g.nb1 * g.nb2 > 1 ? 0 : -1;
     FG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  8 * kSorSolveCells * (int)sizeof(double)));
     FG_LAUNCH(prof, st, "k_sor_solve", 48.0 * dn,
               launch_chained(kernel, 1, threads, smem, st, g, A.s, A.a0, A.a1, A.a2, A.b, x,
                              x_out ? x_out : x, A.n0, A.n1, A.n2, cfg.rtol, cfg.atol, 1.0e4,
-                             cfg.max_it, dst));
+                             cfg.max_it, dst, absent, polls));
     FG_CUDA(cudaGetLastError());
     FG_TRY(fetch_small(hst, dst, sizeof(CgDevState), st));
     FG_CUDA(cudaStreamSynchronize(st));
@@ -1023,6 +1029,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
   const int sweep_threads = sor_sweep_threads(rounded);
   const int sweep_blocks =
       coop_failed ? 1 : std::max(1, sor_sweep_blocks(g, (const void*)kernel, sweep_threads));
+  const int absent = check_polls && sweep_blocks > 1 ? 0 : -1;
   CgDevState init;
   memset(&init, 0, sizeof(init));
   init.rtol = cfg.rtol;
@@ -1046,7 +1053,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
     lc.attrs = at;
     lc.numAttrs = sweep_blocks > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&lc, kernel, g, S, (const double*)r, (const double*)A.s,
-                              (const double*)invd, zs, dst);
+                              (const double*)invd, zs, dst, absent, polls);
   };
   FG_LAUNCH(prof, st, "k_sor_prep", 48.0 * dn,
             launch_chained(k_sor_prep, nb, 256, 0, st, A.s, A.b, invd, xs, r, zs, n));

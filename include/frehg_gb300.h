@@ -293,6 +293,13 @@ int frehg_cg_converged_reason(const frehg_cg* cg, int* reason); /* KSPConvergedR
  * kernels above.  The forms sum the dot products over different block partitions, so their last
  * bits (and, in a borderline case, an iteration count) may differ. */
 int frehg_cg_set_fused_iteration(frehg_cg* cg, int on);
+/* Self-check of the waits between the blocks of a one-launch solve and between the tiles of the SOR
+ * sweeps (not in reference): the solve of A x = b with the last block (SOR: the first tile) staying
+ * away and the others' waits running out after `polls` polls.  *status receives the solve's result,
+ * FREHG_ERR_CUDA (systems of one block or one tile have no waits: FREHG_OK); the handle and the system
+ * serve further solves. */
+int frehg_cg_check_waits(frehg_cg* cg, frehg_system* sys, const double* b, long long polls,
+                         int* status);
 /* Self-check of the one-launch iteration's grid barrier (not in reference): two cooperative
  * blocks meet at one barrier whose wait is bounded by `polls` polls; skip_block = 0 or 1 makes
  * that block return without arriving, so the other's wait runs out, sets the timeout flag and
