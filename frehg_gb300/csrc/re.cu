@@ -61,7 +61,7 @@ struct frehg_re {
   bool constit_fresh = false;
   ReScalars* sc = nullptr;
   ReScalars* sc_host = nullptr;
-  int* unsettled = nullptr;    // (mapped) sweeps after which k_realloc gave up, 0: it did not
+  int* unsettled = nullptr;    // behind sc_host: sweeps after which k_realloc gave up, 0: it did not
   long realloc_limit = -1;     // sweeps of a reallocation before it gives up; -1: more than can be
   double* partials = nullptr;
   double* xch = nullptr;  // surface-exchange staging (eta, bottom, q, total), on first use
@@ -120,7 +120,6 @@ frehg_re::~frehg_re() {
   cudaFree(scratch);
   cudaFree(sc);
   cudaFreeHost(sc_host);
-  cudaFreeHost(unsettled);
   cudaFree(partials);
   cudaFree(cls);
   cudaFree(cid);
@@ -1076,9 +1075,10 @@ int frehg_re_create(int nx, int ny, int nz, const frehg_re_params* p, frehg_re**
   ALLOC(re->sc, sizeof(ReScalars));
   ALLOC(re->partials, 4 * kMaxRedBlocks * sizeof(double));
 #undef ALLOC
-  if (alloc_mapped(reinterpret_cast<void**>(&re->sc_host), sizeof(ReScalars)) != FREHG_OK ||
-      alloc_mapped(reinterpret_cast<void**>(&re->unsettled), sizeof(int)) != FREHG_OK)
+  if (alloc_mapped(reinterpret_cast<void**>(&re->sc_host), sizeof(ReScalars) + sizeof(int)) !=
+      FREHG_OK)
     return fail(FREHG_ERR_CUDA);
+  re->unsettled = reinterpret_cast<int*>(re->sc_host + 1);
   *re->unsettled = 0;
   if (re->A.alloc(nx, ny, nz) != FREHG_OK) return fail(FREHG_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&re->own_stream, cudaStreamNonBlocking) != cudaSuccess)
