@@ -53,8 +53,11 @@ StencilLaunch stencil_launch(int n0, int n1, int n2) {
   // about two waves of 8 resident (32 x 8)-thread blocks per SM, fewer on small grids: 8 cells per
   // thread, down to two blocks per SM, since each block's sums and its uneven share cost the FP64
   // pipe more than the cells do (FP64 assembly of 101 x 77 x 53: 159 us with 1 to 2 cells per
-  // thread, 106 with 8; the FP32 product of 203 x 149 x 96 prefers more blocks, 32 against 33); the
-  // launch shape, and with it the summation tree of the reductions, depends on the grid sizes only
+  // thread, 106 with 8).  Whole passes with 4 / 8 / 16 cells per thread: FP64 Picard of 101 x 77 x 53
+  // 8.44 / 7.74 / 7.75 ms, PCA of 120 x 110 x 90 3.87 / 3.82 / 3.88 and of 90 x 75 x 60 1.85 / 1.79 /
+  // 1.80, float-float Picard of 203 x 149 x 96 11.7 / 11.4 / 12.0; of 100 x 90 x 96, where 4 is the
+  // best, 5.02 / 5.19 / 5.49; 40 x 40 x 100 and 256 x 256 x 128 the same.  The launch shape, and with
+  // it the summation tree of the reductions, depends on the grid sizes only
   const long want = (long)n0 * n1 * n2 / 2048;
   const long target = std::min((long)kNumSMs * 8 * 2, std::max((long)kNumSMs * 2, want));
   long z = target / (tiles > 0 ? tiles : 1);
@@ -958,7 +961,8 @@ int KrylovSolver::ensure(size_t n) {
     FG_TRY(alloc_mapped(reinterpret_cast<void**>(&hst), sizeof(CgDevState)));
     FG_CUDA(cudaMalloc(&solve_words, 4 * kSolveBlocks * sizeof(SolveWord)));
     FG_CUDA(cudaMemset(solve_words, 0, 4 * kSolveBlocks * sizeof(SolveWord)));
-    FG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // (the solves run on streams that do not wait)
+    // (the solves run on streams that do not wait for the legacy one)
+    FG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   }
   cap = n;
   return FREHG_OK;

@@ -792,8 +792,8 @@ __device__ __forceinline__ Float3 split3(double x, int k) {
   return r;
 }
 
-// An exact sum of floats in three levels (the extraction of S. M. Rump, T. Ogita, S. Oishi, "Accurate
-// floating-point summation part I", SIAM J. Sci. Comput. 31(1), 2008): with 2^m above every term,
+// An exact sum of floats in three levels (the extraction of S. M. Rump, T. Ogita, S. Oishi,
+// "Accurate floating-point summation part I", SIAM J. Sci. Comput. 31(1), 2008): with 2^m above every term,
 // s0 collects the terms' bits down to 2^(m-20), s1 (which the products' low parts enter) those
 // down to 2^(m-39), both without rounding for up to 16 and 32 terms, s2 the rest: the sum is within
 // about 2^(m-57), where FP64's partial sums round at 2^(m-54).
@@ -1127,7 +1127,8 @@ __global__ void __launch_bounds__(128) k_scale_mixed(double* __restrict__ a0,
 // This replaces k_diag_rsqrt_sq, k_scale_mixed, the first k_ir_residual and k_ir_scale: the
 // diagonal, the couplings and b are read once.  The assembly wrote
 // the diagonal (dg) and the unscaled couplings (f0-f2) as floats; f0-f2 are overwritten in
-// place by the scaled FP32 copies, and the FP64 scaled couplings go to a0-a2.
+// place by the scaled couplings' leading floats, and their low floats go to l0-l2, where the FP64
+// couplings of other operators are.
 // One cell of the preparation: scale factors sc (its own), sx, sy, sz (the +1 neighbours'), the
 // unscaled couplings e0-e2 (0 towards absent neighbours); writes the scaled operator, s and the
 // first right-hand side and returns the scaled axis-2 coupling.
@@ -1150,7 +1151,7 @@ __device__ __forceinline__ ff prep_cell(const PrepOut& o, size_t c, float e0, fl
   o.l0[c] = v0.l;
   o.l1[c] = v1.l;
   o.l2[c] = v2.l;
-  // first sweep: x~ = 0 (the first k_ir_update writes x~ without reading it), r~ = s b,
+  // first sweep: x~ = 0 (the first k_ir_sweep writes x~ without reading it), r~ = s b,
   // kept only as its FP32 form r~ 2^-e (the inner right-hand side), with the sums of
   // squares of r~ 2^-e and b 2^-e (with x~ = 0 the true residual is b) compensated in FP32
   const float qb = ff_hi_of(bc) * sig;
@@ -1261,12 +1262,13 @@ __global__ void __launch_bounds__(128) k_prep_ff(
 // The same preparation for grids whose columns are too few for a march with one thread each to keep
 // the loads in flight (a microsecond per level): a block owns 32 columns, its eight warps take the
 // cells' part level by level in any order, and only the line factors, which need the level above,
-// are left to one warp, from shared memory. March / split: 40 x 40 x 100 107 / 35 us, 203 x 149 x
-// 96 139 / 80, 256 x 256 x 128 208 / 202; 768 x 768 x 96 846 / 1400, where the march's loads
+// are left to one warp, from shared memory.  March / split: 40 x 40 x 100 107 / 35 us, 200 x 200 x
+// 96 120 / 75, 256 x 256 x 96 129 / 111, 256 x 256 x 128 208 / 202; 300 x 300 x 96 141 / 152, 400 x
+// 400 x 96 200 / 232, 600 x 600 x 96 412 / 497, 768 x 768 x 96 846 / 1400, where the march's loads
 // already fill the memory pipe and this form's barrier between its two parts empties it.
 constexpr int kPrepWarps = 8;
 constexpr int kPrepLevels = 190;         // 48 KB of scaled couplings beside the sums' 4 KB
-constexpr int kPrepSplitGroups = 2048;   // 65,536 columns: above, the march is the faster
+constexpr int kPrepSplitGroups = 2048;   // 65,536 columns (the forms cross at about 80,000)
 __global__ void __launch_bounds__(32 * kPrepWarps) k_prep_ff_split(
     PrepOut o, const float* dg, const double* b, float* lk, float* dinv, int n0, int n1, int n2,
     int line, CgDevState* ir, double* partials, double ir_rtol, CgDevState* in, int sig_exp,
@@ -1405,7 +1407,8 @@ int KrylovSolver::prep_mixed(Stencil64& A, cudaStream_t st, bool line,
   // couplings' low floats)
   if (A.s_in_r) {
     if (!line || ff_line) return FREHG_OK;
-    set_error("operator prepared for another preconditioner of the float-float solve; reassemble it");
+    set_error("operator prepared for another preconditioner of the float-float solve; "
+              "reassemble it");
     return FREHG_ERR_STATE;
   }
   // else derive sq, the FP32 copy and the factors from it
@@ -1677,8 +1680,8 @@ int KrylovSolver::solve_mixed(Stencil64& A, double* x_out, const frehg_solver_co
       }
     }
     if (dbg)
-      fprintf(stderr, "ir sweep %d round %d: launched %d done %d; true |r| %.3e / |b| %.3e status %d\n",
-              sweeps, round, launched, done, hst->ir_rnorm, hst->ir_bnorm, hst->status);
+      fprintf(stderr,
+              "ir sweep %d round %d: launched %d done %d; true |r| %.3e / |b| %.3e status %d\n", sweeps, round, launched, done, hst->ir_rnorm, hst->ir_bnorm, hst->status);
     total += done;
     ++round;
     for (; sweeps < hst->ir_its; ++sweeps, round = hst32->its > 0 ? 1 : 0)

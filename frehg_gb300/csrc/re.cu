@@ -61,8 +61,8 @@ struct frehg_re {
   bool constit_fresh = false;
   ReScalars* sc = nullptr;
   ReScalars* sc_host = nullptr;
-  int* unsettled = nullptr;    // behind sc_host: sweeps after which k_realloc gave up, 0: it did not
-  long realloc_limit = -1;     // sweeps of a reallocation before it gives up; -1: more than can be
+  int* unsettled = nullptr;  // behind sc_host: sweeps after which k_realloc gave up (0: it did not)
+  long realloc_limit = -1;   // sweeps of a reallocation before it gives up; -1: more than can be
   double* partials = nullptr;
   double* xch = nullptr;  // surface-exchange staging (eta, bottom, q, total), on first use
   double* gh_top = nullptr;    // top-layer ghost copies (h then wc) from before an exchange
@@ -679,11 +679,12 @@ static int pca_step(frehg_re* re) {
   re->cnt.realloc_sweeps += sweeps;
   // apply reallocation, clampWaterContent, adaptiveTimeStep: in two halves where a block or two per
   // SM and plane leave the FP64 unit waiting for a chain (100 cells: 18.4 -> 14.3 us, in the
-  // reference's powers 18.4), and in those powers up to kPowCells
+  // reference's powers 18.4), and in those powers, on every grid, up to kPowCells
   const size_t blocks = (size_t)L.grid.x * L.grid.y;
   const bool lanes = re->n <= kPowCells;
   const bool split = lanes || blocks * L.planes <= 2 * (size_t)kNumSMs;
-  const int shares = lanes ? std::max(1, (int)((4 * re->n + 256 * blocks - 1) / (256 * blocks))) : 1;
+  const int shares =
+      lanes ? std::max(1, (int)((4 * re->n + 256 * blocks - 1) / (256 * blocks))) : 1;
   FG_LAUNCH(prof, st, "k_finalize", (25.0 + sb) * n,
             launch_chained(lanes ? k_finalize<2> : (split ? k_finalize<1> : k_finalize<0>),
                            dim3(L.grid.x, L.grid.y * (split ? 1 + shares : 1)), L.block, 0, st, a,
@@ -1249,7 +1250,8 @@ int frehg_re_set_initial_water_content(frehg_re* re, const double* wc) {
   FG_CUDA(cudaStreamSynchronize(re->stream));
   FG_CUDA(cudaMemcpy(re->W[re->cur], wc, re->n * sizeof(double), cudaMemcpyHostToDevice));
   ReArgs a = make_args(re);
-  k_h_of_theta<<<spread_blocks(re->n), kSpreadThreads, 0, re->stream>>>(a, re->W[re->cur], re->H[re->cur]);
+  k_h_of_theta<<<spread_blocks(re->n), kSpreadThreads, 0, re->stream>>>(a, re->W[re->cur],
+                                                                        re->H[re->cur]);
   FG_CUDA(cudaGetLastError());
   FG_CUDA(cudaStreamSynchronize(re->stream));
   re->have_state = true;

@@ -251,7 +251,8 @@ class Placer {
  private:
   double *diag, *up0, *dn0, *up1, *dn1, *up2, *dn2;
   long n, n0, n1, n2, s2;
-  long at = LONG_MIN, k = 0, i = 0, j = 0;  // at: the last row, within the system (none: no row's value)
+  // the last row, one of the system's (none yet: a value that no row has), and its position
+  long at = LONG_MIN, k = 0, i = 0, j = 0;
 };
 }  // namespace
 

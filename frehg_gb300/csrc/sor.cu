@@ -10,8 +10,8 @@
 // with 1/d formed once as PETSc's MatSOR does (a zero diagonal entry taken as 1), the product
 // d y formed as y / (1/d), and the neighbour terms in the reference's column order.
 //
-// Evaluation, larger systems.  With v = D y the two sweeps need one fused multiply-add per
-// neighbour and cell:
+// Evaluation, larger systems of three axes.  With v = D y the two sweeps need one fused multiply-add
+// per neighbour and cell:
 //   v_c = r_c - sum e_m v_m        (m the lower neighbours, e_m = a_m / d_m at the neighbour)
 //   z_c = v_c / d_c - sum e_c z_u  (u the upper neighbours, e_c = a_c / d_c at the cell)
 // with the same e = a / d for both, formed once per solve (a zero diagonal entry taken as 1, as
@@ -19,12 +19,17 @@
 // of MatSOR to rounding; on GB300 a warp issues one FP64 instruction per 64 clocks however few of
 // its lanes are active, so the dependent FP64 instructions per cell are what the sweeps cost
 // (three instead of seven, and no division).  A line of cells (a soil column) takes the same form.
-// Evaluation, small systems of several lines.  MatSOR's products, differences and scalings, each
-// rounded and in its order, and the sums in the order of sor_sum: the results are those of the
-// sequential form (a launch per hyperplane) to the bit.  Such a solve ends after tens of iterations
-// within its own rounding noise (3 % of the residual) of the tolerance: with another rounding one
-// solve in four of a 50 x 30 section stopped an iteration earlier or later, 1e-9 in the head.  It
-// costs 5 FP64 instructions a step instead of 2 (47 us an application of that section, 29 before).
+// Evaluation, systems of two axes (sections) and of up to kSorSolveCells.  MatSOR's products,
+// differences and scalings, each rounded and in its order, and the sums in the order of sor_sum: the
+// results are those of the sequential form (a launch per hyperplane) to the bit.  The one long solve of
+// a dry section under recharge (23 iterations at 50 x 30, 38 at 100 x 60; its others take one or two)
+// ends within its own rounding noise (3 % of the residual) of the tolerance: with another rounding it
+// stopped an iteration earlier or later in one of four runs of 50 x 30, and heads of -500 m moved by up
+// to 1.5e-6 m.  It costs 5 FP64 instructions a step instead of 2 (47 us an application of 50 x 30, 29
+// before; 115 us of 100 x 60, 77 before).  Larger systems of three axes keep the fused form: their
+// runs agree with the sequential form to 1e-14 (ponded loam) and 2e-10 (dry sections a few cells
+// thick) with equal iteration counts, closer than rtol 1e-10 determines those, and rounding every
+// operation takes 1.23 times as long on 90 x 75 x 60.
 //
 // Schedule.  A cell depends only on its lower (backward: upper) neighbours, so the sequential
 // order is a wavefront.  One warp owns a tile of 32 lines (lines run along the longest axis, the
@@ -33,17 +38,16 @@
 // shuffles), the line's own previous value is a register, and the values of the neighbouring
 // tiles are read from memory, where the value itself is the signal that it is there: before a
 // sweep the array holds kSorWait (a NaN that no arithmetic produces), a reader repeats its load
-// until that is gone (bounded).  The loads run a group of steps ahead of
-// their use.  No barrier,
-// no fence and no flag: a handover costs one trip through the L2.
+// until that is gone (bounded).  The loads run a group of steps ahead of their use.  No barrier, no
+// fence and no flag: a handover costs one trip through the L2.
 //   n <= kSorSolveCells: the whole CG solve in one block with its vectors in shared memory.
 //   larger: one cooperative launch (all tiles' blocks resident) per preconditioner application
 //   and the CG kernels around it, captured as graphs.
 // Measured on GB300, one application (both sweeps): 405,000 cells (90 x 75 x 60) 244 us against
 // 1.1 ms for a launch per hyperplane; 4,096 cells 45 us; a whole solve of a 100-cell column (four
-// applications, three iterations) 28 us, of a 50 x 30 section 150 us for 3.2 applications, where
-// one block with a barrier and an L2 round trip per hyperplane took 168 and 228 us for each
-// application.  A step costs about 85 clocks per dependent FP64 instruction, a handover to the next
+// applications, three iterations) 30 us, of a 50 x 30 section 150 us in the mean of twenty (3.2
+// applications), where one block with a barrier and an L2 round trip per hyperplane took 168 and 228 us
+// for each application.  A step costs about 85 clocks per dependent FP64 instruction, a handover to the next
 // tile about 10,000 clocks (the tile's skew, a group of steps and the trip through the L2).
 #include "internal.h"
 #include "reduce.cuh"
@@ -178,8 +182,8 @@ __device__ __forceinline__ bool sor_tile(const SorGeom& g, const SorLane& L, con
 #pragma unroll
     for (int u = 0; u < N; ++u) {
       const int i0 = at(q0 + u), ic = clamp(i0);
-      ops.template load<FWD, AXES>(min(q0 + u, steps - 1), steps, ic, S.a[u], S.c0[u], S.c1[u], S.c2[u],
-                                   S.w[u]);
+      ops.template load<FWD, AXES>(min(q0 + u, steps - 1), steps, ic, S.a[u], S.c0[u], S.c1[u],
+                                   S.c2[u], S.w[u]);
       if (any_far) {
         S.f1[u] = far1 && (unsigned)i0 < len_on ? sor_peek(ops.template near1<FWD>(ic)) : 0.0;
         if (AXES > 1)
@@ -1063,7 +1067,8 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
                            reduction_blocks(slots, 256, 1), 256, 0, st, g, S, ax[g.ax[0]], ax[g.ax[1]],
                            ax[g.ax[2]], invd, slots));
   cudaError_t le = cudaSuccess;
-  FG_LAUNCH(prof, st, "k_sor_sweeps", 16.0 * dn + (rounded ? 96.0 : 72.0) * (double)slots, le = sweeps(st));
+  const double sweep_bytes = 16.0 * dn + (rounded ? 96.0 : 72.0) * (double)slots;
+  FG_LAUNCH(prof, st, "k_sor_sweeps", sweep_bytes, le = sweeps(st));
   if (le != cudaSuccess && sweep_blocks > 1) {
     cudaGetLastError();
     coop_failed = true;
@@ -1082,7 +1087,7 @@ int KrylovSolver::solve_sor(Stencil64& A, double* x_out, const frehg_solver_conf
                                             partials));
     FG_LAUNCH(pr, s, "k_sor_update", 56.0 * dn + 8.0 * (double)slots,
               k_sor_update<<<nb, 256, 0, s>>>(xs, r, p, w, S.v, slots, zs, n, dst));
-    FG_LAUNCH(pr, s, "k_sor_sweeps", 16.0 * dn + (rounded ? 96.0 : 72.0) * (double)slots, FG_CUDA(sweeps(s)));
+    FG_LAUNCH(pr, s, "k_sor_sweeps", sweep_bytes, FG_CUDA(sweeps(s)));
     FG_LAUNCH(pr, s, "k_sor_dots", 16.0 * dn,
               dots<<<nb, 256, 0, s>>>(zs, r, n, dst, partials));
     return FREHG_OK;

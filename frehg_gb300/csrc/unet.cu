@@ -15,10 +15,10 @@
 // the 17 of the output layer.
 //
 // Layout: activations channels-last, BF16, pixel p = x + nx (y + ny z); a layer may read or
-// write a channel slice of a wider buffer (the concatenations).  Convolutions are implicit GEMMs
-// (M = 16 pixels of an x-row per warp, N = output channels, K = 27 taps x input channels) on
-// mma.sync.m16n8k16 BF16 -> FP32; the data gradient is the same kernel with the weights
-// mirrored in space and transposed in channels; weight gradients accumulate in FP32.
+// write a channel slice of a wider buffer.  The convolutions are implicit GEMMs on tcgen05.mma BF16 ->
+// FP32 (unet_tc.cuh), the decoder's reading their upsampled channels from the coarse field; the data
+// gradient is the same kernel with the weights mirrored in space and transposed in channels; the weight
+// gradients run on mma.sync (unet_dw.cuh).  A warp-level form of the convolutions stays for the check.
 #include "internal.h"
 #include "reduce.cuh"
 
@@ -487,15 +487,16 @@ static void conv_dw(const bf16* in, int in_stride, int in_off, const bf16* g, in
                     const bf16* coarse = nullptr) {
   using S = DwShape<COUT>;
   // set on every launch: the attribute belongs to the current device, and the call is cheap
-  cudaFuncSetAttribute(k_conv3_dw<CIN, COUT, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+  cudaFuncSetAttribute(k_conv3_dw<CIN, COUT, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       S::SMEM);
   const long tiles = (long)((nx + kDwT - 1) / kDwT) * ((ny + kDwT - 1) / kDwT);
   const long want = std::max<long>(1, (long)kNumSMs * S::BLOCKS / (CIN / 16));
   int zc = 16;
   while (zc > 4 && tiles * ((nz + zc - 1) / zc) < want) zc /= 2;
   const long items = tiles * ((nz + zc - 1) / zc);
   const dim3 grid((unsigned)std::min(items, want), CIN / 16);
-  k_conv3_dw<CIN, COUT, UP><<<grid, kDwThreads, S::SMEM, st>>>(in, in_stride, in_off, coarse, g, g_stride,
-                                                           g_off, dW, nx, ny, nz, zc);
+  k_conv3_dw<CIN, COUT, UP><<<grid, kDwThreads, S::SMEM, st>>>(
+      in, in_stride, in_off, coarse, g, g_stride, g_off, dW, nx, ny, nz, zc);
 }
 
 }  // namespace unet
@@ -637,7 +638,8 @@ int forward(frehg_unet* net, const float* r, const float* lnk, const float* cap,
   }
   k_pack_input<<<blocks_for(n1), 256, 0, st>>>(r, lnk, cap, net->scal, net->kmean, net->kscale,
                                                net->cscale, net->x0, n1);
-  conv<16, 16>(net->x0, 16, 0, W + net->wboff[0], M + net->boff[0], net->a1, 16, 0, nx, ny, nz, true, st);
+  conv<16, 16>(net->x0, 16, 0, W + net->wboff[0], M + net->boff[0], net->a1, 16, 0, nx, ny, nz,
+               true, st);
   TcExtra pool1, pool2, last;
   pool1.pooled = net->p1;
   pool2.pooled = net->p2;
@@ -646,14 +648,20 @@ int forward(frehg_unet* net, const float* r, const float* lnk, const float* cap,
   last.y = y;
   conv<16, 16, 0, kTcPool>(net->a1, 16, 0, W + net->wboff[1], M + net->boff[1], net->e1, 16, 0, nx,
                            ny, nz, true, st, nullptr, pool1);
-  conv<16, 32>(net->p1, 16, 0, W + net->wboff[2], M + net->boff[2], net->a2, 32, 0, x2, y2, z2, true, st);
+  conv<16, 32>(net->p1, 16, 0, W + net->wboff[2], M + net->boff[2], net->a2, 32, 0, x2, y2, z2,
+               true, st);
   conv<32, 32, 0, kTcPool>(net->a2, 32, 0, W + net->wboff[3], M + net->boff[3], net->e2, 32, 0, x2,
                            y2, z2, true, st, nullptr, pool2);
-  conv<32, 64>(net->p2, 32, 0, W + net->wboff[4], M + net->boff[4], net->a3, 64, 0, x3, y3, z3, true, st);
-  conv<64, 64>(net->a3, 64, 0, W + net->wboff[5], M + net->boff[5], net->e3, 64, 0, x3, y3, z3, true, st);
-  conv<96, 32, 64>(net->e2, 32, 0, W + net->wboff[6], M + net->boff[6], net->d2a, 32, 0, x2, y2, z2, true, st, net->e3);
-  conv<32, 32>(net->d2a, 32, 0, W + net->wboff[7], M + net->boff[7], net->d2, 32, 0, x2, y2, z2, true, st);
-  conv<48, 16, 32>(net->e1, 16, 0, W + net->wboff[8], M + net->boff[8], net->d1a, 16, 0, nx, ny, nz, true, st, net->d2);
+  conv<32, 64>(net->p2, 32, 0, W + net->wboff[4], M + net->boff[4], net->a3, 64, 0, x3, y3, z3,
+               true, st);
+  conv<64, 64>(net->a3, 64, 0, W + net->wboff[5], M + net->boff[5], net->e3, 64, 0, x3, y3, z3,
+               true, st);
+  conv<96, 32, 64>(net->e2, 32, 0, W + net->wboff[6], M + net->boff[6], net->d2a, 32, 0, x2, y2, z2,
+                   true, st, net->e3);
+  conv<32, 32>(net->d2a, 32, 0, W + net->wboff[7], M + net->boff[7], net->d2, 32, 0, x2, y2, z2,
+               true, st);
+  conv<48, 16, 32>(net->e1, 16, 0, W + net->wboff[8], M + net->boff[8], net->d1a, 16, 0, nx, ny, nz,
+                   true, st, net->d2);
   conv<16, 16, 0, kTcOut>(net->d1a, 16, 0, W + net->wboff[9], M + net->boff[9],
                           keep ? net->d1 : nullptr, 16, 0, nx, ny, nz, true, st, nullptr, last);
   FG_CUDA(cudaGetLastError());

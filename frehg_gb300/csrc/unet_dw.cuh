@@ -3,9 +3,9 @@
 //   dW[t][o][i] = sum over pixels p of g[p][o] in[p + off(t)][i]      (zero outside the grid)
 //
 // For every tap a small matrix product whose long dimension is the pixels: M = output channels,
-// N = input channels (both 16 to 96), K = pixels.  tcgen05 needs 64 or 128 rows of M, which
-// COUT = 16 would leave three quarters empty, so the products run on the warp-level
-// mma.m16n8k16 (BF16 operands, FP32 accumulators): one warp owns the nine taps of one dz for 16
+// N = input channels (both 16 to 96), K = pixels, on the warp-level mma.m16n8k16 (BF16 operands,
+// FP32 accumulators).  (tcgen05 has 64 or 128 rows of M, three quarters empty for 16 output
+// channels; with (tap, input channel) along M they would be full, a form not written yet.)  One warp owns the nine taps of one dz for 16
 // input channels and 16 or 32 output channels, 72 or 144 accumulators that stay in registers
 // over all of the block's pixels.  Both operands lie channels-last, that is with the pixel (K)
 // outermost, and reach the fragments by transposing ldmatrix loads; a tap is the same patch read
@@ -72,8 +72,8 @@ __device__ __forceinline__ void dw_mma(float (&d)[4], const uint32_t (&a)[4], ui
 template <int CIN, int COUT, int UP>
 __global__ void __launch_bounds__(kDwThreads, DwShape<COUT>::BLOCKS) k_conv3_dw(
     const __nv_bfloat16* __restrict__ in, int in_stride, int in_off,
-    const __nv_bfloat16* __restrict__ coarse, const __nv_bfloat16* __restrict__ gout, int g_stride, int g_off, float* __restrict__ dW, int nx,
-    int ny, int nz, int zc) {
+    const __nv_bfloat16* __restrict__ coarse, const __nv_bfloat16* __restrict__ gout, int g_stride,
+    int g_off, float* __restrict__ dW, int nx, int ny, int nz, int zc) {
   using S = DwShape<COUT>;
   extern __shared__ __align__(128) unsigned char dw_smem[];
   unsigned char* gbuf = dw_smem + 4 * S::INP;

@@ -7,9 +7,9 @@
 // An MMA of M = 128 takes 32 + N / 4 clocks up to N = 96 (shared-memory reads: 4 KB of A, 32 N bytes
 // of B) and N / 2 above (measured, whatever the alignment of A), so the three dz taps are stacked
 // along N: the weights sit as [t9][chunk][rb COUT + o][8] with row block rb = 2 - dz, and one group
-// of MMAs per INPUT plane z' (9 taps x CIN/16 slices, N = 3 COUT) adds W(dz=2) In(z') to out(z'-1), W(1) In(z') to out(z') and W(0) In(z') to out(z'+1):
-// a third of the MMAs of one group per output plane over three input planes, and each input plane
-// is read once per tile.
+// of MMAs per INPUT plane z' (9 taps x CIN/16 slices, N = 3 COUT) adds W(dz=2) In(z') to out(z'-1),
+// W(1) In(z') to out(z') and W(0) In(z') to out(z'+1): a third of the MMAs of one group per output
+// plane over three input planes, and each input plane is read once per tile.
 // Operands sit in shared memory in the no-swizzle K-major core-matrix layout, which the
 // channels-last activations reach by splitting the channels into 8-channel chunks:
 //   ring slots  [chunk of 2][hy][hx][8]: 16 channels of the 10 x 18 pixels x0-1 .. x0+8,
@@ -31,8 +31,9 @@
 // the copies, which pass through L1.  (Copies past L1 are slower but for 96 channels, 16 copy warps
 // no faster.)  The decoder convolutions read the upsampled half of their input from the coarse
 // field, as the stored concatenation took 170 us more in all at 256 x 256 x 128.  There, against one
-// MMA group per output plane and per-plane barriers of one warpgroup: 16 -> 16 305 -> 153 us, 48 -> 16 617 -> 372; 128 x 128 x 64: 96 -> 32 628 -> 200, 32 ->
-// 32 96 -> 61; 64 x 64 x 32: 64 -> 64 112 -> 33.
+// MMA group per output plane and per-plane barriers of one warpgroup: 16 -> 16 305 -> 153 us,
+// 48 -> 16 617 -> 372; 128 x 128 x 64: 96 -> 32 628 -> 200, 32 -> 32 96 -> 61; 64 x 64 x 32:
+// 64 -> 64 112 -> 33.
 //
 // Every wait is bounded: a wait that runs out records an error word, the block's other waits see
 // the abort word and return, and the MMAs in flight finish (bounded) before the tensor memory is
