@@ -716,8 +716,9 @@ def run_gpu(args):
                 "picard_arith": ("native fp64" if args.scheme != "picard" or w.params.picard_fp64
                                  else "float-float (two fp32, ~48-bit significand) for the "
                                       "constitutive relations, face fluxes and final update; "
-                                      "Picard residual's storage difference and combination, "
-                                      "refinement residual and mass sums fp64"),
+                                      "Picard residual's storage difference and combination "
+                                      "and mass sums fp64; refinement residual from exact "
+                                      "FP32 products (2^-57 of its terms)"),
                 "picard_iterations": cnt["picard_iterations"],
                 "cg_iterations": cnt["ksp_iterations"], "ir_sweeps": cnt["ir_sweeps"],
                 "mass_error_rel": cnt["mass_error_rel"]},
